@@ -19,6 +19,8 @@
 // both operands MN-major, split-K over the CTAs with periodic accumulator flushes.
 // Every mbarrier wait is bounded; a role that gives up sets the status word and the CTA still frees its TMEM.
 #include <cuda.h>
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include "dg_internal.h"
@@ -478,6 +480,55 @@ __global__ void k_tf32_split(const float* __restrict__ src, float* __restrict__ 
     tail[i] = x - h;
 }
 
+// Head and tail of a whole operand, transposed on the way where asked (32 x 32 tiles through shared memory, so that both
+// sides are coalesced), rows zero-filled up to ldb.
+__global__ void __launch_bounds__(256) k_tf32_split_operand(const float* __restrict__ w, int64_t ldw, int transposed, int N, int K,
+                                                            float* __restrict__ head, float* __restrict__ tail, int64_t ldb)
+{
+    __shared__ float tile[32][33];
+    const int k0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r = ty; r < 32; r += 8) {
+        const int n = transposed ? n0 + tx : n0 + r, k = transposed ? k0 + r : k0 + tx;
+        const float x = n < N && k < K ? w[transposed ? (int64_t)k * ldw + n : (int64_t)n * ldw + k] : 0.f;
+        if (transposed) tile[tx][r] = x; else tile[r][tx] = x;
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+        const int n = n0 + r, k = k0 + tx;
+        if (n >= N || k >= ldb) continue;
+        const float x = tile[r][tx];
+        const float h = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
+        head[(int64_t)n * ldb + k] = h;
+        tail[(int64_t)n * ldb + k] = x - h;
+    }
+}
+
+// Raises a kernel's dynamic shared-memory limit to the most a CTA can have, once per device instead of before every launch.
+int allow_smem(const void* kernel, std::atomic<bool>* done)
+{
+    int dev = 0;
+    DG_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return DG_ERR_STATE;
+    if (done[dev].load(std::memory_order_relaxed)) return DG_OK;
+    DG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    done[dev].store(true, std::memory_order_relaxed);
+    return DG_OK;
+}
+
+int sm_count()
+{
+    static std::atomic<int> count[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = count[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+        count[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 }  // namespace
 
 namespace {
@@ -537,6 +588,17 @@ extern "C" int dg_dense_split(const float* src, float* head, float* tail, int64_
     return (int)cudaGetLastError();
 }
 
+extern "C" int dg_dense_split_operand(const float* w, int64_t ldw, int32_t transposed, int32_t N, int32_t K, float* head, float* tail,
+                                      int64_t ldb, void* stream)
+{
+    if (N < 0 || K < 0 || ldb < K || ldw < (transposed ? N : K)) return DG_ERR_DIMS;
+    if (N == 0 || K == 0) return DG_OK;
+    if (!w || !head || !tail) return DG_ERR_NULL;
+    const dim3 grid((unsigned)((ldb + 31) / 32), (unsigned)((N + 31) / 32));
+    k_tf32_split_operand<<<grid, 256, 0, (cudaStream_t)stream>>>(w, ldw, transposed != 0, N, K, head, tail, ldb);
+    return (int)cudaGetLastError();
+}
+
 extern "C" int dg_dense_supported(int64_t M, int32_t N, int32_t K, int64_t lda, int64_t ldb, const void* A, const void* Bh, const void* Bt)
 {
     if (M <= 0 || N <= 0 || K <= 0 || M >= ((int64_t)1 << 31)) return 0;
@@ -586,14 +648,15 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
     // persistent CTA's two stages do (2,449,029 x 256 -> 47: 1.09 ms against 1.28 ms; -> 256: 2.16 against 1.88).
     const bool per_tile = a.n_pad <= 128;
     if (per_tile) {
-        DG_CUDA(cudaFuncSetAttribute(k_dense_nt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        static std::atomic<bool> granted[64];
+        if ((rc = allow_smem((const void*)k_dense_nt, granted))) return rc;
         k_dense_nt<<<(unsigned)n_tiles, kThreads, smem, (cudaStream_t)stream>>>(tmA, tmBh, tmBt, a);
         return (int)cudaGetLastError();
     }
-    int dev = 0, sms = 0;
-    DG_CUDA(cudaGetDevice(&dev));
-    DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    DG_CUDA(cudaFuncSetAttribute(k_dense_nt_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<bool> granted[64];
+    const int sms = sm_count();
+    if (sms <= 0) return DG_ERR_STATE;
+    if ((rc = allow_smem((const void*)k_dense_nt_persistent, granted))) return rc;
     k_dense_nt_persistent<<<(unsigned)(n_tiles < sms ? n_tiles : sms), kThreadsPersistent, smem, (cudaStream_t)stream>>>(tmA, tmBh, tmBt, a, n_tiles);
     return (int)cudaGetLastError();
 }
@@ -969,7 +1032,8 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
     if ((rc = make_map_box(&tmX, X, n, Km, ldx, 32, TN_ROWS)) || (rc = make_map_box(&tmG, G, n, Nn, ldg, 32, TN_ROWS))) return rc;
     const int x_bytes = a.m_halves * 4 * TN_BOX_BYTES, g_bytes = (a.n_pad + 31) / 32 * TN_BOX_BYTES;
     const size_t smem = (size_t)TN_STAGES * (2 * x_bytes + 2 * g_bytes) + 24 * TN_STAGES + 24 + 1024;
-    DG_CUDA(cudaFuncSetAttribute(k_dense_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<bool> granted[64];
+    if ((rc = allow_smem((const void*)k_dense_tn, granted))) return rc;
     k_dense_tn<<<ctas, kThreads, smem, (cudaStream_t)stream>>>(tmX, tmG, a);
     k_dense_tn_reduce<<<(unsigned)((slots + 255) / 256), 256, 0, (cudaStream_t)stream>>>(scratch, ctas, slots, D, ldd, Km, Nn, a.n_pad);
     return (int)cudaGetLastError();

@@ -2,7 +2,7 @@
 
 `timing(key)` is wall clock, as in the reference.  `timing_cuda(key)` does NOT synchronise the device around the
 region the way the reference does (timer.py:16-24; four host syncs per stage there): it records a pair of CUDA
-events on the current stream and adds their elapsed time when a summary is asked for, so timing a region leaves
+events (pooled in the library) on the current stream and adds their elapsed time when a summary is asked for, so timing a region leaves
 the broadcast/SpMM overlap intact.  On a CPU-only process it degrades to wall clock.
 """
 import statistics
@@ -13,27 +13,36 @@ import torch
 
 
 class TimerCtx:
-    def __init__(self, timer, key, cuda):
-        self.timer, self.key, self.cuda = timer, key, cuda and torch.cuda.is_available()
+    """Wall-clock region."""
+
+    def __init__(self, timer, key):
+        self.timer, self.key = timer, key
 
     def __enter__(self):
-        if self.cuda:
-            self.begin = torch.cuda.Event(enable_timing=True)
-            self.begin.record()
-        else:
-            self.t0 = time.time()
+        self.t0 = time.time()
         return self
 
     def __exit__(self, *exc):
-        if self.cuda:
-            end = torch.cuda.Event(enable_timing=True)
-            end.record()
-            self.timer.pending.append((self.key, self.begin, end))
-            if len(self.timer.pending) >= self.timer.MAX_PENDING:       # a long run never holds more than this many event pairs
-                self.timer.resolve()
-        else:
-            self.timer.duration_dict[self.key] += time.time() - self.t0
+        self.timer.duration_dict[self.key] += time.time() - self.t0
         self.timer.count_dict[self.key] += 1
+
+
+class CudaTimerCtx:
+    """Device region between two marks of the library's event pool (spmm_cpp.mark), about 1 us each on the host."""
+
+    def __init__(self, timer, key, mark):
+        self.timer, self.key, self.mark = timer, key, mark
+
+    def __enter__(self):
+        self.begin = self.mark()
+        return self
+
+    def __exit__(self, *exc):
+        timer = self.timer
+        timer.pending.append((self.key, self.begin, self.mark()))
+        if len(timer.pending) >= timer.MAX_PENDING:       # a long run never holds more than this many pairs
+            timer.resolve()
+        timer.count_dict[self.key] += 1
 
 
 class DistTimer:
@@ -45,24 +54,36 @@ class DistTimer:
         self.duration_dict = defaultdict(float)
         self.count_dict = defaultdict(int)
         self.pending = []
+        self._mark = None
 
     def resolve(self, synchronize=True):
-        """Adds the elapsed time of the recorded event pairs to their keys.  The training loop calls it with
+        """Adds the elapsed time of the recorded mark pairs to their keys.  The training loop calls it with
         synchronize=False right after it has read the loss (the device is idle then), so the list never grows."""
         if self.pending:
+            import spmm_cpp
             if synchronize:
                 torch.cuda.synchronize(self.env.device if self.env.device.type == 'cuda' else None)
-            for key, begin, end in self.pending:
-                self.duration_dict[key] += begin.elapsed_time(end) / 1000.0
-            self.pending = []
+            pending, self.pending = self.pending, []
+            for key, begin, end in pending:
+                self.duration_dict[key] += spmm_cpp.mark_elapsed(begin, end) / 1000.0
 
     _resolve = resolve
 
     def timing(self, key):
-        return TimerCtx(self, key, cuda=False)
+        return TimerCtx(self, key)
 
     def timing_cuda(self, key):
-        return TimerCtx(self, key, cuda=True)
+        if self._mark is None:
+            if not torch.cuda.is_available():
+                return TimerCtx(self, key)
+            import spmm_cpp
+            self._mark = spmm_cpp.mark
+        return CudaTimerCtx(self, key, self._mark)
+
+    def empty_region(self, key):
+        """Counts a region in which this layout has nothing to do (a one-rank all-reduce)."""
+        self.duration_dict[key] += 0.0
+        self.count_dict[key] += 1
 
     def start(self, key):
         self.start_time_dict[key] = time.time()

@@ -53,14 +53,24 @@ def _rows(t, keep=False):
         if hit is not None and hit[0]() is t and hit[1] == t._version:
             return hit[2]
     rows, cols = t.shape
-    wide = torch.zeros((rows, cols + (-cols) % 4), dtype=t.dtype, device=t.device)
-    wide[:, :cols] = t
-    view = wide[:, :cols]
+    wide = torch.empty((rows, cols + (-cols) % 4), dtype=t.dtype, device=t.device)
+    view = _pad_into(t, wide)[:, :cols]
     if keep:
         import weakref
         key = id(t)
         _padded_rows[key] = (weakref.ref(t, lambda _r, key=key: _padded_rows.pop(key, None)), t._version, view)
     return view
+
+
+def _pad_into(t, wide):
+    """wide's first columns become t, the rest zero: one launch for fp32 rows on a GPU."""
+    if t.is_cuda and t.dtype == torch.float32 and wide.size(1) % 4 == 0:
+        if t.size(1) > 1 and t.stride(1) != 1 or t.stride(0) < t.size(1):
+            t = t.contiguous()
+        return spmm_cpp.pad_rows(t, wide)
+    wide[:, :t.size(1)] = t
+    wide[:, t.size(1):] = 0
+    return wide
 
 
 def _tf32_split(x):
@@ -112,26 +122,53 @@ def _library_mm(a, b, ta, tb):
 
 
 def broadcast(local_adj_parts, local_feature, tag):
+    return _distributed_spmm(local_adj_parts, local_feature)
+
+
+def _distributed_spmm(local_adj_parts, local_feature, constant=False):
+    """z = sum over the stages of A[rank, s] X_s.  constant: the operand is an input that never changes (where its rows
+    have to be padded, the padded copy is kept)."""
     env = DistEnv.env
     if not local_feature.is_cuda:
         raise RuntimeError('the broadcast-SpMM stage loop runs on CUDA tensors only; there is no CPU path')
+    if env.col_comm is None:
+        return _local_products(env, local_adj_parts, local_feature, constant)
     x = local_feature.contiguous()
     true_width = x.size(1)
     if true_width % 4 and PAD_ODD_WIDTHS:
         # Rows that are not a whole number of 16-byte pieces (47 classes = 188 bytes) cannot be moved with 128-bit loads
         # and start at odd offsets.  The stage loop then runs on a copy whose rows are padded with zero columns to the
         # next multiple of 4; the caller gets the first true_width columns of the wider result.
-        wide = env.recv_buffers(x.size(0), true_width + (-true_width) % 4, nbuf=1, tag='padded')[0]
-        wide[:, :true_width] = x
-        wide[:, true_width:] = 0
-        x = wide
-    n, width = x.shape
-    stages = env.stages()
-    comm = env.col_comm
+        x = _pad_into(x, env.recv_buffers(x.size(0), true_width + (-true_width) % 4, nbuf=1, tag='padded')[0])
     z = torch.empty_like(x)
-    if width != true_width:
-        return _stage_loop(env, local_adj_parts, x, z, stages, comm)[:, :true_width]
-    return _stage_loop(env, local_adj_parts, x, z, stages, comm)
+    _stage_loop(env, local_adj_parts, x, z, env.stages(), env.col_comm)
+    return z if z.size(1) == true_width else z[:, :true_width]
+
+
+def _local_products(env, adj_parts, t, constant):
+    """The stage loop of a rank without peers: its own products, straight on the operand wherever that lies (any row
+    stride of whole 16-byte pieces), else on a padded copy as above.  No communicator, no buffers, no argument tables:
+    on small graphs the host's share of a step is what a step costs."""
+    n, true_width = t.shape
+    width = true_width + (-true_width) % 4 if PAD_ODD_WIDTHS else true_width
+    ld = t.stride(0)
+    if t.stride(1) == 1 and ld % 4 == 0 and ld >= width and t.data_ptr() % 16 == 0 and (
+            width == true_width or t.storage_offset() + (n - 1) * ld + width <= t.untyped_storage().nbytes() // 4):
+        x = t if width == true_width else t.as_strided((n, width), (ld, 1))      # the columns beyond true_width are not looked at
+    elif width == true_width:
+        x = t.contiguous()
+    elif constant:
+        kept = _rows(t, keep=True)
+        x = kept.as_strided((n, width), (kept.stride(0), 1))
+    else:
+        x = _pad_into(t, env.recv_buffers(n, width, nbuf=1, tag='padded')[0])
+    z = torch.empty((n, width), dtype=torch.float32, device=t.device)
+    with env.timer.timing_cuda('broadcast+spmm'):
+        beta = 0.0
+        for st in env.stages():
+            spmm_cpp.plan_for(adj_parts[st.part]).spmm(x, z, 1.0, beta)
+            beta = 1.0
+    return z if width == true_width else z[:, :true_width]
 
 
 def _stage_loop(env, local_adj_parts, x, z, stages, comm, timed=False):
@@ -340,6 +377,15 @@ def group_plans(adj_parts, parts, group):
     return plans
 
 
+def _all_reduce(t):
+    env = DistEnv.env
+    if env.world_size == 1:
+        env.timer.empty_region('all_reduce')
+        return
+    with env.timer.timing_cuda('all_reduce'):
+        env.all_reduce_sum(t)
+
+
 class DistGCNLayer(torch.autograd.Function):
     """forward(features, weight, adj_parts, tag) as in the reference (gcn.py:35-53).  Optional flags let GCN fuse the
     ReLU between two layers into the dense kernels instead of running it (and its backward) as separate passes:
@@ -359,11 +405,13 @@ class DistGCNLayer(torch.autograd.Function):
                     rank's term, and the rounding, differ.
     transform_first for a layer without ReLU whose output is narrower than its input (the last one: 256 -> 47), compute
                     A (X W) instead of (A X) W: the stage loop then runs at the output width.  Same result up to rounding,
-                    same backward pass."""
+                    same backward pass.
+    constant_input  the features are the network's input, which stays as it is from step to step: where its rows have to be
+                    padded, the padded copy is kept until the tensor is modified."""
 
     @staticmethod
     def forward(ctx, features, weight, adj_parts, tag, relu=False, input_is_relu=False, product=None, shortcut=False,
-                transform_first=False):
+                transform_first=False, constant_input=False):
         ctx.adj_parts, ctx.tag, ctx.input_is_relu = adj_parts, tag, input_is_relu
         ctx.weight_key = weight                      # the caller's tensor object: key of the split-weight cache
         ctx.shortcut = bool(shortcut and product is not None)
@@ -374,7 +422,7 @@ class DistGCNLayer(torch.autograd.Function):
             with DistEnv.env.timer.timing_cuda('mm'):
                 y = dense_mm(features, weight, weight_key=weight)
             return broadcast(adj_parts, y, 'Forward' + tag)
-        z_local = product if product is not None else broadcast(adj_parts, features, 'Forward' + tag)
+        z_local = product if product is not None else _distributed_spmm(adj_parts, features, constant_input)
         ctx.save_for_backward(z_local if ctx.shortcut else features, weight)
         with DistEnv.env.timer.timing_cuda('mm'):
             z_local = dense_mm(z_local, weight, relu=relu, weight_key=weight)
@@ -386,9 +434,8 @@ class DistGCNLayer(torch.autograd.Function):
         if ctx.shortcut and not ctx.needs_input_grad[0]:
             with DistEnv.env.timer.timing_cuda('mm'):
                 grad_weight = dense_mm(features, grad_output, ta=True, constant_a=True)      # `features` holds the saved product here
-            with DistEnv.env.timer.timing_cuda('all_reduce'):
-                DistEnv.env.all_reduce_sum(grad_weight)
-            return None, grad_weight, None, None, None, None, None, None, None
+            _all_reduce(grad_weight)
+            return (None, grad_weight) + (None,) * 8
         if ctx.shortcut:
             raise RuntimeError('the gradient shortcut needs an input that requires no gradient')
         ag = broadcast(ctx.adj_parts, grad_output, 'Backward' + ctx.tag)
@@ -397,9 +444,8 @@ class DistGCNLayer(torch.autograd.Function):
             if ctx.needs_input_grad[0]:
                 grad_features = dense_mm(ag, weight, tb=True, mask=features if ctx.input_is_relu else None, weight_key=ctx.weight_key)
             grad_weight = dense_mm(features, ag, ta=True, constant_a=not ctx.needs_input_grad[0])
-        with DistEnv.env.timer.timing_cuda('all_reduce'):
-            DistEnv.env.all_reduce_sum(grad_weight)
-        return grad_features, grad_weight, None, None, None, None, None, None, None
+        _all_reduce(grad_weight)
+        return (grad_features, grad_weight) + (None,) * 8
 
 
 class GCN(nn.Module):
@@ -458,10 +504,10 @@ class GCN(nn.Module):
             product = self.input_product(h) if l == 0 else None
             shortcut = self.input_gradient_shortcut and product is not None
             if FUSE_RELU:
-                h = DistGCNLayer.apply(h, w, self.g.adj_parts, f'L{l + 1}', l < last, l > 0, product, shortcut, self.transform_first)
+                h = DistGCNLayer.apply(h, w, self.g.adj_parts, f'L{l + 1}', l < last, l > 0, product, shortcut, self.transform_first, l == 0)
             else:
                 h = DistGCNLayer.apply(h, w, self.g.adj_parts, f'L{l + 1}', False, False, product, shortcut,
-                                       self.transform_first and l == last)
+                                       self.transform_first and l == last, l == 0)
                 if l < last:
                     h = F.relu(h)
         return h

@@ -17,6 +17,7 @@ _LIB_PATH = os.path.join(_HERE, 'csrc', 'libdist_gnn_b200.so')
 _lib = None
 
 EPI_ROW_SCALE, EPI_BIAS, EPI_RELU = 1, 2, 4
+ERR_UNSUPPORTED = -4
 
 
 class PlanStats(ctypes.Structure):
@@ -82,6 +83,7 @@ def lib():
             'dg_peer_spmm': ([vp, vp, i32, vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, vp, ctypes.c_int, vp], ctypes.c_int),
             'dg_peer_spmm_gather': ([vp, vp, i32, vp, vp, vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, vp, ctypes.c_int, vp], ctypes.c_int),
             'dg_dense_split': ([vp, vp, vp, i64, vp], ctypes.c_int),
+            'dg_dense_split_operand': ([vp, i64, i32, i32, i32, vp, vp, i64, vp], ctypes.c_int),
             'dg_dense_supported': ([i64, i32, i32, i64, i64, vp, vp, vp], ctypes.c_int),
             'dg_dense_nt': ([vp, i64, vp, vp, i64, vp, i64, i64, i32, i32, i32, vp], ctypes.c_int),
             'dg_dense_nt_masked': ([vp, i64, vp, vp, i64, vp, i64, i64, i32, i32, i32, vp, i64, vp], ctypes.c_int),
@@ -90,6 +92,10 @@ def lib():
             'dg_dense_status': ([ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
             'dg_dense_status_reset': ([vp], ctypes.c_int),
             'dg_dense_wait_selftest': ([ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
+            'dg_pad_rows': ([vp, i64, i64, i32, vp, i64, vp], ctypes.c_int),
+            'dg_mark_record': ([vp], ctypes.c_int),
+            'dg_mark_elapsed': ([ctypes.c_int, ctypes.c_int, ctypes.POINTER(f32)], ctypes.c_int),
+            'dg_mark_release': ([ctypes.c_int], ctypes.c_int),
             'dg_profile_begin': ([], ctypes.c_int),
             'dg_profile_end': ([ctypes.POINTER(Profile)], ctypes.c_int),
         }
@@ -105,8 +111,32 @@ def check(code):
         raise RuntimeError(f'dist_gnn_b200 error {code}: {lib().dg_strerror(code).decode()}')
 
 
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+class _NoGuard:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NO_GUARD = _NoGuard()
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, '_cuda_getCurrentRawStream') else None
+_current_device = torch._C._cuda_getDevice if hasattr(torch._C, '_cuda_getDevice') else None
+
+
+def _on(index):
+    """Makes CUDA device `index` current for a block of code; free of charge when it already is (torch.cuda.device costs
+    about 3 us a block, as much as a small kernel's launch)."""
+    return _NO_GUARD if index is None or _current_device() == index else torch.cuda.device(index)
+
+
+def _stream(index=None):
+    """torch's current stream of the device as a plain number (building a torch.cuda.Stream object for it costs 15 us)."""
+    if index is None:
+        if not torch.cuda.is_initialized():
+            torch.cuda.init()
+        index = _current_device()
+    return _raw_stream(index)
 
 
 def _dev_tensor(t, dtype, what):
@@ -122,9 +152,22 @@ def _row_major(t, what):
     length - a column slice of a wider buffer, as the stage loop returns for operands it padded."""
     if not (isinstance(t, torch.Tensor) and t.is_cuda):
         raise RuntimeError(f'{what} must be a CUDA tensor: this library has no CPU path')
-    if t.dtype != torch.float32 or t.dim() != 2 or (t.size(1) > 1 and t.stride(1) != 1) or (t.size(0) > 1 and t.stride(0) < t.size(1)):
-        raise RuntimeError(f'{what} must be a row-major fp32 matrix, got {t.dtype} {tuple(t.shape)} strides {t.stride()}')
-    return t.stride(0) if t.size(0) > 1 else max(t.size(1), 1)
+    if t.dtype == torch.float32 and t.dim() == 2:
+        (n, F), (ld, unit) = t.shape, t.stride()
+        if (F <= 1 or unit == 1) and (n <= 1 or ld >= F):
+            return ld if n > 1 else max(F, 1)
+    raise RuntimeError(f'{what} must be a row-major fp32 matrix, got {t.dtype} {tuple(t.shape)} strides {t.stride()}')
+
+
+def _operand(t, rows, what):
+    """Row stride of a dense operand of a product, which has to have `rows` rows."""
+    if not (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.dim() == 2):
+        raise RuntimeError(f'{what} must be a 2-D fp32 CUDA tensor')
+    n, F = t.shape
+    ld, unit = t.stride()
+    if n != rows or (F > 1 and unit != 1):
+        raise RuntimeError(f'{what} has shape {tuple(t.shape)} / strides {t.stride()}, expected {rows} rows, unit column stride')
+    return ld if n > 1 else max(F, 1)
 
 
 class SpmmPlan:
@@ -137,7 +180,7 @@ class SpmmPlan:
             raise RuntimeError('row, col and value arrays differ in length')
         self.col, self.values, self.m, self.k, self.device = col_i32, values, int(m), int(k), values.device
         handle = ctypes.c_void_p()
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_plan_create_ex(row_i32.data_ptr(), col_i32.data_ptr(), values.numel(), self.m, self.k,
                                           heavy_threshold, chunk, _stream(), ctypes.byref(handle)))
         self.handle = handle
@@ -160,45 +203,42 @@ class SpmmPlan:
 
     def rowptr(self):
         out = torch.empty(self.m + 1, dtype=torch.int64)
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_plan_copy_rowptr(self.handle, out.data_ptr(), _stream()))
         return out
 
     def set_task_size(self, task_nnz):
         """Entries per warp task of the streaming kernel (default 1024; <= 0 restores it)."""
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_plan_set_task_size(self.handle, int(task_nnz), _stream()))
         return self
 
     def device_status(self):
         """0, or non-zero if a kernel of this plan gave up on a bounded wait (its result is then invalid)."""
         out = ctypes.c_int(-1)
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_plan_device_status(self.handle, ctypes.byref(out), _stream()))
         return out.value
 
     def spmm(self, B, C, alpha=1.0, beta=1.0, row_scale=None, bias=None, relu=False, values=None):
         """C <- epilogue(alpha * A @ B + beta * C) in place; B [k, F] and C [m, F] may be row-strided views."""
         val = self.values if values is None else _dev_tensor(values, torch.float32, 'values')
-        for t, rows, what in ((B, self.k, 'B'), (C, self.m, 'C')):
-            if not (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.dim() == 2):
-                raise RuntimeError(f'{what} must be a 2-D fp32 CUDA tensor')
-            if t.size(0) != rows or (t.size(1) > 1 and t.stride(1) != 1):
-                raise RuntimeError(f'{what} has shape {tuple(t.shape)} / strides {t.stride()}, expected {rows} rows, unit column stride')
-        if B.size(1) != C.size(1):
-            raise RuntimeError('B and C differ in width')
-        flags = (EPI_ROW_SCALE if row_scale is not None else 0) | (EPI_BIAS if bias is not None else 0) | (EPI_RELU if relu else 0)
-        if row_scale is not None:
-            _dev_tensor(row_scale, torch.float32, 'row_scale')
-        if bias is not None:
-            _dev_tensor(bias, torch.float32, 'bias')
+        ldb, ldc = _operand(B, self.k, 'B'), _operand(C, self.m, 'C')
         F = B.size(1)
-        ldb = B.stride(0) if B.size(0) > 1 else max(F, 1)
-        ldc = C.stride(0) if C.size(0) > 1 else max(F, 1)
-        with torch.cuda.device(self.device):
-            check(lib().dg_spmm_csr(self.handle, val.data_ptr(), B.data_ptr(), ldb, C.data_ptr(), ldc, F, alpha, beta, flags,
-                                    row_scale.data_ptr() if row_scale is not None else None,
-                                    bias.data_ptr() if bias is not None else None, _stream()))
+        if F != C.size(1):
+            raise RuntimeError('B and C differ in width')
+        flags = EPI_RELU if relu else 0
+        scale_ptr = bias_ptr = None
+        if row_scale is not None:
+            flags |= EPI_ROW_SCALE
+            scale_ptr = _dev_tensor(row_scale, torch.float32, 'row_scale').data_ptr()
+        if bias is not None:
+            flags |= EPI_BIAS
+            bias_ptr = _dev_tensor(bias, torch.float32, 'bias').data_ptr()
+        index = self.device.index
+        with _on(index):
+            check(_lib.dg_spmm_csr(self.handle, val.data_ptr(), B.data_ptr(), ldb, C.data_ptr(), ldc, F, alpha, beta, flags,
+                                   scale_ptr, bias_ptr, _raw_stream(index)))
         return C
 
     def algorithmic_bytes(self, F, beta_nonzero):
@@ -217,6 +257,23 @@ class SpmmPlan:
 def select_kernel(family):
     """0 automatic (row kernels), 1 row kernels only, 2 streaming kernel where eligible; process-wide."""
     check(lib().dg_select_kernel({'auto': 0, 'rows': 1, 'stream': 2}.get(family, family)))
+
+
+def mark():
+    """Records a time mark on the current stream (dg_mark_record) and returns its id."""
+    ident = lib().dg_mark_record(_stream())
+    if ident < 0:
+        check(ident)
+    return ident
+
+
+def mark_elapsed(begin, end):
+    """Milliseconds between two marks that the device has passed; both go back to the pool."""
+    ms = ctypes.c_float()
+    code = lib().dg_mark_elapsed(begin, end, ctypes.byref(ms))
+    _lib.dg_mark_release(begin), _lib.dg_mark_release(end)
+    check(code)
+    return ms.value
 
 
 dense_launches = 0      # kernels launched by dense_split / dense_nt / dense_tn since the last profile_begin
@@ -285,7 +342,7 @@ def spmm_cusparse(A_row_idx, A_col_idx, A_values, A_row, A_col, B, C, alpha, bet
             _dropin_plans.pop(next(iter(_dropin_plans)))
         hit[0].spmm(B, C, float(alpha), float(beta), values=A_values)
         return
-    with torch.cuda.device(C.device):
+    with _on(C.device.index):
         check(lib().dg_spmm_coo(A_row_idx.data_ptr(), A_col_idx.data_ptr(), A_values.data_ptr(), nnz,
                                 int(A_row), int(A_col), B.data_ptr(), C.data_ptr(), B.size(1), float(alpha), float(beta), _stream()))
 
@@ -314,30 +371,30 @@ class Comm:
 
     def split(self, color, key):
         handle = ctypes.c_void_p()
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_split(self.handle, color, key, ctypes.byref(handle)))
         return Comm(handle, self.device) if handle.value else None
 
     def all_reduce_sum(self, t):
         _dev_tensor(t, torch.float32, 'tensor')
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_allreduce_sum(self.handle, t.data_ptr(), t.numel(), _stream()))
 
     def broadcast(self, t, root):
         _dev_tensor(t, torch.float32, 'tensor')
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_broadcast(self.handle, t.data_ptr(), t.numel(), root, _stream()))
 
     def last_times(self):
         s = StageTimes()
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_last_times(self.handle, ctypes.byref(s)))
         return dict(comm_ms=s.comm_ms, spmm_ms=s.spmm_ms, total_ms=s.total_ms, stages=s.stages)
 
     def peer_alloc(self, floats):
         """Allocates this rank's two send buffers of the peer-copy loop; returns their CUDA IPC handles (128 bytes)."""
         buf = ctypes.create_string_buffer(128)
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_peer_alloc(self.handle, int(floats), buf))
         return buf.raw
 
@@ -346,11 +403,11 @@ class Comm:
         blob = b''.join(handles)
         if len(blob) != 128 * self.size:
             raise RuntimeError(f'expected {self.size} handle records of 128 bytes')
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_peer_open(self.handle, blob))
 
     def peer_close(self):
-        with torch.cuda.device(self.device):
+        with _on(self.device.index):
             check(lib().dg_comm_peer_close(self.handle))
 
     def peer_capacity(self):
@@ -382,7 +439,7 @@ def bcast_spmm(comm, roots, plans, x_local, recv, z, row_comm=None, timed=False,
             raise RuntimeError('receive buffer smaller than one group of blocks')
     recv_arr = (ctypes.c_void_p * max(len(recv), 1))(*[b.data_ptr() for b in recv])
     args = (S, roots_arr, group, plan_arr, val_arr, x_local.data_ptr(), n, F, recv_arr, len(recv), z.data_ptr(), int(timed), _stream())
-    with torch.cuda.device(x_local.device):
+    with _on(x_local.device.index):
         if row_comm is None:
             check(lib().dg_bcast_spmm_1d(comm.handle if comm else None, *args))
         else:
@@ -410,7 +467,7 @@ def bcast_spmm_ordered(comm, roots, landing, products, x_local, z, row_comm=None
             raise RuntimeError(f'operand {tuple(operand.shape)} does not match a plan with {plan.k} columns and width {F}')
     op_arr = (ctypes.c_void_p * max(P, 1))(*[t.data_ptr() for _, t, _ in products])
     last_arr = (ctypes.c_int32 * max(P, 1))(*[l for _, _, l in products])
-    with torch.cuda.device(x_local.device):
+    with _on(x_local.device.index):
         if peer_copies:
             check(lib().dg_peer_spmm(comm.handle, row_comm.handle if row_comm else None, S, roots_arr, land_arr, P, plan_arr,
                                      val_arr, op_arr, last_arr, x_local.data_ptr(), n, F, z.data_ptr(), int(timed), _stream()))
@@ -455,7 +512,7 @@ def peer_spmm_packed(comm, packs, roots, stage_offsets, stage_rows, landing, pro
     val_arr = (ctypes.c_void_p * max(P, 1))(*[p.values.data_ptr() for p, _, _ in products])
     op_arr = (ctypes.c_void_p * max(P, 1))(*[t.data_ptr() for _, t, _ in products])
     last_arr = (ctypes.c_int32 * max(P, 1))(*[l for _, _, l in products])
-    with torch.cuda.device(x_local.device):
+    with _on(x_local.device.index):
         check(lib().dg_peer_spmm_packed(comm.handle, row_comm.handle if row_comm else None, Q, pr, pc, po, S, roots_arr, so, sr, land_arr,
                                         P, plan_arr, val_arr, op_arr, last_arr, x_local.data_ptr(), n, F, z.data_ptr(), int(timed), _stream()))
     return z
@@ -487,7 +544,7 @@ def peer_spmm_gather(comm, roots, stage_lists, stage_rows, landing, products, x_
     val_arr = (ctypes.c_void_p * max(P, 1))(*[p.values.data_ptr() for p, _, _ in products])
     op_arr = (ctypes.c_void_p * max(P, 1))(*[t.data_ptr() for _, t, _ in products])
     last_arr = (ctypes.c_int32 * max(P, 1))(*[l for _, _, l in products])
-    with torch.cuda.device(x_local.device):
+    with _on(x_local.device.index):
         check(lib().dg_peer_spmm_gather(comm.handle, row_comm.handle if row_comm else None, S, roots_arr, lists_arr, sr, land_arr,
                                         P, plan_arr, val_arr, op_arr, last_arr, x_local.data_ptr(), n, F, z.data_ptr(), int(timed), _stream()))
     return z
@@ -518,10 +575,23 @@ def allgather_spmm(comm, plan, x_local, pack, area, z, widths, timed=False):
             raise RuntimeError(f'{what} buffer too small')
     pack_arr = (ctypes.c_void_p * 2)(pack[0].data_ptr(), pack[1].data_ptr())
     area_arr = (ctypes.c_void_p * 2)(area[0].data_ptr(), area[1].data_ptr())
-    with torch.cuda.device(x_local.device):
+    with _on(x_local.device.index):
         check(lib().dg_allgather_spmm(comm.handle, plan.handle, plan.values.data_ptr(), x_local.data_ptr(), n, F, len(widths), w_arr,
                                       pack_arr, area_arr, z.data_ptr(), int(timed), _stream()))
     return z
+
+
+def pad_rows(src, dst):
+    """dst[:, :c] = src, dst[:, c:] = 0 in one launch (dg_pad_rows): src [n x c] row-major, dst [n x w] contiguous, w >= c."""
+    ld = _row_major(src, 'src')
+    _dev_tensor(dst, torch.float32, 'dst')
+    (n, c), w = src.shape, dst.size(1)
+    if dst.size(0) != n or w < c:
+        raise RuntimeError(f'cannot pad {tuple(src.shape)} to {tuple(dst.shape)}')
+    index = dst.device.index
+    with _on(index):
+        check(lib().dg_pad_rows(src.data_ptr(), ld, n, c, dst.data_ptr(), w, _raw_stream(index)))
+    return dst
 
 
 def dense_split(w):
@@ -530,7 +600,7 @@ def dense_split(w):
     global dense_launches
     dense_launches += 1
     head, tail = torch.empty_like(w), torch.empty_like(w)
-    with torch.cuda.device(w.device):
+    with _on(w.device.index):
         check(lib().dg_dense_split(w.data_ptr(), head.data_ptr(), tail.data_ptr(), w.numel(), _stream()))
     return head, tail
 
@@ -553,13 +623,18 @@ def split_operand(w, transposed, cache_key=None):
         hit = slot.get(transposed)
         if hit is not None and hit[0] == cache_key._version and hit[1].device == w.device:
             return hit[1], hit[2]
-    bt = w.detach().t() if transposed else w.detach()
-    N, K = bt.shape
-    if K % 4 or not bt.is_contiguous():
-        wide = torch.zeros((N, K + (-K) % 4), dtype=torch.float32, device=w.device)
-        wide[:, :K] = bt
-        bt = wide
-    head, tail = dense_split(bt)
+    w = w.detach()
+    if w.stride(1) != 1 or w.stride(0) < w.size(1):
+        w = w.contiguous()
+    N, K = (w.size(1), w.size(0)) if transposed else w.shape
+    ldb = K + (-K) % 4
+    pair = torch.empty((2, N, ldb), dtype=torch.float32, device=w.device)
+    head, tail = pair[0], pair[1]
+    global dense_launches
+    dense_launches += 1
+    index = w.device.index
+    with _on(index):
+        check(_lib.dg_dense_split_operand(w.data_ptr(), w.stride(0), transposed, N, K, head.data_ptr(), tail.data_ptr(), ldb, _raw_stream(index)))
     if cache_key is not None:
         slot[transposed] = (cache_key._version, head, tail)
     return head, tail
@@ -571,6 +646,7 @@ def dense_nt(a, b, transposed=False, relu=False, mask=None, cache_key=None):
     caller then uses a library GEMM).  relu applies max(x, 0) on the way out; mask [M x N] zeroes the result where
     mask <= 0 (the backward of a ReLU whose output is `mask`); cache_key: see split_operand."""
     lda = _row_major(a, 'a')
+    lib()
     if not (isinstance(b, torch.Tensor) and b.is_cuda and b.dtype == torch.float32 and b.dim() == 2):
         raise RuntimeError('b must be a 2-D fp32 CUDA tensor: this library has no CPU path')
     M, K = a.shape
@@ -580,16 +656,19 @@ def dense_nt(a, b, transposed=False, relu=False, mask=None, cache_key=None):
     ldm = _row_major(mask, 'mask') if mask is not None else 0
     if mask is not None and tuple(mask.shape) != (M, N):
         raise RuntimeError(f'mask is {tuple(mask.shape)}, the product {(M, N)}')
-    ldb = K + (-K) % 4
-    if M == 0 or N == 0 or not lib().dg_dense_supported(M, N, K, lda, ldb, a.data_ptr(), None, None):
+    if M == 0 or N == 0 or K == 0 or lda % 4 or a.data_ptr() % 16 or M >= 1 << 31:
         return None
     head, tail = split_operand(b, transposed, cache_key)
+    c = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    index = a.device.index
+    with _on(index):
+        code = _lib.dg_dense_nt_masked(a.data_ptr(), lda, head.data_ptr(), tail.data_ptr(), head.size(1), c.data_ptr(), N, M, N, K, relu,
+                                       mask.data_ptr() if mask is not None else None, ldm, _raw_stream(index))
+    if code == ERR_UNSUPPORTED:
+        return None
+    check(code)
     global dense_launches
     dense_launches += (N + 255) // 256
-    c = torch.empty((M, N), dtype=torch.float32, device=a.device)
-    with torch.cuda.device(a.device):
-        check(lib().dg_dense_nt_masked(a.data_ptr(), lda, head.data_ptr(), tail.data_ptr(), ldb, c.data_ptr(), N, M, N, K, int(relu),
-                                       mask.data_ptr() if mask is not None else None, ldm, _stream()))
     return c
 
 
@@ -600,22 +679,25 @@ def dense_tn(x, g):
     """x[n x Km]^T @ g[n x Nn] on the tensor cores with fp32 accuracy (dg_dense_tn), or None when the shapes or strides
     are outside what the kernel takes.  Both operands are streamed once; per-CTA partial results are added in CTA order."""
     ldx, ldg = _row_major(x, 'x'), _row_major(g, 'g')
+    lib()
     n, Km = x.shape
     Nn = g.size(1)
     if g.size(0) != n:
         raise RuntimeError(f'row counts differ: {tuple(x.shape)} vs {tuple(g.shape)}')
-    if n == 0 or not lib().dg_dense_tn_supported(n, Km, Nn, ldx, ldg, x.data_ptr(), g.data_ptr()):
+    if not lib().dg_dense_tn_supported(n, Km, Nn, ldx, ldg, x.data_ptr(), g.data_ptr()):
         return None
-    ctas = torch.cuda.get_device_properties(x.device).multi_processor_count
-    scratch = _tn_scratch.get(x.device)
+    index = x.device.index
+    scratch, ctas = _tn_scratch.get(index, (None, 0))
     if scratch is None:
-        scratch = _tn_scratch[x.device] = torch.empty(ctas * 256 * 256, dtype=torch.float32, device=x.device)
+        ctas = torch.cuda.get_device_properties(x.device).multi_processor_count
+        scratch = torch.empty(ctas * 256 * 256, dtype=torch.float32, device=x.device)
+        _tn_scratch[index] = (scratch, ctas)
     global dense_launches
     dense_launches += 2 * ((Km + 255) // 256) * ((Nn + 255) // 256)      # per 256 x 256 panel: the product and the reduction over the CTAs' partials
     d = torch.empty((Km, Nn), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        check(lib().dg_dense_tn(x.data_ptr(), ldx, g.data_ptr(), ldg, d.data_ptr(), Nn, n, Km, Nn, scratch.data_ptr(), scratch.numel(),
-                                ctas, _stream()))
+    with _on(index):
+        check(_lib.dg_dense_tn(x.data_ptr(), ldx, g.data_ptr(), ldg, d.data_ptr(), Nn, n, Km, Nn, scratch.data_ptr(), scratch.numel(),
+                               ctas, _raw_stream(index)))
     return d
 
 

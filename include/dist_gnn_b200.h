@@ -249,6 +249,10 @@ int dg_comm_last_times(dg_comm* comm, dg_stage_times* host_out);
  * memory, waits a few thousand polls on a barrier nothing arrives at, reports that the wait ran out (*host_gave_up = 1),
  * frees its tensor memory and returns; the status word of the real kernels is not touched. */
 int dg_dense_split(const float* src, float* head, float* tail, int64_t count, void* stream);
+/* The same for a whole operand of dg_dense_nt in one launch: Bt [N x K] is w as given (transposed == 0, ldw >= K) or the
+ * transpose of w [K x N] (transposed != 0, ldw >= N); head and tail get rows of ldb >= K floats, zero beyond column K. */
+int dg_dense_split_operand(const float* w, int64_t ldw, int32_t transposed, int32_t N, int32_t K, float* head, float* tail,
+                           int64_t ldb, void* stream);
 int dg_dense_supported(int64_t M, int32_t N, int32_t K, int64_t lda, int64_t ldb, const void* A, const void* Bt_head, const void* Bt_tail);
 int dg_dense_nt(const float* A, int64_t lda, const float* Bt_head, const float* Bt_tail, int64_t ldb, float* C, int64_t ldc,
                 int64_t M, int32_t N, int32_t K, int32_t relu, void* stream);
@@ -281,6 +285,18 @@ int dg_dense_wait_selftest(int* host_gave_up, void* stream);
  * algorithmic traffic  8*nnz + 4*(m+1) + 4*F*touched_columns + 4*F*m*(1 + [beta != 0])  in bytes, the no-reuse gather
  * volume  8*nnz + 4*(m+1) + 4*F*nnz + 4*F*m*(1 + [beta != 0]),  2*nnz*F flops, and how many kernels of this library
  * were launched (products only; NCCL's own kernels are not counted). */
+/* dst[i, 0..cols) = src[i, 0..cols), dst[i, cols..ld_dst) = 0 for n rows: an operand whose rows are not 16-byte multiples is
+ * copied once into rows that are (ld_dst a multiple of 4, dst 16-byte aligned). */
+int dg_pad_rows(const float* src, int64_t ld_src, int64_t n, int32_t cols, float* dst, int64_t ld_dst, void* stream);
+
+/* Time marks: CUDA events from a pool, named by small ids, for timers around regions that are too short for anything
+ * dearer.  dg_mark_record records one on `stream` (a stream of the current device) and returns its id, or a negative
+ * DG_ERR_*; dg_mark_elapsed gives the milliseconds between two recorded marks that have both been reached (cudaErrorNotReady
+ * otherwise); dg_mark_release puts a mark back into the pool. */
+int dg_mark_record(void* stream);
+int dg_mark_elapsed(int begin, int end, float* host_ms);
+int dg_mark_release(int id);
+
 typedef struct dg_profile {
     double spmm_ms;
     double alg_bytes;

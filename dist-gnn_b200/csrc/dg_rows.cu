@@ -1,6 +1,8 @@
 // Row-wise helpers either side of the distributed SpMM.
 #include "dg_internal.h"
 
+#define DG_ROWS_LOSS_PARTS (148 * 8)      // most CTAs of the loss, and the partial sums they leave
+
 namespace {
 
 // One 16-byte piece of a destination row per thread: 4 source floats (neighbouring threads read neighbouring floats), one
@@ -22,7 +24,155 @@ __global__ void __launch_bounds__(256) k_pad_rows(const float* __restrict__ src,
     }
 }
 
+// ---- mean cross-entropy over the rows that carry a target --------------------------------------------------------------
+// The step's loss reads the logits of the train rows once and its gradient reads them once more and writes n x C floats:
+// memory bound, 12 bytes per row and class.  As separate passes (row gather, log-softmax, a one-CTA loss reduction, its
+// backward, the softmax backward, a scatter into zeros) it took 5.5 ms of a 66 ms step at 2,449,029 x 47.
+// A group of LPR lanes owns a row; lanes read neighbouring classes.  Sums are taken in a fixed order (rows of a thread in
+// order, lanes and warps by a tree, CTAs in order), so the loss is bit-reproducible.
+constexpr int kLossThreads = 256;
+
+template <int LPR> __device__ __forceinline__ float group_max(float v)
+{
+#pragma unroll
+    for (int off = LPR / 2; off > 0; off >>= 1) {
+        const float o = __shfl_xor_sync(0xffffffffu, v, off);
+        v = o > v || o != o ? o : v;
+    }
+    return v;
+}
+template <int LPR> __device__ __forceinline__ float group_sum(float v)
+{
+#pragma unroll
+    for (int off = LPR / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
+}
+
+template <int LPR>
+__global__ void __launch_bounds__(kLossThreads) k_rows_ce_forward(const float* __restrict__ x, int64_t ld, int64_t n, int32_t C,
+                                                                  const int32_t* __restrict__ target, float* __restrict__ lse,
+                                                                  double* __restrict__ partial)
+{
+    constexpr int RPB = kLossThreads / LPR;
+    const int lane = threadIdx.x % LPR;
+    double loss = 0.0;
+    for (int64_t base = (int64_t)blockIdx.x * RPB; base < n; base += (int64_t)gridDim.x * RPB) {
+        const int64_t row = base + threadIdx.x / LPR;
+        const int32_t t = row < n ? __ldg(target + row) : -1;
+        const bool on = t >= 0;                                   // the same in every lane of a row's group
+        const float* r = x + row * ld;
+        float mx = __int_as_float(0xff800000);
+        if (on)
+            for (int c = lane; c < C; c += LPR) {
+                const float v = __ldg(r + c);
+                mx = v > mx || v != v ? v : mx;                   // a NaN stays
+            }
+        mx = group_max<LPR>(mx);
+        float sum = 0.f;
+        if (on)
+            for (int c = lane; c < C; c += LPR) sum += expf(__ldg(r + c) - mx);
+        sum = group_sum<LPR>(sum);
+        if (on && lane == 0) {
+            const float l = logf(sum);
+            lse[row] = mx + l;
+            loss += (double)(l - (__ldg(r + t) - mx));
+        }
+    }
+    __shared__ double warp_sum[kLossThreads / 32];
+    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = loss;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < kLossThreads / 32; ++w) s += warp_sum[w];
+        partial[blockIdx.x] = s;
+    }
+}
+
+__global__ void __launch_bounds__(kLossThreads) k_rows_ce_mean(const double* __restrict__ partial, int parts, double inv_count, float* __restrict__ loss)
+{
+    __shared__ double warp_sum[kLossThreads / 32];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < parts; i += kLossThreads) s += partial[i];
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.0;
+        for (int w = 0; w < kLossThreads / 32; ++w) s += warp_sum[w];
+        *loss = (float)(s * inv_count);
+    }
+}
+
+// grad[row, c] = (softmax(x[row])[c] - [c == target]) * upstream / count, zero for rows without a target and beyond C.
+template <int LPR>
+__global__ void __launch_bounds__(kLossThreads) k_rows_ce_backward(const float* __restrict__ x, int64_t ld, int64_t n, int32_t C,
+                                                                   const int32_t* __restrict__ target, const float* __restrict__ lse,
+                                                                   const float* __restrict__ upstream, float inv_count,
+                                                                   float* __restrict__ grad, int64_t ldg)
+{
+    constexpr int RPB = kLossThreads / LPR;
+    const int lane = threadIdx.x % LPR;
+    const float scale = __ldg(upstream) * inv_count;
+    for (int64_t row = (int64_t)blockIdx.x * RPB + threadIdx.x / LPR; row < n; row += (int64_t)gridDim.x * RPB) {
+        const int32_t t = __ldg(target + row);
+        const float l = t >= 0 ? __ldg(lse + row) : 0.f;
+        const float* r = x + row * ld;
+        float* g = grad + row * ldg;
+        for (int c = lane; c < ldg; c += LPR) {
+            float v = 0.f;
+            if (t >= 0 && c < C) v = (expf(__ldg(r + c) - l) - (c == t ? 1.f : 0.f)) * scale;
+            g[c] = v;
+        }
+    }
+}
+
+// Lanes per row: the least power of two that leaves a lane no more than four classes, 4 to 32.
+int lanes_per_row(int32_t C) { return C <= 16 ? 4 : C <= 32 ? 8 : C <= 64 ? 16 : 32; }
+
+unsigned loss_blocks(int64_t n, int lpr)
+{
+    const int64_t rows_per_block = kLossThreads / lpr, blocks = (n + rows_per_block - 1) / rows_per_block;
+    return (unsigned)(blocks < DG_ROWS_LOSS_PARTS ? blocks : DG_ROWS_LOSS_PARTS);
+}
+
 }  // namespace
+
+extern "C" int dg_rows_cross_entropy(const float* x, int64_t ld, int64_t n, int32_t C, const int32_t* target, int64_t count, float* lse,
+                                     double* scratch, float* loss, void* stream)
+{
+    if (n <= 0 || C <= 0 || count <= 0 || ld < C) return DG_ERR_DIMS;
+    if (!x || !target || !lse || !scratch || !loss) return DG_ERR_NULL;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int lpr = lanes_per_row(C);
+    const unsigned blocks = loss_blocks(n, lpr);
+    switch (lpr) {
+        case 4: k_rows_ce_forward<4><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
+        case 8: k_rows_ce_forward<8><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
+        case 16: k_rows_ce_forward<16><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
+        default: k_rows_ce_forward<32><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
+    }
+    k_rows_ce_mean<<<1, kLossThreads, 0, s>>>(scratch, (int)blocks, 1.0 / (double)count, loss);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int dg_rows_cross_entropy_grad(const float* x, int64_t ld, int64_t n, int32_t C, const int32_t* target, int64_t count,
+                                          const float* lse, const float* upstream, float* grad, int64_t ldg, void* stream)
+{
+    if (n <= 0 || C <= 0 || count <= 0 || ld < C || ldg < C) return DG_ERR_DIMS;
+    if (!x || !target || !lse || !upstream || !grad) return DG_ERR_NULL;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int lpr = lanes_per_row(C);
+    const unsigned blocks = loss_blocks(n, lpr);
+    const float inv = (float)(1.0 / (double)count);
+    switch (lpr) {
+        case 4: k_rows_ce_backward<4><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
+        case 8: k_rows_ce_backward<8><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
+        case 16: k_rows_ce_backward<16><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
+        default: k_rows_ce_backward<32><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
+    }
+    return (int)cudaGetLastError();
+}
 
 extern "C" int dg_pad_rows(const float* src, int64_t ld_src, int64_t n, int32_t cols, float* dst, int64_t ld_dst, void* stream)
 {
@@ -34,3 +184,5 @@ extern "C" int dg_pad_rows(const float* src, int64_t ld_src, int64_t n, int32_t 
     k_pad_rows<<<(unsigned)(blocks < 148 * 32 ? blocks : 148 * 32), 256, 0, (cudaStream_t)stream>>>(src, ld_src, n, cols, dst, (int32_t)(ld_dst / 4));
     return (int)cudaGetLastError();
 }
+
+extern "C" int32_t dg_rows_loss_scratch(void) { return DG_ROWS_LOSS_PARTS; }

@@ -22,16 +22,42 @@ def f1(y_true, y_pred, multilabel=True):
 
 def local_loss(g, outputs, loss_func):
     """Mean loss over this rank's LOCAL train rows (dist_train.py:39-43); a rank without train rows still
-    back-propagates a zero so that it takes part in every collective."""
+    back-propagates a zero so that it takes part in every collective.  The plain cross-entropy of class labels runs as
+    one pass over the logits (spmm_cpp.RowCrossEntropy); any other loss function gets the gathered train rows."""
     cached = getattr(g, '_train_rows', None)
     if cached is None:      # the mask never changes: find the rows once instead of a host sync per epoch
         rows = g.local_train_mask.nonzero().squeeze(1)
         cached = g._train_rows = (rows, g.local_labels[rows])
     rows, labels = cached
     if rows.numel() > 0:
+        targets = _class_targets(g, outputs, loss_func, rows, labels)
+        if targets is not None:
+            return spmm_cpp.RowCrossEntropy.apply(outputs, *targets)
         return loss_func(outputs.index_select(0, rows), labels)
     DistEnv.env.logger.log('Warning: no training nodes in this partition! Backward fake loss.')
     return (outputs * 0).sum()
+
+
+def _class_targets(g, outputs, loss_func, rows, labels):
+    """(target class of every local row or -1, number of rows that have one) when loss_func is the unweighted mean
+    cross-entropy of valid class labels on fp32 logits of this GPU, else None.  The targets are kept like the train rows."""
+    if not (type(loss_func) is nn.CrossEntropyLoss and loss_func.weight is None and loss_func.reduction == 'mean'
+            and loss_func.label_smoothing == 0.0 and outputs.is_cuda and outputs.dtype == torch.float32 and outputs.dim() == 2
+            and outputs.stride(1) == 1 and outputs.stride(0) >= outputs.size(1) and not torch.is_autocast_enabled('cuda')):
+        return None
+    cached = getattr(g, '_train_targets', None)
+    if cached is None or cached[0] != loss_func.ignore_index:
+        used = labels != loss_func.ignore_index
+        count = int(used.sum())
+        valid = labels.dim() == 1 and labels.dtype == torch.long and count > 0 and int(labels[used].min()) >= 0
+        targets = torch.full((g.local_train_mask.numel(),), -1, dtype=torch.int32, device=labels.device)
+        if valid:
+            targets[rows[used]] = labels[used].to(torch.int32)
+        cached = g._train_targets = (loss_func.ignore_index, targets, count, int(labels[used].max()) if valid else 2**31)
+    _, targets, count, highest = cached
+    if highest >= outputs.size(1) or outputs.size(0) != targets.numel() or targets.device != outputs.device:
+        return None         # labels that are no classes of these logits: the loss function reports them
+    return targets, count
 
 
 def train(g, env, total_epoch, hidden_dim=256, num_layers=3, weights=None, log_every=10, **model_options):

@@ -93,6 +93,9 @@ def lib():
             'dg_dense_status_reset': ([vp], ctypes.c_int),
             'dg_dense_wait_selftest': ([ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
             'dg_pad_rows': ([vp, i64, i64, i32, vp, i64, vp], ctypes.c_int),
+            'dg_rows_loss_scratch': ([], i32),
+            'dg_rows_cross_entropy': ([vp, i64, i64, i32, vp, i64, vp, vp, vp, vp], ctypes.c_int),
+            'dg_rows_cross_entropy_grad': ([vp, i64, i64, i32, vp, i64, vp, vp, vp, i64, vp], ctypes.c_int),
             'dg_mark_record': ([vp], ctypes.c_int),
             'dg_mark_elapsed': ([ctypes.c_int, ctypes.c_int, ctypes.POINTER(f32)], ctypes.c_int),
             'dg_mark_release': ([ctypes.c_int], ctypes.c_int),
@@ -592,6 +595,41 @@ def pad_rows(src, dst):
     with _on(index):
         check(lib().dg_pad_rows(src.data_ptr(), ld, n, c, dst.data_ptr(), w, _raw_stream(index)))
     return dst
+
+
+class RowCrossEntropy(torch.autograd.Function):
+    """apply(x, targets, count): mean cross-entropy of x [n x C] over the rows with targets[i] >= 0 (int32, all below C), of
+    which there are `count` (dg_rows_cross_entropy).  The gradient's rows are padded to whole 16-byte pieces, which is
+    what the products behind it read."""
+
+    @staticmethod
+    def forward(ctx, x, targets, count):
+        ld = _row_major(x, 'logits')
+        n, C = x.shape
+        _dev_tensor(targets, torch.int32, 'targets')
+        index, parts = x.device.index, lib().dg_rows_loss_scratch()
+        work = torch.empty(2 * parts + n + 1, dtype=torch.float32, device=x.device)       # partial sums, logsumexp per row, loss
+        base = work.data_ptr()
+        loss = work[2 * parts + n]
+        with _on(index):
+            check(_lib.dg_rows_cross_entropy(x.data_ptr(), ld, n, C, targets.data_ptr(), count, base + 8 * parts, base, loss.data_ptr(),
+                                             _raw_stream(index)))
+        ctx.save_for_backward(x, targets, work)
+        ctx.count, ctx.parts = count, parts
+        return loss.clone()
+
+    @staticmethod
+    def backward(ctx, upstream):
+        x, targets, work = ctx.saved_tensors
+        n, C = x.shape
+        width = C + (-C) % 4
+        grad = torch.empty((n, width), dtype=torch.float32, device=x.device)
+        index = x.device.index
+        with _on(index):
+            check(_lib.dg_rows_cross_entropy_grad(x.data_ptr(), _row_major(x, 'logits'), n, C, targets.data_ptr(), ctx.count,
+                                                  work.data_ptr() + 8 * ctx.parts, upstream.contiguous().data_ptr(), grad.data_ptr(), width,
+                                                  _raw_stream(index)))
+        return grad if width == C else grad[:, :C], None, None
 
 
 def dense_split(w):

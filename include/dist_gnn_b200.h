@@ -289,6 +289,17 @@ int dg_dense_wait_selftest(int* host_gave_up, void* stream);
  * copied once into rows that are (ld_dst a multiple of 4, dst 16-byte aligned). */
 int dg_pad_rows(const float* src, int64_t ld_src, int64_t n, int32_t cols, float* dst, int64_t ld_dst, void* stream);
 
+/* Mean cross-entropy over the rows with a target (replaces the loss of light_dist_gnn/dist_train.py:39-43 on the local train
+ * rows): loss = sum over rows with target[i] >= 0 of (logsumexp(x[i, 0..C)) - x[i, target[i]]) / count, where count is the
+ * number of such rows and every target is below C.  lse (n floats) keeps the rows' logsumexp for the gradient; scratch holds
+ * dg_rows_loss_scratch() doubles.  The gradient is (softmax - onehot) * upstream / count (upstream: one float on the device),
+ * zero in rows without a target and in columns C..ldg.  Bit-reproducible. */
+int32_t dg_rows_loss_scratch(void);
+int dg_rows_cross_entropy(const float* x, int64_t ld, int64_t n, int32_t C, const int32_t* target, int64_t count, float* lse,
+                          double* scratch, float* loss, void* stream);
+int dg_rows_cross_entropy_grad(const float* x, int64_t ld, int64_t n, int32_t C, const int32_t* target, int64_t count,
+                               const float* lse, const float* upstream, float* grad, int64_t ldg, void* stream);
+
 /* Time marks: CUDA events from a pool, named by small ids, for timers around regions that are too short for anything
  * dearer.  dg_mark_record records one on `stream` (a stream of the current device) and returns its id, or a negative
  * DG_ERR_*; dg_mark_elapsed gives the milliseconds between two recorded marks that have both been reached (cudaErrorNotReady

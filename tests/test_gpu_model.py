@@ -351,3 +351,24 @@ def test_transform_first_matches_within_rounding(golden, env1):
         assert_close(b.detach().cpu().numpy(), a.detach().cpu().numpy(), 1e-4, 'weights with transform_first')
     with torch.no_grad():
         assert_close(first_model(g.features).cpu().numpy(), plain_model(g.features).cpu().numpy(), 1e-4, 'outputs')
+
+
+@pytest.mark.parametrize('n,C,ld', [(1, 1, 1), (37, 2, 2), (1000, 10, 12), (5003, 47, 47), (999, 41, 44), (700, 64, 64), (300, 130, 130)])
+def test_row_cross_entropy_matches_the_library_loss(n, C, ld):
+    """The one-pass loss over the rows with a target and its gradient against the float64 loss of the gathered rows, for
+    every lane split, with rows that carry no target and a scaled upstream gradient."""
+    import spmm_cpp
+    gen = torch.Generator(device='cuda').manual_seed(n + C)
+    x = (torch.randn(n, ld, device='cuda', generator=gen) * 3)[:, :C].requires_grad_(True)
+    t = torch.randint(0, C, (n,), device='cuda', generator=gen, dtype=torch.int32)
+    t[torch.rand(n, device='cuda', generator=gen) < 0.4] = -1
+    t[0] = C - 1
+    rows = (t >= 0).nonzero().squeeze(1)
+    loss = spmm_cpp.RowCrossEntropy.apply(x, t, rows.numel())
+    grad, = torch.autograd.grad(loss * 2.5, x)
+    xd = x.detach().double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(xd[rows], t[rows].long())
+    want_grad, = torch.autograd.grad(want * 2.5, xd)
+    assert abs(loss.item() - want.item()) <= 1e-6 * max(1.0, abs(want.item()))
+    assert_close(grad.cpu().numpy(), want_grad.cpu().numpy(), TOL, 'gradient of the loss')
+    assert torch.equal(loss, spmm_cpp.RowCrossEntropy.apply(x, t, rows.numel()))

@@ -480,27 +480,38 @@ __global__ void k_tf32_split(const float* __restrict__ src, float* __restrict__ 
     tail[i] = x - h;
 }
 
-// Head and tail of a whole operand, transposed on the way where asked (32 x 32 tiles through shared memory, so that both
-// sides are coalesced), rows zero-filled up to ldb.
-__global__ void __launch_bounds__(256) k_tf32_split_operand(const float* __restrict__ w, int64_t ldw, int transposed, int N, int K,
-                                                            float* __restrict__ head, float* __restrict__ tail, int64_t ldb)
+// Heads and tails of whole operands, transposed on the way where asked (32 x 32 tiles through shared memory, so that both
+// sides are coalesced), rows zero-filled up to ldb.  One launch splits every weight of a network: the operands are a few
+// hundred kilobytes, so a launch each costs more than the work.
+constexpr int kSplitJobs = 16;
+struct SplitJobs {
+    dg_split_job job[kSplitJobs];
+    int first_tile[kSplitJobs + 1];                               // running count of 32 x 32 tiles
+    int count;
+};
+
+__global__ void __launch_bounds__(256) k_tf32_split_operands(const __grid_constant__ SplitJobs jobs)
 {
     __shared__ float tile[32][33];
-    const int k0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
+    int j = 0;
+    while (j + 1 < jobs.count && (int)blockIdx.x >= jobs.first_tile[j + 1]) ++j;
+    const dg_split_job& s = jobs.job[j];
+    const int local = (int)blockIdx.x - jobs.first_tile[j], k_tiles = (int)((s.ldb + 31) / 32);
+    const int k0 = local % k_tiles * 32, n0 = local / k_tiles * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int r = ty; r < 32; r += 8) {
-        const int n = transposed ? n0 + tx : n0 + r, k = transposed ? k0 + r : k0 + tx;
-        const float x = n < N && k < K ? w[transposed ? (int64_t)k * ldw + n : (int64_t)n * ldw + k] : 0.f;
-        if (transposed) tile[tx][r] = x; else tile[r][tx] = x;
+        const int n = s.transposed ? n0 + tx : n0 + r, k = s.transposed ? k0 + r : k0 + tx;
+        const float x = n < s.N && k < s.K ? s.w[s.transposed ? (int64_t)k * s.ldw + n : (int64_t)n * s.ldw + k] : 0.f;
+        if (s.transposed) tile[tx][r] = x; else tile[r][tx] = x;
     }
     __syncthreads();
     for (int r = ty; r < 32; r += 8) {
         const int n = n0 + r, k = k0 + tx;
-        if (n >= N || k >= ldb) continue;
+        if (n >= s.N || k >= s.ldb) continue;
         const float x = tile[r][tx];
         const float h = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-        head[(int64_t)n * ldb + k] = h;
-        tail[(int64_t)n * ldb + k] = x - h;
+        s.head[(int64_t)n * s.ldb + k] = h;
+        s.tail[(int64_t)n * s.ldb + k] = x - h;
     }
 }
 
@@ -588,14 +599,28 @@ extern "C" int dg_dense_split(const float* src, float* head, float* tail, int64_
     return (int)cudaGetLastError();
 }
 
-extern "C" int dg_dense_split_operand(const float* w, int64_t ldw, int32_t transposed, int32_t N, int32_t K, float* head, float* tail,
-                                      int64_t ldb, void* stream)
+extern "C" int dg_dense_split_operands(const dg_split_job* host_jobs, int32_t count, void* stream)
 {
-    if (N < 0 || K < 0 || ldb < K || ldw < (transposed ? N : K)) return DG_ERR_DIMS;
-    if (N == 0 || K == 0) return DG_OK;
-    if (!w || !head || !tail) return DG_ERR_NULL;
-    const dim3 grid((unsigned)((ldb + 31) / 32), (unsigned)((N + 31) / 32));
-    k_tf32_split_operand<<<grid, 256, 0, (cudaStream_t)stream>>>(w, ldw, transposed != 0, N, K, head, tail, ldb);
+    if (count < 0) return DG_ERR_DIMS;
+    if (count > 0 && !host_jobs) return DG_ERR_NULL;
+    for (int32_t i = 0; i < count; ++i) {
+        const dg_split_job& s = host_jobs[i];
+        if (s.N < 0 || s.K < 0 || s.ldb < s.K || s.ldb >= ((int64_t)1 << 24) || s.ldw < (s.transposed ? s.N : s.K)) return DG_ERR_DIMS;
+        if (s.N > 0 && s.K > 0 && (!s.w || !s.head || !s.tail)) return DG_ERR_NULL;
+    }
+    for (int32_t i0 = 0; i0 < count; i0 += kSplitJobs) {
+        SplitJobs jobs{};
+        int64_t tiles = 0;
+        for (int32_t i = i0; i < count && i < i0 + kSplitJobs; ++i) {
+            if (host_jobs[i].N == 0 || host_jobs[i].K == 0) continue;
+            jobs.job[jobs.count] = host_jobs[i];
+            jobs.first_tile[jobs.count++] = (int)tiles;
+            tiles += (host_jobs[i].ldb + 31) / 32 * ((host_jobs[i].N + 31) / 32);
+            if (tiles >= ((int64_t)1 << 31)) return DG_ERR_UNSUPPORTED;
+            jobs.first_tile[jobs.count] = (int)tiles;
+        }
+        if (tiles > 0) k_tf32_split_operands<<<(unsigned)tiles, 256, 0, (cudaStream_t)stream>>>(jobs);
+    }
     return (int)cudaGetLastError();
 }
 

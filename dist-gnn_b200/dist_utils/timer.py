@@ -80,6 +80,15 @@ class DistTimer:
             self._mark = spmm_cpp.mark
         return CudaTimerCtx(self, key, self._mark)
 
+    def add_regions(self, regions):
+        """Device regions whose marks were recorded elsewhere: (key, begin mark, end mark) each."""
+        for key, begin, end in regions:
+            if begin >= 0 and end >= 0:
+                self.pending.append((key, begin, end))
+            self.count_dict[key] += 1
+        if len(self.pending) >= self.MAX_PENDING:
+            self.resolve()
+
     def empty_region(self, key):
         """Counts a region in which this layout has nothing to do (a one-rank all-reduce)."""
         self.duration_dict[key] += 0.0

@@ -9,7 +9,9 @@ the reuse of the un-transposed row block of A in backward, which is exact only f
 
 There is no CPU implementation: CPU tensors raise.
 """
+import ctypes
 import os
+import weakref
 
 import torch
 import torch.nn as nn
@@ -56,7 +58,6 @@ def _rows(t, keep=False):
     wide = torch.empty((rows, cols + (-cols) % 4), dtype=t.dtype, device=t.device)
     view = _pad_into(t, wide)[:, :cols]
     if keep:
-        import weakref
         key = id(t)
         _padded_rows[key] = (weakref.ref(t, lambda _r, key=key: _padded_rows.pop(key, None)), t._version, view)
     return view
@@ -145,30 +146,34 @@ def _distributed_spmm(local_adj_parts, local_feature, constant=False):
     return z if z.size(1) == true_width else z[:, :true_width]
 
 
-def _local_products(env, adj_parts, t, constant):
-    """The stage loop of a rank without peers: its own products, straight on the operand wherever that lies (any row
-    stride of whole 16-byte pieces), else on a padded copy as above.  No communicator, no buffers, no argument tables:
-    on small graphs the host's share of a step is what a step costs."""
+def _product_operand(env, t, constant):
+    """t [n x w] as an operand whose rows are whole 16-byte pieces, [n x pad4(w)]: t itself wherever it lies (any row stride
+    of whole pieces; the columns beyond w are read and their results dropped), else a padded copy as above."""
     n, true_width = t.shape
     width = true_width + (-true_width) % 4 if PAD_ODD_WIDTHS else true_width
     ld = t.stride(0)
     if t.stride(1) == 1 and ld % 4 == 0 and ld >= width and t.data_ptr() % 16 == 0 and (
             width == true_width or t.storage_offset() + (n - 1) * ld + width <= t.untyped_storage().nbytes() // 4):
-        x = t if width == true_width else t.as_strided((n, width), (ld, 1))      # the columns beyond true_width are not looked at
-    elif width == true_width:
-        x = t.contiguous()
-    elif constant:
+        return t if width == true_width else t.as_strided((n, width), (ld, 1))
+    if width == true_width:
+        return t.contiguous()
+    if constant:
         kept = _rows(t, keep=True)
-        x = kept.as_strided((n, width), (kept.stride(0), 1))
-    else:
-        x = _pad_into(t, env.recv_buffers(n, width, nbuf=1, tag='padded')[0])
-    z = torch.empty((n, width), dtype=torch.float32, device=t.device)
+        return kept.as_strided((n, width), (kept.stride(0), 1))
+    return _pad_into(t, env.recv_buffers(n, width, nbuf=1, tag='padded')[0])
+
+
+def _local_products(env, adj_parts, t, constant):
+    """The stage loop of a rank without peers: its own products, straight on the operand.  No communicator, no buffers, no
+    argument tables: on small graphs the host's share of a step is what a step costs."""
+    x = _product_operand(env, t, constant)
+    z = torch.empty(x.shape, dtype=torch.float32, device=t.device)
     with env.timer.timing_cuda('broadcast+spmm'):
         beta = 0.0
         for st in env.stages():
             spmm_cpp.plan_for(adj_parts[st.part]).spmm(x, z, 1.0, beta)
             beta = 1.0
-    return z if width == true_width else z[:, :true_width]
+    return z if x.size(1) == t.size(1) else z[:, :t.size(1)]
 
 
 def _stage_loop(env, local_adj_parts, x, z, stages, comm, timed=False):
@@ -448,6 +453,76 @@ class DistGCNLayer(torch.autograd.Function):
         return (grad_features, grad_weight) + (None,) * 8
 
 
+class _OneRankGCN(torch.autograd.Function):
+    """All layers of a GCN on a rank without peers, forward and backward, from one library call each (dg_gcn_forward,
+    dg_gcn_backward): the products and transforms of the chained DistGCNLayers in the same order on the same operands, the
+    same bits, without the host's work between them."""
+
+    @staticmethod
+    def forward(ctx, env, plan, features, *weights):
+        n, L, device = features.size(0), len(weights), features.device
+        train = any(ctx.needs_input_grad)
+        dims = [features.size(1)] + [w.size(1) for w in weights]
+        pad = [d + (-d) % 4 for d in dims]
+        x = _product_operand(env, features, True)
+        splits = spmm_cpp.split_operands([(w, True, w) for w in weights] + ([(w, False, w) for w in weights[1:]] if train else []))
+        # hidden activations in one buffer: side by side while a backward pass will read them, else every layer over the last
+        starts = [n * sum(pad[1:l + 1]) if train else 0 for l in range(L - 1)]
+        hidden = torch.empty((n * sum(pad[1:L]) if train else n * max(pad[1:L])) if L > 1 else 0, dtype=torch.float32, device=device)
+        out = torch.empty((n, dims[L]), dtype=torch.float32, device=device)
+        base = hidden.data_ptr()
+        act = [base + 4 * s for s in starts] + [out.data_ptr()]
+        net, keep = _gcn_net(plan, x, dims, pad, act, pad[1:L] + [dims[L]])
+        z = torch.empty(n * max(pad[:L]), dtype=torch.float32, device=device)
+        heads = (ctypes.c_void_p * L)(*[s[1] for s in splits[:L]])
+        marks = (ctypes.c_int32 * (4 * L))(*[-1] * (4 * L))
+        net.z, net.fwd_split, net.marks = z.data_ptr(), ctypes.addressof(heads), ctypes.addressof(marks)
+        spmm_cpp.gcn_call('dg_gcn_forward', net, device.index)
+        spmm_cpp.dense_launches += sum((d + 255) // 256 for d in dims[1:])
+        env.timer.add_regions([r for l in range(L) for r in (('broadcast+spmm', marks[4 * l], marks[4 * l + 1]), ('mm', marks[4 * l + 2], marks[4 * l + 3]))])
+        if train:
+            ctx.save_for_backward(features, x, hidden, *weights)
+            ctx.env, ctx.plan, ctx.dims, ctx.pad, ctx.starts, ctx.splits = env, plan, dims, pad, starts, splits[L:]
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_output):
+        features, x, hidden, *weights = ctx.saved_tensors
+        env, dims, pad, L, n, device = ctx.env, ctx.dims, ctx.pad, len(weights), x.size(0), x.device
+        g = _product_operand(env, grad_output, False)
+        base = hidden.data_ptr()
+        net, keep = _gcn_net(ctx.plan, x, dims, pad, [base + 4 * s for s in ctx.starts] + [base or x.data_ptr()], pad[1:L] + [dims[L]])
+        work = torch.empty(n * (max(pad[1:]) + max(pad[1:L], default=0)), dtype=torch.float32, device=device)
+        net.z = work.data_ptr()
+        if L > 1:
+            net.g = net.z + 4 * n * max(pad[1:])
+        grads = [torch.empty_like(w) if need else None for w, need in zip(weights, ctx.needs_input_grad[3:])]
+        dw = (ctypes.c_void_p * L)(*[None if t is None else t.data_ptr() for t in grads])
+        heads = (ctypes.c_void_p * L)(None, *[s[1] for s in ctx.splits])
+        scratch, ctas = spmm_cpp.tn_scratch(device.index)
+        marks = (ctypes.c_int32 * (4 * L))(*[-1] * (4 * L))
+        net.grad, net.ld_grad = g.data_ptr(), g.stride(0) if n > 1 else pad[L]
+        net.dw, net.bwd_split = ctypes.addressof(dw), ctypes.addressof(heads)
+        net.tn_scratch, net.tn_scratch_floats, net.max_ctas, net.marks = scratch.data_ptr(), scratch.numel(), ctas, ctypes.addressof(marks)
+        spmm_cpp.gcn_call('dg_gcn_backward', net, device.index)
+        panels = [(d + 255) // 256 for d in dims]
+        spmm_cpp.dense_launches += sum(panels[1:L]) + sum(2 * panels[l] * panels[l + 1] for l in range(L) if grads[l] is not None)
+        env.timer.add_regions([r for l in range(L) for r in (('broadcast+spmm', marks[4 * l], marks[4 * l + 1]), ('mm', marks[4 * l + 2], marks[4 * l + 3]))])
+        for _ in range(L):
+            env.timer.empty_region('all_reduce')
+        return (None, None, None, *grads)
+
+
+def _gcn_net(plan, x, dims, pad, act, ld_act):
+    """The dg_gcn_net of a call, and the arrays it points into."""
+    L = len(act)
+    arrays = (ctypes.c_int32 * (L + 1))(*dims), (ctypes.c_void_p * L)(*act), (ctypes.c_int64 * L)(*ld_act)
+    net = spmm_cpp.GcnNet(plan=plan.handle, val=plan.values.data_ptr(), x=x.data_ptr(), ldx=x.stride(0) if x.size(0) > 1 else pad[0],
+                          n=x.size(0), layers=L)
+    net.dims, net.act, net.ld_act = (ctypes.addressof(a) for a in arrays)
+    return net, arrays
+
+
 class GCN(nn.Module):
     """num_layers DistGCNLayers with ReLU between them, no bias (gcn.py:56-72).  Weights are drawn as the reference
     draws them - torch.rand on the host after manual_seed(0), layer by layer - unless `weights` injects them.
@@ -497,10 +572,31 @@ class GCN(nn.Module):
             self._product = hit = (features, features._version, z)
         return hit[2]
 
+    def _one_rank_plan(self, features, weights):
+        """The plan to run all layers on in one call, or None when a layer has to be called by itself: a rank with peers, one of
+        the options above, another dense mode, an input that wants a gradient, or operands the kernels do not take."""
+        env, parts = DistEnv.env, self.g.adj_parts
+        if (env is None or env.world_size != 1 or len(parts) != 1 or not FUSE_RELU or not PAD_ODD_WIDTHS or DENSE_MODE != 'tcgen05'
+                or self.cache_input_product or self.transform_first or not features.is_cuda or features.requires_grad
+                or features.dtype != torch.float32 or features.dim() != 2 or features.size(0) < 1 or features.size(1) < 1):
+            return None
+        width = features.size(1)
+        for w in weights:
+            if (w.device != features.device or w.dtype != torch.float32 or w.dim() != 2 or w.size(0) != width or w.size(1) < 1
+                    or not w.is_contiguous()):
+                return None
+            width = w.size(1)
+        plan = spmm_cpp.plan_for(parts[0])
+        return plan if plan.m == plan.k == features.size(0) and plan.device == features.device else None
+
     def forward(self, features):
         h = features
         last = self.num_layers - 1
-        for l, w in enumerate(self.weights()):
+        weights = self.weights()
+        plan = self._one_rank_plan(features, weights)
+        if plan is not None:
+            return _OneRankGCN.apply(DistEnv.env, plan, features, *weights)
+        for l, w in enumerate(weights):
             product = self.input_product(h) if l == 0 else None
             shortcut = self.input_gradient_shortcut and product is not None
             if FUSE_RELU:

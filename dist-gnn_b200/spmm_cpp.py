@@ -9,6 +9,7 @@ without CUDA tensors they raise.
 """
 import ctypes
 import os
+import weakref
 
 import torch
 
@@ -35,6 +36,18 @@ class StageTimes(ctypes.Structure):
 class Profile(ctypes.Structure):
     _fields_ = [('spmm_ms', ctypes.c_double), ('alg_bytes', ctypes.c_double), ('gather_bytes', ctypes.c_double),
                 ('flops', ctypes.c_double), ('products', ctypes.c_int64), ('kernel_launches', ctypes.c_int64)]
+
+
+class SplitJob(ctypes.Structure):
+    _fields_ = [('w', ctypes.c_void_p), ('ldw', ctypes.c_int64), ('head', ctypes.c_void_p), ('tail', ctypes.c_void_p),
+                ('ldb', ctypes.c_int64), ('N', ctypes.c_int32), ('K', ctypes.c_int32), ('transposed', ctypes.c_int32), ('pad', ctypes.c_int32)]
+
+
+class GcnNet(ctypes.Structure):
+    _fields_ = [(name, ctypes.c_void_p) for name in ('plan', 'val', 'dims', 'x')] + [('ldx', ctypes.c_int64)] + [
+        (name, ctypes.c_void_p) for name in ('act', 'ld_act', 'fwd_split', 'bwd_split', 'grad')] + [('ld_grad', ctypes.c_int64)] + [
+        (name, ctypes.c_void_p) for name in ('z', 'g', 'dw', 'tn_scratch')] + [('tn_scratch_floats', ctypes.c_int64), ('marks', ctypes.c_void_p)] + [
+        (name, ctypes.c_int32) for name in ('n', 'layers', 'max_ctas', 'pad')]
 
 
 def lib():
@@ -83,7 +96,9 @@ def lib():
             'dg_peer_spmm': ([vp, vp, i32, vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, vp, ctypes.c_int, vp], ctypes.c_int),
             'dg_peer_spmm_gather': ([vp, vp, i32, vp, vp, vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, vp, ctypes.c_int, vp], ctypes.c_int),
             'dg_dense_split': ([vp, vp, vp, i64, vp], ctypes.c_int),
-            'dg_dense_split_operand': ([vp, i64, i32, i32, i32, vp, vp, i64, vp], ctypes.c_int),
+            'dg_dense_split_operands': ([ctypes.POINTER(SplitJob), i32, vp], ctypes.c_int),
+            'dg_gcn_forward': ([ctypes.POINTER(GcnNet), vp], ctypes.c_int),
+            'dg_gcn_backward': ([ctypes.POINTER(GcnNet), vp], ctypes.c_int),
             'dg_dense_supported': ([i64, i32, i32, i64, i64, vp, vp, vp], ctypes.c_int),
             'dg_dense_nt': ([vp, i64, vp, vp, i64, vp, i64, i64, i32, i32, i32, vp], ctypes.c_int),
             'dg_dense_nt_masked': ([vp, i64, vp, vp, i64, vp, i64, i64, i32, i32, i32, vp, i64, vp], ctypes.c_int),
@@ -303,7 +318,6 @@ _plan_cache = {}
 
 def plan_for(A):
     """The cached SpmmPlan of a sparse COO block, built on first use and dropped when the tensor dies."""
-    import weakref
     key = id(A)
     hit = _plan_cache.get(key)
     if hit is not None and hit[0]() is A:
@@ -643,46 +657,64 @@ def dense_split(w):
     return head, tail
 
 
-_split_cache = {}       # id(weight object) -> (weak reference to it, {transposed flag: (version, head, tail)})
+_split_cache = {}       # id(weight object) -> (weak reference to it, {transposed flag: (version, buffer, head, tail, ldb)})
 
 
-def split_operand(w, transposed, cache_key=None):
-    """The small operand of dense_nt, laid out [N x K] (rows padded to a multiple of 4 floats) and split into TF32 head
-    and tail.  transposed=True takes w as [K x N] and transposes it.  With cache_key (the weight object the caller holds,
-    e.g. the nn.Parameter) the result is kept until that tensor is modified in place - its version counter moves with every
-    optimiser step - so a weight is transposed and split once per step, not once per product."""
-    if cache_key is not None:
-        import weakref
-        ident = id(cache_key)
-        entry = _split_cache.get(ident)
-        if entry is None or entry[0]() is not cache_key:       # tensors compare element-wise, so the table is keyed by identity
-            entry = _split_cache[ident] = (weakref.ref(cache_key, lambda _r, ident=ident: _split_cache.pop(ident, None)), {})
-        slot = entry[1]
-        hit = slot.get(transposed)
-        if hit is not None and hit[0] == cache_key._version and hit[1].device == w.device:
-            return hit[1], hit[2]
-    w = w.detach()
-    if w.stride(1) != 1 or w.stride(0) < w.size(1):
-        w = w.contiguous()
-    N, K = (w.size(1), w.size(0)) if transposed else w.shape
-    ldb = K + (-K) % 4
-    pair = torch.empty((2, N, ldb), dtype=torch.float32, device=w.device)
-    head, tail = pair[0], pair[1]
-    global dense_launches
-    dense_launches += 1
-    index = w.device.index
-    with _on(index):
-        check(_lib.dg_dense_split_operand(w.data_ptr(), w.stride(0), transposed, N, K, head.data_ptr(), tail.data_ptr(), ldb, _raw_stream(index)))
-    if cache_key is not None:
-        slot[transposed] = (cache_key._version, head, tail)
-    return head, tail
+def split_operands(requests):
+    """Small operands of dense_nt, each laid out [N x K] (rows padded to a multiple of 4 floats) and split into TF32 head and
+    tail, all of them by one launch.  requests: (w, transposed, cache_key) each; transposed=True takes w as [K x N] and
+    transposes it.  With a cache_key (the weight object the caller holds, e.g. the nn.Parameter) the result is kept until
+    that tensor is modified in place - its version counter moves with every optimiser step - so a weight is transposed and
+    split once per step, not once per product.  Returns (buffer that holds them, head address, tail address, row stride)
+    per request; the tail lies right behind the head."""
+    out, stale, floats = [None] * len(requests), [], 0
+    for i, (w, transposed, cache_key) in enumerate(requests):
+        slot = None
+        if cache_key is not None:
+            ident = id(cache_key)
+            entry = _split_cache.get(ident)
+            if entry is None or entry[0]() is not cache_key:   # tensors compare element-wise, so the table is keyed by identity
+                entry = _split_cache[ident] = (weakref.ref(cache_key, lambda _r, ident=ident: _split_cache.pop(ident, None)), {})
+            slot = entry[1]
+            hit = slot.get(transposed)
+            if hit is not None and hit[0] == cache_key._version and hit[1].device == w.device:
+                out[i] = hit[1:]
+                continue
+        w = w.detach()
+        if w.stride(1) != 1 or w.stride(0) < w.size(1):
+            w = w.contiguous()
+        N, K = w.shape
+        if transposed:
+            N, K = K, N
+        ldb = K + (-K) % 4
+        stale.append((i, w, transposed, cache_key, slot, N, K, ldb, floats))
+        floats += 2 * N * ldb
+    if stale:
+        device = stale[0][1].device
+        buffer = torch.empty(floats, dtype=torch.float32, device=device)
+        base = buffer.data_ptr()
+        jobs = (SplitJob * len(stale))()
+        for job, (i, w, transposed, cache_key, slot, N, K, ldb, first) in zip(jobs, stale):
+            head = base + 4 * first
+            tail = head + 4 * N * ldb
+            job.w, job.ldw, job.head, job.tail, job.ldb = w.data_ptr(), w.stride(0), head, tail, ldb
+            job.N, job.K, job.transposed = N, K, transposed
+            out[i] = (buffer, head, tail, ldb)
+            if cache_key is not None:
+                slot[transposed] = (cache_key._version,) + out[i]
+        global dense_launches
+        dense_launches += 1
+        index = device.index
+        with _on(index):
+            check(lib().dg_dense_split_operands(jobs, len(stale), _raw_stream(index)))
+    return out
 
 
 def dense_nt(a, b, transposed=False, relu=False, mask=None, cache_key=None):
     """a [M x K] @ op(b) on the tensor cores with fp32 accuracy (dg_dense_nt): b is the small operand, [N x K] as given
     or [K x N] with transposed=True.  Returns None when the shapes or strides are outside what the kernel takes (the
     caller then uses a library GEMM).  relu applies max(x, 0) on the way out; mask [M x N] zeroes the result where
-    mask <= 0 (the backward of a ReLU whose output is `mask`); cache_key: see split_operand."""
+    mask <= 0 (the backward of a ReLU whose output is `mask`); cache_key: see split_operands."""
     lda = _row_major(a, 'a')
     lib()
     if not (isinstance(b, torch.Tensor) and b.is_cuda and b.dtype == torch.float32 and b.dim() == 2):
@@ -696,11 +728,11 @@ def dense_nt(a, b, transposed=False, relu=False, mask=None, cache_key=None):
         raise RuntimeError(f'mask is {tuple(mask.shape)}, the product {(M, N)}')
     if M == 0 or N == 0 or K == 0 or lda % 4 or a.data_ptr() % 16 or M >= 1 << 31:
         return None
-    head, tail = split_operand(b, transposed, cache_key)
+    kept, head, tail, ldb = split_operands(((b, transposed, cache_key),))[0]
     c = torch.empty((M, N), dtype=torch.float32, device=a.device)
     index = a.device.index
     with _on(index):
-        code = _lib.dg_dense_nt_masked(a.data_ptr(), lda, head.data_ptr(), tail.data_ptr(), head.size(1), c.data_ptr(), N, M, N, K, relu,
+        code = _lib.dg_dense_nt_masked(a.data_ptr(), lda, head, tail, ldb, c.data_ptr(), N, M, N, K, relu,
                                        mask.data_ptr() if mask is not None else None, ldm, _raw_stream(index))
     if code == ERR_UNSUPPORTED:
         return None
@@ -711,6 +743,15 @@ def dense_nt(a, b, transposed=False, relu=False, mask=None, cache_key=None):
 
 
 _tn_scratch = {}
+
+
+def tn_scratch(index):
+    """(partial-result area of dense_tn on CUDA device `index`, number of CTAs it serves)."""
+    hit = _tn_scratch.get(index)
+    if hit is None:
+        ctas = torch.cuda.get_device_properties(index).multi_processor_count
+        hit = _tn_scratch[index] = (torch.empty(ctas * 256 * 256, dtype=torch.float32, device=torch.device('cuda', index)), ctas)
+    return hit
 
 
 def dense_tn(x, g):
@@ -725,11 +766,7 @@ def dense_tn(x, g):
     if not lib().dg_dense_tn_supported(n, Km, Nn, ldx, ldg, x.data_ptr(), g.data_ptr()):
         return None
     index = x.device.index
-    scratch, ctas = _tn_scratch.get(index, (None, 0))
-    if scratch is None:
-        ctas = torch.cuda.get_device_properties(x.device).multi_processor_count
-        scratch = torch.empty(ctas * 256 * 256, dtype=torch.float32, device=x.device)
-        _tn_scratch[index] = (scratch, ctas)
+    scratch, ctas = tn_scratch(index)
     global dense_launches
     dense_launches += 2 * ((Km + 255) // 256) * ((Nn + 255) // 256)      # per 256 x 256 panel: the product and the reduction over the CTAs' partials
     d = torch.empty((Km, Nn), dtype=torch.float32, device=x.device)
@@ -737,6 +774,12 @@ def dense_tn(x, g):
         check(_lib.dg_dense_tn(x.data_ptr(), ldx, g.data_ptr(), ldg, d.data_ptr(), Nn, n, Km, Nn, scratch.data_ptr(), scratch.numel(),
                                ctas, _raw_stream(index)))
     return d
+
+
+def gcn_call(name, net, index):
+    """dg_gcn_forward / dg_gcn_backward on the current stream of CUDA device `index`."""
+    with _on(index):
+        check(getattr(lib(), name)(ctypes.byref(net), _raw_stream(index)))
 
 
 def dense_status(reset=False):

@@ -249,10 +249,18 @@ int dg_comm_last_times(dg_comm* comm, dg_stage_times* host_out);
  * memory, waits a few thousand polls on a barrier nothing arrives at, reports that the wait ran out (*host_gave_up = 1),
  * frees its tensor memory and returns; the status word of the real kernels is not touched. */
 int dg_dense_split(const float* src, float* head, float* tail, int64_t count, void* stream);
-/* The same for a whole operand of dg_dense_nt in one launch: Bt [N x K] is w as given (transposed == 0, ldw >= K) or the
- * transpose of w [K x N] (transposed != 0, ldw >= N); head and tail get rows of ldb >= K floats, zero beyond column K. */
-int dg_dense_split_operand(const float* w, int64_t ldw, int32_t transposed, int32_t N, int32_t K, float* head, float* tail,
-                           int64_t ldb, void* stream);
+/* The same for whole operands of dg_dense_nt, all of them in one launch: Bt [N x K] is w as given (transposed == 0,
+ * ldw >= K) or the transpose of w [K x N] (transposed != 0, ldw >= N); head and tail get rows of ldb >= K floats, zero beyond
+ * column K. */
+typedef struct dg_split_job {
+    const float* w;
+    int64_t ldw;
+    float* head;
+    float* tail;
+    int64_t ldb;
+    int32_t N, K, transposed, pad;
+} dg_split_job;
+int dg_dense_split_operands(const dg_split_job* host_jobs, int32_t count, void* stream);
 int dg_dense_supported(int64_t M, int32_t N, int32_t K, int64_t lda, int64_t ldb, const void* A, const void* Bt_head, const void* Bt_tail);
 int dg_dense_nt(const float* A, int64_t lda, const float* Bt_head, const float* Bt_tail, int64_t ldb, float* C, int64_t ldc,
                 int64_t M, int32_t N, int32_t K, int32_t relu, void* stream);
@@ -285,6 +293,46 @@ int dg_dense_wait_selftest(int* host_gave_up, void* stream);
  * algorithmic traffic  8*nnz + 4*(m+1) + 4*F*touched_columns + 4*F*m*(1 + [beta != 0])  in bytes, the no-reuse gather
  * volume  8*nnz + 4*(m+1) + 4*F*nnz + 4*F*m*(1 + [beta != 0]),  2*nnz*F flops, and how many kernels of this library
  * were launched (products only; NCCL's own kernels are not counted). */
+/* ---- a whole GCN on one rank, forward or backward in one call (no counterpart in the reference, which issues every
+ * product and every torch.mm of light_dist_gnn/models/gcn.py:35-72 from Python) -----------------------------------------
+ * Layer l computes act[l] = A (input W_l), with max(x, 0) behind every layer but the last; input is x for l = 0, act[l-1]
+ * after it.  The calls are those of dg_spmm_csr, dg_dense_nt_masked and dg_dense_tn, in the order the layers issue them
+ * one by one, so the results are the same bits; what goes is the host's work between them.
+ *   dims           layers + 1 widths; pad4(w) below is w rounded up to a multiple of 4
+ *   x, ldx         n rows of pad4(dims[0]) readable floats, ldx a multiple of 4, 16-byte aligned (columns beyond dims[0]
+ *                  are read and ignored)
+ *   act, ld_act    output of layer l, ld_act[l] >= dims[l+1]; for l < layers - 1 a multiple of 4, >= pad4(dims[l+1]), 16-byte
+ *                  aligned.  Forward without a backward pass may give every hidden layer the same buffer.
+ *   fwd_split[l]   head of W_l^T [dims[l+1] x pad4(dims[l])], its tail right behind it (dg_dense_split_operands)
+ *   bwd_split[l]   head of W_l [dims[l] x pad4(dims[l+1])], its tail right behind it; backward only, l >= 1
+ *   grad, ld_grad  gradient of act[layers-1], as x; backward only
+ *   z, g           work areas of n * pad4(widest dims) floats; g: backward of two or more layers only
+ *   dw[l]          gradient of W_l [dims[l] x dims[l+1]], contiguous; NULL skips it
+ *   tn_scratch     as `scratch` of dg_dense_tn, for max_ctas CTAs
+ *   marks          NULL, or 4 * layers ids that receive time marks: begin and end of every product, then of every transform */
+typedef struct dg_gcn_net {
+    const dg_plan* plan;
+    const float* val;
+    const int32_t* dims;
+    const float* x;
+    int64_t ldx;
+    float* const* act;
+    const int64_t* ld_act;
+    const float* const* fwd_split;
+    const float* const* bwd_split;
+    const float* grad;
+    int64_t ld_grad;
+    float* z;
+    float* g;
+    float* const* dw;
+    float* tn_scratch;
+    int64_t tn_scratch_floats;
+    int32_t* marks;
+    int32_t n, layers, max_ctas, pad;
+} dg_gcn_net;
+int dg_gcn_forward(const dg_gcn_net* net, void* stream);
+int dg_gcn_backward(const dg_gcn_net* net, void* stream);
+
 /* dst[i, 0..cols) = src[i, 0..cols), dst[i, cols..ld_dst) = 0 for n rows: an operand whose rows are not 16-byte multiples is
  * copied once into rows that are (ld_dst a multiple of 4, dst 16-byte aligned). */
 int dg_pad_rows(const float* src, int64_t ld_src, int64_t n, int32_t cols, float* dst, int64_t ld_dst, void* stream);

@@ -372,3 +372,42 @@ def test_row_cross_entropy_matches_the_library_loss(n, C, ld):
     assert abs(loss.item() - want.item()) <= 1e-6 * max(1.0, abs(want.item()))
     assert_close(grad.cpu().numpy(), want_grad.cpu().numpy(), TOL, 'gradient of the loss')
     assert torch.equal(loss, spmm_cpp.RowCrossEntropy.apply(x, t, rows.numel()))
+
+
+@pytest.mark.parametrize('dims', [(33, 7), (45, 73, 42), (100, 64, 20, 3), (602, 16, 5, 300, 2)])
+def test_one_call_network_equals_chained_layers(golden, env1, dims):
+    """All layers in one library call against the same layers called one by one (the path a rank with peers takes): same
+    bits in outputs and weight gradients, for widths that are no whole 16-byte pieces, one to four layers, more than one
+    panel, a weight that wants no gradient, and without autograd."""
+    from coo_graph import COO_Graph, Parted_COO_Graph
+    from models import GCN
+    from models.gcn import DistGCNLayer
+    z = golden('graph_small')
+    g = Parted_COO_Graph.from_full(COO_Graph.from_dict('gsmall', _fixture_dataset(z), device='cuda'), 0, 1)
+    gen = torch.Generator(device='cuda').manual_seed(len(dims))
+    n, L = g.local_num_nodes, len(dims) - 1
+    x = torch.randn(n, dims[0], device='cuda', generator=gen)
+    up = torch.randn(n, dims[-1], device='cuda', generator=gen)
+    g.features, g.num_classes = x, dims[-1]
+    model = GCN(g, env1, hidden_dim=8, num_layers=1)
+    for l in range(L):
+        setattr(model, f'weight{l + 1}', torch.nn.Parameter(torch.randn(dims[l], dims[l + 1], device='cuda', generator=gen) * 0.2))
+    model.num_layers = L
+    weights = model.weights()
+    if L > 2:
+        weights[1].requires_grad_(False)
+    out = model(x)
+    assert type(out.grad_fn).__name__.startswith('_OneRankGCN')
+    out.backward(up)
+    got = [None if w.grad is None else w.grad.clone() for w in weights]
+    with torch.no_grad():
+        assert torch.equal(model(x), out)
+    for w in weights:
+        w.grad = None
+    h = x
+    for l, w in enumerate(weights):
+        h = DistGCNLayer.apply(h, w, g.adj_parts, f'L{l + 1}', l < L - 1, l > 0)
+    h.backward(up)
+    assert torch.equal(h, out)
+    for a, w in zip(got, weights):
+        assert (a is None) == (w.grad is None) and (a is None or torch.equal(a, w.grad))

@@ -190,8 +190,8 @@ int dg_plan_build(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m
     if (nnz < 0 || m < 0 || k < 0) return DG_ERR_DIMS;
     if (nnz > 0 && (!row || !col)) return DG_ERR_NULL;
     if (nnz > 0 && (m == 0 || k == 0)) return DG_ERR_DIMS;
-    if (heavy_threshold <= 0) heavy_threshold = DG_DEFAULT_HEAVY_THRESHOLD;
-    if (chunk <= 0) chunk = DG_DEFAULT_CHUNK;
+    if (heavy_threshold <= 0) heavy_threshold = dg_default_chunk(nnz);
+    if (chunk <= 0) chunk = dg_default_chunk(nnz);
     cudaStream_t stream = (cudaStream_t)stream_;
 
     dg_plan* p = new (std::nothrow) dg_plan();
@@ -251,20 +251,18 @@ int dg_plan_build(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m
         if ((rc = (int)cudaMemcpy(rows.data(), d_heavy, rows.size() * sizeof(HeavyTriple), cudaMemcpyDeviceToHost))) return fail(rc);
         std::sort(rows.begin(), rows.end(), [](const HeavyTriple& a, const HeavyTriple& b) { return a.row < b.row; });
         std::vector<dg_chunk> chunks;
-        std::vector<dg_heavy_row> heavy;
-        for (const HeavyTriple& r : rows) {
-            dg_heavy_row h{r.row, (int32_t)chunks.size(), 0, 0};
+        for (size_t i = 0; i < rows.size(); ++i) {
+            const HeavyTriple& r = rows[i];
+            const int32_t slot0 = (int32_t)chunks.size(), nchunks = (int32_t)((r.e1 - r.e0 + chunk - 1) / chunk);
             for (int64_t e = r.e0; e < r.e1; e += chunk)
-                chunks.push_back(dg_chunk{e, std::min<int64_t>(e + chunk, r.e1), r.row, (int32_t)chunks.size()});
-            h.nchunks = (int32_t)chunks.size() - h.slot0;
-            heavy.push_back(h);
+                chunks.push_back(dg_chunk{e, (int32_t)std::min<int64_t>(chunk, r.e1 - e), r.row, (int32_t)chunks.size(), slot0, nchunks, (int32_t)i});
         }
         p->n_chunks = (int32_t)chunks.size();
-        p->n_heavy = (int32_t)heavy.size();
+        p->n_heavy = (int32_t)rows.size();
+        const size_t counts = rows.size() * DG_FINISH_TILES * sizeof(int);
         if ((rc = (int)cudaMalloc((void**)&p->chunks, chunks.size() * sizeof(dg_chunk))) ||
-            (rc = (int)cudaMalloc((void**)&p->heavy, heavy.size() * sizeof(dg_heavy_row))) ||
-            (rc = (int)cudaMemcpy(p->chunks, chunks.data(), chunks.size() * sizeof(dg_chunk), cudaMemcpyHostToDevice)) ||
-            (rc = (int)cudaMemcpy(p->heavy, heavy.data(), heavy.size() * sizeof(dg_heavy_row), cudaMemcpyHostToDevice)))
+            (rc = (int)cudaMalloc((void**)&p->arrived, counts)) || (rc = (int)cudaMemsetAsync(p->arrived, 0, counts, stream)) ||
+            (rc = (int)cudaMemcpy(p->chunks, chunks.data(), chunks.size() * sizeof(dg_chunk), cudaMemcpyHostToDevice)))
             return fail(rc);
         // Visiting order of the chunks.  A chunk's scratch slot is fixed above, so the list itself may be walked in any order
         // without changing a bit of the result.  Chunks are handed to warps in list order, eight per CTA, CTAs in launch
@@ -313,7 +311,7 @@ extern "C" int dg_plan_destroy(dg_plan* p)
     if (prev != p->device) cudaSetDevice(p->device);
     cudaFree(p->rowptr);
     cudaFree(p->chunks);
-    cudaFree(p->heavy);
+    cudaFree(p->arrived);
     cudaFree(p->scratch);
     cudaFree(p->task_first_row);
     cudaFree(p->split);

@@ -3,29 +3,17 @@
 // Replaces cusparseSpMM(COO_ALG4) as called by the reference (light_dist_gnn/spmm_cpp/spmm.cpp:26-28).
 //
 // The product is a gather: every stored entry (i, j, a) pulls the F-float row j of B and adds a * B[j,:] into
-// row i of C.  HBM / L2 bandwidth bounds it, tensor cores have nothing to do here.  Scheduling:
-//   * light rows (<= heavy_threshold entries): one warp per row.  A CTA owns a contiguous range of rows and
-//     its warps fetch the next row from a shared-memory counter, so a long row does not idle the other warps.
-//   * heavy rows: cut into chunks of `chunk` entries at plan time; one warp per chunk writes a partial sum to
-//     scratch, then one CTA per heavy row adds the partials in chunk order and applies the epilogue.  No float
+// row i of C.  HBM / L2 bandwidth bounds it.  Scheduling (k_spmm):
+//   * light rows (<= heavy_threshold entries): a group of 4 to 32 lanes per row, out of CTA-local windows sorted by length;
+//   * heavy rows: cut into chunks of `chunk` entries at plan time; one lane group per chunk leaves a partial sum in
+//     scratch, and the last one to arrive adds the partials in chunk order and applies the epilogue.  No float
 //     atomics anywhere: the result is bit-reproducible.
-// Inside a warp the 32 lanes are G groups of LPR lanes.  The lanes of a group hold TPL vectors (VEC floats each)
-// of the output row at columns (t*LPR + lane)*VEC, so one gathered row of B is read with fully coalesced 64/128-bit
-// loads.  The warp reads 32 (col, val) pairs with one coalesced load each and hands them out by shuffle; with
-// G > 1 (narrow F) the groups take interleaved entries of the same row and are summed by shuffle at the end.
-// U entries are in flight per group before the first FMA, which is what keeps the memory system busy.
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
 #include <vector>
 #include "dg_internal.h"
-
-// Launch shapes, fixed after measurement on B200: 256-thread CTAs, 8 resident per SM (64 warps, <= 32 registers per thread),
-// one gathered row in flight per warp (two or four were slower: 11.9 / 12.2 / 14.5 ms on the benchmark graph at F = 256).
-#define DG_ROWS_MIN_BLOCKS 8
-#define DG_V4_MIN_BLOCKS 8
-#define DG_V4_UNROLL 1
 
 namespace {
 
@@ -62,21 +50,17 @@ struct SpmmArgs {
     const float* row_scale;
     const float* bias;
     const dg_chunk* chunks;
-    const dg_heavy_row* heavy;
+    int* arrived;               // [n_heavy x DG_FINISH_TILES] partial sums of a split row that are in place; zero between products
     float* scratch;
-    int64_t ldb, ldc;
-    int32_t m, F, nvec;         // nvec = F / VEC
+    int64_t ldb, ldc, lds;      // lds: row stride of the partial sums
+    int32_t m, F;
     int32_t heavy_threshold;
-    int32_t n_chunks, n_heavy;
+    int32_t n_chunks;
     int32_t rows_per_cta;
+    int32_t vec_first, vec_end; // the vectors of a row this launch covers
     float alpha, beta;
     uint32_t flags;
 };
-
-template <int VEC> struct VecT;
-template <> struct VecT<1> { using type = float; };
-template <> struct VecT<2> { using type = float2; };
-template <> struct VecT<4> { using type = float4; };
 
 template <int VEC> __device__ __forceinline__ void load_vec(const float* p, float (&out)[VEC])
 {
@@ -91,329 +75,326 @@ template <int VEC> __device__ __forceinline__ void load_vec(const float* p, floa
     }
 }
 
-template <int VEC> __device__ __forceinline__ void store_vec(float* p, const float (&v)[VEC])
+// What is left to do with a sum before it is stored: alpha * sum + beta * C (alpha == 1 has beta * C in the sum already), row
+// scale, bias, ReLU.
+__device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const float* c, int32_t row, int32_t colidx)
 {
-    if constexpr (VEC == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    else if constexpr (VEC == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
-    else *p = v[0];
-}
-
-// Adds sum_{e in [e0,e1)} val[e] * B[col[e], columns of this lane] into acc.  Warp-uniform e0, e1.
-template <int VEC, int LPR, int TPL, int U>
-__device__ __forceinline__ void gather_range(const SpmmArgs& a, int64_t e0, int64_t e1, const int (&coff)[TPL],
-                                             const bool (&act)[TPL], int lane, float (&acc)[TPL][VEC])
-{
-    constexpr int G = 32 / LPR;
-    const int grp = lane / LPR;
-    for (int64_t e = e0; e < e1; e += 32) {
-        const int cnt = (int)min((int64_t)32, e1 - e);
-        int32_t c = 0;
-        float v = 0.f;
-        if (lane < cnt) {
-            c = __ldcs(a.col + e + lane);       // streamed once: keep it from displacing B rows in cache
-            v = __ldcs(a.val + e + lane);
-        }
-        for (int kk = 0; kk < cnt; kk += G * U) {
-            float x[U][TPL][VEC];
-            float w[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int k = kk + u * G + grp;
-                const bool ok = k < cnt;
-                const int32_t j = __shfl_sync(0xffffffffu, c, k & 31);
-                const float wv = __shfl_sync(0xffffffffu, v, k & 31);
-                w[u] = ok ? wv : 0.f;
-                const float* brow = a.B + (size_t)j * (size_t)a.ldb;
-#pragma unroll
-                for (int t = 0; t < TPL; ++t) {
-                    if (ok && act[t]) {
-                        load_vec<VEC>(brow + coff[t], x[u][t]);
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < VEC; ++q) x[u][t][q] = 0.f;
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int t = 0; t < TPL; ++t)
-#pragma unroll
-                    for (int q = 0; q < VEC; ++q) acc[t][q] = fmaf(w[u], x[u][t][q], acc[t][q]);
-        }
+    float out = sum;
+    if (a.alpha != 1.f) {
+        out *= a.alpha;
+        if (a.beta != 0.f) out = fmaf(a.beta, *c, out);
     }
-    if constexpr (G > 1) {
-#pragma unroll
-        for (int off = LPR; off < 32; off <<= 1)
-#pragma unroll
-            for (int t = 0; t < TPL; ++t)
-#pragma unroll
-                for (int q = 0; q < VEC; ++q) acc[t][q] += __shfl_xor_sync(0xffffffffu, acc[t][q], off);
-    }
-}
-
-__device__ __forceinline__ float finish(const SpmmArgs& a, float sum, float cold, int32_t row, int32_t colidx)
-{
-    float out = a.alpha * sum;
-    if (a.beta != 0.f) out = fmaf(a.beta, cold, out);
     if (a.flags & DG_EPI_ROW_SCALE) out *= __ldg(a.row_scale + row);
     if (a.flags & DG_EPI_BIAS) out += __ldg(a.bias + colidx);
     if (a.flags & DG_EPI_RELU) out = fmaxf(out, 0.f);
     return out;
 }
 
-template <int VEC, int LPR, int TPL>
-__device__ __forceinline__ void lane_columns(const SpmmArgs& a, int lane, int (&coff)[TPL], bool (&act)[TPL])
+// ---- the product -------------------------------------------------------------------------------------------------------
+// A warp is G = 32 / LPR groups of LPR lanes, and every group works on an item of its own: a row, or a chunk of a split
+// row.  Lane gl of a group owns the TPL vectors (VEC floats each) gl, gl + LPR, ... of the column tile blockIdx.y, so a
+// gathered row of B is read with coalesced loads of up to 128 bits; the group reads LPR (col, val) pairs at a time, the next
+// LPR while it works on these, and hands them out by shuffle, U gathers in flight before the first FMA.  A row is summed
+// in entry order by one group, whatever LPR is.
+//
+// The first `chunk_ctas` CTAs take the chunks of the split rows, NG = 256 / LPR at a time; each group leaves its partial
+// sum in scratch and adds one to its row's count, and the group that finds the count complete adds the row's partial sums in
+// chunk order and writes the row (no second launch, no float atomics, the same bits every time).
+//
+// The other CTAs own `rows_per_cta` <= 256 consecutive rows each.  They read the window's row offsets with one coalesced
+// load (a warp that fetches its own row's offsets waits a memory latency per row), sort the rows by length class in shared
+// memory and hand them out longest first, G at a time, so that the rows a warp works on together are about equally long and
+// the last rows of a CTA are short ones.  The first entries of the next G rows are requested before the current ones are
+// gathered.
+//
+// What bounds it: the gathers.  512-byte rows that miss nothing but the L1 move at 18.8 TB/s (64 bytes a clock and SM), and
+// large graphs run at that rate times their L2 hit rate; small ones and short rows are bound by latency, which the offsets in
+// shared memory, the look-ahead and U hide.  Against separate kernels with a warp per row (B200, us per product):
+//   10,000 nodes, 210 k entries, F = 64: 74 -> 17      150,001 nodes, 2.6 M entries, F = 256: 263 -> 204; F = 48: 156 -> 79
+//   1 M nodes, 17 M entries, F = 64: 748 -> 475, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 219
+//   2,449,029 nodes, 126 M entries, F = 256: 10,000 -> 9,800, F = 100: 5,760 -> 5,120, F = 48: 3,620 -> 2,570
+// PADDED: the operand is the padded copy of a matrix whose rows are not 16-byte multiples; C is then written float by float.
+template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED>
+__global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int chunk_ctas)
 {
-    const int gl = lane % LPR;
-    const int vec0 = blockIdx.y * (LPR * TPL);
+    constexpr int G = 32 / LPR, NG = 256 / LPR;
+    static_assert(U <= LPR, "a batch of U gathers comes from one set of LPR entries");
+    const int gl = threadIdx.x % LPR, grp = (threadIdx.x & 31) / LPR;
+    const int vec0 = a.vec_first + blockIdx.y * (LPR * TPL) + gl;
+    bool on[TPL];
 #pragma unroll
-    for (int t = 0; t < TPL; ++t) {
-        const int v = vec0 + t * LPR + gl;
-        act[t] = v < a.nvec;
-        coff[t] = v * VEC;
-    }
-}
+    for (int t = 0; t < TPL; ++t) on[t] = vec0 + t * LPR < a.vec_end;
+    const float* bl = a.B + (int64_t)vec0 * VEC;
+    const int64_t ldb = a.ldb;
+    float acc[TPL][VEC];
 
-// Light rows.  grid.x = ceil(m / rows_per_cta), grid.y = column chunks of LPR*TPL vectors, 256 threads.
-template <int VEC, int LPR, int TPL, int U>
-__global__ void __launch_bounds__(256, DG_ROWS_MIN_BLOCKS) k_spmm_rows(const SpmmArgs a)
-{
-    __shared__ int next_row;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int coff[TPL];
-    bool act[TPL];
-    lane_columns<VEC, LPR, TPL>(a, lane, coff, act);
-    const int64_t row0 = (int64_t)blockIdx.x * a.rows_per_cta;
-    const int nrows = (int)min((int64_t)a.rows_per_cta, (int64_t)a.m - row0);
-    if (threadIdx.x == 0) next_row = blockDim.x >> 5;
-    __syncthreads();
-    int r = warp;
-    while (r < nrows) {
-        const int32_t i = (int32_t)(row0 + r);
-        const int64_t e0 = __ldg(a.rowptr + i), e1 = __ldg(a.rowptr + i + 1);
-        if (e1 - e0 <= a.heavy_threshold) {
-            float acc[TPL][VEC];
+    // acc += sum over this group's `len` entries; `e` is this lane's first entry, c / v hold it already
+    auto gather = [&](int64_t e, int len, int c, float v) {
+        const int longest = G == 1 ? len : __reduce_max_sync(0xffffffffu, len);
+#pragma unroll 1
+        for (int base = 0; base < longest; base += LPR) {
+            int c_next = 0;
+            float v_next = 0.f;
+            if (base + LPR + gl < len) {
+                c_next = __ldcs(a.col + e + base + LPR);          // streamed once: keep it from displacing rows of B in cache
+                v_next = __ldcs(a.val + e + base + LPR);
+            }
+            const int cnt = len - base, steps = min(LPR, longest - base);
+#pragma unroll 1
+            for (int k = 0; k < steps; k += U) {
+                float x[U][TPL][VEC], w[U];
 #pragma unroll
-            for (int t = 0; t < TPL; ++t)
+                for (int u = 0; u < U; ++u) {
+                    const int j = __shfl_sync(0xffffffffu, c, k + u, LPR);
+                    w[u] = __shfl_sync(0xffffffffu, v, k + u, LPR);          // 0 beyond the last entry
+                    const float* row = bl + j * ldb;
 #pragma unroll
-                for (int q = 0; q < VEC; ++q) acc[t][q] = 0.f;
-            gather_range<VEC, LPR, TPL, U>(a, e0, e1, coff, act, lane, acc);
-            if (lane < LPR) {
-                float* crow = a.C + (size_t)i * (size_t)a.ldc;
+                    for (int t = 0; t < TPL; ++t) {
+                        if (k + u < cnt && on[t]) {
+                            load_vec<VEC>(row + t * LPR * VEC, x[u][t]);
+                        } else {
 #pragma unroll
-                for (int t = 0; t < TPL; ++t) {
-                    if (!act[t]) continue;
-                    float old[VEC], outv[VEC];
-                    if (a.beta != 0.f) {
-                        if constexpr (VEC == 4) { const float4 o = *reinterpret_cast<const float4*>(crow + coff[t]); old[0] = o.x; old[1] = o.y; old[2] = o.z; old[3] = o.w; }
-                        else if constexpr (VEC == 2) { const float2 o = *reinterpret_cast<const float2*>(crow + coff[t]); old[0] = o.x; old[1] = o.y; }
-                        else old[0] = crow[coff[t]];
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < VEC; ++q) old[q] = 0.f;
+                            for (int q = 0; q < VEC; ++q) x[u][t][q] = 0.f;
+                        }
                     }
-#pragma unroll
-                    for (int q = 0; q < VEC; ++q) outv[q] = finish(a, acc[t][q], old[q], i, coff[t] + q);
-                    store_vec<VEC>(crow + coff[t], outv);
                 }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int t = 0; t < TPL; ++t)
+#pragma unroll
+                        for (int q = 0; q < VEC; ++q) acc[t][q] = fmaf(w[u], x[u][t][q], acc[t][q]);
+            }
+            c = c_next;
+            v = v_next;
+        }
+    };
+    // acc = beta * C[row] where the product starts from it (alpha == 1: no registers for the old row beside the sum, and its
+    // latency runs under the first gathers'), else 0
+    auto begin_row = [&](int32_t row, bool add) {
+        const float* cp = a.C + (int64_t)row * a.ldc + (int64_t)vec0 * VEC;
+#pragma unroll
+        for (int t = 0; t < TPL; ++t) {
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) acc[t][q] = 0.f;
+            if (!add || !on[t]) continue;
+            const float* p = cp + t * LPR * VEC;
+            if constexpr (PADDED) {
+#pragma unroll
+                for (int q = 0; q < VEC; ++q)
+                    if ((vec0 + t * LPR) * VEC + q < a.F) acc[t][q] = a.beta * __ldcs(p + q);
+            } else if constexpr (VEC == 4) {
+                const float4 o = __ldcs(reinterpret_cast<const float4*>(p));
+                acc[t][0] = a.beta * o.x; acc[t][1] = a.beta * o.y; acc[t][2] = a.beta * o.z; acc[t][3] = a.beta * o.w;
+            } else if constexpr (VEC == 2) {
+                const float2 o = __ldcs(reinterpret_cast<const float2*>(p));
+                acc[t][0] = a.beta * o.x; acc[t][1] = a.beta * o.y;
+            } else {
+                acc[t][0] = a.beta * __ldcs(p);
             }
         }
-        int nxt = 0;
-        if (lane == 0) nxt = atomicAdd(&next_row, 1);
-        r = __shfl_sync(0xffffffffu, nxt, 0);
-    }
-}
-
-// Heavy rows, pass 1: one warp per chunk, partial sums (no alpha) to scratch[slot, 0..F).
-template <int VEC, int LPR, int TPL, int U>
-__global__ void __launch_bounds__(256, DG_ROWS_MIN_BLOCKS) k_spmm_chunks(const SpmmArgs a)
-{
-    const int lane = threadIdx.x & 31;
-    const int chunk_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (chunk_id >= a.n_chunks) return;
-    int coff[TPL];
-    bool act[TPL];
-    lane_columns<VEC, LPR, TPL>(a, lane, coff, act);
-    const dg_chunk ch = a.chunks[chunk_id];
-    float acc[TPL][VEC];
+    };
+    const bool add_first = a.beta != 0.f && a.alpha == 1.f;
+    auto store_row = [&](int32_t row) {
+        float* cp = a.C + (int64_t)row * a.ldc + (int64_t)vec0 * VEC;
 #pragma unroll
-    for (int t = 0; t < TPL; ++t)
+        for (int t = 0; t < TPL; ++t) {
+            if (!on[t]) continue;
+            const int c0 = (vec0 + t * LPR) * VEC;
+            float* p = cp + t * LPR * VEC;
+            if (a.alpha != 1.f || a.flags) {
 #pragma unroll
-        for (int q = 0; q < VEC; ++q) acc[t][q] = 0.f;
-    gather_range<VEC, LPR, TPL, U>(a, ch.e0, ch.e1, coff, act, lane, acc);
-    if (lane < LPR) {
-        float* srow = a.scratch + (size_t)ch.slot * (size_t)a.F;
-#pragma unroll
-        for (int t = 0; t < TPL; ++t)
-            if (act[t]) {
-#pragma unroll
-                for (int q = 0; q < VEC; ++q) srow[coff[t] + q] = acc[t][q];
+                for (int q = 0; q < VEC; ++q)
+                    if (!PADDED || c0 + q < a.F) acc[t][q] = finish(a, acc[t][q], p + q, row, c0 + q);
             }
-    }
-}
+            if constexpr (PADDED) {
+#pragma unroll
+                for (int q = 0; q < VEC; ++q)
+                    if (c0 + q < a.F) __stcs(p + q, acc[t][q]);
+            } else if constexpr (VEC == 4) {
+                __stcs(reinterpret_cast<float4*>(p), make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]));
+            } else if constexpr (VEC == 2) {
+                __stcs(reinterpret_cast<float2*>(p), make_float2(acc[t][0], acc[t][1]));
+            } else {
+                __stcs(p, acc[t][0]);
+            }
+        }
+    };
 
-// Heavy rows, pass 2: one CTA per heavy row adds its partials in chunk order and applies the epilogue.
-__global__ void __launch_bounds__(256) k_spmm_heavy_finish(const SpmmArgs a)
-{
-    const dg_heavy_row h = a.heavy[blockIdx.x];
-    float* crow = a.C + (size_t)h.row * (size_t)a.ldc;
-    for (int f = threadIdx.x; f < a.F; f += blockDim.x) {
-        float sum = 0.f;
-        for (int c = 0; c < h.nchunks; ++c) sum += a.scratch[(size_t)(h.slot0 + c) * (size_t)a.F + f];
-        const float old = a.beta != 0.f ? crow[f] : 0.f;
-        crow[f] = finish(a, sum, old, h.row, f);
-    }
-}
-
-// ---- lean kernel for 16-byte aligned rows: float4 gathers, 32-bit offsets, one launch per product ---------------------
-// Same scheduling and the same sum order as the generic kernels above, written to need few registers: on B200 the gather
-// runs fastest at full occupancy (64 warps per SM, one gathered row per warp in flight).  A warp covers a column tile of
-// 128 floats (every lane one float4; blockIdx.y walks the tiles, tile-major, so the CTAs resident at one time gather from
-// the same 512-byte slice of B's rows), `on` masks the lanes of a partial last tile.  Row offsets col * (ldb / 4) are 32-bit
-// (the host checks k * ldb / 4 < 2^31).  Measured on the 2,449,029-node benchmark graph (F = 256; whole graph / the eight
-// 306 k-row stage blocks of one rank): two float4 per lane in separate row and chunk kernels 12.83 / 2.73 ms, this kernel
-// 12.16 / 2.50 ms; F = 100: 6.15 / 1.82 -> 6.09 / 1.39 ms.
-template <int U>
-__device__ __forceinline__ void gather_v4(const float4* __restrict__ bl, int ld4, const int32_t* __restrict__ colp,
-                                          const float* __restrict__ valp, int len, bool on, float4& acc)
-{
-    // colp / valp point at this lane's first entry (entry `lane` of the range); len = entries in the range (a light row or
-    // one chunk of a split row, so it fits 32 bits with room to spare)
-    for (int base = 0; base < len; base += 32) {
-        const int cnt = min(32, len - base);
+    if ((int)blockIdx.x < chunk_ctas) {
+        const int id = blockIdx.x * NG + threadIdx.x / LPR;
+        const bool valid = id < a.n_chunks;
+        dg_chunk ch{};
+        if (valid) ch = a.chunks[id];
         int c = 0;
         float v = 0.f;
-        if ((int)(threadIdx.x & 31) < cnt) {
-            c = __ldcs(colp + base) * ld4;        // streamed once: keep it from displacing rows of B in cache
-            v = __ldcs(valp + base);
+        if (gl < ch.len) {
+            c = __ldcs(a.col + ch.e0 + gl);
+            v = __ldcs(a.val + ch.e0 + gl);
         }
-        for (int k = 0; k < cnt; k += U) {
-            float4 x[U];
-            float w[U];
+        begin_row(0, false);
+        gather(ch.e0 + gl, ch.len, c, v);
+        if (valid) {
+            float* sp = a.scratch + (int64_t)ch.slot * a.lds + (int64_t)vec0 * VEC;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int idx = __shfl_sync(0xffffffffu, c, (k + u) & 31);
-                w[u] = __shfl_sync(0xffffffffu, v, (k + u) & 31);     // lanes >= cnt hold 0: a zero weight ...
-                x[u] = k + u < cnt && on ? __ldg(bl + idx) : make_float4(0.f, 0.f, 0.f, 0.f);   // ... and nothing is loaded
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                acc.x = fmaf(w[u], x[u].x, acc.x); acc.y = fmaf(w[u], x[u].y, acc.y);
-                acc.z = fmaf(w[u], x[u].z, acc.z); acc.w = fmaf(w[u], x[u].w, acc.w);
+            for (int t = 0; t < TPL; ++t) {
+                if (!on[t]) continue;
+                float* p = sp + t * LPR * VEC;
+                if constexpr (VEC == 4) __stcg(reinterpret_cast<float4*>(p), make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]));
+                else if constexpr (VEC == 2) __stcg(reinterpret_cast<float2*>(p), make_float2(acc[t][0], acc[t][1]));
+                else __stcg(p, acc[t][0]);
             }
         }
-    }
-}
-
-// One launch for a whole product: the first `chunk_ctas` CTAs take the chunks of the split rows (one warp per chunk, partial
-// sums to scratch), the others the light rows.  A chunk is a chain of `chunk` gathers walked by one warp, so on a small
-// block the chunk work is a fixed latency that does not fill the GPU (385 CTAs for a 306 k-row stage block of the 8-rank
-// partition: 0.09 ms on its own next to 0.25 ms of light rows); issued first in the same grid it runs underneath the light
-// rows instead of after them.  k_spmm_heavy_finish follows as a second launch.
-// PLAIN: alpha == 1 and no row scale, bias or ReLU - what the stage loops run; fmaf(beta, old, sum) with old = 0 is sum, so
-// it gives the bits of the general epilogue.
-template <int U, bool PLAIN>
-__global__ void __launch_bounds__(256, DG_V4_MIN_BLOCKS) k_spmm_v4(const SpmmArgs a, const int chunk_ctas)
-{
-    __shared__ int next_row;
-    const int lane = threadIdx.x & 31;
-    const int vec0 = blockIdx.y * 32 + lane;                          // this lane's float4 of the row
-    const bool on = vec0 < a.nvec;
-    const float4* bl = reinterpret_cast<const float4*>(a.B) + vec0;
-    const int ld4 = (int)(a.ldb >> 2);
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if ((int)blockIdx.x < chunk_ctas) {
-        const int chunk_id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-        if (chunk_id >= a.n_chunks) return;
-        const dg_chunk ch = a.chunks[chunk_id];
-        gather_v4<U>(bl, ld4, a.col + ch.e0 + lane, a.val + ch.e0 + lane, (int)(ch.e1 - ch.e0), on, acc);
-        if (on) __stcs(reinterpret_cast<float4*>(a.scratch + (size_t)ch.slot * (size_t)a.F) + vec0, acc);
-        return;
-    }
-    const int32_t row0 = ((int)blockIdx.x - chunk_ctas) * a.rows_per_cta;     // m < 2^31
-    const int nrows = min(a.rows_per_cta, a.m - row0);
-    if (threadIdx.x == 0) next_row = blockDim.x >> 5;
-    __syncthreads();
-    int r = threadIdx.x >> 5;
-    while (r < nrows) {
-        const int32_t i = row0 + r;
-        const int64_t e0 = __ldg(a.rowptr + i);
-        const int64_t len = __ldg(a.rowptr + i + 1) - e0;
-        if (len <= a.heavy_threshold) {
-            float4* cp = reinterpret_cast<float4*>(a.C + (size_t)i * (size_t)a.ldc) + vec0;
-            float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (on && a.beta != 0.f) old = __ldcs(cp);          // requested before the gather; streams through, must not displace rows of B in L2
-            gather_v4<U>(bl, ld4, a.col + e0 + lane, a.val + e0 + lane, (int)len, on, acc);
-            if (on) {
-                if constexpr (PLAIN) {
-                    __stcs(cp, make_float4(fmaf(a.beta, old.x, acc.x), fmaf(a.beta, old.y, acc.y), fmaf(a.beta, old.z, acc.z),
-                                           fmaf(a.beta, old.w, acc.w)));
+        __threadfence();                                          // the partial sum is in place before the count says so
+        __syncwarp();
+        int before = -1;
+        if (valid && gl == 0) before = atomicAdd(a.arrived + (int64_t)ch.heavy * DG_FINISH_TILES + blockIdx.y, 1);
+        before = __shfl_sync(0xffffffffu, before, 0, LPR);
+        if (!valid || before != ch.nchunks - 1) return;
+        __threadfence();
+        if (gl == 0) a.arrived[(int64_t)ch.heavy * DG_FINISH_TILES + blockIdx.y] = 0;
+        begin_row(ch.row, add_first);
+        const float* sp = a.scratch + (int64_t)ch.slot0 * a.lds + (int64_t)vec0 * VEC;
+#pragma unroll
+        for (int t = 0; t < TPL; ++t) {
+            if (!on[t]) continue;
+            const float* p = sp + t * LPR * VEC;
+#pragma unroll 4
+            for (int s = 0; s < ch.nchunks; ++s) {
+                const float* ps = p + s * a.lds;
+                if constexpr (VEC == 4) {
+                    const float4 x = __ldcg(reinterpret_cast<const float4*>(ps));
+                    acc[t][0] += x.x; acc[t][1] += x.y; acc[t][2] += x.z; acc[t][3] += x.w;
+                } else if constexpr (VEC == 2) {
+                    const float2 x = __ldcg(reinterpret_cast<const float2*>(ps));
+                    acc[t][0] += x.x; acc[t][1] += x.y;
                 } else {
-                    const int c = vec0 * 4;
-                    __stcs(cp, make_float4(finish(a, acc.x, old.x, i, c), finish(a, acc.y, old.y, i, c + 1),
-                                           finish(a, acc.z, old.z, i, c + 2), finish(a, acc.w, old.w, i, c + 3)));
+                    acc[t][0] += __ldcg(ps);
                 }
             }
-            acc = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        int nxt = 0;
-        if (lane == 0) nxt = atomicAdd(&next_row, 1);
-        r = __shfl_sync(0xffffffffu, nxt, 0);
+        store_row(ch.row);
+        return;
+    }
+
+    constexpr int kClasses = 24;
+    __shared__ int64_t first[257];                                // row offsets of the window
+    __shared__ uint8_t order[256];                                // its light rows, longest class first
+    __shared__ int count[kClasses], start[kClasses + 1], next;
+    const int32_t row0 = ((int)blockIdx.x - chunk_ctas) * a.rows_per_cta;
+    const int nrows = min(a.rows_per_cta, a.m - row0);
+    if (threadIdx.x < kClasses) count[threadIdx.x] = 0;
+    if (threadIdx.x == 0) next = 0;
+    for (int i = threadIdx.x; i <= nrows; i += 256) first[i] = __ldg(a.rowptr + row0 + i);
+    __syncthreads();
+    int cls = -1, place = 0;
+    if ((int)threadIdx.x < nrows) {
+        const int64_t len = first[threadIdx.x + 1] - first[threadIdx.x];
+        if (len <= a.heavy_threshold) {
+            const int s = ((int)len + LPR - 1) / LPR;             // batches of LPR entries: classes 0, 1, 2, 3, 4-5, 6-7, 8-11, ...
+            const int rank = s < 4 ? s : 2 * (31 - __clz(s)) + ((s >> (30 - __clz(s))) & 1);
+            cls = kClasses - 1 - min(rank, kClasses - 1);
+            place = atomicAdd(&count[cls], 1);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int n = threadIdx.x < kClasses ? count[threadIdx.x] : 0, sum = n;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, sum, off);
+            if ((int)threadIdx.x >= off) sum += o;
+        }
+        if (threadIdx.x <= kClasses) start[threadIdx.x] = sum - n;
+    }
+    __syncthreads();
+    if (cls >= 0) order[start[cls] + place] = (uint8_t)threadIdx.x;
+    __syncthreads();
+    const int total = start[kClasses];
+
+    int r = -1, c = 0;
+    float v = 0.f;
+    auto take = [&] {                                             // the next G rows, one per group, and their first entries
+        int b = 0;
+        if ((threadIdx.x & 31) == 0) b = atomicAdd(&next, G);
+        b = __shfl_sync(0xffffffffu, b, 0);
+        r = -1; c = 0; v = 0.f;
+        if (b + grp < total) {
+            r = order[b + grp];
+            const int64_t e = first[r] + gl;
+            if (e < first[r + 1]) {
+                c = __ldcs(a.col + e);
+                v = __ldcs(a.val + e);
+            }
+        }
+        return b < total;
+    };
+    bool more = take();
+    while (more) {
+        const int cur = r, cur_c = c;
+        const float cur_v = v;
+        more = take();
+        const bool valid = cur >= 0;
+        begin_row(row0 + cur, add_first && valid);
+        const int64_t e = valid ? first[cur] : 0;
+        gather(e + gl, valid ? (int)(first[cur + 1] - e) : 0, cur_c, cur_v);
+        if (valid) store_row(row0 + cur);
     }
 }
 
-int launch_v4(const SpmmArgs& a, cudaStream_t stream)
+template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED>
+int launch(SpmmArgs a, cudaStream_t stream)
 {
-    constexpr int U = DG_V4_UNROLL;
-    const int col_tiles = (a.nvec + 31) / 32;
-    const int chunk_ctas = (a.n_chunks + 7) / 8;
+    constexpr int NG = 256 / LPR, tile = LPR * TPL;
+    const int chunk_ctas = (a.n_chunks + NG - 1) / NG;
     const int64_t row_ctas = ((int64_t)a.m + a.rows_per_cta - 1) / a.rows_per_cta;
-    if (chunk_ctas + row_ctas > 0) {
-        dim3 grid((unsigned)(chunk_ctas + row_ctas), (unsigned)col_tiles);
-        if (a.flags == 0u && a.alpha == 1.f) k_spmm_v4<U, true><<<grid, 256, 0, stream>>>(a, chunk_ctas);
-        else k_spmm_v4<U, false><<<grid, 256, 0, stream>>>(a, chunk_ctas);
-        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    }
-    if (a.n_heavy > 0) {
-        k_spmm_heavy_finish<<<(unsigned)a.n_heavy, 256, 0, stream>>>(a);
+    for (; a.vec_first < a.vec_end; a.vec_first += tile * DG_FINISH_TILES) {
+        const dim3 grid((unsigned)(chunk_ctas + row_ctas), (unsigned)std::min((a.vec_end - a.vec_first + tile - 1) / tile, DG_FINISH_TILES));
+        k_spmm<VEC, LPR, TPL, U, MINB, PADDED><<<grid, 256, 0, stream>>>(a, chunk_ctas);
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     }
     return (int)cudaGetLastError();
 }
 
-template <int VEC, int LPR, int TPL>
-int launch_variant(const SpmmArgs& a, cudaStream_t stream)
+// Lanes per item and gathers in flight by the number of vectors in a row.  Tiles of 64 float4 go two per lane: half the index
+// traffic and half the chains of row latencies of one per lane, 10 to 25 % faster at every size although only 40 warps fit
+// an SM; two gathers in flight there (one or four are slower, four much).  What is left behind whole tiles of 64 takes launches
+// of its own in the forms that suit it, 32 vectors and then up to 32 more, unless it fills most of a tile (115 M entries,
+// F = 604: 18.4 -> 16.6 ms).  With 17 to 32 float4 a product that fills the GPU for long runs best on 64 warps with one gather
+// each, a short one on four gathers per warp; narrower rows take four.
+template <int VEC, bool PADDED>
+int launch_vec(SpmmArgs a, bool large, cudaStream_t stream)
 {
-    constexpr int U = (TPL * VEC >= 8) ? 1 : 2;          // gathers in flight per lane group before the first FMA
-    const int col_chunks = (a.nvec + LPR * TPL - 1) / (LPR * TPL);
-    if (a.m > 0) {
-        dim3 grid((unsigned)(((int64_t)a.m + a.rows_per_cta - 1) / a.rows_per_cta), (unsigned)col_chunks);
-        k_spmm_rows<VEC, LPR, TPL, U><<<grid, 256, 0, stream>>>(a);
-        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    const int end = a.vec_end, wide = end % 64 > 48 ? end : end / 64 * 64;
+    int rc = DG_OK;
+    if (wide > 0) {
+        a.vec_end = wide;
+        rc = launch<VEC, 32, 2, VEC == 4 ? 2 : 4, VEC == 4 && !PADDED ? 5 : 4, PADDED>(a, stream);
+        a.vec_first = wide;
     }
-    if (a.n_chunks > 0) {
-        dim3 grid((unsigned)((a.n_chunks + 7) / 8), (unsigned)col_chunks);
-        k_spmm_chunks<VEC, LPR, TPL, U><<<grid, 256, 0, stream>>>(a);
-        k_spmm_heavy_finish<<<(unsigned)a.n_heavy, 256, 0, stream>>>(a);
-        g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
+    while (rc == DG_OK && a.vec_first < end) {
+        a.vec_end = std::min(end, a.vec_first + 32);
+        const int nvec = a.vec_end - a.vec_first;
+        if (nvec <= 4) rc = launch<VEC, 4, 1, 4, 5, PADDED>(a, stream);
+        else if (nvec <= 8) rc = launch<VEC, 8, 1, 4, 5, PADDED>(a, stream);
+        else if (nvec <= 16) rc = launch<VEC, 16, 1, 4, 5, PADDED>(a, stream);
+        else if (VEC == 4 && large) rc = launch<VEC, 32, 1, 1, 8, PADDED>(a, stream);
+        else rc = launch<VEC, 32, 1, 4, 5, PADDED>(a, stream);
+        a.vec_first = a.vec_end;
     }
-    return (int)cudaGetLastError();
-}
-
-template <int VEC>
-int launch_vec(const SpmmArgs& a, cudaStream_t stream)
-{
-    const int nvec = a.nvec;
-    if (nvec <= 4) return launch_variant<VEC, 4, 1>(a, stream);
-    if (nvec <= 8) return launch_variant<VEC, 8, 1>(a, stream);
-    if (nvec <= 16) return launch_variant<VEC, 16, 1>(a, stream);
-    if (nvec <= 32) return launch_variant<VEC, 32, 1>(a, stream);
-    if (nvec <= 64) return launch_variant<VEC, 32, 2>(a, stream);
-    return launch_variant<VEC, 32, 4>(a, stream);       // wider rows take ceil(nvec/128) column chunks
+    return rc;
 }
 
 bool aligned(const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) % bytes) == 0; }
+
+// Floats of scratch behind the partial sums for a padded copy of the operand, 0 where none is made.  The copy costs a pass
+// over B and pays where its rows are gathered several times: 200,003 nodes, 10.2 M entries, F = 41: 336 -> 235 us.
+int64_t pad_floats(const dg_plan* plan, int32_t F)
+{
+    return F % 4 && F > 4 && plan->nnz >= 4 * (int64_t)plan->k ? (int64_t)plan->k * ((F + 3) / 4 * 4) : 0;
+}
+
+int64_t partial_floats(const dg_plan* plan, int32_t F) { return (int64_t)plan->n_chunks * ((F + 3) / 4 * 4); }
 
 }  // namespace
 
@@ -434,30 +415,39 @@ int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, in
 
 int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                         int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                        float* scratch, cudaStream_t stream)
+                        float* scratch, int64_t scratch_floats, cudaStream_t stream)
 {
     if (plan->m == 0 || F == 0) return DG_OK;
     SpmmArgs a{};
     a.rowptr = plan->rowptr; a.col = plan->col; a.val = val; a.B = B; a.C = C;
-    a.row_scale = row_scale; a.bias = bias; a.chunks = plan->chunks; a.heavy = plan->heavy; a.scratch = scratch;
-    a.ldb = ldb; a.ldc = ldc; a.m = plan->m; a.F = F;
-    a.heavy_threshold = plan->heavy_threshold; a.n_chunks = plan->n_chunks; a.n_heavy = plan->n_heavy;
-    a.rows_per_cta = 64;
+    a.row_scale = row_scale; a.bias = bias; a.chunks = plan->chunks; a.arrived = plan->arrived; a.scratch = scratch;
+    a.ldb = ldb; a.ldc = ldc; a.lds = F; a.m = plan->m; a.F = F;
+    a.heavy_threshold = plan->heavy_threshold; a.n_chunks = plan->n_chunks;
+    // Rows per CTA: as wide a window as still gives every SM a dozen CTAs (wider windows sort better and share their offsets;
+    // 64 rows are best at 150 k rows, 128 at 300 k, 256 from 1 M).
+    a.rows_per_cta = 32;
+    while (a.rows_per_cta < 256 && (int64_t)a.rows_per_cta * 2 * 2000 <= plan->m) a.rows_per_cta *= 2;
     a.alpha = alpha; a.beta = beta; a.flags = flags;
     // widest vector the shapes and addresses allow (B may be NULL only when there is nothing to gather)
     int vec = 1;
     if (F % 4 == 0 && ldb % 4 == 0 && ldc % 4 == 0 && aligned(B, 16) && aligned(C, 16)) vec = 4;
     else if (F % 2 == 0 && ldb % 2 == 0 && ldc % 2 == 0 && aligned(B, 8) && aligned(C, 8)) vec = 2;
-    a.nvec = F / vec;
-    // The lean kernel takes rows of more than 64 floats, and narrower ones (36 to 64 floats) when the rows are short: there
-    // (stage blocks of a partition, about 6 entries per row) it is 18 % faster than the generic kernel, which wins on long
-    // rows by walking two entries per warp at a time (whole graph, F = 48: 4.1 against 4.9 ms).
-    const bool narrow_ok = a.nvec > 8 && plan->nnz < (int64_t)16 * plan->m;
-    if (vec == 4 && (a.nvec > 16 || narrow_ok) && (int64_t)plan->k * (ldb / 4) + a.nvec < (int64_t)INT32_MAX) return launch_v4(a, stream);
+    const bool large = plan->nnz >= (int64_t)4 << 20;
+    const int64_t copy = pad_floats(plan, F), sums = partial_floats(plan, F);
+    if (vec < 4 && copy > 0 && sums + copy <= scratch_floats && aligned(scratch, 16)) {
+        float* wide = scratch + sums;
+        const int64_t ld = (F + 3) / 4 * 4;
+        const int rc = dg_pad_rows(B, ldb, plan->k, F, wide, ld, stream);
+        if (rc) return rc;
+        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        a.B = wide; a.ldb = ld; a.lds = ld; a.vec_end = (int32_t)(ld / 4);
+        return launch_vec<4, true>(a, large, stream);
+    }
+    a.vec_end = F / vec;
     switch (vec) {
-        case 4: return launch_vec<4>(a, stream);
-        case 2: return launch_vec<2>(a, stream);
-        default: return launch_vec<1>(a, stream);
+        case 4: return launch_vec<4, false>(a, large, stream);
+        case 2: return launch_vec<2, false>(a, large, stream);
+        default: return launch_vec<1, false>(a, large, stream);
     }
 }
 
@@ -465,7 +455,7 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
 // profile events while a profile is open.
 int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                    int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                   float* scratch, cudaStream_t stream)
+                   float* scratch, int64_t scratch_floats, cudaStream_t stream)
 {
     if (plan->m == 0 || F == 0) return DG_OK;
     bool profiled = false;
@@ -486,7 +476,7 @@ int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_
         rc = dg_spmm_stream_launch(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, stream, &launches);
         g_kernel_launches.fetch_add(launches, std::memory_order_relaxed);
     } else {
-        rc = dg_spmm_launch_rows(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, stream);
+        rc = dg_spmm_launch_rows(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, scratch_floats, stream);
     }
     if (profiled) {
         std::lock_guard<std::mutex> lock(g_profile.mu);
@@ -531,7 +521,8 @@ int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream)
 {
     if (!plan) return DG_ERR_NULL;
     dg_plan* p = const_cast<dg_plan*>(plan);
-    const int64_t need = dg_stream_selected() ? dg_scratch_floats(plan, F) : (int64_t)plan->n_chunks * F;
+    const int64_t rows = partial_floats(plan, F) + pad_floats(plan, F), tasks = dg_stream_selected() ? 2 * (int64_t)plan->n_tasks * F : 0;
+    const int64_t need = rows > tasks ? rows : tasks;
     if (need > p->scratch_floats) {
         DG_CUDA(cudaStreamSynchronize(stream));
         cudaFree(p->scratch);
@@ -549,17 +540,9 @@ extern "C" int dg_spmm_csr(const dg_plan* plan, const float* val, const float* B
 {
     int rc = dg_check_spmm_args(plan, val, B, ldb, C, ldc, F, flags, row_scale, bias);
     if (rc) return rc;
-    dg_plan* p = const_cast<dg_plan*>(plan);
-    const int64_t need = dg_spmm_stream_eligible(plan, B, ldb, C, ldc, F) ? 2 * (int64_t)p->n_tasks * F : (int64_t)p->n_chunks * F;
-    if (need > p->scratch_floats) {     // first use at this width: grow the plan's scratch (allocates, synchronises)
-        DG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-        cudaFree(p->scratch);
-        p->scratch = nullptr;
-        p->scratch_floats = 0;
-        DG_CUDA(cudaMalloc((void**)&p->scratch, (size_t)need * sizeof(float)));
-        p->scratch_floats = need;
-    }
-    return dg_spmm_launch(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, p->scratch, (cudaStream_t)stream);
+    if ((rc = dg_spmm_prepare(plan, F, (cudaStream_t)stream))) return rc;      // first use at this width may grow the scratch
+    return dg_spmm_launch(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, plan->scratch, plan->scratch_floats,
+                          (cudaStream_t)stream);
 }
 
 extern "C" int dg_spmm_coo(const int32_t* row, const int32_t* col, const float* val, int64_t nnz, int32_t m, int32_t k,

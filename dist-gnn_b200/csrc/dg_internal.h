@@ -52,7 +52,7 @@ struct dg_plan {
     int64_t heavy_nnz, max_row_nnz, touched_columns;
     float* scratch;           // device, grown on demand by dg_spmm_prepare
     int64_t scratch_floats;
-    // streaming kernel: the entry list cut into tasks of task_nnz entries, one warp each
+    // streaming kernel: the entry list cut into tasks of task_nnz entries, one warp each (0 until that family is first used)
     int32_t task_nnz, n_tasks, n_split;
     int32_t* task_first_row;  // device, n_tasks: the row that holds entry t * task_nnz
     dg_split_row* split;      // device, n_split rows that span tasks, ascending
@@ -73,8 +73,11 @@ int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_
 int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                         int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
                         float* scratch, int64_t scratch_floats, cudaStream_t stream);
-int dg_plan_build(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k, int32_t heavy_threshold,
-                  int32_t chunk, bool lean, void* stream, dg_plan** out);
+int dg_plan_build_lean(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k, void* stream, dg_plan** out);
+int dg_plan_ensure_tasks(dg_plan* plan, cudaStream_t stream);
+// Device memory of plans (dg_pool.cu), on the current device.  A block may be freed once the device is done with it.
+int dg_pool_alloc(void** out, size_t bytes);
+void dg_pool_free(void* ptr);
 int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream);
 int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, int64_t ldb, const float* C, int64_t ldc,
                        int32_t F, uint32_t flags, const float* row_scale, const float* bias);

@@ -1,0 +1,99 @@
+// Device memory of plans: blocks that outlive the plan that used them.
+//
+// cudaMalloc and cudaFree cost tens of microseconds at best and, on a device whose memory is mostly mapped, now and then
+// milliseconds; building a plan took 45 of the former and 54 of the latter, most of the 8 to 30 ms that plan construction
+// and one product of a 300 k-row block cost.  Freed blocks are kept per device, at most kKeepBytes of them, and handed out
+// again to requests of a similar size.  A block may come back only when the device is done with it: callers synchronise
+// first (dg_plan_destroy the device, as cudaFree did; plan construction its stream).  A failed allocation gives everything
+// back and tries again; dg_pool_trim gives everything back on request.
+#include <map>
+#include <mutex>
+#include <unordered_map>
+#include "dg_internal.h"
+
+namespace {
+
+constexpr size_t kKeepBytes = (size_t)512 << 20;
+constexpr int kMaxDevices = 64;
+
+struct Pool {
+    std::mutex mu;
+    std::multimap<size_t, void*> unused[kMaxDevices];
+    size_t unused_bytes[kMaxDevices] = {};
+    std::unordered_map<void*, size_t> size[kMaxDevices];
+};
+Pool& pool() { static Pool* p = new Pool(); return *p; }      // never destroyed: the driver may be gone first
+
+// Sizes in steps of an eighth of their power of two, so that blocks of nearly equal plans fit one another.
+size_t rounded(size_t bytes)
+{
+    size_t step = 512;
+    while (step * 16 < bytes) step *= 2;
+    return (bytes + step - 1) / step * step;
+}
+
+void release_unused(Pool& p, int dev)                             // caller holds the mutex and has dev current
+{
+    for (auto& b : p.unused[dev]) {
+        cudaFree(b.second);
+        p.size[dev].erase(b.second);
+    }
+    p.unused[dev].clear();
+    p.unused_bytes[dev] = 0;
+}
+
+}  // namespace
+
+int dg_pool_alloc(void** out, size_t bytes)
+{
+    int dev = -1;
+    DG_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) return DG_ERR_STATE;
+    const size_t want = rounded(bytes ? bytes : 1);
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    auto it = p.unused[dev].lower_bound(want);
+    if (it != p.unused[dev].end() && it->first <= want + want / 4) {
+        *out = it->second;
+        p.unused_bytes[dev] -= it->first;
+        p.unused[dev].erase(it);
+        return DG_OK;
+    }
+    cudaError_t e = cudaMalloc(out, want);
+    if (e == cudaErrorMemoryAllocation && !p.unused[dev].empty()) {
+        cudaGetLastError();
+        release_unused(p, dev);
+        e = cudaMalloc(out, want);
+    }
+    if (e != cudaSuccess) return (int)e;
+    p.size[dev][*out] = want;
+    return DG_OK;
+}
+
+void dg_pool_free(void* ptr)
+{
+    int dev = -1;
+    if (!ptr || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    auto it = p.size[dev].find(ptr);
+    if (it == p.size[dev].end()) return;
+    if (p.unused_bytes[dev] + it->second > kKeepBytes) {
+        p.size[dev].erase(it);
+        cudaFree(ptr);
+        return;
+    }
+    p.unused[dev].emplace(it->second, ptr);
+    p.unused_bytes[dev] += it->second;
+}
+
+extern "C" int dg_pool_trim(void)
+{
+    int dev = -1;
+    DG_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices) return DG_ERR_STATE;
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    release_unused(p, dev);
+    return DG_OK;
+}

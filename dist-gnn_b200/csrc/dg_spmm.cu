@@ -521,14 +521,19 @@ int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream)
 {
     if (!plan) return DG_ERR_NULL;
     dg_plan* p = const_cast<dg_plan*>(plan);
+    if (dg_stream_selected()) {
+        const int rc = dg_plan_ensure_tasks(p, stream);
+        if (rc) return rc;
+    }
     const int64_t rows = partial_floats(plan, F) + pad_floats(plan, F), tasks = dg_stream_selected() ? 2 * (int64_t)plan->n_tasks * F : 0;
     const int64_t need = rows > tasks ? rows : tasks;
     if (need > p->scratch_floats) {
         DG_CUDA(cudaStreamSynchronize(stream));
-        cudaFree(p->scratch);
+        dg_pool_free(p->scratch);
         p->scratch = nullptr;
         p->scratch_floats = 0;
-        DG_CUDA(cudaMalloc((void**)&p->scratch, (size_t)need * sizeof(float)));
+        const int rc = dg_pool_alloc((void**)&p->scratch, (size_t)need * sizeof(float));
+        if (rc) return rc;
         p->scratch_floats = need;
     }
     return DG_OK;
@@ -549,7 +554,7 @@ extern "C" int dg_spmm_coo(const int32_t* row, const int32_t* col, const float* 
                            const float* B, float* C, int32_t F, float alpha, float beta, void* stream)
 {
     dg_plan* plan = nullptr;
-    int rc = dg_plan_build(row, col, nnz, m, k, 0, 0, /*lean=*/true, stream, &plan);
+    int rc = dg_plan_build_lean(row, col, nnz, m, k, stream, &plan);
     if (rc) return rc;
     rc = dg_spmm_csr(plan, val, B, F, C, F, F, alpha, beta, 0u, nullptr, nullptr, stream);
     if (rc == DG_OK) rc = (int)cudaStreamSynchronize((cudaStream_t)stream);   // the plan's buffers die below

@@ -65,7 +65,17 @@ int dg_plan_create(const int32_t* row, const int32_t* col, int64_t nnz, int32_t 
                    void* stream, dg_plan** out);
 int dg_plan_create_ex(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k,
                       int32_t heavy_threshold, int32_t chunk, void* stream, dg_plan** out);
+/* The same from int64 ids, as a loader's coalesced block holds them: they are read once, and the column ids are narrowed into
+ * col32 (nnz ints of the caller's, BORROWED like `col` above).  Ids are range-checked before they are narrowed. */
+int dg_plan_create_i64(const int64_t* row, const int64_t* col, int64_t nnz, int32_t m, int32_t k, int32_t heavy_threshold,
+                       int32_t chunk, int32_t* col32, void* stream, dg_plan** out);
 int dg_plan_destroy(dg_plan* plan);
+/* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device; this gives all of it on the current
+ * device back (a failed allocation of the library does so by itself). */
+int dg_pool_trim(void);
+/* *host_equal = 1 if both id lists hold the same nnz entries, else 0 (one pass; waits for `stream`). */
+int dg_ids_equal(const int32_t* row_a, const int32_t* col_a, const int32_t* row_b, const int32_t* col_b, int64_t nnz,
+                 int* host_equal, void* stream);
 int dg_plan_get_stats(const dg_plan* plan, dg_plan_stats* host_out);
 /* The streaming kernel cuts the entry list into tasks of `task_nnz` entries (one warp each; default 1024).  This
  * rebuilds the task tables for another size (<= 0 restores the default); synchronises `stream`. */

@@ -350,3 +350,33 @@ def test_streaming_kernel_epilogue_and_reproducibility():
     assert_close(outs[0].numpy(), want, TOL, 'streaming epilogue')
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     assert plan.device_status() == 0
+
+
+@pytest.mark.parametrize('m,k,nnz', [(1, 1, 1), (300, 190, 5000), (4099, 257, 1024), (5000, 100003, 70001)])
+def test_plan_from_int64_ids_equals_the_int32_plan(m, k, nnz):
+    """The loader's int64 block narrowed while the plan is built: same offsets, columns and census as from int32 arrays
+    (with empty first and last rows, split rows, and entry counts around a CTA's share), ids beyond int32 are refused, and a
+    plan built in the blocks an earlier one left behind is none the wiser."""
+    import spmm_cpp
+    rng = np.random.Generator(np.random.PCG64(m + k))
+    A = random_coo(rng, m, k, min(nnz, m * k)) if m * k < 10**8 else ref_graph.Coo(
+        np.sort(rng.integers(0, m // 50, nnz)), rng.integers(0, k, nnz), np.ones(nnz, np.float32), (m, k))
+    if m > 1:
+        keep = (A.row > 2) & (A.row < m - 2)
+        A = ref_graph.Coo(A.row[keep], A.col[keep], A.val[keep], A.shape)
+    t = torch.sparse_coo_tensor(torch.from_numpy(np.stack((A.row, A.col))), torch.from_numpy(A.val), A.shape, is_coalesced=True).cuda()
+    for _ in range(2):
+        wide, narrow = spmm_cpp.SpmmPlan.from_coo(t, 40, 16), make_plan(A, heavy_threshold=40, chunk=16)
+        assert torch.equal(wide.col, narrow.col) and torch.equal(wide.rowptr(), narrow.rowptr()) and wide.stats() == narrow.stats()
+        assert np.array_equal(wide.rowptr().numpy(), ref_graph.rowptr_of(A))
+        deg = np.bincount(A.row, minlength=m)
+        st = wide.stats()
+        assert st['heavy_rows'] == int((deg > 40).sum()) and st['heavy_chunks'] == sum(-(-int(d) // 16) for d in deg if d > 40)
+        assert st['touched_columns'] == np.unique(A.col).size and st['max_row_nnz'] == deg.max()
+        B, C, D = torch.randn(k, 20, device='cuda'), torch.zeros(m, 20, device='cuda'), torch.zeros(m, 20, device='cuda')
+        assert torch.equal(wide.spmm(B, C, 1.0, 0.0), narrow.spmm(B, D, 1.0, 0.0))
+        del wide, narrow
+    row, col = torch.zeros(1, dtype=torch.int64, device='cuda'), torch.tensor([2**32], dtype=torch.int64, device='cuda')
+    out, narrowed = ctypes.c_void_p(), torch.empty(1, dtype=torch.int32, device='cuda')
+    assert spmm_cpp.lib().dg_plan_create_i64(row.data_ptr(), col.data_ptr(), 1, m, k, 0, 0, narrowed.data_ptr(), None, ctypes.byref(out)) == -3
+    spmm_cpp.empty_cache()

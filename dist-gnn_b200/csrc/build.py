@@ -9,7 +9,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(os.path.dirname(HERE))
-SOURCES = ['dg_pool.cu', 'dg_plan.cu', 'dg_spmm.cu', 'dg_spmm_stream.cu', 'dg_spmm_static.cu', 'dg_dense.cu', 'dg_pipeline.cu', 'dg_peer.cu', 'dg_rows.cu', 'dg_marks.cu', 'dg_gcn.cu']
+SOURCES = ['dg_pool.cu', 'dg_plan.cu', 'dg_tiles.cu', 'dg_spmm.cu', 'dg_spmm_stream.cu', 'dg_spmm_static.cu', 'dg_dense.cu', 'dg_pipeline.cu', 'dg_peer.cu', 'dg_rows.cu', 'dg_marks.cu', 'dg_gcn.cu']
 OUTPUT = os.path.join(HERE, 'libdist_gnn_b200.so')
 
 
@@ -37,7 +37,7 @@ def command(verbose=False):
 def up_to_date(srcs):
     if not os.path.exists(OUTPUT):
         return False
-    deps = srcs + [os.path.join(HERE, 'dg_internal.h'), os.path.join(HERE, 'dg_comm.h'), os.path.join(ROOT, 'include', 'dist_gnn_b200.h'), __file__]
+    deps = srcs + [os.path.join(HERE, 'dg_internal.h'), os.path.join(HERE, 'dg_comm.h'), os.path.join(HERE, 'dg_tiles.h'), os.path.join(HERE, 'dg_umma.h'), os.path.join(ROOT, 'include', 'dist_gnn_b200.h'), __file__]
     return all(os.path.getmtime(d) <= os.path.getmtime(OUTPUT) for d in deps)
 
 

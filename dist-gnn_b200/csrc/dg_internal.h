@@ -39,6 +39,8 @@ struct dg_split_row {
 
 #define DG_DEFAULT_TASK_NNZ 1024
 
+struct dg_tiles;      // dg_tiles.h
+
 struct dg_plan {
     int device;
     int32_t m, k;
@@ -56,6 +58,7 @@ struct dg_plan {
     int32_t task_nnz, n_tasks, n_split;
     int32_t* task_first_row;  // device, n_tasks: the row that holds entry t * task_nnz
     dg_split_row* split;      // device, n_split rows that span tasks, ascending
+    dg_tiles* tiles;          // tensor-core part of the split rows, or null
     int* status;              // device word: set non-zero by a kernel that gave up on a bounded wait
 };
 

@@ -11,6 +11,7 @@
 #include <new>
 #include <vector>
 #include "dg_internal.h"
+#include "dg_tiles.h"
 
 namespace {
 
@@ -439,6 +440,7 @@ extern "C" int dg_plan_destroy(dg_plan* p)
     cudaDeviceSynchronize();              // products on any stream are done with the blocks before the pool may hand them out
     for (void* b : {(void*)p->rowptr, (void*)p->chunks, (void*)p->arrived, (void*)p->scratch, (void*)p->task_first_row, (void*)p->split, (void*)p->status})
         dg_pool_free(b);
+    dg_tiles_free(p->tiles);
     if (prev != p->device && prev >= 0) cudaSetDevice(prev);
     delete p;
     return DG_OK;

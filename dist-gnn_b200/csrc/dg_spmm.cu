@@ -14,6 +14,7 @@
 #include <mutex>
 #include <vector>
 #include "dg_internal.h"
+#include "dg_tiles.h"
 
 namespace {
 
@@ -50,6 +51,11 @@ struct SpmmArgs {
     const float* row_scale;
     const float* bias;
     const dg_chunk* chunks;
+    const int32_t* chunk_col;   // entries of the chunks: the matrix's own, or what the tiles leave of the split rows
+    const float* chunk_val;
+    const int2* parts;          // partial results of the tiles per split row (dg_tiles.h), or null
+    const float4* part_area;
+    int64_t part_ld4;           // 16-byte pieces of a partial row
     int* arrived;               // [n_heavy x DG_FINISH_TILES] partial sums of a split row that are in place; zero between products
     float* scratch;
     int64_t ldb, ldc, lds;      // lds: row stride of the partial sums
@@ -129,15 +135,15 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
     float acc[TPL][VEC];
 
     // acc += sum over this group's `len` entries; `e` is this lane's first entry, c / v hold it already
-    auto gather = [&](int64_t e, int len, int c, float v) {
+    auto gather = [&](const int32_t* col, const float* val, int64_t e, int len, int c, float v) {
         const int longest = G == 1 ? len : __reduce_max_sync(0xffffffffu, len);
 #pragma unroll 1
         for (int base = 0; base < longest; base += LPR) {
             int c_next = 0;
             float v_next = 0.f;
             if (base + LPR + gl < len) {
-                c_next = __ldcs(a.col + e + base + LPR);          // streamed once: keep it from displacing rows of B in cache
-                v_next = __ldcs(a.val + e + base + LPR);
+                c_next = __ldcs(col + e + base + LPR);            // streamed once: keep it from displacing rows of B in cache
+                v_next = __ldcs(val + e + base + LPR);
             }
             const int cnt = len - base, steps = min(LPR, longest - base);
 #pragma unroll 1
@@ -229,11 +235,11 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
         int c = 0;
         float v = 0.f;
         if (gl < ch.len) {
-            c = __ldcs(a.col + ch.e0 + gl);
-            v = __ldcs(a.val + ch.e0 + gl);
+            c = __ldcs(a.chunk_col + ch.e0 + gl);
+            v = __ldcs(a.chunk_val + ch.e0 + gl);
         }
         begin_row(0, false);
-        gather(ch.e0 + gl, ch.len, c, v);
+        gather(a.chunk_col, a.chunk_val, ch.e0 + gl, ch.len, c, v);
         if (valid) {
             float* sp = a.scratch + (int64_t)ch.slot * a.lds + (int64_t)vec0 * VEC;
 #pragma unroll
@@ -271,6 +277,19 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
                 } else {
                     acc[t][0] += __ldcg(ps);
                 }
+            }
+        }
+        if constexpr (VEC == 4) {
+            if (a.parts) {
+                const int2 part = a.parts[ch.heavy];
+                const float4* p = a.part_area + ((int64_t)(part.x >> 7) * a.part_ld4 + vec0) * 128 + (part.x & 127);
+                for (int s = 0; s < part.y; ++s, p += a.part_ld4 * 128)
+#pragma unroll
+                    for (int t = 0; t < TPL; ++t) {
+                        if (!on[t]) continue;
+                        const float4 x = __ldcg(p + t * LPR * 128);
+                        acc[t][0] += x.x; acc[t][1] += x.y; acc[t][2] += x.z; acc[t][3] += x.w;
+                    }
             }
         }
         store_row(ch.row);
@@ -337,7 +356,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
         const bool valid = cur >= 0;
         begin_row(row0 + cur, add_first && valid);
         const int64_t e = valid ? first[cur] : 0;
-        gather(e + gl, valid ? (int)(first[cur + 1] - e) : 0, cur_c, cur_v);
+        gather(a.col, a.val, e + gl, valid ? (int)(first[cur + 1] - e) : 0, cur_c, cur_v);
         if (valid) store_row(row0 + cur);
     }
 }
@@ -394,6 +413,12 @@ int64_t pad_floats(const dg_plan* plan, int32_t F)
     return F % 4 && F > 4 && plan->nnz >= 4 * (int64_t)plan->k ? (int64_t)plan->k * ((F + 3) / 4 * 4) : 0;
 }
 
+// Floats of scratch behind those for the tensor-core part, 0 where it is not used: the tiles hold these very values.
+int64_t tile_floats(const dg_plan* plan, const float* val, int32_t F)
+{
+    return plan->tiles && (!val || plan->tiles->val == val) ? dg_tiles_scratch_floats(plan, F) : 0;
+}
+
 int64_t partial_floats(const dg_plan* plan, int32_t F) { return (int64_t)plan->n_chunks * ((F + 3) / 4 * 4); }
 
 }  // namespace
@@ -421,6 +446,7 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     SpmmArgs a{};
     a.rowptr = plan->rowptr; a.col = plan->col; a.val = val; a.B = B; a.C = C;
     a.row_scale = row_scale; a.bias = bias; a.chunks = plan->chunks; a.arrived = plan->arrived; a.scratch = scratch;
+    a.chunk_col = plan->col; a.chunk_val = val;
     a.ldb = ldb; a.ldc = ldc; a.lds = F; a.m = plan->m; a.F = F;
     a.heavy_threshold = plan->heavy_threshold; a.n_chunks = plan->n_chunks;
     // Rows per CTA: as wide a window as still gives every SM a dozen CTAs (wider windows sort better and share their offsets;
@@ -433,8 +459,19 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     if (F % 4 == 0 && ldb % 4 == 0 && ldc % 4 == 0 && aligned(B, 16) && aligned(C, 16)) vec = 4;
     else if (F % 2 == 0 && ldb % 2 == 0 && ldc % 2 == 0 && aligned(B, 8) && aligned(C, 8)) vec = 2;
     const bool large = plan->nnz >= (int64_t)4 << 20;
-    const int64_t copy = pad_floats(plan, F), sums = partial_floats(plan, F);
-    if (vec < 4 && copy > 0 && sums + copy <= scratch_floats && aligned(scratch, 16)) {
+    const int64_t copy = pad_floats(plan, F), sums = partial_floats(plan, F), tiled = tile_floats(plan, val, F);
+    const bool padded = vec < 4 && copy > 0 && sums + copy <= scratch_floats && aligned(scratch, 16);
+    if (tiled > 0 && (vec == 4 || padded) && sums + copy + tiled <= scratch_floats && aligned(scratch, 16)) {
+        float* area = scratch + sums + copy;
+        int launches = 0;
+        const int rc = dg_tiles_launch(plan, B, ldb, F, area, stream, &launches);
+        if (rc) return rc;
+        g_kernel_launches.fetch_add(launches, std::memory_order_relaxed);
+        const dg_tiles* t = plan->tiles;
+        a.chunks = t->rest_chunks; a.n_chunks = t->n_rest_chunks; a.chunk_col = t->rest_col; a.chunk_val = t->rest_val;
+        a.parts = t->parts; a.part_area = reinterpret_cast<const float4*>(area); a.part_ld4 = (F + 3) / 4;
+    }
+    if (padded) {
         float* wide = scratch + sums;
         const int64_t ld = (F + 3) / 4 * 4;
         const int rc = dg_pad_rows(B, ldb, plan->k, F, wide, ld, stream);
@@ -525,7 +562,7 @@ int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream)
         const int rc = dg_plan_ensure_tasks(p, stream);
         if (rc) return rc;
     }
-    const int64_t rows = partial_floats(plan, F) + pad_floats(plan, F), tasks = dg_stream_selected() ? 2 * (int64_t)plan->n_tasks * F : 0;
+    const int64_t rows = partial_floats(plan, F) + pad_floats(plan, F) + tile_floats(plan, nullptr, F), tasks = dg_stream_selected() ? 2 * (int64_t)plan->n_tasks * F : 0;
     const int64_t need = rows > tasks ? rows : tasks;
     if (need > p->scratch_floats) {
         DG_CUDA(cudaStreamSynchronize(stream));

@@ -305,7 +305,7 @@ def compact_exchange(env, adj_parts, stages, owner_packs=True):
     first = 0
     for count in group_sizes(len(kept), env.stage_group):
         row, col, val, rows_total = schedule.join_packed_blocks(blocks, lay['area_offsets'], first, count)
-        plans.append(spmm_cpp.SpmmPlan(row.to(torch.int32), col.to(torch.int32).contiguous(), val.contiguous(), n, rows_total))
+        plans.append(spmm_cpp.SpmmPlan(row.to(torch.int32), col.to(torch.int32).contiguous(), val.contiguous(), n, rows_total).tile())
         plan_slices.append((lay['area_offsets'][first], rows_total))
         plan_last.append(first + count - 1)
         first += count
@@ -377,7 +377,7 @@ def group_plans(adj_parts, parts, group):
         col = torch.cat([b.indices()[1] + off for b, off in zip(blocks, offsets)])
         val = torch.cat([b.values() for b in blocks])
         order = torch.sort(row * total + col).indices
-        plans.append(spmm_cpp.SpmmPlan(row[order].to(torch.int32), col[order].to(torch.int32), val[order].contiguous(), n, total))
+        plans.append(spmm_cpp.SpmmPlan(row[order].to(torch.int32), col[order].to(torch.int32), val[order].contiguous(), n, total).tile())
     _group_plan_cache[key] = (adj_parts, plans)
     return plans
 
@@ -517,7 +517,7 @@ def _gcn_net(plan, x, dims, pad, act, ld_act):
     """The dg_gcn_net of a call, and the arrays it points into."""
     L = len(act)
     arrays = (ctypes.c_int32 * (L + 1))(*dims), (ctypes.c_void_p * L)(*act), (ctypes.c_int64 * L)(*ld_act)
-    net = spmm_cpp.GcnNet(plan=plan.handle, val=plan.values.data_ptr(), x=x.data_ptr(), ldx=x.stride(0) if x.size(0) > 1 else pad[0],
+    net = spmm_cpp.GcnNet(plan=plan.handle, val=plan.value_ptr(), x=x.data_ptr(), ldx=x.stride(0) if x.size(0) > 1 else pad[0],
                           n=x.size(0), layers=L)
     net.dims, net.act, net.ld_act = (ctypes.addressof(a) for a in arrays)
     return net, arrays

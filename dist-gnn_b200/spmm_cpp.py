@@ -17,6 +17,13 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB_PATH = os.path.join(_HERE, 'csrc', 'libdist_gnn_b200.so')
 _lib = None
 
+# Blocks of at least TILE_NNZ entries whose plans are kept for many products (plan_for, the joined blocks of the stage loops) get
+# tensor-core tiles: below that the images of the frequent columns and two more launches cost what the tiles save (2.5 M
+# entries: nothing gained; 15.8 M: a fifth).  From TILE_ALWAYS entries on every plan made from a loader's block gets them:
+# normalising and sorting such a block took ten times as long as finding its tiles.
+TILE_NNZ = 8 << 20
+TILE_ALWAYS = 48 << 20
+
 EPI_ROW_SCALE, EPI_BIAS, EPI_RELU = 1, 2, 4
 ERR_UNSUPPORTED = -4
 
@@ -66,6 +73,9 @@ def lib():
             'dg_plan_create': ([vp, vp, i64, i32, i32, vp, pp], ctypes.c_int),
             'dg_plan_create_ex': ([vp, vp, i64, i32, i32, i32, i32, vp, pp], ctypes.c_int),
             'dg_plan_create_i64': ([vp, vp, i64, i32, i32, i32, i32, vp, vp, pp], ctypes.c_int),
+            'dg_plan_add_tiles': ([vp, vp, vp], ctypes.c_int),
+            'dg_plan_drop_tiles': ([vp, vp], ctypes.c_int),
+            'dg_plan_tiled_entries': ([vp], i64),
             'dg_pool_trim': ([], ctypes.c_int),
             'dg_ids_equal': ([vp, vp, vp, vp, i64, ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
             'dg_plan_destroy': ([vp], ctypes.c_int),
@@ -205,6 +215,7 @@ class SpmmPlan:
             check(lib().dg_plan_create_ex(row_i32.data_ptr(), col_i32.data_ptr(), values.numel(), self.m, self.k,
                                           heavy_threshold, chunk, _stream(), ctypes.byref(handle)))
         self.handle = handle
+        self._tiled = None
 
     @classmethod
     def from_coo(cls, A, heavy_threshold=0, chunk=0):
@@ -226,7 +237,33 @@ class SpmmPlan:
             check(lib().dg_plan_create_i64(base, base + 8 * idx.stride(0), nnz, self.m, self.k, heavy_threshold, chunk, self.col.data_ptr(),
                                            _raw_stream(index), ctypes.byref(handle)))
         self.handle = handle
+        self._tiled = None
+        return self.tile() if nnz >= TILE_ALWAYS else self
+
+    def tile(self):
+        """Moves the densest part of the block to the tensor cores for the products to come (dg_plan_add_tiles): worth its few
+        milliseconds for a block that is multiplied again and again, and done where it pays (at least TILE_NNZ entries, enough
+        of them in dense tiles).  The tiles hold the values as they are now; changing them in place afterwards is noticed by
+        the tensor's version counter, and the products then gather everything again."""
+        if self.values.numel() >= TILE_NNZ and self._tiled is None:
+            index = self.device.index
+            with _on(index):
+                check(lib().dg_plan_add_tiles(self.handle, self.values.data_ptr(), _raw_stream(index)))
+            if _lib.dg_plan_tiled_entries(self.handle):
+                self._tiled = self.values._version
         return self
+
+    def tiled_entries(self):
+        """Entries that products with this plan's own values take on the tensor cores."""
+        return int(lib().dg_plan_tiled_entries(self.handle))
+
+    def value_ptr(self):
+        """Address of the plan's values for the calls that take it beside the plan; drops tiles that the values have left behind."""
+        if self._tiled is not None and self._tiled != self.values._version:
+            self._tiled = None
+            with _on(self.device.index):
+                check(_lib.dg_plan_drop_tiles(self.handle, _raw_stream(self.device.index)))
+        return self.values.data_ptr()
 
     def stats(self):
         s = PlanStats()
@@ -254,7 +291,9 @@ class SpmmPlan:
 
     def spmm(self, B, C, alpha=1.0, beta=1.0, row_scale=None, bias=None, relu=False, values=None):
         """C <- epilogue(alpha * A @ B + beta * C) in place; B [k, F] and C [m, F] may be row-strided views."""
-        val = self.values if values is None else _dev_tensor(values, torch.float32, 'values')
+        if values is not None and values is not self.values:
+            _dev_tensor(values, torch.float32, 'values')
+        val = self.value_ptr() if values is None or values.data_ptr() == self.values.data_ptr() else values.data_ptr()
         ldb, ldc = _operand(B, self.k, 'B'), _operand(C, self.m, 'C')
         F = B.size(1)
         if F != C.size(1):
@@ -269,7 +308,7 @@ class SpmmPlan:
             bias_ptr = _dev_tensor(bias, torch.float32, 'bias').data_ptr()
         index = self.device.index
         with _on(index):
-            check(_lib.dg_spmm_csr(self.handle, val.data_ptr(), B.data_ptr(), ldb, C.data_ptr(), ldc, F, alpha, beta, flags,
+            check(_lib.dg_spmm_csr(self.handle, val, B.data_ptr(), ldb, C.data_ptr(), ldc, F, alpha, beta, flags,
                                    scale_ptr, bias_ptr, _raw_stream(index)))
         return C
 
@@ -341,7 +380,7 @@ def plan_for(A):
     hit = _plan_cache.get(key)
     if hit is not None and hit[0]() is A:
         return hit[1]
-    plan = SpmmPlan.from_coo(A)
+    plan = SpmmPlan.from_coo(A).tile()
     _plan_cache[key] = (weakref.ref(A, lambda _ref, key=key: _plan_cache.pop(key, None)), plan)
     return plan
 
@@ -472,7 +511,7 @@ def bcast_spmm(comm, roots, plans, x_local, recv, z, row_comm=None, timed=False,
         raise RuntimeError(f'{S} stages in groups of {group} need {(S + group - 1) // group} plans, got {len(plans)}')
     roots_arr = (ctypes.c_int32 * max(S, 1))(*roots)
     plan_arr = (ctypes.c_void_p * max(len(plans), 1))(*[p.handle for p in plans])
-    val_arr = (ctypes.c_void_p * max(len(plans), 1))(*[p.values.data_ptr() for p in plans])
+    val_arr = (ctypes.c_void_p * max(len(plans), 1))(*[p.value_ptr() for p in plans])
     recv = recv or []
     for b in recv:
         _dev_tensor(b, torch.float32, 'receive buffer')
@@ -501,7 +540,7 @@ def bcast_spmm_ordered(comm, roots, landing, products, x_local, z, row_comm=None
     roots_arr = (ctypes.c_int32 * max(S, 1))(*roots)
     land_arr = (ctypes.c_void_p * max(S, 1))(*[None if t is None else _dev_tensor(t, torch.float32, 'landing block').data_ptr() for t in landing])
     plan_arr = (ctypes.c_void_p * max(P, 1))(*[p.handle for p, _, _ in products])
-    val_arr = (ctypes.c_void_p * max(P, 1))(*[p.values.data_ptr() for p, _, _ in products])
+    val_arr = (ctypes.c_void_p * max(P, 1))(*[p.value_ptr() for p, _, _ in products])
     for plan, operand, _ in products:
         _dev_tensor(operand, torch.float32, 'operand')
         if operand.size(0) != plan.k or operand.size(1) != F:
@@ -550,7 +589,7 @@ def peer_spmm_packed(comm, packs, roots, stage_offsets, stage_rows, landing, pro
         if operand.size(0) != plan.k or operand.size(1) != F:
             raise RuntimeError(f'operand {tuple(operand.shape)} does not match a plan with {plan.k} columns and width {F}')
     plan_arr = (ctypes.c_void_p * max(P, 1))(*[p.handle for p, _, _ in products])
-    val_arr = (ctypes.c_void_p * max(P, 1))(*[p.values.data_ptr() for p, _, _ in products])
+    val_arr = (ctypes.c_void_p * max(P, 1))(*[p.value_ptr() for p, _, _ in products])
     op_arr = (ctypes.c_void_p * max(P, 1))(*[t.data_ptr() for _, t, _ in products])
     last_arr = (ctypes.c_int32 * max(P, 1))(*[l for _, _, l in products])
     with _on(x_local.device.index):
@@ -582,7 +621,7 @@ def peer_spmm_gather(comm, roots, stage_lists, stage_rows, landing, products, x_
         if operand.size(0) != plan.k or operand.size(1) != F:
             raise RuntimeError(f'operand {tuple(operand.shape)} does not match a plan with {plan.k} columns and width {F}')
     plan_arr = (ctypes.c_void_p * max(P, 1))(*[p.handle for p, _, _ in products])
-    val_arr = (ctypes.c_void_p * max(P, 1))(*[p.values.data_ptr() for p, _, _ in products])
+    val_arr = (ctypes.c_void_p * max(P, 1))(*[p.value_ptr() for p, _, _ in products])
     op_arr = (ctypes.c_void_p * max(P, 1))(*[t.data_ptr() for _, t, _ in products])
     last_arr = (ctypes.c_int32 * max(P, 1))(*[l for _, _, l in products])
     with _on(x_local.device.index):
@@ -617,7 +656,7 @@ def allgather_spmm(comm, plan, x_local, pack, area, z, widths, timed=False):
     pack_arr = (ctypes.c_void_p * 2)(pack[0].data_ptr(), pack[1].data_ptr())
     area_arr = (ctypes.c_void_p * 2)(area[0].data_ptr(), area[1].data_ptr())
     with _on(x_local.device.index):
-        check(lib().dg_allgather_spmm(comm.handle, plan.handle, plan.values.data_ptr(), x_local.data_ptr(), n, F, len(widths), w_arr,
+        check(lib().dg_allgather_spmm(comm.handle, plan.handle, plan.value_ptr(), x_local.data_ptr(), n, F, len(widths), w_arr,
                                       pack_arr, area_arr, z.data_ptr(), int(timed), _stream()))
     return z
 

@@ -70,6 +70,15 @@ int dg_plan_create_ex(const int32_t* row, const int32_t* col, int64_t nnz, int32
 int dg_plan_create_i64(const int64_t* row, const int64_t* col, int64_t nnz, int32_t m, int32_t k, int32_t heavy_threshold,
                        int32_t chunk, int32_t* col32, void* stream, dg_plan** out);
 int dg_plan_destroy(dg_plan* plan);
+/* Lets products on this plan multiply the densest part of the block - long rows x frequent columns - on the tensor cores
+ * (six bf16 passes on three-piece splits: fp32 accuracy).  A one-off step for a block that will be multiplied many times: it
+ * makes a second copy of the split rows' entries (8 bytes each) WITH their values `val`; products with another `val` pointer
+ * are gathered as before, and a caller that changes the values in place calls this again or dg_plan_drop_tiles.  Returns
+ * DG_OK without doing anything where the block has too few dense tiles.  Synchronises `stream`; no product on the plan may be
+ * in flight.  dg_plan_tiled_entries: how many entries the tensor cores take (0: no tiles). */
+int dg_plan_add_tiles(dg_plan* plan, const float* val, void* stream);
+int dg_plan_drop_tiles(dg_plan* plan, void* stream);
+int64_t dg_plan_tiled_entries(const dg_plan* plan);
 /* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device; this gives all of it on the current
  * device back (a failed allocation of the library does so by itself). */
 int dg_pool_trim(void);
@@ -84,8 +93,8 @@ int dg_plan_set_task_size(dg_plan* plan, int32_t task_nnz, void* stream);
  * (asynchronous copies through shared memory, entry-balanced tasks) wherever the operands allow it (rows of B and C
  * 16-byte aligned and at least 64 floats wide).  Process-wide; also settable with DG_SPMM_KERNEL=rows|stream. */
 int dg_select_kernel(int family);
-/* Reads the plan's device status word (synchronises `stream`).  Reserved for kernels with bounded device-side waits;
- * no current kernel waits on anything, so it reads 0. */
+/* Reads the plan's device status word (synchronises `stream`).  Non-zero if the tensor-core part of a product
+ * (dg_plan_add_tiles) gave up on one of its bounded waits; its result is then invalid. */
 int dg_plan_device_status(const dg_plan* plan, int* host_status, void* stream);
 /* copies the m+1 row offsets to host memory (synchronises `stream`); used to check CSR indexing bit for bit */
 int dg_plan_copy_rowptr(const dg_plan* plan, int64_t* host_rowptr, void* stream);

@@ -380,3 +380,53 @@ def test_plan_from_int64_ids_equals_the_int32_plan(m, k, nnz):
     out, narrowed = ctypes.c_void_p(), torch.empty(1, dtype=torch.int32, device='cuda')
     assert spmm_cpp.lib().dg_plan_create_i64(row.data_ptr(), col.data_ptr(), 1, m, k, 0, 0, narrowed.data_ptr(), None, ctypes.byref(out)) == -3
     spmm_cpp.empty_cache()
+
+
+@pytest.mark.parametrize('F', [32, 41, 64, 100, 256, 260, 604])
+def test_tensor_core_tiles_against_float64(F):
+    """A block with a dense corner (rows of 40 to 3,000 entries, columns as skewed) whose tiles run on the tensor cores: all
+    widths' panels, odd rows through the padded copy, accumulation into C, the epilogue, and the same bits every time.  The
+    values span six orders of magnitude; the error is held to a tenth of the parity tolerance."""
+    import spmm_cpp
+    rng = np.random.Generator(np.random.PCG64(4000 + F))
+    m, k = 3001, 2600
+    deg = np.minimum((40 * (m / (1 + np.arange(m))) ** 0.7).astype(np.int64) + 1, 2400)
+    p = 1.0 / (1 + np.arange(k)) ** 0.8
+    p /= p.sum()
+    row = np.repeat(rng.permutation(m), deg)
+    col = np.concatenate([rng.choice(k, d, replace=False, p=p) for d in deg])
+    col = rng.permutation(k)[col]
+    val = (rng.standard_normal(row.size) * 10.0 ** rng.uniform(-3, 3, row.size)).astype(np.float32)
+    A = ref_graph.fast_coalesce_sorted(row.astype(np.int64), col.astype(np.int64), val, (m, k))
+    plan = make_plan(A)
+    keep = spmm_cpp.TILE_NNZ
+    try:
+        spmm_cpp.TILE_NNZ = 0
+        plan.tile()
+    finally:
+        spmm_cpp.TILE_NNZ = keep
+    assert plan.tiled_entries() > A.nnz // 8
+    B = torch.randn(k, F, device='cuda', generator=torch.Generator(device='cuda').manual_seed(F))
+    C0 = torch.randn(m, F, device='cuda', generator=torch.Generator(device='cuda').manual_seed(F + 1))
+    dense = torch.zeros(m, k, dtype=torch.float64, device='cuda')
+    dense[torch.from_numpy(A.row).cuda(), torch.from_numpy(A.col).cuda()] = dev(A.val).double()
+    want = (dense @ B.double()).cpu().numpy()
+    C = plan.spmm(B, torch.full((m, F), float('nan'), device='cuda'), 1.0, 0.0)
+    assert plan.device_status() == 0
+    assert_close(C.cpu().numpy(), want, TOL / 10, 'tiles, beta = 0')
+    plain = make_plan(A).spmm(B, torch.empty_like(C), 1.0, 0.0)
+    err = lambda t: np.linalg.norm(t.cpu().numpy() - want) / np.linalg.norm(want)
+    assert err(C) <= 4 * err(plain) + 1e-7                         # no worse than gathering beyond rounding
+    assert torch.equal(C, plan.spmm(B, torch.empty_like(C), 1.0, 0.0))
+    scale = torch.rand(m, device='cuda')
+    got = plan.spmm(B, C0.clone(), 0.5, -2.0, row_scale=scale, relu=True)
+    full = ((0.5 * dense @ B.double() - 2.0 * C0.double()) * scale.double()[:, None]).clamp(min=0)
+    assert_close(got.cpu().numpy(), full.cpu().numpy(), TOL, 'tiles with the epilogue')
+    acc = plan.spmm(B, C0.clone(), 1.0, 1.0)
+    assert_close(acc.cpu().numpy(), (dense @ B.double() + C0.double()).cpu().numpy(), TOL / 10, 'tiles, beta = 1')
+    # other values, or the same changed in place, are gathered
+    other = plan.values * 2
+    assert_close(plan.spmm(B, torch.empty_like(C), 1.0, 0.0, values=other).cpu().numpy(), 2 * want, TOL / 10, 'other values')
+    plan.values.mul_(3.0)
+    assert_close(plan.spmm(B, torch.empty_like(C), 1.0, 0.0).cpu().numpy(), 3 * want, TOL / 10, 'values changed in place')
+    assert plan.tiled_entries() == 0

@@ -361,7 +361,7 @@ def measure(args, rank, world, keep_process_group=False):
                                      + 'traffic_est: captured bytes per (stored entry x float) of '
                                      + ('the whole-graph products' if world == 1 else 'the 8-rank stage-block products at F = 256') + ' x this run\'s nnz x F',
                      'peak_source': peaks['source'],
-                     'kernel': 'k_spmm_v4 (+ generic row kernels for narrow widths on long rows) + k_spmm_heavy_finish, all local products of the slowest rank',
+                     'kernel': 'k_spmm (gather) + k_tile_columns, k_tile_mma (dense tiles on the tensor cores), all local products of the slowest rank',
                      'products_per_step': slow['products'] // args.steps, 'spmm_ms_per_step': round(slow['spmm_ms'] / args.steps, 4),
                      'alg_bytes_per_step': slow['alg_bytes'] / args.steps,
                      'gather_gbs': round(slow['gather_bytes'] / (slow['spmm_ms'] * 1e-3) / 1e9, 2) if slow['spmm_ms'] > 0 else 0.0,

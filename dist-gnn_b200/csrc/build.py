@@ -1,4 +1,4 @@
-"""Builds libdist_gnn_b200.so (sm_100a only) in place with nvcc.  Usage: python dist-gnn_b200/csrc/build.py [-v]
+"""Builds libdist_gnn_b200.so (sm_100a only) with nvcc and the PyTorch binding beside it with g++, in place.  Usage: python dist-gnn_b200/csrc/build.py [-v]
 
 The library links the NCCL that PyTorch bundles (headers and libnccl.so.2 from the `nvidia.nccl` wheel) so the
 stage loop and torch.distributed share one NCCL in the process.
@@ -41,15 +41,41 @@ def up_to_date(srcs):
     return all(os.path.getmtime(d) <= os.path.getmtime(OUTPUT) for d in deps)
 
 
+BINDING_SOURCE, BINDING = os.path.join(HERE, 'torch_binding.cpp'), os.path.join(HERE, '_dist_gnn_torch.so')
+
+
+def build_binding(force=False):
+    """The C++ autograd side (host code only): g++ against the installed PyTorch, linked to the library beside it."""
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    deps = [BINDING_SOURCE, os.path.join(ROOT, 'include', 'dist_gnn_b200.h'), __file__]
+    if not force and os.path.exists(BINDING) and all(os.path.getmtime(d) <= os.path.getmtime(BINDING) for d in deps):
+        return BINDING
+    cmd = ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', '-DTORCH_EXTENSION_NAME=_dist_gnn_torch', '-DTORCH_API_INCLUDE_EXTENSION_H',
+           f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', '-I', os.path.join(ROOT, 'include'),
+           '-isystem', os.path.join(base, 'include'), '-isystem', os.path.join(base, 'include', 'torch', 'csrc', 'api', 'include'),
+           '-isystem', sysconfig.get_paths()['include'], '-isystem', '/usr/local/cuda/include', BINDING_SOURCE, '-o', BINDING,
+           '-L', HERE, '-l:libdist_gnn_b200.so', '-L', os.path.join(base, 'lib'), '-lc10', '-lc10_cuda', '-ltorch_cpu', '-ltorch_cuda', '-ltorch', '-ltorch_python',
+           '-Wl,-rpath,$ORIGIN', f"-Wl,-rpath,{os.path.join(base, 'lib')}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError('g++ failed: ' + ' '.join(cmd))
+    return BINDING
+
+
 def build(verbose=False, force=False):
     cmd, srcs = command(verbose)
     if not force and not verbose and up_to_date(srcs):
+        build_binding()
         return OUTPUT
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode:
         sys.stderr.write(res.stdout + res.stderr)
     if res.returncode:
         raise RuntimeError('nvcc failed: ' + ' '.join(cmd))
+    build_binding(force)
     return OUTPUT
 
 

@@ -23,7 +23,7 @@ def f1(y_true, y_pred, multilabel=True):
 def local_loss(g, outputs, loss_func):
     """Mean loss over this rank's LOCAL train rows (dist_train.py:39-43); a rank without train rows still
     back-propagates a zero so that it takes part in every collective.  The plain cross-entropy of class labels runs as
-    one pass over the logits (spmm_cpp.RowCrossEntropy); any other loss function gets the gathered train rows."""
+    one pass over the logits (spmm_cpp.row_cross_entropy); any other loss function gets the gathered train rows."""
     cached = getattr(g, '_train_rows', None)
     if cached is None:      # the mask never changes: find the rows once instead of a host sync per epoch
         rows = g.local_train_mask.nonzero().squeeze(1)
@@ -32,7 +32,7 @@ def local_loss(g, outputs, loss_func):
     if rows.numel() > 0:
         targets = _class_targets(g, outputs, loss_func, rows, labels)
         if targets is not None:
-            return spmm_cpp.RowCrossEntropy.apply(outputs, *targets)
+            return spmm_cpp.row_cross_entropy(outputs, *targets)
         return loss_func(outputs.index_select(0, rows), labels)
     DistEnv.env.logger.log('Warning: no training nodes in this partition! Backward fake loss.')
     return (outputs * 0).sum()

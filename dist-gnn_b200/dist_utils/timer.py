@@ -5,7 +5,9 @@ region the way the reference does (timer.py:16-24; four host syncs per stage the
 events (pooled in the library) on the current stream and adds their elapsed time when a summary is asked for, so timing a region leaves
 the broadcast/SpMM overlap intact.  On a CPU-only process it degrades to wall clock.
 """
+import itertools
 import statistics
+import sys
 import time
 from collections import defaultdict
 
@@ -47,6 +49,8 @@ class CudaTimerCtx:
 
 class DistTimer:
     MAX_PENDING = 4096
+    NATIVE_KEYS = ('broadcast+spmm', 'mm', 'all_reduce')     # what the library's own regions are called
+    _idents = itertools.count()
 
     def __init__(self, env):
         self.env = env
@@ -55,17 +59,34 @@ class DistTimer:
         self.count_dict = defaultdict(int)
         self.pending = []
         self._mark = None
+        self.ident = next(self._idents)
 
     def resolve(self, synchronize=True):
-        """Adds the elapsed time of the recorded mark pairs to their keys.  The training loop calls it with
-        synchronize=False right after it has read the loss (the device is idle then), so the list never grows."""
+        """Adds the elapsed time of the recorded mark pairs to their keys, those of regions inside the library's calls
+        included.  The training loop calls it with synchronize=False right after it has read the loss (the device is idle
+        then), so the list never grows."""
+        spmm_cpp = sys.modules.get('spmm_cpp')
+        if spmm_cpp is None:                                # nothing was ever timed on a device
+            return
+        if spmm_cpp._binding is not None:
+            for key, begin, end in spmm_cpp._binding.take_regions(self.ident):
+                key = self.NATIVE_KEYS[key]
+                self.count_dict[key] += 1
+                if begin >= 0 and end >= 0:
+                    self.pending.append((key, begin, end))
+                else:
+                    self.duration_dict[key] += 0.0
         if self.pending:
-            import spmm_cpp
             if synchronize:
                 torch.cuda.synchronize(self.env.device if self.env.device.type == 'cuda' else None)
             pending, self.pending = self.pending, []
             for key, begin, end in pending:
                 self.duration_dict[key] += spmm_cpp.mark_elapsed(begin, end) / 1000.0
+
+    def bound_regions(self):
+        """Called after a library call that times regions by itself: never more than MAX_PENDING of them are kept."""
+        if sys.modules['spmm_cpp']._binding.pending_regions(self.ident) >= self.MAX_PENDING:
+            self.resolve()
 
     _resolve = resolve
 
@@ -79,15 +100,6 @@ class DistTimer:
             import spmm_cpp
             self._mark = spmm_cpp.mark
         return CudaTimerCtx(self, key, self._mark)
-
-    def add_regions(self, regions):
-        """Device regions whose marks were recorded elsewhere: (key, begin mark, end mark) each."""
-        for key, begin, end in regions:
-            if begin >= 0 and end >= 0:
-                self.pending.append((key, begin, end))
-            self.count_dict[key] += 1
-        if len(self.pending) >= self.MAX_PENDING:
-            self.resolve()
 
     def empty_region(self, key):
         """Counts a region in which this layout has nothing to do (a one-rank all-reduce)."""

@@ -9,7 +9,6 @@ the reuse of the un-transposed row block of A in backward, which is exact only f
 
 There is no CPU implementation: CPU tensors raise.
 """
-import ctypes
 import os
 import weakref
 
@@ -453,76 +452,6 @@ class DistGCNLayer(torch.autograd.Function):
         return (grad_features, grad_weight) + (None,) * 8
 
 
-class _OneRankGCN(torch.autograd.Function):
-    """All layers of a GCN on a rank without peers, forward and backward, from one library call each (dg_gcn_forward,
-    dg_gcn_backward): the products and transforms of the chained DistGCNLayers in the same order on the same operands, the
-    same bits, without the host's work between them."""
-
-    @staticmethod
-    def forward(ctx, env, plan, features, *weights):
-        n, L, device = features.size(0), len(weights), features.device
-        train = any(ctx.needs_input_grad)
-        dims = [features.size(1)] + [w.size(1) for w in weights]
-        pad = [d + (-d) % 4 for d in dims]
-        x = _product_operand(env, features, True)
-        splits = spmm_cpp.split_operands([(w, True, w) for w in weights] + ([(w, False, w) for w in weights[1:]] if train else []))
-        # hidden activations in one buffer: side by side while a backward pass will read them, else every layer over the last
-        starts = [n * sum(pad[1:l + 1]) if train else 0 for l in range(L - 1)]
-        hidden = torch.empty((n * sum(pad[1:L]) if train else n * max(pad[1:L])) if L > 1 else 0, dtype=torch.float32, device=device)
-        out = torch.empty((n, dims[L]), dtype=torch.float32, device=device)
-        base = hidden.data_ptr()
-        act = [base + 4 * s for s in starts] + [out.data_ptr()]
-        net, keep = _gcn_net(plan, x, dims, pad, act, pad[1:L] + [dims[L]])
-        z = torch.empty(n * max(pad[:L]), dtype=torch.float32, device=device)
-        heads = (ctypes.c_void_p * L)(*[s[1] for s in splits[:L]])
-        marks = (ctypes.c_int32 * (4 * L))(*[-1] * (4 * L))
-        net.z, net.fwd_split, net.marks = z.data_ptr(), ctypes.addressof(heads), ctypes.addressof(marks)
-        spmm_cpp.gcn_call('dg_gcn_forward', net, device.index)
-        spmm_cpp.dense_launches += sum((d + 255) // 256 for d in dims[1:])
-        env.timer.add_regions([r for l in range(L) for r in (('broadcast+spmm', marks[4 * l], marks[4 * l + 1]), ('mm', marks[4 * l + 2], marks[4 * l + 3]))])
-        if train:
-            ctx.save_for_backward(features, x, hidden, *weights)
-            ctx.env, ctx.plan, ctx.dims, ctx.pad, ctx.starts, ctx.splits = env, plan, dims, pad, starts, splits[L:]
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        features, x, hidden, *weights = ctx.saved_tensors
-        env, dims, pad, L, n, device = ctx.env, ctx.dims, ctx.pad, len(weights), x.size(0), x.device
-        g = _product_operand(env, grad_output, False)
-        base = hidden.data_ptr()
-        net, keep = _gcn_net(ctx.plan, x, dims, pad, [base + 4 * s for s in ctx.starts] + [base or x.data_ptr()], pad[1:L] + [dims[L]])
-        work = torch.empty(n * (max(pad[1:]) + max(pad[1:L], default=0)), dtype=torch.float32, device=device)
-        net.z = work.data_ptr()
-        if L > 1:
-            net.g = net.z + 4 * n * max(pad[1:])
-        grads = [torch.empty_like(w) if need else None for w, need in zip(weights, ctx.needs_input_grad[3:])]
-        dw = (ctypes.c_void_p * L)(*[None if t is None else t.data_ptr() for t in grads])
-        heads = (ctypes.c_void_p * L)(None, *[s[1] for s in ctx.splits])
-        scratch, ctas = spmm_cpp.tn_scratch(device.index)
-        marks = (ctypes.c_int32 * (4 * L))(*[-1] * (4 * L))
-        net.grad, net.ld_grad = g.data_ptr(), g.stride(0) if n > 1 else pad[L]
-        net.dw, net.bwd_split = ctypes.addressof(dw), ctypes.addressof(heads)
-        net.tn_scratch, net.tn_scratch_floats, net.max_ctas, net.marks = scratch.data_ptr(), scratch.numel(), ctas, ctypes.addressof(marks)
-        spmm_cpp.gcn_call('dg_gcn_backward', net, device.index)
-        panels = [(d + 255) // 256 for d in dims]
-        spmm_cpp.dense_launches += sum(panels[1:L]) + sum(2 * panels[l] * panels[l + 1] for l in range(L) if grads[l] is not None)
-        env.timer.add_regions([r for l in range(L) for r in (('broadcast+spmm', marks[4 * l], marks[4 * l + 1]), ('mm', marks[4 * l + 2], marks[4 * l + 3]))])
-        for _ in range(L):
-            env.timer.empty_region('all_reduce')
-        return (None, None, None, *grads)
-
-
-def _gcn_net(plan, x, dims, pad, act, ld_act):
-    """The dg_gcn_net of a call, and the arrays it points into."""
-    L = len(act)
-    arrays = (ctypes.c_int32 * (L + 1))(*dims), (ctypes.c_void_p * L)(*act), (ctypes.c_int64 * L)(*ld_act)
-    net = spmm_cpp.GcnNet(plan=plan.handle, val=plan.value_ptr(), x=x.data_ptr(), ldx=x.stride(0) if x.size(0) > 1 else pad[0],
-                          n=x.size(0), layers=L)
-    net.dims, net.act, net.ld_act = (ctypes.addressof(a) for a in arrays)
-    return net, arrays
-
-
 class GCN(nn.Module):
     """num_layers DistGCNLayers with ReLU between them, no bias (gcn.py:56-72).  Weights are drawn as the reference
     draws them - torch.rand on the host after manual_seed(0), layer by layer - unless `weights` injects them.
@@ -589,13 +518,25 @@ class GCN(nn.Module):
         plan = spmm_cpp.plan_for(parts[0])
         return plan if plan.m == plan.k == features.size(0) and plan.device == features.device else None
 
+    def _one_rank_forward(self, plan, features, weights):
+        """All layers on a rank without peers, forward and backward, from one library call each (dg_gcn_forward,
+        dg_gcn_backward behind the binding's autograd node): the products and transforms of the chained DistGCNLayers in the
+        same order on the same operands, the same bits, without the host's work between them."""
+        env = DistEnv.env
+        plan.value_ptr()                                    # values changed in place: their tiles go first
+        scratch, ctas = spmm_cpp.tn_scratch(features.device.index)
+        timer = env.timer
+        out = spmm_cpp.binding().gcn(plan.ref, features, _product_operand(env, features, True), weights, scratch, ctas, timer.ident)
+        timer.bound_regions()
+        return out
+
     def forward(self, features):
         h = features
         last = self.num_layers - 1
         weights = self.weights()
         plan = self._one_rank_plan(features, weights)
         if plan is not None:
-            return _OneRankGCN.apply(DistEnv.env, plan, features, *weights)
+            return self._one_rank_forward(plan, features, weights)
         for l, w in enumerate(weights):
             product = self.input_product(h) if l == 0 else None
             shortcut = self.input_gradient_shortcut and product is not None

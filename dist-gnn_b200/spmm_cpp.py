@@ -50,13 +50,6 @@ class SplitJob(ctypes.Structure):
                 ('ldb', ctypes.c_int64), ('N', ctypes.c_int32), ('K', ctypes.c_int32), ('transposed', ctypes.c_int32), ('pad', ctypes.c_int32)]
 
 
-class GcnNet(ctypes.Structure):
-    _fields_ = [(name, ctypes.c_void_p) for name in ('plan', 'val', 'dims', 'x')] + [('ldx', ctypes.c_int64)] + [
-        (name, ctypes.c_void_p) for name in ('act', 'ld_act', 'fwd_split', 'bwd_split', 'grad')] + [('ld_grad', ctypes.c_int64)] + [
-        (name, ctypes.c_void_p) for name in ('z', 'g', 'dw', 'tn_scratch')] + [('tn_scratch_floats', ctypes.c_int64), ('marks', ctypes.c_void_p)] + [
-        (name, ctypes.c_int32) for name in ('n', 'layers', 'max_ctas', 'pad')]
-
-
 def lib():
     """The loaded C library; raises if it has not been built (python dist-gnn_b200/csrc/build.py)."""
     global _lib
@@ -110,8 +103,6 @@ def lib():
             'dg_peer_spmm_gather': ([vp, vp, i32, vp, vp, vp, vp, i32, vp, vp, vp, vp, vp, i32, i32, vp, ctypes.c_int, vp], ctypes.c_int),
             'dg_dense_split': ([vp, vp, vp, i64, vp], ctypes.c_int),
             'dg_dense_split_operands': ([ctypes.POINTER(SplitJob), i32, vp], ctypes.c_int),
-            'dg_gcn_forward': ([ctypes.POINTER(GcnNet), vp], ctypes.c_int),
-            'dg_gcn_backward': ([ctypes.POINTER(GcnNet), vp], ctypes.c_int),
             'dg_dense_supported': ([i64, i32, i32, i64, i64, vp, vp, vp], ctypes.c_int),
             'dg_dense_nt': ([vp, i64, vp, vp, i64, vp, i64, i64, i32, i32, i32, vp], ctypes.c_int),
             'dg_dense_nt_masked': ([vp, i64, vp, vp, i64, vp, i64, i64, i32, i32, i32, vp, i64, vp], ctypes.c_int),
@@ -121,9 +112,6 @@ def lib():
             'dg_dense_status_reset': ([vp], ctypes.c_int),
             'dg_dense_wait_selftest': ([ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
             'dg_pad_rows': ([vp, i64, i64, i32, vp, i64, vp], ctypes.c_int),
-            'dg_rows_loss_scratch': ([], i32),
-            'dg_rows_cross_entropy': ([vp, i64, i64, i32, vp, i64, vp, vp, vp, vp], ctypes.c_int),
-            'dg_rows_cross_entropy_grad': ([vp, i64, i64, i32, vp, i64, vp, vp, vp, i64, vp], ctypes.c_int),
             'dg_mark_record': ([vp], ctypes.c_int),
             'dg_mark_elapsed': ([ctypes.c_int, ctypes.c_int, ctypes.POINTER(f32)], ctypes.c_int),
             'dg_mark_release': ([ctypes.c_int], ctypes.c_int),
@@ -135,6 +123,27 @@ def lib():
             fn.argtypes, fn.restype = argtypes, restype
         _lib = L
     return _lib
+
+
+_BINDING_PATH = os.path.join(_HERE, 'csrc', '_dist_gnn_torch.so')
+_binding = None
+
+
+def binding():
+    """The C++ autograd side of the library (csrc/torch_binding.cpp); raises if it has not been built."""
+    global _binding
+    if _binding is None:
+        lib()
+        if not os.path.exists(_BINDING_PATH):
+            raise RuntimeError(f'{_BINDING_PATH} is missing: build it with `python dist-gnn_b200/csrc/build.py`; '
+                               'there is no fallback implementation')
+        import importlib.machinery
+        import importlib.util
+        loader = importlib.machinery.ExtensionFileLoader('_dist_gnn_torch', _BINDING_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location('_dist_gnn_torch', _BINDING_PATH, loader=loader))
+        loader.exec_module(module)
+        _binding = module
+    return _binding
 
 
 def check(code):
@@ -190,17 +199,6 @@ def _row_major(t, what):
     raise RuntimeError(f'{what} must be a row-major fp32 matrix, got {t.dtype} {tuple(t.shape)} strides {t.stride()}')
 
 
-def _operand(t, rows, what):
-    """Row stride of a dense operand of a product, which has to have `rows` rows."""
-    if not (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.dim() == 2):
-        raise RuntimeError(f'{what} must be a 2-D fp32 CUDA tensor')
-    n, F = t.shape
-    ld, unit = t.stride()
-    if n != rows or (F > 1 and unit != 1):
-        raise RuntimeError(f'{what} has shape {tuple(t.shape)} / strides {t.stride()}, expected {rows} rows, unit column stride')
-    return ld if n > 1 else max(F, 1)
-
-
 class SpmmPlan:
     """Device CSR plan of one sparse block (dg_plan).  Keeps the int32 column ids and fp32 values alive."""
 
@@ -214,8 +212,7 @@ class SpmmPlan:
         with _on(self.device.index):
             check(lib().dg_plan_create_ex(row_i32.data_ptr(), col_i32.data_ptr(), values.numel(), self.m, self.k,
                                           heavy_threshold, chunk, _stream(), ctypes.byref(handle)))
-        self.handle = handle
-        self._tiled = None
+        self._own(handle)
 
     @classmethod
     def from_coo(cls, A, heavy_threshold=0, chunk=0):
@@ -236,9 +233,13 @@ class SpmmPlan:
         with _on(index):
             check(lib().dg_plan_create_i64(base, base + 8 * idx.stride(0), nnz, self.m, self.k, heavy_threshold, chunk, self.col.data_ptr(),
                                            _raw_stream(index), ctypes.byref(handle)))
-        self.handle = handle
-        self._tiled = None
+        self._own(handle)
         return self.tile() if nnz >= TILE_ALWAYS else self
+
+    def _own(self, handle):
+        # the binding's reference destroys the plan when this object and every autograd graph that uses it are gone
+        self.handle, self._tiled = handle, None
+        self.ref = binding().PlanRef(handle.value, self.col, self.values)
 
     def tile(self):
         """Moves the densest part of the block to the tensor cores for the products to come (dg_plan_add_tiles): worth its few
@@ -291,25 +292,12 @@ class SpmmPlan:
 
     def spmm(self, B, C, alpha=1.0, beta=1.0, row_scale=None, bias=None, relu=False, values=None):
         """C <- epilogue(alpha * A @ B + beta * C) in place; B [k, F] and C [m, F] may be row-strided views."""
-        if values is not None and values is not self.values:
+        if values is None or values is self.values:
+            val = self.value_ptr()
+        else:
             _dev_tensor(values, torch.float32, 'values')
-        val = self.value_ptr() if values is None or values.data_ptr() == self.values.data_ptr() else values.data_ptr()
-        ldb, ldc = _operand(B, self.k, 'B'), _operand(C, self.m, 'C')
-        F = B.size(1)
-        if F != C.size(1):
-            raise RuntimeError('B and C differ in width')
-        flags = EPI_RELU if relu else 0
-        scale_ptr = bias_ptr = None
-        if row_scale is not None:
-            flags |= EPI_ROW_SCALE
-            scale_ptr = _dev_tensor(row_scale, torch.float32, 'row_scale').data_ptr()
-        if bias is not None:
-            flags |= EPI_BIAS
-            bias_ptr = _dev_tensor(bias, torch.float32, 'bias').data_ptr()
-        index = self.device.index
-        with _on(index):
-            check(_lib.dg_spmm_csr(self.handle, val, B.data_ptr(), ldb, C.data_ptr(), ldc, F, alpha, beta, flags,
-                                   scale_ptr, bias_ptr, _raw_stream(index)))
+            val = values.data_ptr() if values.data_ptr() != self.values.data_ptr() else self.value_ptr()
+        _binding.spmm(self.ref, self.m, self.k, val, B, C, alpha, beta, row_scale, bias, relu)
         return C
 
     def algorithmic_bytes(self, F, beta_nonzero):
@@ -319,10 +307,6 @@ class SpmmPlan:
         s = self.stats()
         return 8 * s['nnz'] + 4 * (s['m'] + 1) + 4 * F * s['touched_columns'] + 4 * F * s['m'] * (2 if beta_nonzero else 1)
 
-    def __del__(self):
-        h, self.handle = getattr(self, 'handle', None), None
-        if h and _lib is not None:
-            _lib.dg_plan_destroy(h)
 
 
 def empty_cache():
@@ -359,6 +343,8 @@ def profile_begin():
     """Start bracketing every local product with CUDA events (dg_profile_begin)."""
     global dense_launches
     dense_launches = 0
+    if _binding is not None:
+        _binding.take_launches()
     check(lib().dg_profile_begin())
 
 
@@ -367,7 +353,7 @@ def profile_end():
     p = Profile()
     check(lib().dg_profile_end(ctypes.byref(p)))
     out = {name: getattr(p, name) for name, _ in Profile._fields_}
-    out['dense_launches'] = dense_launches
+    out['dense_launches'] = dense_launches + (_binding.take_launches() if _binding is not None else 0)
     return out
 
 
@@ -674,39 +660,11 @@ def pad_rows(src, dst):
     return dst
 
 
-class RowCrossEntropy(torch.autograd.Function):
-    """apply(x, targets, count): mean cross-entropy of x [n x C] over the rows with targets[i] >= 0 (int32, all below C), of
-    which there are `count` (dg_rows_cross_entropy).  The gradient's rows are padded to whole 16-byte pieces, which is
-    what the products behind it read."""
-
-    @staticmethod
-    def forward(ctx, x, targets, count):
-        ld = _row_major(x, 'logits')
-        n, C = x.shape
-        _dev_tensor(targets, torch.int32, 'targets')
-        index, parts = x.device.index, lib().dg_rows_loss_scratch()
-        work = torch.empty(2 * parts + n + 1, dtype=torch.float32, device=x.device)       # partial sums, logsumexp per row, loss
-        base = work.data_ptr()
-        loss = work[2 * parts + n]
-        with _on(index):
-            check(_lib.dg_rows_cross_entropy(x.data_ptr(), ld, n, C, targets.data_ptr(), count, base + 8 * parts, base, loss.data_ptr(),
-                                             _raw_stream(index)))
-        ctx.save_for_backward(x, targets, work)
-        ctx.count, ctx.parts = count, parts
-        return loss.clone()
-
-    @staticmethod
-    def backward(ctx, upstream):
-        x, targets, work = ctx.saved_tensors
-        n, C = x.shape
-        width = C + (-C) % 4
-        grad = torch.empty((n, width), dtype=torch.float32, device=x.device)
-        index = x.device.index
-        with _on(index):
-            check(_lib.dg_rows_cross_entropy_grad(x.data_ptr(), _row_major(x, 'logits'), n, C, targets.data_ptr(), ctx.count,
-                                                  work.data_ptr() + 8 * ctx.parts, upstream.contiguous().data_ptr(), grad.data_ptr(), width,
-                                                  _raw_stream(index)))
-        return grad if width == C else grad[:, :C], None, None
+def row_cross_entropy(x, targets, count):
+    """Mean cross-entropy of x [n x C] over the rows with targets[i] >= 0 (int32, all below C), of which there are `count`
+    (dg_rows_cross_entropy), differentiable in x.  The gradient's rows are padded to whole 16-byte pieces, which is what
+    the products behind it read."""
+    return binding().row_cross_entropy(x, targets, count)
 
 
 def dense_split(w):
@@ -837,12 +795,6 @@ def dense_tn(x, g):
         check(_lib.dg_dense_tn(x.data_ptr(), ldx, g.data_ptr(), ldg, d.data_ptr(), Nn, n, Km, Nn, scratch.data_ptr(), scratch.numel(),
                                ctas, _raw_stream(index)))
     return d
-
-
-def gcn_call(name, net, index):
-    """dg_gcn_forward / dg_gcn_backward on the current stream of CUDA device `index`."""
-    with _on(index):
-        check(getattr(lib(), name)(ctypes.byref(net), _raw_stream(index)))
 
 
 def dense_status(reset=False):

@@ -43,8 +43,6 @@ struct DenseArgs {
     uint32_t relu;
     const float* mask;              // optional [M x N]: the result is zeroed where mask <= 0 (ReLU backward), else nullptr
     int64_t ldm;
-    int32_t raw_head;               // persistent kernel: 0 = masked head copy; 1 = the fp32 tile itself serves as head;
-                                    // 2 = as 1, and the two head passes of a slab are issued before its tail is ready
     int* status;
 };
 
@@ -64,6 +62,11 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr)
     d |= (uint64_t)1 << 46;                                   // descriptor version for sm_100
     d |= (uint64_t)2 << 61;                                   // layout type: SWIZZLE_128B
     return d;
+}
+// The same for rows of 64 bytes with the 64B swizzle: 8-row groups are 512 bytes apart.
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t smem_addr)
+{
+    return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
 }
 // Instruction descriptor for kind::tf32: fp32 accumulator, TF32 A and B, both K-major, shape 128 x n_pad.
 __device__ __forceinline__ uint32_t umma_idesc_tf32(int n_pad)
@@ -87,6 +90,71 @@ __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t a_desc, uint
 }  // namespace
 
 namespace {
+
+// Epilogue of one warp: 32 rows of the accumulator (tensor-memory address `acc`, this warp's lane quarter included) to
+// rows row0.. of C, with the optional ReLU and ReLU-backward mask.  A lane holds one row, so stores straight from the
+// registers touch 32 cache lines an instruction (and so do the mask's loads); the piece goes through `stage` in shared memory
+// (32 rows of 36 floats, conflict-free both ways) and leaves as whole 128-byte row pieces, four rows an instruction.
+constexpr int kStagePitch = 36, kStageBytes = 32 * kStagePitch * 4;
+__device__ __forceinline__ void store_rows(const DenseArgs& a, uint32_t acc, float* stage, int64_t row0, int lane)
+{
+    const bool vec = a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0 &&
+                     (!a.mask || (a.ldm % 4 == 0 && (reinterpret_cast<uintptr_t>(a.mask) & 15) == 0));
+    const int rows = (int)min((int64_t)32, a.M - row0);
+    for (int c0 = 0; c0 < a.n_pad; c0 += 32) {
+        const bool pieces = vec && c0 + 32 <= a.N;                // whole 128-byte pieces of every row
+        const int r4 = lane >> 3, col4 = c0 + (lane & 7) * 4;
+        float4 mk[8];
+        if (pieces && a.mask) {                                   // requested before the accumulator read so that both are in flight
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i * 4 + r4 < rows) mk[i] = __ldg(reinterpret_cast<const float4*>(a.mask + (row0 + i * 4 + r4) * a.ldm + col4));
+        }
+        uint32_t r[32];
+        tmem_ld16(acc + (uint32_t)c0, r);
+        if (c0 + 16 < a.n_pad) tmem_ld16(acc + (uint32_t)c0 + 16, r + 16);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float4* mine = reinterpret_cast<float4*>(stage + lane * kStagePitch);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            mine[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+        __syncwarp();
+        if (pieces) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (i * 4 + r4 >= rows) continue;
+                float4 v = *reinterpret_cast<const float4*>(stage + (i * 4 + r4) * kStagePitch + (lane & 7) * 4);
+                if (a.relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+                if (a.mask) {
+                    if (!(mk[i].x > 0.f)) v.x = 0.f;
+                    if (!(mk[i].y > 0.f)) v.y = 0.f;
+                    if (!(mk[i].z > 0.f)) v.z = 0.f;
+                    if (!(mk[i].w > 0.f)) v.w = 0.f;
+                }
+                __stcs(reinterpret_cast<float4*>(a.C + (row0 + i * 4 + r4) * a.ldc + col4), v);
+            }
+        } else if (c0 + lane < a.N) {                             // odd strides and the last columns: a row's floats side by side
+            const int c = c0 + lane;
+            for (int i0 = 0; i0 < rows; i0 += 8) {                // eight rows' mask values in flight
+                float mrow[8];
+                if (a.mask) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i0 + i < rows) mrow[i] = __ldg(a.mask + (row0 + i0 + i) * a.ldm + c);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (i0 + i >= rows) break;
+                    float v = stage[(i0 + i) * kStagePitch + lane];
+                    if (a.relu) v = fmaxf(v, 0.f);
+                    if (a.mask && !(mrow[i] > 0.f)) v = 0.f;
+                    __stcs(a.C + (row0 + i0 + i) * a.ldc + c, v);
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
 
 __global__ void __launch_bounds__(kThreads, 1)
 k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
@@ -185,50 +253,9 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int q = warp & 3;                               // a warp may only read its own quarter of the TMEM lanes
-            const int64_t row = m0 + q * 32 + lane;
-            float* crow = a.C + row * a.ldc;
-            const bool vec_ok = (a.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0);
-            const bool mvec_ok = a.mask && (a.ldm % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.mask) & 15) == 0);
-            const float* mrow = a.mask ? a.mask + row * a.ldm : nullptr;
-            for (int c0 = 0; c0 < a.n_pad; c0 += 16) {
-                float mk[16];
-                if (mrow && row < a.M) {                          // issued before the accumulator read so that both are in flight
-                    if (mvec_ok && c0 + 16 <= a.N) {
-#pragma unroll
-                        for (int j = 0; j < 16; j += 4) {
-                            const float4 m4 = __ldg(reinterpret_cast<const float4*>(mrow + c0 + j));
-                            mk[j] = m4.x; mk[j + 1] = m4.y; mk[j + 2] = m4.z; mk[j + 3] = m4.w;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) mk[j] = c0 + j < a.N ? __ldg(mrow + c0 + j) : 0.f;
-                    }
-                }
-                uint32_t r[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                    : "r"(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row < a.M) {
-                    float v[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        v[j] = __uint_as_float(r[j]);
-                        if (a.relu) v[j] = fmaxf(v[j], 0.f);
-                        if (mrow && !(mk[j] > 0.f)) v[j] = 0.f;
-                    }
-                    if (vec_ok && c0 + 16 <= a.N) {
-#pragma unroll
-                        for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(crow + c0 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < a.N) crow[c0 + j] = v[j];
-                    }
-                }
-            }
+            // every load has landed and every MMA has read its operands: the stages are free for the staging of the rows
+            if (m0 + q * 32 < a.M)
+                store_rows(a, tmem + ((uint32_t)(q * 32) << 16), reinterpret_cast<float*>(gbase + q * kStageBytes), m0 + q * 32, lane);
         }
     }
     if (!ok) atomicExch(a.status, 1);
@@ -242,7 +269,12 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 // memory (columns 0 and 256) and separate warps for the operand split and for the epilogue, so that tile t is read out
 // of tensor memory and stored while tile t+1 is already being loaded, split and multiplied.
 // Warps: 0 TMA, 1 MMA issue + tensor-memory allocation, 2-5 split A, 6-9 epilogue (warp w reads lane quarter w % 4).
+// The ring holds four half slabs of 16 columns (64-byte rows, 64B swizzle) instead of two slabs of 32: a stage is refilled
+// from the L2 (Bt's 512 KB come back for every tile), split and multiplied one after the other, and with two stages in that
+// circle the tensor cores waited for it more than half of the time.  A slab's MMAs keep their order - both head passes of its
+// four k-steps, then the tail passes - so the sums are the same bits.
 constexpr int kThreadsPersistent = 320;
+constexpr int PK = 16, PSTAGES = 4;
 
 __global__ void __launch_bounds__(kThreadsPersistent, 1)
 k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
@@ -252,18 +284,20 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* gbase = smem_raw + (base - raw);
-    const int b_bytes = a.n_pad * 128;
-    const int stage_bytes = 2 * BM * 128 + 2 * b_bytes;
-    const uint32_t bars = base + STAGES * stage_bytes;
-    const uint32_t full0 = bars, ready0 = bars + 8 * STAGES, empty0 = bars + 16 * STAGES;
-    const uint32_t acc_full0 = bars + 24 * STAGES, acc_empty0 = acc_full0 + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + STAGES * stage_bytes + 24 * STAGES + 32);
+    constexpr int a_bytes = BM * PK * 4;
+    const int b_bytes = a.n_pad * PK * 4;
+    const int stage_bytes = 2 * a_bytes + 2 * b_bytes;            // A head, A tail, Bt head, Bt tail
+    const int staging = PSTAGES * stage_bytes;                    // the epilogue warps' row pieces
+    const uint32_t bars = base + staging + 4 * kStageBytes;
+    const uint32_t full0 = bars, ready0 = bars + 8 * PSTAGES, empty0 = bars + 16 * PSTAGES;
+    const uint32_t acc_full0 = bars + 24 * PSTAGES, acc_empty0 = acc_full0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + staging + 4 * kStageBytes + 24 * PSTAGES + 32);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nslabs = (a.K + BK - 1) / BK;
+    const int nhalves = (a.K + PK - 1) / PK;
     constexpr int kTmemCols = 512;                                // two accumulators of up to 256 columns
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < PSTAGES; ++s) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(ready0 + 8 * s, 128);
             mbar_init(empty0 + 8 * s, 1);
@@ -288,15 +322,15 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (lane == 0) {                                          // TMA producer: one ring of stages across all tiles
             int it = 0;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                for (int i = 0; i < nslabs; ++i, ++it) {
-                    const int s = it % STAGES, u = it / STAGES;
+                for (int i = 0; i < nhalves; ++i, ++it) {
+                    const int s = it % PSTAGES, u = it / PSTAGES;
                     if (u > 0) ok = mbar_wait(empty0 + 8 * s, (u - 1) & 1);
                     if (!ok) break;
                     const uint32_t st = base + s * stage_bytes;
-                    mbar_expect_tx(full0 + 8 * s, BM * 128 + 2 * b_bytes);
-                    tma_load_2d(st, &tmA, i * BK, tile * BM, full0 + 8 * s);
-                    tma_load_2d(st + 2 * BM * 128, &tmBh, i * BK, 0, full0 + 8 * s);
-                    tma_load_2d(st + 2 * BM * 128 + b_bytes, &tmBt, i * BK, 0, full0 + 8 * s);
+                    mbar_expect_tx(full0 + 8 * s, a_bytes + 2 * b_bytes);
+                    tma_load_2d(st, &tmA, i * PK, tile * BM, full0 + 8 * s);
+                    tma_load_2d(st + 2 * a_bytes, &tmBh, i * PK, 0, full0 + 8 * s);
+                    tma_load_2d(st + 2 * a_bytes + b_bytes, &tmBt, i * PK, 0, full0 + 8 * s);
                 }
             }
         }
@@ -310,62 +344,56 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + (uint32_t)(b * 256);
-                for (int i = 0; i < nslabs; ++i, ++it) {
-                    const int s = it % STAGES, u = it / STAGES;
-                    const uint32_t st = base + s * stage_bytes;
-                    const uint64_t a_head = umma_desc_sw128(st), a_tail = umma_desc_sw128(st + BM * 128);
-                    const uint64_t b_head = umma_desc_sw128(st + 2 * BM * 128), b_tail = umma_desc_sw128(st + 2 * BM * 128 + b_bytes);
-                    if (a.raw_head == 2) {
-                        // The tensor cores read a TF32 operand from a 32-bit container and ignore its low 13 bits, so the
-                        // tile as TMA delivered it IS the head: both head passes go out as soon as the data has landed,
-                        // and only the tail pass waits for the split warps.
+                for (int i = 0; i < nhalves && ok; i += 2, it += 2) {
+                    const int halves = min(2, nhalves - i);
+                    // The tensor cores read a TF32 operand from a 32-bit container and ignore its low 13 bits (verified: identical
+                    // bits with a masked copy), so the tile as TMA delivered it IS the head: both head passes go out as soon as
+                    // the data has landed, and only the tail pass waits for the split warps.
+                    for (int h = 0; h < halves && ok; ++h) {
+                        const int s = (it + h) % PSTAGES, u = (it + h) / PSTAGES;
                         ok = mbar_wait(full0 + 8 * s, u & 1);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t st = base + s * stage_bytes;
+                        const uint64_t a_head = umma_desc_sw64(st), b_head = umma_desc_sw64(st + 2 * a_bytes), b_tail = umma_desc_sw64(st + 2 * a_bytes + b_bytes);
 #pragma unroll
-                        for (int k = 0; k < BK / 8; ++k) {
-                            umma_tf32(acc, a_head + 2 * k, b_tail + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < PK / 8; ++k) {        // 8 TF32 columns = 32 bytes per MMA: +2 in 16-byte units
+                            umma_tf32(acc, a_head + 2 * k, b_tail + 2 * k, idesc, (i + h > 0 || k > 0) ? 1u : 0u);
                             umma_tf32(acc, a_head + 2 * k, b_head + 2 * k, idesc, 1u);
                         }
+                    }
+                    for (int h = 0; h < halves && ok; ++h) {
+                        const int s = (it + h) % PSTAGES, u = (it + h) / PSTAGES;
                         ok = mbar_wait(ready0 + 8 * s, u & 1);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t st = base + s * stage_bytes;
+                        const uint64_t a_tail = umma_desc_sw64(st + a_bytes), b_head = umma_desc_sw64(st + 2 * a_bytes);
 #pragma unroll
-                        for (int k = 0; k < BK / 8; ++k) umma_tf32(acc, a_tail + 2 * k, b_head + 2 * k, idesc, 1u);
+                        for (int k = 0; k < PK / 8; ++k) umma_tf32(acc, a_tail + 2 * k, b_head + 2 * k, idesc, 1u);
                         umma_commit(empty0 + 8 * s);
-                        continue;
                     }
-                    ok = mbar_wait(ready0 + 8 * s, u & 1);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-                    for (int k = 0; k < BK / 8; ++k) {
-                        umma_tf32(acc, a_tail + 2 * k, b_head + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                        umma_tf32(acc, a_head + 2 * k, b_tail + 2 * k, idesc, 1u);
-                        umma_tf32(acc, a_head + 2 * k, b_head + 2 * k, idesc, 1u);
-                    }
-                    umma_commit(empty0 + 8 * s);
+                    if (halves == 1) --it;                        // the last slab of an odd count takes one stage
                 }
                 if (ok) umma_commit(acc_full0 + 8 * b);
             }
         }
     } else if (warp < 6) {
-        const int t = threadIdx.x - 64;                           // 0..127: split the A slab of every stage
+        const int t = threadIdx.x - 64;                           // 0..127: split the A half slab of every stage
         int it = 0;
         for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            for (int i = 0; i < nslabs; ++i, ++it) {
-                const int s = it % STAGES, u = it / STAGES;
+            for (int i = 0; i < nhalves; ++i, ++it) {
+                const int s = it % PSTAGES, u = it / PSTAGES;
                 ok = mbar_wait(full0 + 8 * s, u & 1);
                 if (!ok) break;
-                float4* head = reinterpret_cast<float4*>(gbase + (size_t)s * stage_bytes);
-                float4* tail = head + BM * 128 / 16;
-#pragma unroll 4
-                for (int j = t; j < BM * 128 / 16; j += 128) {
+                const float4* head = reinterpret_cast<const float4*>(gbase + (size_t)s * stage_bytes);
+                float4* tail = reinterpret_cast<float4*>(gbase + (size_t)s * stage_bytes + a_bytes);
+#pragma unroll
+                for (int j = t; j < a_bytes / 16; j += 128) {
                     const float4 x = head[j];
                     float4 h;
                     h.x = __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u); h.y = __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
                     h.z = __uint_as_float(__float_as_uint(x.z) & 0xFFFFE000u); h.w = __uint_as_float(__float_as_uint(x.w) & 0xFFFFE000u);
-                    if (!a.raw_head) head[j] = h;
                     tail[j] = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -374,53 +402,15 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
     } else {
         const int q = warp & 3;                                   // a warp may only read its own quarter of the TMEM lanes
-        const bool vec_ok = (a.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0);
-        const bool mvec_ok = a.mask && (a.ldm % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.mask) & 15) == 0);
         int lt = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++lt) {
             const int b = lt & 1, v = lt >> 1;
             ok = __all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * b, v & 1));     // tcgen05.ld is warp-collective
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int64_t row = (int64_t)tile * BM + q * 32 + lane;
-            float* crow = a.C + row * a.ldc;
-            const float* mrow = a.mask ? a.mask + row * a.ldm : nullptr;
-            for (int c0 = 0; c0 < a.n_pad; c0 += 16) {
-                float mk[16];
-                if (mrow && row < a.M) {
-                    if (mvec_ok && c0 + 16 <= a.N) {
-#pragma unroll
-                        for (int j = 0; j < 16; j += 4) {
-                            const float4 m4 = __ldg(reinterpret_cast<const float4*>(mrow + c0 + j));
-                            mk[j] = m4.x; mk[j + 1] = m4.y; mk[j + 2] = m4.z; mk[j + 3] = m4.w;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) mk[j] = c0 + j < a.N ? __ldg(mrow + c0 + j) : 0.f;
-                    }
-                }
-                uint32_t r[16];
-                tmem_ld16(tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row < a.M) {
-                    float v16[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        v16[j] = __uint_as_float(r[j]);
-                        if (a.relu) v16[j] = fmaxf(v16[j], 0.f);
-                        if (mrow && !(mk[j] > 0.f)) v16[j] = 0.f;
-                    }
-                    if (vec_ok && c0 + 16 <= a.N) {
-#pragma unroll
-                        for (int j = 0; j < 16; j += 4)
-                            __stcs(reinterpret_cast<float4*>(crow + c0 + j), make_float4(v16[j], v16[j + 1], v16[j + 2], v16[j + 3]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (c0 + j < a.N) crow[c0 + j] = v16[j];
-                    }
-                }
-            }
+            const int64_t row0 = (int64_t)tile * BM + q * 32;
+            if (row0 < a.M)
+                store_rows(a, tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16), reinterpret_cast<float*>(gbase + staging + q * kStageBytes), row0, lane);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(acc_empty0 + 8 * b);
         }
@@ -522,18 +512,19 @@ EncodeTiledFn encode_tiled()
     return fn;
 }
 
-// 2-D fp32 row-major matrix [rows x cols] with leading dimension ld, boxes of 32 columns x box_rows rows, 128B swizzle,
+// 2-D fp32 row-major matrix [rows x cols] with leading dimension ld, boxes of box_cols (32: 128B swizzle, 16: 64B swizzle) columns x box_rows rows,
 // out-of-range elements read as zero.
-int make_map(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows)
+int make_map(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, int box_cols = BK)
 {
     EncodeTiledFn fn = encode_tiled();
     if (!fn) return DG_ERR_UNSUPPORTED;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(float)};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), dims, strides, box, elem,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == BK ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? DG_OK : DG_ERR_UNSUPPORTED;
 }
@@ -618,22 +609,22 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
     DenseArgs a{};
     a.C = C; a.ldc = ldc; a.M = M; a.N = N; a.K = K; a.n_pad = (N + 15) / 16 * 16; a.relu = relu ? 1u : 0u;
     a.mask = mask; a.ldm = ldm;
-    // Measured: the tensor cores ignore the low 13 bits of a TF32 operand (results with and without the masked head copy are
-    // bit-identical), so the tile as loaded serves as head; issuing the head passes before the split is 4 % faster.
-    a.raw_head = 2;
     a.status = dense_status_word();
     if (!a.status) return DG_ERR_STATE;
-    CUtensorMap tmA, tmBh, tmBt;
-    int rc;
-    if ((rc = make_map(&tmA, A, M, K, lda, BM)) || (rc = make_map(&tmBh, Bt_head, N, K, ldb, a.n_pad)) ||
-        (rc = make_map(&tmBt, Bt_tail, N, K, ldb, a.n_pad)))
-        return rc;
-    const size_t smem = (size_t)STAGES * (2 * BM * 128 + 2 * a.n_pad * 128) + 24 * STAGES + 48 + 1024;
     const int n_tiles = (int)((M + BM - 1) / BM);
     // two kernels: one tile per CTA, or one persistent CTA per SM walking the tiles
     // Narrow results leave room for two one-tile CTAs per SM, which overlap each other's load latency better than the
-    // persistent CTA's two stages do (2,449,029 x 256 -> 47: 1.09 ms against 1.28 ms; -> 256: 2.16 against 1.88).
+    // persistent CTA's stages do (2,449,029 x 256 -> 47: 1.09 ms against 1.28 ms; -> 256: 2.16 against 1.88, before either
+    // kernel stored whole row pieces).
     const bool per_tile = a.n_pad <= 128;
+    const int box = per_tile ? BK : PK;
+    CUtensorMap tmA, tmBh, tmBt;
+    int rc;
+    if ((rc = make_map(&tmA, A, M, K, lda, BM, box)) || (rc = make_map(&tmBh, Bt_head, N, K, ldb, a.n_pad, box)) ||
+        (rc = make_map(&tmBt, Bt_tail, N, K, ldb, a.n_pad, box)))
+        return rc;
+    const size_t stage = (size_t)box * 4 * (2 * BM + 2 * a.n_pad);
+    const size_t smem = per_tile ? STAGES * stage + 24 * STAGES + 48 + 1024 : PSTAGES * stage + 4 * kStageBytes + 24 * PSTAGES + 64 + 1024;
     if (per_tile) {
         static std::atomic<bool> granted[64];
         if ((rc = allow_smem((const void*)k_dense_nt, granted))) return rc;
@@ -728,22 +719,17 @@ constexpr int TN_STAGES = 3;
 constexpr int TN_BOX_BYTES = TN_ROWS * 128;     // one 32-column box
 
 struct DenseTnArgs {
-    float* partial;                             // [gridDim.x][m_halves][n_pad / 16][4][128][4], see tn_partial_index
+    float* partial;                             // [gridDim.x][m_halves][n_pad / 16][4][128][4]
     int64_t n;                                  // rows to reduce over
     int64_t rows_per_cta;                       // multiple of TN_ROWS
     int32_t Km, Nn, n_pad, m_halves;            // n_pad: Nn rounded up to 16; m_halves: 1 (Km <= 128) or 2
     int32_t flush_slabs;                        // slabs accumulated in tensor memory between two flushes
-    int32_t raw_head;                           // as DenseArgs::raw_head
     int* status;
 };
 
-// Where element (m, c) of a CTA's partial D lives: the 128 rows of an accumulator half are the fastest index above a
-// float4 of columns, so that a warp that holds 32 rows of tensor memory moves 512 contiguous bytes per access.
-__host__ __device__ __forceinline__ int64_t tn_partial_index(int m, int c, int n_pad)
-{
-    return ((((int64_t)(m >> 7) * (n_pad >> 4) + (c >> 4)) * 4 + ((c & 15) >> 2)) * 128 + (m & 127)) * 4 + (c & 3);
-}
-
+// A CTA's partial D: the 128 rows of an accumulator half are the fastest index above a float4 of columns,
+// [half][16-column group][float4][row][4], so that a warp that holds 32 rows of tensor memory moves 512 contiguous bytes per
+// access.
 // MN-major tile of 32-bit elements.  The tensor cores read such operands only in the "128B swizzle with 32-byte atoms"
 // layout (32-byte chunks of a 128-byte row XOR-ed with the row index modulo 4), which TMA writes in its
 // SWIZZLE_128B_ATOM_32B mode: 4-row groups are 512 bytes apart (stride byte offset), the 32-column boxes 2048 bytes
@@ -829,36 +815,6 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
                 if (!ok) break;
                 const uint32_t st = base + s * stage_bytes;
                 const uint64_t g_head = umma_desc_mn_sw128(st + 2 * x_bytes), g_tail = umma_desc_mn_sw128(st + 2 * x_bytes + g_bytes);
-                if (a.raw_head == 2) {
-                    // the tiles as TMA delivered them serve as heads (the low 13 bits of a TF32 operand are ignored): the
-                    // head x head pass does not wait for the split
-                    ok = mbar_wait(full0 + 8 * s, u & 1);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int h = 0; h < a.m_halves; ++h) {
-                        const uint64_t x_head = umma_desc_mn_sw128(st + h * 4 * TN_BOX_BYTES);
-#pragma unroll
-                        for (int k = 0; k < TN_ROWS / 8; ++k)
-                            umma_tf32(tmem + (uint32_t)(h * 256), x_head + (uint64_t)(k * (1024 >> 4)), g_head + (uint64_t)(k * (1024 >> 4)), idesc,
-                                      (in_grp > 0 || k > 0) ? 1u : 0u);
-                    }
-                    ok = mbar_wait(ready0 + 8 * s, u & 1);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int h = 0; h < a.m_halves; ++h) {
-                        const uint64_t x_head = umma_desc_mn_sw128(st + h * 4 * TN_BOX_BYTES);
-                        const uint64_t x_tail = umma_desc_mn_sw128(st + x_bytes + h * 4 * TN_BOX_BYTES);
-#pragma unroll
-                        for (int k = 0; k < TN_ROWS / 8; ++k) {
-                            const uint64_t adv = (uint64_t)(k * (1024 >> 4));
-                            umma_tf32(tmem + (uint32_t)(h * 256), x_tail + adv, g_head + adv, idesc, 1u);
-                            umma_tf32(tmem + (uint32_t)(h * 256), x_head + adv, g_tail + adv, idesc, 1u);
-                        }
-                    }
-                    umma_commit(empty0 + 8 * s);
-                    if (in_grp == T - 1 || i == nslabs - 1) umma_commit(acc_full);
-                    continue;
-                }
                 ok = mbar_wait(ready0 + 8 * s, u & 1);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -887,7 +843,7 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
             ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, u & 1));        // warp-uniform: tcgen05.ld below is .aligned
             if (!ok) break;
             unsigned char* st = gbase + (size_t)s * stage_bytes;
-            for (int part = 0; part < 2; ++part) {                // X then G: head in place, tail behind it
+            for (int part = 0; part < 2; ++part) {                // X then G: the tile as loaded serves as head, its tail goes behind it
                 float4* head = reinterpret_cast<float4*>(st + (part ? 2 * x_bytes : 0));
                 const int count = (part ? g_bytes : x_bytes) / 16;
                 float4* tail = head + count;
@@ -896,7 +852,6 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
                     float4 h;
                     h.x = __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u); h.y = __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
                     h.z = __uint_as_float(__float_as_uint(x.z) & 0xFFFFE000u); h.w = __uint_as_float(__float_as_uint(x.w) & 0xFFFFE000u);
-                    if (!a.raw_head) head[j] = h;
                     tail[j] = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
                 }
             }
@@ -1009,7 +964,6 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
     a.rows_per_cta = (slabs + ctas - 1) / ctas * TN_ROWS;
     const int64_t slots = (int64_t)a.m_halves * 128 * a.n_pad;    // one CTA's partial, padding included
     if (ctas * slots > scratch_floats) return DG_ERR_SCRATCH;
-    a.raw_head = 1;     // no masked head copies (bit-identical results, fewer shared-memory writes); issuing head x head before the split is not faster here
     a.flush_slabs = 16;                                           // 256 rows = 96 tensor-core accumulations per chain
     a.partial = scratch;
     a.status = dense_status_word();

@@ -375,30 +375,32 @@ int launch(SpmmArgs a, cudaStream_t stream)
     return (int)cudaGetLastError();
 }
 
-// Lanes per item and gathers in flight by the number of vectors in a row.  Tiles of 64 float4 go two per lane: half the index
-// traffic and half the chains of row latencies of one per lane, 10 to 25 % faster at every size although only 40 warps fit
-// an SM; two gathers in flight there (one or four are slower, four much).  What is left behind whole tiles of 64 takes launches
-// of its own in the forms that suit it, 32 vectors and then up to 32 more, unless it fills most of a tile (115 M entries,
-// F = 604: 18.4 -> 16.6 ms).  With 17 to 32 float4 a product that fills the GPU for long runs best on 64 warps with one gather
-// each, a short one on four gathers per warp; narrower rows take four.
+// Lanes per item and gathers in flight by the number of vectors in a row and the size of the matrix.  Whole tiles of 64
+// float4 first; what is left behind them takes launches of its own, 32 vectors and then up to 32 more, unless it fills most
+// of a tile (115 M entries, F = 604: 18.4 -> 16.6 ms).
+// Large matrices (from 4 M entries) run best with half the lanes and twice the vectors each: two (or four) rows are in flight
+// per warp, a gather is several independent loads, and index traffic and shuffles are shared by more of them; small ones
+// have too few rows for that and want a row spread over more lanes.  us per product, this form against twice the lanes:
+//   F = 256: 1 M nodes / 17 M entries 1,545 -> 1,296, 2.4 M / 126 M 9,850 -> 8,640; 10,000 nodes / 210 k entries 27 -> 41 (not taken)
+//   F = 100: 936 -> 717, 5,540 -> 4,350, 150 k nodes / 2.6 M entries 131 -> 115; F = 48: 470 -> 389, 2,750 -> 2,250
 template <int VEC, bool PADDED>
-int launch_vec(SpmmArgs a, bool large, cudaStream_t stream)
+int launch_vec(SpmmArgs a, int64_t nnz, cudaStream_t stream)
 {
+    const bool large = nnz >= (int64_t)4 << 20, small = nnz < (int64_t)1 << 20;
     const int end = a.vec_end, wide = end % 64 > 48 ? end : end / 64 * 64;
     int rc = DG_OK;
     if (wide > 0) {
         a.vec_end = wide;
-        rc = launch<VEC, 32, 2, VEC == 4 ? 2 : 4, VEC == 4 && !PADDED ? 5 : 4, PADDED>(a, stream);
+        rc = large ? launch<VEC, 16, 4, 2, 4, PADDED>(a, stream) : launch<VEC, 32, 2, 4, 4, PADDED>(a, stream);
         a.vec_first = wide;
     }
     while (rc == DG_OK && a.vec_first < end) {
         a.vec_end = std::min(end, a.vec_first + 32);
         const int nvec = a.vec_end - a.vec_first;
         if (nvec <= 4) rc = launch<VEC, 4, 1, 4, 5, PADDED>(a, stream);
-        else if (nvec <= 8) rc = launch<VEC, 8, 1, 4, 5, PADDED>(a, stream);
-        else if (nvec <= 16) rc = launch<VEC, 16, 1, 4, 5, PADDED>(a, stream);
-        else if (VEC == 4 && large) rc = launch<VEC, 32, 1, 1, 8, PADDED>(a, stream);
-        else rc = launch<VEC, 32, 1, 4, 5, PADDED>(a, stream);
+        else if (nvec <= 8) rc = launch<VEC, 8, 1, 8, 4, PADDED>(a, stream);
+        else if (nvec <= 16) rc = large ? launch<VEC, 8, 2, 8, 3, PADDED>(a, stream) : launch<VEC, 16, 1, 4, 5, PADDED>(a, stream);
+        else rc = small ? launch<VEC, 32, 1, 4, 5, PADDED>(a, stream) : launch<VEC, 16, 2, 4, 4, PADDED>(a, stream);
         a.vec_first = a.vec_end;
     }
     return rc;
@@ -458,7 +460,6 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     int vec = 1;
     if (F % 4 == 0 && ldb % 4 == 0 && ldc % 4 == 0 && aligned(B, 16) && aligned(C, 16)) vec = 4;
     else if (F % 2 == 0 && ldb % 2 == 0 && ldc % 2 == 0 && aligned(B, 8) && aligned(C, 8)) vec = 2;
-    const bool large = plan->nnz >= (int64_t)4 << 20;
     const int64_t copy = pad_floats(plan, F), sums = partial_floats(plan, F), tiled = tile_floats(plan, val, F);
     const bool padded = vec < 4 && copy > 0 && sums + copy <= scratch_floats && aligned(scratch, 16);
     if (tiled > 0 && (vec == 4 || padded) && sums + copy + tiled <= scratch_floats && aligned(scratch, 16)) {
@@ -478,13 +479,13 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
         if (rc) return rc;
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
         a.B = wide; a.ldb = ld; a.lds = ld; a.vec_end = (int32_t)(ld / 4);
-        return launch_vec<4, true>(a, large, stream);
+        return launch_vec<4, true>(a, plan->nnz, stream);
     }
     a.vec_end = F / vec;
     switch (vec) {
-        case 4: return launch_vec<4, false>(a, large, stream);
-        case 2: return launch_vec<2, false>(a, large, stream);
-        default: return launch_vec<1, false>(a, large, stream);
+        case 4: return launch_vec<4, false>(a, plan->nnz, stream);
+        case 2: return launch_vec<2, false>(a, plan->nnz, stream);
+        default: return launch_vec<1, false>(a, plan->nnz, stream);
     }
 }
 

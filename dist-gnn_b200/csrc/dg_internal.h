@@ -12,9 +12,9 @@
 
 // Rows longer than the threshold are cut into chunks, one lane group each.  A group walks its entries a few dependent gathers
 // at a time, so the longest row or chunk bounds a kernel's duration from below, and a small block has too few rows to hide it:
-// 64 entries below 1 M, 128 below 32 M (F = 256, 150,001 nodes: 204 us against 224 with 256 and 221 with 64), 256 beyond,
-// where shorter chunks gain nothing and their partial sums take twice the memory.
-static inline int32_t dg_default_chunk(int64_t nnz) { return nnz < (1 << 20) ? 64 : nnz < (1 << 25) ? 128 : 256; }
+// 64 entries below 1 M, 128 beyond (F = 256, 150,001 nodes: 199 us against 221 with 64; 2.4 M nodes, F = 48: 2.28 ms against 2.52
+// with 256), and 256 where rows are long on average (dense graph, F = 256: 5.6 ms against 6.3 with 128).
+static inline int32_t dg_default_chunk(int64_t nnz, int32_t m) { return nnz < (1 << 20) ? 64 : nnz < 128 * (int64_t)m ? 128 : 256; }
 
 #define DG_FINISH_TILES 16        // column tiles of one launch: arrival counts are kept per split row and tile
 

@@ -339,8 +339,8 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     if (nnz < 0 || m < 0 || k < 0) return DG_ERR_DIMS;
     if (nnz > 0 && (!row || !col || (sizeof(Id) == 8 && !col32))) return DG_ERR_NULL;
     if (nnz > 0 && (m == 0 || k == 0)) return DG_ERR_DIMS;
-    if (heavy_threshold <= 0) heavy_threshold = dg_default_chunk(nnz);
-    if (chunk <= 0) chunk = dg_default_chunk(nnz);
+    if (heavy_threshold <= 0) heavy_threshold = dg_default_chunk(nnz, m);
+    if (chunk <= 0) chunk = dg_default_chunk(nnz, m);
     cudaStream_t stream = (cudaStream_t)stream_;
 
     dg_plan* p = new (std::nothrow) dg_plan();

@@ -32,10 +32,9 @@ import torch  # noqa: E402
 METRIC, UNIT = 'gcn_epoch_ms', 'ms'
 # DRAM traffic of the local products (dram__bytes_read + dram__bytes_write, ncu, one pass, --clock-control none):
 #   the N = 1 default workload itself, one epoch of `bench.py --steps 1 --warmup 3 --no-cpu-baseline --profiler-range`:
-#   128.18 GB for 147.87 G (stored entry x float) = 0.867 B each;
-#   the 8 products of one distributed SpMM of rank 0 of 8 at F = 256 (spmm_sweep.py --block-of 8): 6.41 GB for 4.02 G = 1.594 B each.
-MEASURED_TRAFFIC = {('sparse2m', 1, 3): 128.18e9}     # (config, ranks, layers) -> bytes per step, captured on that very workload
-TRAFFIC_PER_ENTRY_FLOAT = {'whole_graph': 0.867, 'stage_blocks': 1.594}
+#   158.4 GB for 147.87 G (stored entry x float) = 1.071 B each; no capture of these kernels on the blocks of several ranks.
+MEASURED_TRAFFIC = {('sparse2m', 1, 3): 158.4e9}      # (config, ranks, layers) -> bytes per step, captured on that very workload
+TRAFFIC_PER_ENTRY_FLOAT = 1.071
 CONFIG3_DEADLINE_S = 150      # the extra 1.5D measurement of an 8-GPU default run gives up after this long (it takes about 20 s)
 
 
@@ -354,12 +353,11 @@ def measure(args, rank, world, keep_process_group=False):
         'roofline': {'bound': 'hbm', 'achieved': round(achieved, 2), 'peak': peaks['hbm_gbs'], 'unit': 'GB/s',
                      'frac': round(achieved / peaks['hbm_gbs'], 4),
                      # measured DRAM bytes of all products of one step where this very workload was captured under ncu, else
-                     # null with an estimate beside it: captured bytes per (stored entry x float) x this run's nnz x F (= flops / 2)
+                     # null; on one rank an estimate beside it: captured bytes per (stored entry x float) x this run's nnz x F (= flops / 2)
                      'traffic': traffic,
-                     'traffic_est': round(TRAFFIC_PER_ENTRY_FLOAT['whole_graph' if world == 1 else 'stage_blocks'] * slow['flops'] / 2 / args.steps),
+                     'traffic_est': round(TRAFFIC_PER_ENTRY_FLOAT * slow['flops'] / 2 / args.steps) if world == 1 else None,
                      'traffic_note': ('traffic: ncu dram__bytes of this workload\'s products, one epoch; ' if traffic else 'traffic: no capture of this workload; ')
-                                     + 'traffic_est: captured bytes per (stored entry x float) of '
-                                     + ('the whole-graph products' if world == 1 else 'the 8-rank stage-block products at F = 256') + ' x this run\'s nnz x F',
+                                     + 'traffic_est: captured bytes per (stored entry x float) of the whole-graph products x this run\'s nnz x F, one rank only',
                      'peak_source': peaks['source'],
                      'kernel': 'k_spmm (gather) + k_tile_columns, k_tile_mma (dense tiles on the tensor cores), all local products of the slowest rank',
                      'products_per_step': slow['products'] // args.steps, 'spmm_ms_per_step': round(slow['spmm_ms'] / args.steps, 4),

@@ -117,8 +117,8 @@ __device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const floa
 // large graphs run at that rate times their L2 hit rate; small ones and short rows are bound by latency, which the offsets in
 // shared memory, the look-ahead and U hide.  Against separate kernels with a warp per row (B200, us per product):
 //   10,000 nodes, 210 k entries, F = 64: 74 -> 17      150,001 nodes, 2.6 M entries, F = 256: 263 -> 204; F = 48: 156 -> 79
-//   1 M nodes, 17 M entries, F = 64: 748 -> 475, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 219
-//   2,449,029 nodes, 126 M entries, F = 256: 10,000 -> 9,800, F = 100: 5,760 -> 5,120, F = 48: 3,620 -> 2,570
+//   1 M nodes, 17 M entries, F = 64: 748 -> 400, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 182
+//   2,449,029 nodes, 126 M entries, F = 256: 10,000 -> 8,640, F = 100: 5,760 -> 4,350, F = 48: 3,620 -> 2,230
 // PADDED: the operand is the padded copy of a matrix whose rows are not 16-byte multiples; C is then written float by float.
 template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED>
 __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int chunk_ctas)
@@ -302,6 +302,9 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
     __shared__ int count[kClasses], start[kClasses + 1], next;
     const int32_t row0 = ((int)blockIdx.x - chunk_ctas) * a.rows_per_cta;
     const int nrows = min(a.rows_per_cta, a.m - row0);
+    // An empty row of a product that is added to C stays as it is, neither read nor written: three fifths of the rows of a stage block
+    // on power-law graphs (eight 306,129-row blocks into one result, F = 256: 1,819 -> 1,459 us).
+    const bool keeps = add_first && a.beta == 1.f && !a.flags;
     if (threadIdx.x < kClasses) count[threadIdx.x] = 0;
     if (threadIdx.x == 0) next = 0;
     for (int i = threadIdx.x; i <= nrows; i += 256) first[i] = __ldg(a.rowptr + row0 + i);
@@ -309,7 +312,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
     int cls = -1, place = 0;
     if ((int)threadIdx.x < nrows) {
         const int64_t len = first[threadIdx.x + 1] - first[threadIdx.x];
-        if (len <= a.heavy_threshold) {
+        if (len <= a.heavy_threshold && (len > 0 || !keeps)) {
             const int s = ((int)len + LPR - 1) / LPR;             // batches of LPR entries: classes 0, 1, 2, 3, 4-5, 6-7, 8-11, ...
             const int rank = s < 4 ? s : 2 * (31 - __clz(s)) + ((s >> (30 - __clz(s))) & 1);
             cls = kClasses - 1 - min(rank, kClasses - 1);

@@ -430,3 +430,25 @@ def test_tensor_core_tiles_against_float64(F):
     plan.values.mul_(3.0)
     assert_close(plan.spmm(B, torch.empty_like(C), 1.0, 0.0).cpu().numpy(), 3 * want, TOL / 10, 'values changed in place')
     assert plan.tiled_entries() == 0
+
+
+@pytest.mark.parametrize('alpha,beta,epilogue', [(1.0, 1.0, False), (1.0, 1.0, True), (0.5, 1.0, False), (1.0, -2.0, False), (1.0, 0.0, False)])
+@pytest.mark.parametrize('F', [3, 41, 48, 256])
+def test_empty_rows(F, alpha, beta, epilogue):
+    """Rows without entries, windows without any row that has one: left alone where the product adds to C, else scaled, finished or cleared."""
+    rng = np.random.Generator(np.random.PCG64(F))
+    A = random_coo(rng, 1001, 700, 300, heavy=[(5, 600), (999, 1)])
+    keep = (A.row < 256) | (A.row > 700)
+    A = ref_graph.fast_coalesce_sorted(A.row[keep], A.col[keep], A.val[keep], A.shape)
+    B, C0 = rng.standard_normal((700, F), dtype=np.float32), rng.standard_normal((1001, F), dtype=np.float32)
+    want = ref_gcn.spmm_coo(A, B, C0.copy(), alpha, beta)
+    options = {}
+    if epilogue:
+        scale, bias = rng.random(1001, dtype=np.float32), rng.standard_normal(F, dtype=np.float32)
+        want = np.maximum(want * scale[:, None] + bias, 0)
+        options = dict(row_scale=dev(scale), bias=dev(bias), relu=True)
+    got = make_plan(A).spmm(dev(B), dev(C0), alpha, beta, **options).cpu().numpy()
+    assert_close(got, want, TOL, f'F={F}')
+    if (alpha, beta, epilogue) == (1.0, 1.0, False):
+        empty = np.setdiff1d(np.arange(1001), A.row)
+        assert np.array_equal(got[empty], C0[empty])

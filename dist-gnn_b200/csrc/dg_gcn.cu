@@ -10,7 +10,7 @@ namespace {
 int64_t pad4(int64_t w) { return (w + 3) / 4 * 4; }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-struct Marks {          // begin / end ids of the regions of one call; a failed record is reported by its negative id
+struct Marks {          // ids of the points between the regions of one call; a failed record is reported by its negative id
     int32_t* at;
     void* stream;
     void operator()() { if (at) *at++ = dg_mark_record(stream); }
@@ -49,14 +49,14 @@ extern "C" int dg_gcn_forward(const dg_gcn_net* a, void* stream)
     int rc = check_net(a, false);
     if (rc || a->n == 0) return rc;
     Marks mark{a->marks, stream};
+    mark();
     const float* in = a->x;
     int64_t ld_in = a->ldx;
     for (int l = 0; l < a->layers; ++l) {
         const int32_t K = a->dims[l], N = a->dims[l + 1];
         const int64_t width = pad4(K);
-        mark();
         if ((rc = product(a, in, ld_in, (int32_t)width, stream))) return rc;
-        mark(), mark();
+        mark();
         const float* head = a->fwd_split[l];
         rc = dg_dense_nt_masked(a->z, width, head, head + (int64_t)N * width, width, a->act[l], a->ld_act[l], a->n, N, K, l + 1 < a->layers,
                                 nullptr, 0, stream);
@@ -73,6 +73,7 @@ extern "C" int dg_gcn_backward(const dg_gcn_net* a, void* stream)
     int rc = check_net(a, true);
     if (rc || a->n == 0) return rc;
     Marks mark{a->marks, stream};
+    mark();
     const float* g = a->grad;
     int64_t ld_g = a->ld_grad;
     for (int l = a->layers - 1; l >= 0; --l) {
@@ -80,9 +81,8 @@ extern "C" int dg_gcn_backward(const dg_gcn_net* a, void* stream)
         const int64_t width = pad4(N);
         const float* in = l ? a->act[l - 1] : a->x;
         const int64_t ld_in = l ? a->ld_act[l - 1] : a->ldx;
-        mark();
         if ((rc = product(a, g, ld_g, (int32_t)width, stream))) return rc;
-        mark(), mark();
+        mark();
         if (l > 0) {        // the next gradient; g itself has been read by the product above
             const float* head = a->bwd_split[l];
             rc = dg_dense_nt_masked(a->z, width, head, head + (int64_t)K * width, width, a->g, pad4(K), a->n, K, N, 0, in, ld_in, stream);

@@ -31,37 +31,60 @@ void check(int code)
 void* stream_of(const Tensor& t) { return (void*)at::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 int64_t pad4(int64_t w) { return (w + 3) / 4 * 4; }
 
-// ---- time marks of regions that no Python code sees: drained by the timer they belong to -------------------------------
-struct Region { int key, begin, end; };
+// ---- time marks of regions that no Python code sees: kept until the timer they belong to asks ---------------------------
+// One list per call: the points between its products and transforms, which alternate.  A region read out one by one from the
+// interpreter was 5 us of host work, a quarter of a small training step; here it is what cudaEventElapsedTime takes.
+struct Regions {
+    std::vector<int32_t> marks;
+    bool backward;                        // every layer then counts an all-reduce that a rank without peers has not to do
+};
 std::mutex g_regions_mu;
-std::unordered_map<int64_t, std::vector<Region>> g_regions;
+std::unordered_map<int64_t, std::vector<Regions>> g_regions;
 
-void add_regions(int64_t timer, const std::vector<int32_t>& marks, int layers, bool backward)
+void add_regions(int64_t timer, std::vector<int32_t>&& marks, bool backward)
 {
     std::lock_guard<std::mutex> lock(g_regions_mu);
-    auto& list = g_regions[timer];
-    for (int l = 0; l < layers; ++l) {
-        list.push_back({0, marks[4 * l], marks[4 * l + 1]});
-        list.push_back({1, marks[4 * l + 2], marks[4 * l + 3]});
-        if (backward) list.push_back({2, -1, -1});
-    }
+    g_regions[timer].push_back({std::move(marks), backward});
 }
 int64_t pending_regions(int64_t timer)
 {
     std::lock_guard<std::mutex> lock(g_regions_mu);
-    auto it = g_regions.find(timer);
-    return it == g_regions.end() ? 0 : (int64_t)it->second.size();
+    int64_t n = 0;
+    const auto it = g_regions.find(timer);
+    if (it != g_regions.end())
+        for (const Regions& r : it->second) n += (int64_t)r.marks.size() - 1;
+    return n;
 }
-std::vector<std::tuple<int, int, int>> take_regions(int64_t timer)
+// (seconds, regions) of the products, the transforms and the all-reduces since the last call.  The device has passed the marks.
+std::vector<std::pair<double, int64_t>> resolve_regions(int64_t timer)
 {
-    std::lock_guard<std::mutex> lock(g_regions_mu);
-    std::vector<std::tuple<int, int, int>> out;
-    auto it = g_regions.find(timer);
-    if (it != g_regions.end()) {
-        for (const Region& r : it->second) out.emplace_back(r.key, r.begin, r.end);
-        g_regions.erase(it);
+    std::vector<Regions> calls;
+    {
+        std::lock_guard<std::mutex> lock(g_regions_mu);
+        const auto it = g_regions.find(timer);
+        if (it != g_regions.end()) {
+            calls = std::move(it->second);
+            g_regions.erase(it);
+        }
     }
-    return out;
+    std::vector<std::pair<double, int64_t>> sums(3, {0.0, 0});
+    int failed = DG_OK;
+    for (const Regions& r : calls) {
+        for (size_t i = 0; i + 1 < r.marks.size(); ++i) {
+            auto& sum = sums[i & 1];
+            ++sum.second;
+            float ms = 0.f;
+            if (r.marks[i] < 0 || r.marks[i + 1] < 0) continue;
+            const int rc = dg_mark_elapsed(r.marks[i], r.marks[i + 1], &ms);
+            if (rc != DG_OK) failed = rc;
+            else sum.first += ms / 1000.0;
+        }
+        for (int32_t id : r.marks)
+            if (id >= 0) dg_mark_release(id);
+        if (r.backward) sums[2].second += (int64_t)r.marks.size() / 2;
+    }
+    check(failed);
+    return sums;
 }
 
 // ---- a plan that the autograd graph can keep alive ----------------------------------------------------------------------
@@ -129,7 +152,7 @@ struct Net {                              // shapes and buffers of one call
     std::vector<int64_t> ld_act;
     std::vector<int32_t> marks;
     dg_gcn_net net{};
-    Net(const PlanRef& plan, const Tensor& x, const std::vector<int32_t>& d, std::vector<float*> a) : dims(d), act(std::move(a)), marks(4 * (d.size() - 1), -1)
+    Net(const PlanRef& plan, const Tensor& x, const std::vector<int32_t>& d, std::vector<float*> a) : dims(d), act(std::move(a)), marks(2 * d.size() - 1, -1)
     {
         const int L = (int)dims.size() - 1;
         for (int l = 0; l < L; ++l) ld_act.push_back(l + 1 < L ? pad4(dims[l + 1]) : dims[l + 1]);
@@ -208,7 +231,7 @@ struct GcnNode : public torch::autograd::Node {
         call.net.max_ctas = ctas;
         check(dg_gcn_backward(&call.net, stream_of(x)));
         g_launches += launches;
-        add_regions(timer, call.marks, L, true);
+        add_regions(timer, std::move(call.marks), true);
         return out;
     }
 };
@@ -275,7 +298,7 @@ Tensor gcn(const std::shared_ptr<PlanRef>& plan, const Tensor& features, const T
         int64_t launches = 1;
         for (int l = 1; l <= L; ++l) launches += (dims[l] + 255) / 256;
         g_launches += launches;
-        add_regions(timer, call.marks, L, false);
+        add_regions(timer, std::move(call.marks), false);
     }
     if (train) {
         auto node = std::shared_ptr<GcnNode>(new GcnNode(), torch::autograd::deleteNode);
@@ -363,6 +386,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     m.def("gcn", &gcn);
     m.def("row_cross_entropy", &row_cross_entropy);
     m.def("pending_regions", &pending_regions);
-    m.def("take_regions", &take_regions);
+    m.def("resolve_regions", &resolve_regions);
     m.def("take_launches", [] { return g_launches.exchange(0); });
 }

@@ -68,17 +68,15 @@ class DistTimer:
         spmm_cpp = sys.modules.get('spmm_cpp')
         if spmm_cpp is None:                                # nothing was ever timed on a device
             return
-        if spmm_cpp._binding is not None:
-            for key, begin, end in spmm_cpp._binding.take_regions(self.ident):
-                key = self.NATIVE_KEYS[key]
-                self.count_dict[key] += 1
-                if begin >= 0 and end >= 0:
-                    self.pending.append((key, begin, end))
-                else:
-                    self.duration_dict[key] += 0.0
+        native = spmm_cpp._binding is not None and spmm_cpp._binding.pending_regions(self.ident) > 0
+        if synchronize and (native or self.pending):
+            torch.cuda.synchronize(self.env.device if self.env.device.type == 'cuda' else None)
+        if native:
+            for key, (seconds, count) in zip(self.NATIVE_KEYS, spmm_cpp._binding.resolve_regions(self.ident)):
+                if count:
+                    self.duration_dict[key] += seconds
+                    self.count_dict[key] += count
         if self.pending:
-            if synchronize:
-                torch.cuda.synchronize(self.env.device if self.env.device.type == 'cuda' else None)
             pending, self.pending = self.pending, []
             for key, begin, end in pending:
                 self.duration_dict[key] += spmm_cpp.mark_elapsed(begin, end) / 1000.0

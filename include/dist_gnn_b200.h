@@ -328,7 +328,8 @@ int dg_dense_wait_selftest(int* host_gave_up, void* stream);
  *   z, g           work areas of n * pad4(widest dims) floats; g: backward of two or more layers only
  *   dw[l]          gradient of W_l [dims[l] x dims[l+1]], contiguous; NULL skips it
  *   tn_scratch     as `scratch` of dg_dense_tn, for max_ctas CTAs
- *   marks          NULL, or 4 * layers ids that receive time marks: begin and end of every product, then of every transform */
+ *   marks          NULL, or 2 * layers + 1 ids that receive time marks: one at the beginning, then one behind every product and every
+ *                  transform in the order they are issued (a layer's product comes before its transform) */
 typedef struct dg_gcn_net {
     const dg_plan* plan;
     const float* val;

@@ -59,7 +59,9 @@ struct dg_plan {
     int32_t* task_first_row;  // device, n_tasks: the row that holds entry t * task_nnz
     dg_split_row* split;      // device, n_split rows that span tasks, ascending
     dg_tiles* tiles;          // tensor-core part of the split rows, or null
-    int* status;              // device word: set non-zero by a kernel that gave up on a bounded wait
+    int* status;              // device words: [0] set non-zero by a kernel that gave up on a bounded wait, [1] the last check
+                              // (by number) that found other ids than the plan's
+    int checks;               // checks issued so far
 };
 
 int dg_stream_selected();     // non-zero while dg_select_kernel(2) is in force
@@ -70,12 +72,13 @@ int dg_spmm_stream_launch(const dg_plan* plan, const float* val, const float* B,
 
 // Launches the product with an explicit scratch area (at least n_chunks x F floats; room for a padded copy of an odd-width
 // operand behind it is used where it is there); shared by the plan-owned and the fixed-scratch entry points.
+// `check` != 0: C stays as it is if that check has failed (row kernels only).
 int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                    int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                   float* scratch, int64_t scratch_floats, cudaStream_t stream);
+                   float* scratch, int64_t scratch_floats, cudaStream_t stream, int check = 0);
 int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                         int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                        float* scratch, int64_t scratch_floats, cudaStream_t stream);
+                        float* scratch, int64_t scratch_floats, cudaStream_t stream, int check = 0);
 int dg_plan_build_lean(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k, void* stream, dg_plan** out);
 int dg_plan_ensure_tasks(dg_plan* plan, cudaStream_t stream);
 // Device memory of plans (dg_pool.cu), on the current device.  A block may be freed once the device is done with it.

@@ -66,6 +66,8 @@ struct SpmmArgs {
     int32_t vec_first, vec_end; // the vectors of a row this launch covers
     float alpha, beta;
     uint32_t flags;
+    int check;                  // non-zero: nothing is written if *failed_check says that this check failed
+    const int* failed_check;
 };
 
 template <int VEC> __device__ __forceinline__ void load_vec(const float* p, float (&out)[VEC])
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
     const float* bl = a.B + (int64_t)vec0 * VEC;
     const int64_t ldb = a.ldb;
     float acc[TPL][VEC];
+    const int failed = a.check ? __ldcg(a.failed_check) : 0;      // under way while the first offsets and entries are
 
     // acc += sum over this group's `len` entries; `e` is this lane's first entry, c / v hold it already
     auto gather = [&](const int32_t* col, const float* val, int64_t e, int len, int c, float v) {
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
             c = __ldcs(a.chunk_col + ch.e0 + gl);
             v = __ldcs(a.chunk_val + ch.e0 + gl);
         }
+        if (a.check && failed == a.check) return;
         begin_row(0, false);
         gather(a.chunk_col, a.chunk_val, ch.e0 + gl, ch.len, c, v);
         if (valid) {
@@ -332,6 +336,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
     __syncthreads();
     if (cls >= 0) order[start[cls] + place] = (uint8_t)threadIdx.x;
     __syncthreads();
+    if (a.check && failed == a.check) return;
     const int total = start[kClasses];
 
     int r = -1, c = 0;
@@ -445,10 +450,11 @@ int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, in
 
 int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                         int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                        float* scratch, int64_t scratch_floats, cudaStream_t stream)
+                        float* scratch, int64_t scratch_floats, cudaStream_t stream, int check)
 {
     if (plan->m == 0 || F == 0) return DG_OK;
     SpmmArgs a{};
+    a.check = check; a.failed_check = plan->status + 1;
     a.rowptr = plan->rowptr; a.col = plan->col; a.val = val; a.B = B; a.C = C;
     a.row_scale = row_scale; a.bias = bias; a.chunks = plan->chunks; a.arrived = plan->arrived; a.scratch = scratch;
     a.chunk_col = plan->col; a.chunk_val = val;
@@ -496,7 +502,7 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
 // profile events while a profile is open.
 int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                    int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                   float* scratch, int64_t scratch_floats, cudaStream_t stream)
+                   float* scratch, int64_t scratch_floats, cudaStream_t stream, int check)
 {
     if (plan->m == 0 || F == 0) return DG_OK;
     bool profiled = false;
@@ -517,7 +523,7 @@ int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_
         rc = dg_spmm_stream_launch(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, stream, &launches);
         g_kernel_launches.fetch_add(launches, std::memory_order_relaxed);
     } else {
-        rc = dg_spmm_launch_rows(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, scratch_floats, stream);
+        rc = dg_spmm_launch_rows(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, scratch_floats, stream, check);
     }
     if (profiled) {
         std::lock_guard<std::mutex> lock(g_profile.mu);

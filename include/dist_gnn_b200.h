@@ -82,9 +82,11 @@ int64_t dg_plan_tiled_entries(const dg_plan* plan);
 /* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device; this gives all of it on the current
  * device back (a failed allocation of the library does so by itself). */
 int dg_pool_trim(void);
-/* *host_equal = 1 if both id lists hold the same nnz entries, else 0 (one pass; waits for `stream`). */
-int dg_ids_equal(const int32_t* row_a, const int32_t* col_a, const int32_t* row_b, const int32_t* col_b, int64_t nnz,
-                 int* host_equal, void* stream);
+/* dg_spmm_csr if the ids `row`, `col` (plan's nnz entries) equal `plan_row`, `plan_col`, those the plan was built from: *host_equal
+ * says so.  Otherwise C is left alone.  Waits on the host for the comparison (one pass over both lists), not for the product. */
+int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row, const int32_t* plan_col, const int32_t* row, const int32_t* col,
+                        const float* val, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t F, float alpha, float beta,
+                        int* host_equal, void* stream);
 int dg_plan_get_stats(const dg_plan* plan, dg_plan_stats* host_out);
 /* The streaming kernel cuts the entry list into tasks of `task_nnz` entries (one warp each; default 1024).  This
  * rebuilds the task tables for another size (<= 0 restores the default); synchronises `stream`. */

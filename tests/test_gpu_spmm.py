@@ -452,3 +452,30 @@ def test_empty_rows(F, alpha, beta, epilogue):
     if (alpha, beta, epilogue) == (1.0, 1.0, False):
         empty = np.setdiff1d(np.arange(1001), A.row)
         assert np.array_equal(got[empty], C0[empty])
+
+
+@pytest.mark.parametrize('where', [0, -1])
+@pytest.mark.parametrize('F', [1, 41, 100, 256])
+def test_checked_product_writes_nothing_for_other_ids(F, where):
+    """The product behind the id check, through the C ABI: the plan's own ids, then lists that differ in one entry - C untouched -
+    and the plan still works afterwards."""
+    import spmm_cpp
+    rng = np.random.Generator(np.random.PCG64(700 + F))
+    A = random_coo(rng, 500, 333, 4000, heavy=[(17, 300), (499, 90)])
+    plan = make_plan(A)
+    row, col, val = dev(A.row, torch.int32), dev(A.col, torch.int32), plan.values
+    other = col.clone()
+    other[where] += 1
+    B, C0 = rng.standard_normal((333, F), dtype=np.float32), rng.standard_normal((500, F), dtype=np.float32)
+    want = ref_gcn.spmm_coo(A, B, C0.copy(), 1.0, 1.0)
+    b, same = dev(B), ctypes.c_int(-1)
+    for ids, equal in ((col, 1), (other, 0), (col, 1)):
+        C = dev(C0)
+        spmm_cpp.check(spmm_cpp.lib().dg_spmm_csr_checked(plan.handle, row.data_ptr(), col.data_ptr(), row.data_ptr(), ids.data_ptr(), val.data_ptr(), b.data_ptr(),
+                                                          F, C.data_ptr(), F, F, 1.0, 1.0, ctypes.byref(same), torch.cuda.current_stream().cuda_stream))
+        assert same.value == equal
+        got = C.cpu().numpy()
+        if equal:
+            assert_close(got, want, TOL, f'F={F}')
+        else:
+            assert np.array_equal(got, C0)

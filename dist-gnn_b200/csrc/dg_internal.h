@@ -54,6 +54,7 @@ struct dg_plan {
     int64_t heavy_nnz, max_row_nnz, touched_columns;
     float* scratch;           // device, grown on demand by dg_spmm_prepare
     int64_t scratch_floats;
+    bool no_padded_copy;      // there was no memory for one
     // streaming kernel: the entry list cut into tasks of task_nnz entries, one warp each (0 until that family is first used)
     int32_t task_nnz, n_tasks, n_split;
     int32_t* task_first_row;  // device, n_tasks: the row that holds entry t * task_nnz
@@ -83,6 +84,7 @@ int dg_plan_build_lean(const int32_t* row, const int32_t* col, int64_t nnz, int3
 int dg_plan_ensure_tasks(dg_plan* plan, cudaStream_t stream);
 // Device memory of plans (dg_pool.cu), on the current device.  A block may be freed once the device is done with it.
 int dg_pool_alloc(void** out, size_t bytes);
+int dg_device_alloc(void** out, size_t bytes);      // not from the pool, freed with cudaFree
 void dg_pool_free(void* ptr);
 int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream);
 int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, int64_t ldb, const float* C, int64_t ldc,

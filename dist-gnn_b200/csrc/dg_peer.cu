@@ -96,7 +96,8 @@ extern "C" int dg_comm_peer_alloc(dg_comm* c, int64_t floats, char host_handles_
     }
     static_assert(sizeof(cudaIpcMemHandle_t) == 64, "a CUDA IPC memory handle is expected to be 64 bytes");
     for (int b = 0; b < 2; ++b) {
-        DG_CUDA(cudaMalloc(&c->peer_send[b], (size_t)floats * sizeof(float)));
+        const int rc = dg_device_alloc((void**)&c->peer_send[b], (size_t)floats * sizeof(float));
+        if (rc) return rc;
         cudaIpcMemHandle_t h;
         DG_CUDA(cudaIpcGetMemHandle(&h, c->peer_send[b]));
         memcpy(host_handles_out + 64 * b, &h, 64);

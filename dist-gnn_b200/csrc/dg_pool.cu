@@ -6,8 +6,12 @@
 // again to requests of a similar size.  A block that does not fit any more pushes out those that have lain idle longest: what
 // earlier, larger plans left behind must not keep the blocks of those in use now from staying (plan and product of a 55,160-node
 // matrix after others had filled the pool: 930 -> 180 us).  A block may come back only when the device is done with it: callers synchronise
-// first (dg_plan_destroy the device, as cudaFree did; plan construction its stream).  A failed allocation gives everything
-// back and tries again; dg_pool_trim gives everything back on request.
+// first (dg_plan_destroy the device, as cudaFree did; plan construction its stream).
+//
+// The program around the library usually has a caching allocator of its own, which may hold the whole device without using it.
+// So an allocation that the driver refuses is tried three times: as it is, after the pool has given its idle blocks back, and
+// after the program has been asked to (dg_on_low_memory).  dg_pool_trim gives the pool's idle blocks back on request.
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -28,6 +32,8 @@ struct Pool {
 };
 Pool& pool() { static Pool* p = new Pool(); return *p; }      // never destroyed: the driver may be gone first
 
+std::atomic<void (*)(void)> g_give_back{nullptr};                 // the program's own cache
+
 // Sizes in steps of an eighth of their power of two, so that blocks of nearly equal plans fit one another.
 size_t rounded(size_t bytes)
 {
@@ -46,7 +52,47 @@ void release_unused(Pool& p, int dev)                             // caller hold
     p.unused_bytes[dev] = 0;
 }
 
+int trim(int dev)
+{
+    if (dev < 0 || dev >= kMaxDevices) return DG_ERR_STATE;
+    Pool& p = pool();
+    std::lock_guard<std::mutex> lock(p.mu);
+    release_unused(p, dev);
+    return DG_OK;
+}
+
 }  // namespace
+
+// cudaMalloc that makes room where there is none.  No lock is held while the program gives its memory back, and a refusal leaves
+// nothing behind for the next cudaGetLastError() to report.
+int dg_device_alloc(void** out, size_t bytes)
+{
+    int dev = -1;
+    DG_CUDA(cudaGetDevice(&dev));
+    cudaError_t e = cudaMalloc(out, bytes);
+    for (int attempt = 0; attempt < 2 && e == cudaErrorMemoryAllocation; ++attempt) {
+        cudaGetLastError();
+        if (attempt == 0) {
+            trim(dev);
+        } else {
+            void (*give_back)(void) = g_give_back.load();
+            if (!give_back) break;
+            give_back();
+        }
+        e = cudaMalloc(out, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *out = nullptr;
+    }
+    return (int)e;
+}
+
+extern "C" int dg_on_low_memory(void (*give_back)(void))
+{
+    g_give_back.store(give_back);
+    return DG_OK;
+}
 
 int dg_pool_alloc(void** out, size_t bytes)
 {
@@ -55,21 +101,19 @@ int dg_pool_alloc(void** out, size_t bytes)
     if (dev < 0 || dev >= kMaxDevices) return DG_ERR_STATE;
     const size_t want = rounded(bytes ? bytes : 1);
     Pool& p = pool();
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        auto it = p.unused[dev].lower_bound(want);
+        if (it != p.unused[dev].end() && it->first <= want + want / 4) {
+            *out = it->second.ptr;
+            p.unused_bytes[dev] -= it->first;
+            p.unused[dev].erase(it);
+            return DG_OK;
+        }
+    }
+    const int rc = dg_device_alloc(out, want);
+    if (rc) return rc;
     std::lock_guard<std::mutex> lock(p.mu);
-    auto it = p.unused[dev].lower_bound(want);
-    if (it != p.unused[dev].end() && it->first <= want + want / 4) {
-        *out = it->second.ptr;
-        p.unused_bytes[dev] -= it->first;
-        p.unused[dev].erase(it);
-        return DG_OK;
-    }
-    cudaError_t e = cudaMalloc(out, want);
-    if (e == cudaErrorMemoryAllocation && !p.unused[dev].empty()) {
-        cudaGetLastError();
-        release_unused(p, dev);
-        e = cudaMalloc(out, want);
-    }
-    if (e != cudaSuccess) return (int)e;
     p.size[dev][*out] = want;
     return DG_OK;
 }
@@ -105,9 +149,5 @@ extern "C" int dg_pool_trim(void)
 {
     int dev = -1;
     DG_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices) return DG_ERR_STATE;
-    Pool& p = pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    release_unused(p, dev);
-    return DG_OK;
+    return trim(dev);
 }

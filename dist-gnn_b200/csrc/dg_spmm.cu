@@ -420,7 +420,7 @@ bool aligned(const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(
 // over B and pays where its rows are gathered several times: 200,003 nodes, 10.2 M entries, F = 41: 336 -> 235 us.
 int64_t pad_floats(const dg_plan* plan, int32_t F)
 {
-    return F % 4 && F > 4 && plan->nnz >= 4 * (int64_t)plan->k ? (int64_t)plan->k * ((F + 3) / 4 * 4) : 0;
+    return !plan->no_padded_copy && F % 4 && F > 4 && plan->nnz >= 4 * (int64_t)plan->k ? (int64_t)plan->k * ((F + 3) / 4 * 4) : 0;
 }
 
 // Floats of scratch behind those for the tensor-core part, 0 where it is not used: the tiles hold these very values.
@@ -563,7 +563,8 @@ extern "C" int dg_profile_end(dg_profile* out)
 
 // Grows the plan's scratch to what a product of width F may need (either kernel family); allocates and synchronises
 // `stream` only when it has to grow.  The stage loops call it for every plan before they enqueue anything, so that an
-// allocation failure cannot leave a loop half issued.
+// allocation failure cannot leave a loop half issued.  Only the partial sums of the split rows are indispensable: a plan that cannot have
+// more goes on without its tiles, and then without padded copies, for good (asking again would stall every product).
 int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream)
 {
     if (!plan) return DG_ERR_NULL;
@@ -572,18 +573,26 @@ int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream)
         const int rc = dg_plan_ensure_tasks(p, stream);
         if (rc) return rc;
     }
-    const int64_t rows = partial_floats(plan, F) + pad_floats(plan, F) + tile_floats(plan, nullptr, F), tasks = dg_stream_selected() ? 2 * (int64_t)plan->n_tasks * F : 0;
-    const int64_t need = rows > tasks ? rows : tasks;
-    if (need > p->scratch_floats) {
+    for (;;) {
+        const int64_t rows = partial_floats(plan, F) + pad_floats(plan, F) + tile_floats(plan, nullptr, F), tasks = dg_stream_selected() ? 2 * (int64_t)plan->n_tasks * F : 0;
+        const int64_t need = rows > tasks ? rows : tasks;
+        if (need <= p->scratch_floats) return DG_OK;
         DG_CUDA(cudaStreamSynchronize(stream));
         dg_pool_free(p->scratch);
         p->scratch = nullptr;
         p->scratch_floats = 0;
         const int rc = dg_pool_alloc((void**)&p->scratch, (size_t)need * sizeof(float));
-        if (rc) return rc;
-        p->scratch_floats = need;
+        if (rc == DG_OK) p->scratch_floats = need;
+        if (rc != (int)cudaErrorMemoryAllocation) return rc;
+        if (tile_floats(plan, nullptr, F) > 0) {
+            dg_tiles_free(p->tiles);
+            p->tiles = nullptr;
+        } else if (pad_floats(plan, F) > 0) {
+            p->no_padded_copy = true;
+        } else {
+            return rc;
+        }
     }
-    return DG_OK;
 }
 
 extern "C" int dg_spmm_csr(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,

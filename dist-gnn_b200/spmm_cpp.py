@@ -9,6 +9,7 @@ without CUDA tensors they raise.
 """
 import ctypes
 import os
+import warnings
 import weakref
 
 import torch
@@ -26,6 +27,7 @@ TILE_ALWAYS = 48 << 20
 
 EPI_ROW_SCALE, EPI_BIAS, EPI_RELU = 1, 2, 4
 ERR_UNSUPPORTED = -4
+CUDA_OUT_OF_MEMORY = 2
 
 
 class PlanStats(ctypes.Structure):
@@ -50,6 +52,11 @@ class SplitJob(ctypes.Structure):
                 ('ldb', ctypes.c_int64), ('N', ctypes.c_int32), ('K', ctypes.c_int32), ('transposed', ctypes.c_int32), ('pad', ctypes.c_int32)]
 
 
+_GiveBack = ctypes.CFUNCTYPE(None)
+# PyTorch keeps freed memory, up to the whole device; the library's plans and scratch live beside it
+_give_back = _GiveBack(torch.cuda.empty_cache)
+
+
 def lib():
     """The loaded C library; raises if it has not been built (python dist-gnn_b200/csrc/build.py)."""
     global _lib
@@ -70,6 +77,7 @@ def lib():
             'dg_plan_drop_tiles': ([vp, vp], ctypes.c_int),
             'dg_plan_tiled_entries': ([vp], i64),
             'dg_pool_trim': ([], ctypes.c_int),
+            'dg_on_low_memory': ([_GiveBack], ctypes.c_int),
             'dg_spmm_csr_checked': ([vp, vp, vp, vp, vp, vp, vp, i64, vp, i64, i32, f32, f32, ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
             'dg_plan_destroy': ([vp], ctypes.c_int),
             'dg_plan_get_stats': ([vp, ctypes.POINTER(PlanStats)], ctypes.c_int),
@@ -121,6 +129,7 @@ def lib():
         for name, (argtypes, restype) in sig.items():
             fn = getattr(L, name)
             fn.argtypes, fn.restype = argtypes, restype
+        L.dg_on_low_memory(_give_back)
         _lib = L
     return _lib
 
@@ -249,7 +258,11 @@ class SpmmPlan:
         if self.values.numel() >= TILE_NNZ and self._tiled is None:
             index = self.device.index
             with _on(index):
-                check(lib().dg_plan_add_tiles(self.handle, self.values.data_ptr(), _raw_stream(index)))
+                code = lib().dg_plan_add_tiles(self.handle, self.values.data_ptr(), _raw_stream(index))
+            if code < 0 or code == CUDA_OUT_OF_MEMORY:                # the products are right without them
+                warnings.warn(f'no tensor-core tiles for a block of {self.values.numel()} entries: {_lib.dg_strerror(code).decode()}')
+            else:
+                check(code)
             if _lib.dg_plan_tiled_entries(self.handle):
                 self._tiled = self.values._version
         return self

@@ -75,13 +75,18 @@ int dg_plan_destroy(dg_plan* plan);
  * makes a second copy of the split rows' entries (8 bytes each) WITH their values `val`; products with another `val` pointer
  * are gathered as before, and a caller that changes the values in place calls this again or dg_plan_drop_tiles.  Returns
  * DG_OK without doing anything where the block has too few dense tiles.  Synchronises `stream`; no product on the plan may be
- * in flight.  dg_plan_tiled_entries: how many entries the tensor cores take (0: no tiles). */
+ * in flight.  dg_plan_tiled_entries: how many entries the tensor cores take (0: no tiles).  Where it fails, for lack of memory
+ * (cudaErrorMemoryAllocation) or otherwise, the plan is as it was without tiles; a plan whose scratch finds no memory drops them. */
 int dg_plan_add_tiles(dg_plan* plan, const float* val, void* stream);
 int dg_plan_drop_tiles(dg_plan* plan, void* stream);
 int64_t dg_plan_tiled_entries(const dg_plan* plan);
 /* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device; this gives all of it on the current
  * device back (a failed allocation of the library does so by itself). */
 int dg_pool_trim(void);
+/* `give_back` is called (on the allocating thread, with the allocating device current and none of the library's locks held) when
+ * the driver refuses device memory that the library's own idle blocks cannot make up for; then the allocation is tried once
+ * more.  A program whose allocator keeps freed memory returns it to the driver there, as spmm_cpp does with PyTorch's.  NULL: none. */
+int dg_on_low_memory(void (*give_back)(void));
 /* dg_spmm_csr if the ids `row`, `col` (plan's nnz entries) equal `plan_row`, `plan_col`, those the plan was built from: *host_equal
  * says so.  Otherwise C is left alone.  Waits on the host for the comparison (one pass over both lists), not for the product. */
 int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row, const int32_t* plan_col, const int32_t* row, const int32_t* col,

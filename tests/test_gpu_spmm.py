@@ -479,3 +479,116 @@ def test_checked_product_writes_nothing_for_other_ids(F, where):
             assert_close(got, want, TOL, f'F={F}')
         else:
             assert np.array_equal(got, C0)
+
+
+def skewed_block(seed, m=3001, k=2600):
+    """Rows of 40 to 2,400 entries, columns as skewed: a block with a dense corner."""
+    rng = np.random.Generator(np.random.PCG64(seed))
+    deg = np.minimum((40 * (m / (1 + np.arange(m))) ** 0.7).astype(np.int64) + 1, 2400)
+    p = 1.0 / (1 + np.arange(k)) ** 0.8
+    row = np.repeat(rng.permutation(m), deg)
+    col = np.concatenate([rng.choice(k, d, replace=False, p=p / p.sum()) for d in deg])
+    val = rng.standard_normal(row.size, dtype=np.float32)
+    return ref_graph.fast_coalesce_sorted(row.astype(np.int64), rng.permutation(k)[col].astype(np.int64), val, (m, k))
+
+
+def tiled_plan(A):
+    import spmm_cpp
+    keep = spmm_cpp.TILE_NNZ
+    try:
+        spmm_cpp.TILE_NNZ = 0
+        return make_plan(A).tile()
+    finally:
+        spmm_cpp.TILE_NNZ = keep
+
+
+def leave_free(mib):
+    """Takes all but about `mib` MiB of the device's free memory."""
+    import spmm_cpp
+    spmm_cpp.empty_cache()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.empty(torch.cuda.mem_get_info()[0] - (mib << 20), dtype=torch.uint8, device='cuda')
+
+
+def test_plan_and_scratch_beside_a_framework_that_keeps_the_whole_device():
+    """PyTorch holds all but a few MiB as freed blocks: the plan, its tiles and its scratch get theirs all the same."""
+    A = skewed_block(5)
+    F = 1024
+    B = np.random.Generator(np.random.PCG64(6)).standard_normal((2600, F), dtype=np.float32)
+    b, C = dev(B), torch.empty(3001, F, device='cuda')
+    held = leave_free(8)
+    del held                                                       # kept by torch's cache
+    assert torch.cuda.mem_get_info()[0] < 64 << 20
+    plan = tiled_plan(A)
+    assert plan.tiled_entries() > 0
+    plan.spmm(b, C, 1.0, 0.0)
+    assert plan.device_status() == 0
+    assert_close(C.cpu().numpy(), ref_gcn.spmm_coo(A, B, np.zeros((3001, F), np.float32), 1.0, 0.0), TOL, 'beside a full cache')
+    torch.cuda.empty_cache()
+
+
+def test_product_without_memory_for_its_tiles():
+    """The device is really full: the scratch of the tiles finds no room, the product gathers everything; later launches see no stale error."""
+    A = skewed_block(7)
+    F = 1024
+    B = np.random.Generator(np.random.PCG64(8)).standard_normal((2600, F), dtype=np.float32)
+    plan = tiled_plan(A)
+    assert plan.tiled_entries() > 0
+    b, C = dev(B), torch.empty(3001, F, device='cuda')
+    partial = plan.stats()['heavy_chunks'] * F * 4 >> 20
+    assert partial < 40                                            # the tiles' partial results and images take 100 MiB and more
+    held = leave_free(partial + 24)
+    plan.spmm(b, C, 1.0, 0.0)
+    assert plan.tiled_entries() == 0
+    b.add_(0)
+    del held
+    torch.cuda.empty_cache()
+    assert_close(C.cpu().numpy(), ref_gcn.spmm_coo(A, B, np.zeros((3001, F), np.float32), 1.0, 0.0), TOL, 'without tiles')
+
+
+@pytest.mark.parametrize('code', [2, -5])
+def test_tile_search_that_fails_leaves_the_plan_without_tiles(monkeypatch, code):
+    import spmm_cpp
+    A = skewed_block(9)
+    B = np.random.Generator(np.random.PCG64(10)).standard_normal((2600, 64), dtype=np.float32)
+    monkeypatch.setattr(spmm_cpp.lib(), 'dg_plan_add_tiles', lambda *a: code)
+    with pytest.warns(UserWarning, match='no tensor-core tiles'):
+        plan = tiled_plan(A)
+    assert plan.tiled_entries() == 0
+    C = plan.spmm(dev(B), torch.empty(3001, 64, device='cuda'), 1.0, 0.0)
+    assert_close(C.cpu().numpy(), ref_gcn.spmm_coo(A, B, np.zeros((3001, 64), np.float32), 1.0, 0.0), TOL, 'without tiles')
+
+
+LARGEST = """
+import sys, torch
+sys.path.insert(0, sys.argv[1])
+import spmm_cpp
+from coo_graph import graph_utils, synthetic
+n, F, seed = 4_000_000, 256, int(sys.argv[2])
+A = graph_utils.sym_normalization(synthetic.rmat_edge_index(n, 256_000_000, seed, device='cuda'), n)
+b = torch.randn(n, F, device='cuda', generator=torch.Generator(device='cuda').manual_seed(seed))
+plan = spmm_cpp.SpmmPlan.from_coo(A)
+C = plan.spmm(b, torch.empty(n, F, device='cuda'), 1.0, 0.0)
+assert plan.device_status() == 0
+first = plan.rowptr()
+length = first[1:] - first[:-1]
+rows = torch.cat((torch.topk(length, 128).indices, torch.randint(n, (256,), generator=torch.Generator().manual_seed(seed))))
+col, val = A.indices()[1], A.values()
+for r in rows.tolist():
+    e = slice(int(first[r]), int(first[r + 1]))
+    want = val[e].double() @ b[col[e]].double()
+    err = float((C[r].double() - want).norm() / want.norm())
+    assert err < 1e-5, (r, int(length[r]), err)
+print('rows agree')
+"""
+
+
+@pytest.mark.parametrize('seed', [1, 2])
+def test_largest_graph_in_a_fresh_process(seed):
+    """4 M nodes, 260 M entries, operand and result of 4 GB: the longest rows and a sample against float64."""
+    import subprocess
+    import sys
+    from conftest import PKG
+    done = subprocess.run([sys.executable, '-c', LARGEST, PKG, str(seed)], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and 'rows agree' in done.stdout, done.stdout + done.stderr[-2000:]

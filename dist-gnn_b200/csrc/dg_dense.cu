@@ -529,18 +529,6 @@ int make_map(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int
     return r == CUDA_SUCCESS ? DG_OK : DG_ERR_UNSUPPORTED;
 }
 
-int* dense_status_word()
-{
-    static int* word[64] = {nullptr};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    if (!word[dev]) {
-        if (cudaMalloc((void**)&word[dev], sizeof(int)) != cudaSuccess) return nullptr;
-        cudaMemset(word[dev], 0, sizeof(int));
-    }
-    return word[dev];
-}
-
 }  // namespace
 
 extern "C" int dg_dense_split(const float* src, float* head, float* tail, int64_t count, void* stream)
@@ -609,7 +597,7 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
     DenseArgs a{};
     a.C = C; a.ldc = ldc; a.M = M; a.N = N; a.K = K; a.n_pad = (N + 15) / 16 * 16; a.relu = relu ? 1u : 0u;
     a.mask = mask; a.ldm = ldm;
-    a.status = dense_status_word();
+    a.status = dg_status_word();
     if (!a.status) return DG_ERR_STATE;
     const int n_tiles = (int)((M + BM - 1) / BM);
     // two kernels: one tile per CTA, or one persistent CTA per SM walking the tiles
@@ -642,7 +630,7 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
 extern "C" int dg_dense_status(int* host_status, void* stream)
 {
     if (!host_status) return DG_ERR_NULL;
-    int* w = dense_status_word();
+    int* w = dg_status_word();
     if (!w) return DG_ERR_STATE;
     DG_CUDA(cudaMemcpyAsync(host_status, w, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     DG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
@@ -651,7 +639,7 @@ extern "C" int dg_dense_status(int* host_status, void* stream)
 
 extern "C" int dg_dense_status_reset(void* stream)
 {
-    int* w = dense_status_word();
+    int* w = dg_status_word();
     if (!w) return DG_ERR_STATE;
     DG_CUDA(cudaMemsetAsync(w, 0, sizeof(int), (cudaStream_t)stream));
     return DG_OK;
@@ -966,7 +954,7 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
     if (ctas * slots > scratch_floats) return DG_ERR_SCRATCH;
     a.flush_slabs = 16;                                           // 256 rows = 96 tensor-core accumulations per chain
     a.partial = scratch;
-    a.status = dense_status_word();
+    a.status = dg_status_word();
     if (!a.status) return DG_ERR_STATE;
     CUtensorMap tmX, tmG;
     int rc;

@@ -88,6 +88,26 @@ int dg_device_alloc(void** out, size_t bytes)
     return (int)e;
 }
 
+// One word per device, zero until a tensor-core kernel gives up on a bounded wait.
+int* dg_status_word()
+{
+    static std::mutex mu;
+    static int* word[kMaxDevices] = {};
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!word[dev]) {
+        int* w = nullptr;
+        if (dg_device_alloc((void**)&w, sizeof(int)) != DG_OK) return nullptr;
+        if (cudaMemset(w, 0, sizeof(int)) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+            cudaFree(w);
+            return nullptr;
+        }
+        word[dev] = w;
+    }
+    return word[dev];
+}
+
 extern "C" int dg_on_low_memory(void (*give_back)(void))
 {
     g_give_back.store(give_back);

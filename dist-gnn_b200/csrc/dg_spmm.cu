@@ -15,6 +15,7 @@
 #include <vector>
 #include "dg_internal.h"
 #include "dg_tiles.h"
+#include "dg_umma.h"
 
 namespace {
 
@@ -474,7 +475,7 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     if (tiled > 0 && (vec == 4 || padded) && sums + copy + tiled <= scratch_floats && aligned(scratch, 16)) {
         float* area = scratch + sums + copy;
         int launches = 0;
-        const int rc = dg_tiles_launch(plan, B, ldb, F, area, stream, &launches);
+        const int rc = dg_tiles_launch(plan, B, ldb, F, area, stream, &launches, dg::kWaitLimit);
         if (rc) return rc;
         g_kernel_launches.fetch_add(launches, std::memory_order_relaxed);
         const dg_tiles* t = plan->tiles;

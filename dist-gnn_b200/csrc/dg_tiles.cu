@@ -39,7 +39,6 @@ constexpr int kFlushSlabs = 16;
 constexpr int kTileStages = 3;
 constexpr int kScatterThreads = 256, kGroupThreads = 128, kTileThreads = kScatterThreads + 64;
 constexpr int kAhead = 8;                 // records a thread holds for its group's next tile
-constexpr int kTileWaitLimit = 1 << 16;   // polls of a wait, a fraction of a second
 constexpr int T = 256;
 constexpr int kBands = 4096;
 
@@ -108,7 +107,8 @@ struct TileArgs {
     const uint16_t* images;
     float4* partial;                      // [slot][ld4][128]
     int32_t ld4, F4, n_pad, col_tiles;    // 16-byte pieces of a partial row; of those, how many are wanted
-    int* status;
+    int *status, *device_status;          // the plan's word and the device's
+    int wait_limit;                       // polls of a wait
 };
 
 // blockIdx.x: the CTA's share of the tiles, blockIdx.y: panel of n_pad columns.  Warps 0-3 and 4-7: the two scatter groups
@@ -160,15 +160,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
     if (warp == 8) {                                              // copies of B's slabs
         const uint16_t* images = a.images + (int64_t)blockIdx.y * a.col_tiles * 3 * n * kTileCols;
         int next = lane < total ? __ldg(&slabs[lane].col_tile) : 0, cur = 0;
-        for (int t = 0; t < total && ok; ++t) {
+        int t = 0;
+        for (; t < total; ++t) {
             const int s = t % kTileStages, u = t / kTileStages;
             if ((t & 31) == 0) {
                 cur = next;
                 next = t + 32 + lane < total ? __ldg(&slabs[t + 32 + lane].col_tile) : 0;
             }
             const int tile = __shfl_sync(0xffffffffu, cur, t & 31);
-            if (u > 0) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (u - 1) & 1, kTileWaitLimit));
-            if (ok && lane == 0) {
+            if (u > 0) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (u - 1) & 1, a.wait_limit));
+            if (!ok) break;
+            if (lane == 0) {
                 mbar_expect_tx(full_b + 8 * s, b_bytes);
                 bulk_load(base + s * stage_bytes + a_bytes, images + (int64_t)tile * 3 * n * kTileCols, b_bytes, full_b + 8 * s);
             }
@@ -183,8 +185,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
                 const int count = a.segments[seg].slab1 - a.segments[seg].slab0;
                 for (int i = 0; i < count && ok; ++i, ++t) {
                     const int s = t % kTileStages, u = t / kTileStages, in_run = i % kFlushSlabs;
-                    if (in_run == 0 && run > 0) ok = mbar_wait(acc_empty, (run - 1) & 1, kTileWaitLimit);
-                    ok = ok && mbar_wait(full_b + 8 * s, u & 1, kTileWaitLimit) && mbar_wait(ready_a + 8 * s, u & 1, kTileWaitLimit);
+                    if (in_run == 0 && run > 0) ok = mbar_wait(acc_empty, (run - 1) & 1, a.wait_limit);
+                    ok = ok && mbar_wait(full_b + 8 * s, u & 1, a.wait_limit) && mbar_wait(ready_a + 8 * s, u & 1, a.wait_limit);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t A = base + s * stage_bytes, Bs = A + a_bytes;
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
         // Adds the accumulators into the partial result of the segment.  Only this thread ever touches these 16-byte pieces, in
         // program order, so the sum order is fixed; the reduction is sent to L2 and not waited for.
         auto drain = [&](bool first, bool last) {
-            ok = __all_sync(0xffffffffu, mbar_wait(acc_full, run & 1, kTileWaitLimit));      // tcgen05.ld is warp-collective
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_full, run & 1, a.wait_limit));      // tcgen05.ld is warp-collective
             ++run;
             if (!ok) return;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
         int filled = -1;                                          // the last tile this group filled
         for (int t = group; t < total; t += 2) {                  // no way out of this loop: its barrier wants all four warps
             const int s = t % kTileStages, u = t / kTileStages;
-            if (ok && u > 0) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (u - 1) & 1, kTileWaitLimit));
+            if (ok && u > 0) ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * s, (u - 1) & 1, a.wait_limit));
             unsigned char* A = gbase + s * stage_bytes;
             if (ok) {
 #pragma unroll
@@ -311,7 +313,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
         }
         for (int t = filled >= 0 ? filled - 1 : 0; t < total; ++t) drain_if_end(t);
     }
-    if (!ok) atomicExch(a.status, 1);
+    if (!ok) {
+        atomicExch(a.status, 1);
+        atomicExch(a.device_status, 1);
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -690,7 +695,8 @@ extern "C" int dg_plan_add_tiles(dg_plan* p, const float* val, void* stream)
     dg_tiles* t = new (std::nothrow) dg_tiles();
     if (!t) return (int)cudaErrorMemoryAllocation;
     *t = dg_tiles{};
-    const int rc = build_tiles(p, val, (cudaStream_t)stream, t);
+    t->status = dg_status_word();
+    const int rc = t->status ? build_tiles(p, val, (cudaStream_t)stream, t) : DG_ERR_STATE;
     if (rc != DG_OK || t->entries == 0) {
         cudaStreamSynchronize((cudaStream_t)stream);
         dg_tiles_free(t);
@@ -710,6 +716,19 @@ extern "C" int dg_plan_drop_tiles(dg_plan* p, void* stream)
     return DG_OK;
 }
 
+// The give-up path on purpose: the tensor-core part of a product, with waits of no polls at all.
+extern "C" int dg_tiles_wait_selftest(const dg_plan* p, const float* B, int64_t ldb, int32_t F, void* stream)
+{
+    if (!p || !B) return DG_ERR_NULL;
+    if (F < 1 || ldb < F) return DG_ERR_DIMS;
+    int rc = dg_spmm_prepare(p, F, (cudaStream_t)stream);
+    if (rc) return rc;
+    const int64_t need = dg_tiles_scratch_floats(p, F);
+    if (need == 0 || need > p->scratch_floats) return DG_ERR_STATE;
+    int launches = 0;
+    return dg_tiles_launch(p, B, ldb, F, p->scratch, (cudaStream_t)stream, &launches, 0);
+}
+
 extern "C" int64_t dg_plan_tiled_entries(const dg_plan* p) { return p && p->tiles ? p->tiles->entries : 0; }
 
 // Narrow operands are gathered: a tile costs at least its six passes over A whatever the width is.
@@ -721,13 +740,13 @@ int64_t dg_tiles_scratch_floats(const dg_plan* p, int32_t F)
     return (int64_t)t->n_segments * kTileRows * F4 + (int64_t)panels_of(F) * t->col_tiles * 3 * panel_width(F) * kTileCols / 2;
 }
 
-int dg_tiles_launch(const dg_plan* p, const float* B, int64_t ldb, int32_t F, float* area, cudaStream_t stream, int* launches)
+int dg_tiles_launch(const dg_plan* p, const float* B, int64_t ldb, int32_t F, float* area, cudaStream_t stream, int* launches, int wait_limit)
 {
     const dg_tiles* t = p->tiles;
     const int32_t F4 = (F + 3) / 4, panels = panels_of(F), n_pad = panel_width(F);
     uint16_t* images = reinterpret_cast<uint16_t*>(area + (int64_t)t->n_segments * kTileRows * F4 * 4);
     k_tile_columns<<<dim3((unsigned)t->col_tiles, (unsigned)panels), T, 0, stream>>>(B, ldb, t->columns, t->n_columns, t->col_tiles, F, n_pad, images);
-    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status};
+    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, wait_limit};
     const size_t smem = kTileStages * (3 * kTileElems * 2 + (size_t)3 * n_pad * kTileCols * 2) + 24 * kTileStages + 32 + 128;
     static std::atomic<bool> allowed[64];
     if (p->device < 0 || p->device >= 64) return DG_ERR_STATE;

@@ -27,10 +27,11 @@ struct dg_tiles {
     float* rest_val;
     dg_chunk* rest_chunks;
     int32_t n_rest_chunks;
+    int* status;                  // the device's word of kernels that gave up (dg_status_word)
 };
 
 // Scratch floats that a product of width F takes for the tiles (0: the tiles are not used at this width).
 int64_t dg_tiles_scratch_floats(const dg_plan* plan, int32_t F);
 // Launches the tensor-core part: partial results of the tiled rows land at `area`, 16-byte pieces of 128 rows side by side.
-int dg_tiles_launch(const dg_plan* plan, const float* B, int64_t ldb, int32_t F, float* area, cudaStream_t stream, int* launches);
+int dg_tiles_launch(const dg_plan* plan, const float* B, int64_t ldb, int32_t F, float* area, cudaStream_t stream, int* launches, int wait_limit);
 void dg_tiles_free(dg_tiles* t);      // the device is done with it

@@ -84,6 +84,7 @@ def lib():
             'dg_plan_copy_rowptr': ([vp, vp, vp], ctypes.c_int),
             'dg_plan_set_task_size': ([vp, i32, vp], ctypes.c_int),
             'dg_plan_device_status': ([vp, ctypes.POINTER(ctypes.c_int), vp], ctypes.c_int),
+            'dg_tiles_wait_selftest': ([vp, vp, i64, i32, vp], ctypes.c_int),
             'dg_spmm_csr': ([vp, vp, vp, i64, vp, i64, i32, f32, f32, u32, vp, vp, vp], ctypes.c_int),
             'dg_spmm_csr_static': ([vp, vp, vp, i64, vp, i64, i32, f32, f32, u32, vp, vp, vp], ctypes.c_int),
             'dg_static_scratch_capacity': ([], ctypes.c_int64),
@@ -813,8 +814,9 @@ def dense_tn(x, g):
 
 
 def dense_status(reset=False):
-    """0, or non-zero if a dense-transform kernel gave up on one of its bounded waits since the last reset (its output is
-    then invalid).  Synchronises the current stream.  reset=True clears the word after reading it."""
+    """0, or non-zero if a tensor-core kernel - a dense transform's or a tiled product's - gave up on one of its bounded waits
+    since the last reset (its output is then invalid).  Synchronises the current stream.  reset=True clears the word after
+    reading it."""
     out = ctypes.c_int(-1)
     check(lib().dg_dense_status(ctypes.byref(out), _stream()))
     if reset and out.value:
@@ -823,10 +825,11 @@ def dense_status(reset=False):
 
 
 def check_dense_status():
-    """Raises if a dense kernel gave up since the last check (and clears the word, so the next check starts fresh)."""
+    """Raises if a tensor-core kernel gave up since the last check (and clears the word, so the next check starts fresh)."""
     status = dense_status(reset=True)
     if status:
-        raise RuntimeError('a dense-transform kernel gave up on a bounded wait: the activations or gradients of this step are invalid')
+        raise RuntimeError('a dense-transform or tile kernel gave up on a bounded wait: the products, activations or gradients '
+                           'computed since the last check are invalid')
 
 
 def dense_wait_selftest():

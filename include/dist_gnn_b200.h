@@ -101,8 +101,12 @@ int dg_plan_set_task_size(dg_plan* plan, int32_t task_nnz, void* stream);
  * 16-byte aligned and at least 64 floats wide).  Process-wide; also settable with DG_SPMM_KERNEL=rows|stream. */
 int dg_select_kernel(int family);
 /* Reads the plan's device status word (synchronises `stream`).  Non-zero if the tensor-core part of a product
- * (dg_plan_add_tiles) gave up on one of its bounded waits; its result is then invalid. */
+ * (dg_plan_add_tiles) gave up on one of its bounded waits; its result is then invalid.  Such a kernel also sets the device's
+ * word that dg_dense_status reads, which is the one to look at after a step. */
 int dg_plan_device_status(const dg_plan* plan, int* host_status, void* stream);
+/* Runs the tensor-core part of a product on a plan with tiles with waits that run out at once: the kernel gives up, sets both
+ * words and returns (DG_ERR_STATE without tiles at this width).  For tests of the callers that read them. */
+int dg_tiles_wait_selftest(const dg_plan* plan, const float* B, int64_t ldb, int32_t F, void* stream);
 /* copies the m+1 row offsets to host memory (synchronises `stream`); used to check CSR indexing bit for bit */
 int dg_plan_copy_rowptr(const dg_plan* plan, int64_t* host_rowptr, void* stream);
 

@@ -592,3 +592,22 @@ def test_largest_graph_in_a_fresh_process(seed):
     from conftest import PKG
     done = subprocess.run([sys.executable, '-c', LARGEST, PKG, str(seed)], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0 and 'rows agree' in done.stdout, done.stdout + done.stderr[-2000:]
+
+
+def test_tile_kernel_that_gives_up_is_noticed():
+    """A tile kernel whose waits run out sets the word that training reads after every step; other plans' products are unharmed."""
+    import spmm_cpp
+    A = skewed_block(11)
+    b = torch.randn(2600, 256, device='cuda')
+    plan = tiled_plan(A)
+    spmm_cpp.check_dense_status()
+    spmm_cpp.check(spmm_cpp.lib().dg_tiles_wait_selftest(plan.handle, b.data_ptr(), 256, 256, torch.cuda.current_stream().cuda_stream))
+    assert plan.device_status() != 0
+    with pytest.raises(RuntimeError, match='gave up'):
+        spmm_cpp.check_dense_status()
+    spmm_cpp.check_dense_status()
+    fresh, plain = tiled_plan(A), make_plan(A)
+    C = fresh.spmm(b, torch.empty(3001, 256, device='cuda'), 1.0, 0.0)
+    assert fresh.device_status() == 0
+    assert_close(C.cpu().numpy(), plain.spmm(b, torch.empty_like(C), 1.0, 0.0).cpu().numpy(), TOL / 10, 'after a kernel that gave up')
+    assert spmm_cpp.lib().dg_tiles_wait_selftest(plain.handle, b.data_ptr(), 256, 256, None) == -5

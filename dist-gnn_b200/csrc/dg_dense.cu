@@ -167,8 +167,8 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
     const int b_bytes = a.n_pad * 128;                            // one slab of Bt: n_pad rows x 128 bytes
     const int stage_bytes = 2 * BM * 128 + 2 * b_bytes;           // A head, A tail, Bt head, Bt tail
     const uint32_t bars = base + STAGES * stage_bytes;
-    const uint32_t full0 = bars, ready0 = bars + 8 * STAGES, empty0 = bars + 16 * STAGES, acc_full = bars + 24 * STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + STAGES * stage_bytes + 24 * STAGES + 8);
+    const uint32_t full0 = bars, ready0 = bars + 8 * STAGES, empty0 = bars + 16 * STAGES, acc_full = bars + 24 * STAGES, done = acc_full + 8;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + STAGES * stage_bytes + 24 * STAGES + 16);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t m0 = (int64_t)blockIdx.x * BM;
     const int nslabs = (a.K + BK - 1) / BK;
@@ -182,6 +182,7 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
             mbar_init(empty0 + 8 * s, 1);
         }
         mbar_init(acc_full, 1);
+        mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {                                              // one warp allocates the accumulator columns
@@ -196,7 +197,8 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 
     if (warp == 0) {
         if (lane == 0) {                                          // TMA producer
-            for (int i = 0; i < nslabs && ok; ++i) {
+            int i = 0;
+            for (; i < nslabs && ok; ++i) {
                 const int s = i % STAGES, u = i / STAGES;
                 if (u > 0) ok = mbar_wait(empty0 + 8 * s, (u - 1) & 1);
                 if (!ok) break;
@@ -206,6 +208,7 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 tma_load_2d(st + 2 * BM * 128, &tmBh, i * BK, 0, full0 + 8 * s);
                 tma_load_2d(st + 2 * BM * 128 + b_bytes, &tmBt, i * BK, 0, full0 + 8 * s);
             }
+            await_loads(full0, i, STAGES);
         }
     } else if (warp == 1) {
         if (lane == 0) {                                          // MMA issuer
@@ -227,6 +230,7 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
                 umma_commit(empty0 + 8 * s);                      // the stage is free once these MMAs have read it
             }
             if (ok) umma_commit(acc_full);
+            await_mmas(done);
         }
     } else {
         const int t = threadIdx.x - 64;                           // 0..127: split A, then drain the accumulator
@@ -290,8 +294,8 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int staging = PSTAGES * stage_bytes;                    // the epilogue warps' row pieces
     const uint32_t bars = base + staging + 4 * kStageBytes;
     const uint32_t full0 = bars, ready0 = bars + 8 * PSTAGES, empty0 = bars + 16 * PSTAGES;
-    const uint32_t acc_full0 = bars + 24 * PSTAGES, acc_empty0 = acc_full0 + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + staging + 4 * kStageBytes + 24 * PSTAGES + 32);
+    const uint32_t acc_full0 = bars + 24 * PSTAGES, acc_empty0 = acc_full0 + 16, done = acc_empty0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + staging + 4 * kStageBytes + 24 * PSTAGES + 40);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nhalves = (a.K + PK - 1) / PK;
     constexpr int kTmemCols = 512;                                // two accumulators of up to 256 columns
@@ -306,6 +310,7 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             mbar_init(acc_full0 + 8 * b, 1);
             mbar_init(acc_empty0 + 8 * b, 128);
         }
+        mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -333,6 +338,7 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                     tma_load_2d(st + 2 * a_bytes + b_bytes, &tmBt, i * PK, 0, full0 + 8 * s);
                 }
             }
+            await_loads(full0, it, PSTAGES);
         }
     } else if (warp == 1) {
         if (lane == 0) {                                          // MMA issuer
@@ -377,6 +383,7 @@ k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                 }
                 if (ok) umma_commit(acc_full0 + 8 * b);
             }
+            await_mmas(done);
         }
     } else if (warp < 6) {
         const int t = threadIdx.x - 64;                           // 0..127: split the A half slab of every stage
@@ -750,8 +757,8 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
     const int stage_bytes = 2 * x_bytes + 2 * g_bytes;            // X head, X tail, G head, G tail
     const uint32_t bars = base + TN_STAGES * stage_bytes;
     const uint32_t full0 = bars, ready0 = bars + 8 * TN_STAGES, empty0 = bars + 16 * TN_STAGES, acc_full = bars + 24 * TN_STAGES;
-    const uint32_t acc_empty = acc_full + 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + TN_STAGES * stage_bytes + 24 * TN_STAGES + 16);
+    const uint32_t acc_empty = acc_full + 8, done = acc_full + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + TN_STAGES * stage_bytes + 24 * TN_STAGES + 24);
     const int T = a.flush_slabs;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t r_begin = (int64_t)blockIdx.x * a.rows_per_cta;
@@ -768,6 +775,7 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
         }
         mbar_init(acc_full, 1);
         mbar_init(acc_empty, 128);
+        mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -782,7 +790,8 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
 
     if (warp == 0) {
         if (lane == 0) {                                          // TMA producer
-            for (int i = 0; i < nslabs && ok; ++i) {
+            int i = 0;
+            for (; i < nslabs && ok; ++i) {
                 const int s = i % TN_STAGES, u = i / TN_STAGES;
                 if (u > 0) ok = mbar_wait(empty0 + 8 * s, (u - 1) & 1);
                 if (!ok) break;
@@ -792,6 +801,7 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
                 for (int j = 0; j < x_boxes; ++j) tma_load_2d(st + j * TN_BOX_BYTES, &tmX, 32 * j, r0, full0 + 8 * s);
                 for (int j = 0; j < g_boxes; ++j) tma_load_2d(st + 2 * x_bytes + j * TN_BOX_BYTES, &tmG, 32 * j, r0, full0 + 8 * s);
             }
+            await_loads(full0, i, TN_STAGES);
         }
     } else if (warp == 1) {
         if (lane == 0) {                                          // MMA issuer
@@ -821,6 +831,7 @@ k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUte
                 umma_commit(empty0 + 8 * s);
                 if (in_grp == T - 1 || i == nslabs - 1) umma_commit(acc_full);
             }
+            await_mmas(done);
         }
     } else {
         const int t = threadIdx.x - 64;
@@ -960,7 +971,7 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
     int rc;
     if ((rc = make_map_box(&tmX, X, n, Km, ldx, 32, TN_ROWS)) || (rc = make_map_box(&tmG, G, n, Nn, ldg, 32, TN_ROWS))) return rc;
     const int x_bytes = a.m_halves * 4 * TN_BOX_BYTES, g_bytes = (a.n_pad + 31) / 32 * TN_BOX_BYTES;
-    const size_t smem = (size_t)TN_STAGES * (2 * x_bytes + 2 * g_bytes) + 24 * TN_STAGES + 24 + 1024;
+    const size_t smem = (size_t)TN_STAGES * (2 * x_bytes + 2 * g_bytes) + 24 * TN_STAGES + 32 + 1024;
     static std::atomic<bool> granted[64];
     if ((rc = allow_smem((const void*)k_dense_tn, granted))) return rc;
     k_dense_tn<<<ctas, kThreads, smem, (cudaStream_t)stream>>>(tmX, tmG, a);

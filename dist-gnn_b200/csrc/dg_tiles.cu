@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
     constexpr uint32_t a_piece = kTileElems * 2, a_bytes = 3 * a_piece;
     const uint32_t stage_bytes = a_bytes + b_bytes, bars = base + kTileStages * stage_bytes;
     const uint32_t full_b = bars, ready_a = bars + 8 * kTileStages, empty = bars + 16 * kTileStages, acc_full = bars + 24 * kTileStages,
-                   acc_empty = acc_full + 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + kTileStages * stage_bytes + 24 * kTileStages + 16);
+                   acc_empty = acc_full + 8, done = acc_full + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + kTileStages * stage_bytes + 24 * kTileStages + 24);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
         }
         mbar_init(acc_full, 1);
         mbar_init(acc_empty, 8);
+        mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 9) {
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
             }
             __syncwarp();
         }
+        await_loads(full_b, t, kTileStages);
     } else if (warp == 9) {
         if (lane == 0) {                                          // MMA issue
             // fp32 accumulator, bf16 A and B, both K-major, 128 x n
@@ -212,6 +214,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
                     }
                 }
             }
+            await_mmas(done);
         }
     } else {
         const int group = warp >> 2, q = warp & 3, tid = threadIdx.x & (kGroupThreads - 1);

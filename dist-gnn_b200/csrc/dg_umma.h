@@ -45,5 +45,18 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// What a role waits for before it leaves the CTA, whether its loop came to its end or gave up: a copy that lands, or an MMA that
+// reads, after the CTA is gone would do so in the shared and tensor memory of the next one.
+// The loads of stages 0 .. issued - 1 of a ring (one full barrier a stage): the last round of every stage.
+__device__ __forceinline__ void await_loads(uint32_t full0, int issued, int stages)
+{
+    for (int t = issued > stages ? issued - stages : 0; t < issued; ++t) mbar_wait(full0 + 8 * (t % stages), (t / stages) & 1);
+}
+// All MMAs this thread has issued; `done` is a barrier of its own, with a count of 1.
+__device__ __forceinline__ void await_mmas(uint32_t done)
+{
+    umma_commit(done);
+    mbar_wait(done, 0);
+}
 
 }  // namespace dg

@@ -39,6 +39,11 @@ struct dg_split_row {
 
 #define DG_DEFAULT_TASK_NNZ 1024
 
+#define DG_STATUS_WORDS 4
+#define DG_TILE_WORDS 2           // from here: whether the product under way may use its tiles (dg_tiles.h)
+#define DG_UNFIT_OPERAND 0
+#define DG_GATHER_ALL 1
+
 struct dg_tiles;      // dg_tiles.h
 
 struct dg_plan {
@@ -61,7 +66,7 @@ struct dg_plan {
     dg_split_row* split;      // device, n_split rows that span tasks, ascending
     dg_tiles* tiles;          // tensor-core part of the split rows, or null
     int* status;              // device words: [0] set non-zero by a kernel that gave up on a bounded wait, [1] the last check
-                              // (by number) that found other ids than the plan's
+                              // (by number) that found other ids than the plan's, then the tiles' (DG_TILE_WORDS)
     int checks;               // checks issued so far
 };
 

@@ -363,7 +363,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     int2* block_sums = nullptr;
     dg_chunk* in_row_order = nullptr;
     const size_t zero_bytes = sizeof(PlanCounts) + kBands * sizeof(int32_t) + (size_t)words * sizeof(uint32_t);
-    if ((rc = dg_pool_alloc((void**)&p->rowptr, ((size_t)m + 1) * sizeof(int64_t))) || (rc = dg_pool_alloc((void**)&p->status, 2 * sizeof(int))) ||
+    if ((rc = dg_pool_alloc((void**)&p->rowptr, ((size_t)m + 1) * sizeof(int64_t))) || (rc = dg_pool_alloc((void**)&p->status, DG_STATUS_WORDS * sizeof(int))) ||
         (rc = tmp.alloc(&zeroed, zero_bytes)) || (rc = tmp.alloc(&block_sums, (size_t)row_blocks)))
         return fail(rc);
     if (max_chunks > 0 && ((rc = dg_pool_alloc((void**)&p->chunks, (size_t)max_chunks * sizeof(dg_chunk))) ||
@@ -374,7 +374,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     int32_t* bands = reinterpret_cast<int32_t*>(counts + 1);
     uint32_t* bitmap = words ? reinterpret_cast<uint32_t*>(bands + kBands) : nullptr;
     cudaMemsetAsync(zeroed, 0, zero_bytes, stream);
-    cudaMemsetAsync(p->status, 0, 2 * sizeof(int), stream);
+    cudaMemsetAsync(p->status, 0, DG_STATUS_WORDS * sizeof(int), stream);
     if (max_chunks > 0) cudaMemsetAsync(p->arrived, 0, (size_t)max_heavy * DG_FINISH_TILES * sizeof(int), stream);
 
     const int64_t per_block = (int64_t)T * kEntriesPerThread;

@@ -57,6 +57,7 @@ struct SpmmArgs {
     const int2* parts;          // partial results of the tiles per split row (dg_tiles.h), or null
     const float4* part_area;
     int64_t part_ld4;           // 16-byte pieces of a partial row
+    int* tile_words;            // with tiles: dg_plan::status + DG_TILE_WORDS, else null
     int* arrived;               // [n_heavy x DG_FINISH_TILES] partial sums of a split row that are in place; zero between products
     float* scratch;
     int64_t ldb, ldc, lds;      // lds: row stride of the partial sums
@@ -122,8 +123,10 @@ __device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const floa
 //   10,000 nodes, 210 k entries, F = 64: 74 -> 17      150,001 nodes, 2.6 M entries, F = 256: 263 -> 204; F = 48: 156 -> 79
 //   1 M nodes, 17 M entries, F = 64: 748 -> 400, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 182
 //   2,449,029 nodes, 126 M entries, F = 256: 10,000 -> 8,640, F = 100: 5,760 -> 4,350, F = 48: 3,620 -> 2,230
+// WHOLE: the second launch of a product with tiles.  It does nothing unless the tiles could not be used (dg_tiles.h): then the first
+// one has left the split rows alone, and a few CTAs per SM gather them whole.
 // PADDED: the operand is the padded copy of a matrix whose rows are not 16-byte multiples; C is then written float by float.
-template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED>
+template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED, bool WHOLE>
 __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int chunk_ctas)
 {
     constexpr int G = 32 / LPR, NG = 256 / LPR;
@@ -231,8 +234,9 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
         }
     };
 
-    if ((int)blockIdx.x < chunk_ctas) {
-        const int id = blockIdx.x * NG + threadIdx.x / LPR;
+    // NG chunks of split rows, from chunk id0 on
+    auto run_chunks = [&](int id0) {
+        const int id = id0 + threadIdx.x / LPR;
         const bool valid = id < a.n_chunks;
         dg_chunk ch{};
         if (valid) ch = a.chunks[id];
@@ -298,6 +302,24 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
             }
         }
         store_row(ch.row);
+    };
+    if constexpr (VEC == 4) {
+        if (a.tile_words) {                                       // a product with tiles, which it may turn out not to be able to use
+            const bool whole = __ldcg(a.tile_words + DG_GATHER_ALL) != 0;
+            if constexpr (WHOLE) {
+                if (!whole) return;
+            } else {
+                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.tile_words[DG_UNFIT_OPERAND] = 0;      // for the next product
+                if (whole && (int)blockIdx.x < chunk_ctas) return;
+            }
+        }
+    }
+    if constexpr (WHOLE) {
+        for (int id0 = blockIdx.x * NG; id0 < a.n_chunks; id0 += chunk_ctas * NG) run_chunks(id0);
+        return;
+    }
+    if ((int)blockIdx.x < chunk_ctas) {
+        run_chunks(blockIdx.x * NG);
         return;
     }
 
@@ -371,15 +393,25 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
 }
 
 template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED>
-int launch(SpmmArgs a, cudaStream_t stream)
+int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
 {
     constexpr int NG = 256 / LPR, tile = LPR * TPL;
+    SpmmArgs a = args;
     const int chunk_ctas = (a.n_chunks + NG - 1) / NG;
     const int64_t row_ctas = ((int64_t)a.m + a.rows_per_cta - 1) / a.rows_per_cta;
     for (; a.vec_first < a.vec_end; a.vec_first += tile * DG_FINISH_TILES) {
         const dim3 grid((unsigned)(chunk_ctas + row_ctas), (unsigned)std::min((a.vec_end - a.vec_first + tile - 1) / tile, DG_FINISH_TILES));
-        k_spmm<VEC, LPR, TPL, U, MINB, PADDED><<<grid, 256, 0, stream>>>(a, chunk_ctas);
+        k_spmm<VEC, LPR, TPL, U, MINB, PADDED, false><<<grid, 256, 0, stream>>>(a, chunk_ctas);
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        if constexpr (VEC == 4) {
+            if (!whole) continue;
+            SpmmArgs w = *whole;
+            w.vec_first = a.vec_first;
+            w.vec_end = a.vec_end;
+            const int ctas = std::min((w.n_chunks + NG - 1) / NG, 148 * 4);
+            k_spmm<VEC, LPR, TPL, U, MINB, PADDED, true><<<dim3((unsigned)ctas, grid.y), 256, 0, stream>>>(w, ctas);
+            g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        }
     }
     return (int)cudaGetLastError();
 }
@@ -393,23 +425,23 @@ int launch(SpmmArgs a, cudaStream_t stream)
 //   F = 256: 1 M nodes / 17 M entries 1,545 -> 1,296, 2.4 M / 126 M 9,850 -> 8,640; 10,000 nodes / 210 k entries 27 -> 41 (not taken)
 //   F = 100: 936 -> 717, 5,540 -> 4,350, 150 k nodes / 2.6 M entries 131 -> 115; F = 48: 470 -> 389, 2,750 -> 2,250
 template <int VEC, bool PADDED>
-int launch_vec(SpmmArgs a, int64_t nnz, cudaStream_t stream)
+int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, cudaStream_t stream)
 {
     const bool large = nnz >= (int64_t)4 << 20, small = nnz < (int64_t)1 << 20;
     const int end = a.vec_end, wide = end % 64 > 48 ? end : end / 64 * 64;
     int rc = DG_OK;
     if (wide > 0) {
         a.vec_end = wide;
-        rc = large ? launch<VEC, 16, 4, 2, 4, PADDED>(a, stream) : launch<VEC, 32, 2, 4, 4, PADDED>(a, stream);
+        rc = large ? launch<VEC, 16, 4, 2, 4, PADDED>(a, whole, stream) : launch<VEC, 32, 2, 4, 4, PADDED>(a, whole, stream);
         a.vec_first = wide;
     }
     while (rc == DG_OK && a.vec_first < end) {
         a.vec_end = std::min(end, a.vec_first + 32);
         const int nvec = a.vec_end - a.vec_first;
-        if (nvec <= 4) rc = launch<VEC, 4, 1, 4, 5, PADDED>(a, stream);
-        else if (nvec <= 8) rc = launch<VEC, 8, 1, 8, 4, PADDED>(a, stream);
-        else if (nvec <= 16) rc = large ? launch<VEC, 8, 2, 8, 3, PADDED>(a, stream) : launch<VEC, 16, 1, 4, 5, PADDED>(a, stream);
-        else rc = small ? launch<VEC, 32, 1, 4, 5, PADDED>(a, stream) : launch<VEC, 16, 2, 4, 4, PADDED>(a, stream);
+        if (nvec <= 4) rc = launch<VEC, 4, 1, 4, 5, PADDED>(a, whole, stream);
+        else if (nvec <= 8) rc = launch<VEC, 8, 1, 8, 4, PADDED>(a, whole, stream);
+        else if (nvec <= 16) rc = large ? launch<VEC, 8, 2, 8, 3, PADDED>(a, whole, stream) : launch<VEC, 16, 1, 4, 5, PADDED>(a, whole, stream);
+        else rc = small ? launch<VEC, 32, 1, 4, 5, PADDED>(a, whole, stream) : launch<VEC, 16, 2, 4, 4, PADDED>(a, whole, stream);
         a.vec_first = a.vec_end;
     }
     return rc;
@@ -472,13 +504,16 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     else if (F % 2 == 0 && ldb % 2 == 0 && ldc % 2 == 0 && aligned(B, 8) && aligned(C, 8)) vec = 2;
     const int64_t copy = pad_floats(plan, F), sums = partial_floats(plan, F), tiled = tile_floats(plan, val, F);
     const bool padded = vec < 4 && copy > 0 && sums + copy <= scratch_floats && aligned(scratch, 16);
-    if (tiled > 0 && (vec == 4 || padded) && sums + copy + tiled <= scratch_floats && aligned(scratch, 16)) {
+    SpmmArgs whole;
+    const bool tiles = tiled > 0 && (vec == 4 || padded) && sums + copy + tiled <= scratch_floats && aligned(scratch, 16);
+    if (tiles) {
         float* area = scratch + sums + copy;
         int launches = 0;
         const int rc = dg_tiles_launch(plan, B, ldb, F, area, stream, &launches, dg::kWaitLimit);
         if (rc) return rc;
         g_kernel_launches.fetch_add(launches, std::memory_order_relaxed);
         const dg_tiles* t = plan->tiles;
+        a.tile_words = plan->status + DG_TILE_WORDS;
         a.chunks = t->rest_chunks; a.n_chunks = t->n_rest_chunks; a.chunk_col = t->rest_col; a.chunk_val = t->rest_val;
         a.parts = t->parts; a.part_area = reinterpret_cast<const float4*>(area); a.part_ld4 = (F + 3) / 4;
     }
@@ -488,14 +523,20 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
         const int rc = dg_pad_rows(B, ldb, plan->k, F, wide, ld, stream);
         if (rc) return rc;
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-        a.B = wide; a.ldb = ld; a.lds = ld; a.vec_end = (int32_t)(ld / 4);
-        return launch_vec<4, true>(a, plan->nnz, stream);
+        a.B = wide; a.ldb = ld; a.lds = ld;
     }
-    a.vec_end = F / vec;
+    a.vec_end = padded ? (int32_t)(a.ldb / 4) : F / vec;
+    if (tiles) {                                                  // the same product without them
+        whole = a;
+        whole.chunks = plan->chunks; whole.n_chunks = plan->n_chunks; whole.chunk_col = plan->col; whole.chunk_val = val;
+        whole.parts = nullptr;
+    }
+    const SpmmArgs* w = tiles ? &whole : nullptr;
+    if (padded) return launch_vec<4, true>(a, w, plan->nnz, stream);
     switch (vec) {
-        case 4: return launch_vec<4, false>(a, plan->nnz, stream);
-        case 2: return launch_vec<2, false>(a, plan->nnz, stream);
-        default: return launch_vec<1, false>(a, plan->nnz, stream);
+        case 4: return launch_vec<4, false>(a, w, plan->nnz, stream);
+        case 2: return launch_vec<2, false>(a, w, plan->nnz, stream);
+        default: return launch_vec<1, false>(a, w, plan->nnz, stream);
     }
 }
 

@@ -35,6 +35,7 @@ constexpr int kTileRows = 128, kTileCols = 32;
 constexpr int kTileElems = kTileRows * kTileCols;
 constexpr int kTileMin = 160;             // entries from which a tile is worth multiplying
 constexpr int kMaxColumns = 1 << 16;      // frequent columns considered, at most
+constexpr float kTileBound = 9.2233720e18f;     // 2^63: a product of two smaller numbers is finite, with a factor of 4 to spare for sums
 constexpr int kFlushSlabs = 16;
 constexpr int kTileStages = 3;
 constexpr int kScatterThreads = 256, kGroupThreads = 128, kTileThreads = kScatterThreads + 64;
@@ -79,8 +80,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 
 // Slab images of B: [panel][column tile][piece][k octet][n][8] bf16.  One thread makes one 16-byte octet of all three pieces.
 __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B, int64_t ldb, const int32_t* __restrict__ columns, int32_t n_columns,
-                                                    int32_t col_tiles, int32_t F, int32_t n_pad, uint16_t* __restrict__ out)
+                                                    int32_t col_tiles, int32_t F, int32_t n_pad, uint16_t* __restrict__ out, int* __restrict__ words)
 {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) words[DG_GATHER_ALL] = 0;
+    bool fit = true;
     uint16_t* image = out + ((int64_t)blockIdx.y * col_tiles + blockIdx.x) * 3 * n_pad * kTileCols;
     for (int i = threadIdx.x; i < n_pad * (kTileCols / 8); i += T) {
         const int n = i % n_pad, octet = i / n_pad, f = blockIdx.y * n_pad + n;
@@ -89,6 +92,7 @@ __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B,
         for (int j = 0; j < 8; ++j) {
             const int k = blockIdx.x * kTileCols + octet * 8 + j;
             const float x = k < n_columns && f < F ? __ldg(B + (int64_t)__ldg(columns + k) * ldb + f) : 0.f;
+            fit = fit && fabsf(x) < kTileBound;                   // not so for a NaN
             split3(x, h[j], m[j], l[j]);
         }
         uint4* at = reinterpret_cast<uint4*>(image) + octet * n_pad + n;
@@ -97,6 +101,7 @@ __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B,
         at[piece] = make_uint4(m[0] | m[1] << 16, m[2] | m[3] << 16, m[4] | m[5] << 16, m[6] | m[7] << 16);
         at[2 * piece] = make_uint4(l[0] | l[1] << 16, l[2] | l[3] << 16, l[4] | l[5] << 16, l[6] | l[7] << 16);
     }
+    if (!fit) words[DG_UNFIT_OPERAND] = 1;
 }
 
 struct TileArgs {
@@ -108,6 +113,7 @@ struct TileArgs {
     float4* partial;                      // [slot][ld4][128]
     int32_t ld4, F4, n_pad, col_tiles;    // 16-byte pieces of a partial row; of those, how many are wanted
     int *status, *device_status;          // the plan's word and the device's
+    int* words;                           // dg_plan::status + DG_TILE_WORDS
     int wait_limit;                       // polls of a wait
 };
 
@@ -154,7 +160,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
     const uint32_t tmem = *tmem_slot, acc_small = tmem + 256;
     bool ok = true;
 
-    const int seg0 = a.cta_segment[blockIdx.x], seg1 = a.cta_segment[blockIdx.x + 1];
+    const bool unfit = __ldcg(a.words + DG_UNFIT_OPERAND) != 0;   // the whole product will be gathered: no tiles for anybody
+    if (unfit && threadIdx.x == 0) a.words[DG_GATHER_ALL] = 1;
+    const int seg0 = a.cta_segment[blockIdx.x], seg1 = unfit ? seg0 : a.cta_segment[blockIdx.x + 1];
     const int slab0 = seg0 < seg1 ? a.segments[seg0].slab0 : 0, total = seg0 < seg1 ? a.segments[seg1 - 1].slab1 - slab0 : 0;
     const dg_slab* slabs = a.slabs + slab0;
 
@@ -389,7 +397,7 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
                                                     const float* __restrict__ val, const int32_t* __restrict__ row_rank,
                                                     const int32_t* __restrict__ col_rank, int32_t col_tiles, int32_t* __restrict__ tile,
                                                     int32_t* __restrict__ cursor, int32_t* __restrict__ rest, uint2* __restrict__ records,
-                                                    int32_t* __restrict__ rest_col, float* __restrict__ rest_val)
+                                                    int32_t* __restrict__ rest_col, float* __restrict__ rest_val, int* __restrict__ unfit)
 {
     const int32_t c = blockIdx.x * (T / 32) + (threadIdx.x >> 5);
     if (c >= n_chunks) return;
@@ -416,6 +424,7 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
                     if (slab >= 0) {
                         uint32_t h, m, l;
                         split3(v, h, m, l);
+                        if (!(fabsf(v) < kTileBound)) *unfit = 1;
                         records[atomicAdd(cursor + slab, 1)] =
                             make_uint2(h | m << 16, l | (uint32_t)tile_element(rr % kTileRows, cr % kTileCols) << 16);
                     } else {
@@ -539,7 +548,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     SplitRow* d_rows = nullptr;
     int32_t *first_slot = nullptr, *weight = nullptr, *bins = nullptr, *col_rank = nullptr, *row_rank = nullptr;
     int2* frequent = nullptr;
-    const size_t bins_n = kWeightBins + 1;
+    const size_t bins_n = kWeightBins + 2;
     if ((rc = tmp.alloc(&d_rows, p->n_heavy)) || (rc = tmp.alloc(&first_slot, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&weight, p->k)) ||
         (rc = tmp.alloc(&bins, bins_n)) || (rc = tmp.alloc(&col_rank, p->k)) || (rc = tmp.alloc(&row_rank, p->n_heavy)) ||
         (rc = tmp.alloc(&frequent, kMaxColumns)))
@@ -562,7 +571,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     int64_t columns = h_bins[kWeightBins - 1];
     while (least > 1 + kTileMin / kTileCols && columns + h_bins[least - 1] <= kMaxColumns) columns += h_bins[--least];
     if (columns < kTileCols || columns > kMaxColumns) return DG_OK;
-    int32_t* d_count = bins + kWeightBins;
+    int32_t *d_count = bins + kWeightBins, *unfit = d_count + 1;
     k_frequent_columns<<<grid_of(p->k, T), T, 0, stream>>>(weight, p->k, least, frequent, kMaxColumns, d_count);
     std::vector<int2> h_frequent((size_t)columns);
     DG_CUDA(cudaMemcpyAsync(h_frequent.data(), frequent, h_frequent.size() * sizeof(int2), cudaMemcpyDeviceToHost, stream));
@@ -587,7 +596,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     k_column_ranks<<<grid_of(columns, T), T, 0, stream>>>(t->columns, t->n_columns, col_rank);
     DG_CUDA(cudaMemsetAsync(tile, 0, (size_t)tiles * sizeof(int32_t), stream));
     const unsigned warps = grid_of(p->n_chunks, T / 32);
-    k_tile_entries<0><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, nullptr, nullptr, nullptr, nullptr, nullptr);
+    k_tile_entries<0><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     std::vector<int32_t> h_tile((size_t)tiles);
     DG_CUDA(cudaMemcpyAsync(h_tile.data(), tile, h_tile.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
     DG_CUDA(cudaStreamSynchronize(stream));
@@ -642,7 +651,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     if ((rc = tmp.alloc(&cursor, slabs.size()))) return rc;
     DG_CUDA(cudaMemcpyAsync(tile, h_tile.data(), h_tile.size() * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
     DG_CUDA(cudaMemcpyAsync(cursor, h_cursor.data(), h_cursor.size() * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-    k_tile_entries<1><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, nullptr, rest, nullptr, nullptr, nullptr);
+    k_tile_entries<1><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, nullptr, rest, nullptr, nullptr, nullptr, nullptr);
     k_exclusive_sums<<<1, 1024, 0, stream>>>(rest, p->n_chunks);
     int32_t h_rest = 0;
     DG_CUDA(cudaMemcpyAsync(&h_rest, rest + p->n_chunks, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
@@ -654,7 +663,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
         (rc = upload(&t->segments, segments, stream)) || (rc = upload(&t->cta_segment, cta_segment, stream)) || (rc = upload(&t->parts, parts, stream)))
         return rc;
     k_tile_entries<2><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, cursor, rest, t->records, t->rest_col,
-                                               t->rest_val);
+                                               t->rest_val, unfit);
     // chunks of the rest, in the order of the column band they start in
     int32_t *chunk_first = nullptr, *bands = nullptr;
     if ((rc = tmp.alloc(&chunk_first, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&bands, kBands + 1))) return rc;
@@ -668,8 +677,11 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     DG_CUDA(cudaStreamSynchronize(stream));
     if ((rc = dg_pool_alloc((void**)&t->rest_chunks, (size_t)t->n_rest_chunks * sizeof(dg_chunk)))) return rc;
     k_rest_chunks<2><<<row_blocks, T, 0, stream>>>(d_rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, t->rest_chunks);
+    int h_unfit = 0;
+    DG_CUDA(cudaMemcpyAsync(&h_unfit, unfit, sizeof(int), cudaMemcpyDeviceToHost, stream));
     DG_CUDA(cudaStreamSynchronize(stream));
     DG_CUDA(cudaGetLastError());
+    if (h_unfit) return DG_OK;                                    // an infinity, a NaN or a huge value among them
     t->val = val;
     t->n_slabs = (int32_t)slabs.size();
     t->n_segments = (int32_t)segments.size();
@@ -748,8 +760,8 @@ int dg_tiles_launch(const dg_plan* p, const float* B, int64_t ldb, int32_t F, fl
     const dg_tiles* t = p->tiles;
     const int32_t F4 = (F + 3) / 4, panels = panels_of(F), n_pad = panel_width(F);
     uint16_t* images = reinterpret_cast<uint16_t*>(area + (int64_t)t->n_segments * kTileRows * F4 * 4);
-    k_tile_columns<<<dim3((unsigned)t->col_tiles, (unsigned)panels), T, 0, stream>>>(B, ldb, t->columns, t->n_columns, t->col_tiles, F, n_pad, images);
-    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, wait_limit};
+    k_tile_columns<<<dim3((unsigned)t->col_tiles, (unsigned)panels), T, 0, stream>>>(B, ldb, t->columns, t->n_columns, t->col_tiles, F, n_pad, images, p->status + DG_TILE_WORDS);
+    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, p->status + DG_TILE_WORDS, wait_limit};
     const size_t smem = kTileStages * (3 * kTileElems * 2 + (size_t)3 * n_pad * kTileCols * 2) + 24 * kTileStages + 32 + 128;
     static std::atomic<bool> allowed[64];
     if (p->device < 0 || p->device >= 64) return DG_ERR_STATE;

@@ -1,4 +1,11 @@
 // Dense tiles of a sparse block (dg_tiles.cu): the part of a plan's entries that the tensor cores multiply.
+//
+// A dense tile multiplies its zeros too, and values and operand are cut into bf16 pieces.  Both are right for numbers of a size whose
+// products cannot overflow; an infinity, a NaN or a number beyond kTileBound would reach rows that have no entry there, or turn an
+// infinity into NaN.  So values like that get no tiles, and an operand like that has its whole product gathered: k_tile_columns,
+// which reads every element the tiles use, sets the plan's word DG_UNFIT_OPERAND; k_tile_mma then sets DG_GATHER_ALL, which
+// k_tile_columns cleared, and does nothing else; k_spmm reads DG_GATHER_ALL and clears the other.  Each word is written by one
+// kernel of the three and read by a later one, so that captured graphs can be replayed.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>

@@ -74,7 +74,9 @@ int dg_plan_destroy(dg_plan* plan);
  * (six bf16 passes on three-piece splits: fp32 accuracy).  A one-off step for a block that will be multiplied many times: it
  * makes a second copy of the split rows' entries (8 bytes each) WITH their values `val`; products with another `val` pointer
  * are gathered as before, and a caller that changes the values in place calls this again or dg_plan_drop_tiles.  Returns
- * DG_OK without doing anything where the block has too few dense tiles.  Synchronises `stream`; no product on the plan may be
+ * DG_OK without doing anything where the block has too few dense tiles, or a value of 2^63 or more, an infinity or a NaN among
+ * them.  A product whose operand holds such an element in a column of the tiles is gathered whole, with the bits of a plan
+ * without tiles: the device finds out, at no wait.  Synchronises `stream`; no product on the plan may be
  * in flight.  dg_plan_tiled_entries: how many entries the tensor cores take (0: no tiles).  Where it fails, for lack of memory
  * (cudaErrorMemoryAllocation) or otherwise, the plan is as it was without tiles; a plan whose scratch finds no memory drops them. */
 int dg_plan_add_tiles(dg_plan* plan, const float* val, void* stream);

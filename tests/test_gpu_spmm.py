@@ -611,3 +611,43 @@ def test_tile_kernel_that_gives_up_is_noticed():
     assert fresh.device_status() == 0
     assert_close(C.cpu().numpy(), plain.spmm(b, torch.empty_like(C), 1.0, 0.0).cpu().numpy(), TOL / 10, 'after a kernel that gave up')
     assert spmm_cpp.lib().dg_tiles_wait_selftest(plain.handle, b.data_ptr(), 256, 256, None) == -5
+
+
+@pytest.mark.parametrize('bad', [float('inf'), float('-inf'), float('nan'), 3.4e38, 1e19])
+@pytest.mark.parametrize('F', [41, 100, 256, 300])
+def test_tiles_leave_rows_alone_that_have_no_entry_in_a_column(F, bad):
+    """Infinities, NaN and numbers near the largest in the row of B of the most frequent column (and of the rarest): the bits of
+    a plan without tiles, in every row; and tiles again for the next, ordinary operand."""
+    A = skewed_block(13)
+    plan, plain = tiled_plan(A), make_plan(A)
+    assert plan.tiled_entries() > 0
+    count = np.bincount(A.col, minlength=2600)
+    b = torch.randn(2600, F, device='cuda', generator=torch.Generator(device='cuda').manual_seed(F))
+    usual = plan.spmm(b, torch.empty(3001, F, device='cuda'), 1.0, 0.0)
+    for column in (int(count.argmax()), int(count.argmin())):
+        x = b.clone()
+        x[column, F - 1] = bad
+        for alpha, beta in ((1.0, 0.0), (1.0, 1.0)):
+            C = torch.ones(3001, F, device='cuda')
+            got, want = plan.spmm(x, C.clone(), alpha, beta).cpu().numpy(), plain.spmm(x, C.clone(), alpha, beta).cpu().numpy()
+            if column == int(count.argmax()):
+                assert np.array_equal(got, want, equal_nan=True)
+            else:
+                assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+        if not np.isfinite(bad):
+            touched = np.unique(A.row[A.col == column])
+            assert np.isfinite(np.delete(got, touched, 0)).all() and not np.isfinite(got[touched, F - 1]).any()
+        assert plan.device_status() == 0
+    assert torch.equal(plan.spmm(b, torch.empty_like(usual), 1.0, 0.0), usual)
+
+
+@pytest.mark.parametrize('bad', [float('inf'), float('nan'), 1e19])
+def test_values_that_cannot_be_cut_get_no_tiles(bad):
+    A = skewed_block(14)
+    longest, widest = np.bincount(A.row).argmax(), np.bincount(A.col).argmax()
+    A.val[np.flatnonzero((A.row == longest))[0]] = bad
+    A.val[np.flatnonzero((A.col == widest))[:50]] = bad
+    plan = tiled_plan(A)
+    assert plan.tiled_entries() == 0
+    b = torch.randn(2600, 64, device='cuda')
+    assert torch.equal(plan.spmm(b, torch.zeros(3001, 64, device='cuda'), 1.0, 0.0).isnan(), make_plan(A).spmm(b, torch.zeros(3001, 64, device='cuda'), 1.0, 0.0).isnan())

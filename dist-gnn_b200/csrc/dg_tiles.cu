@@ -38,7 +38,8 @@ constexpr int kMaxColumns = 1 << 16;      // frequent columns considered, at mos
 constexpr float kTileBound = 9.2233720e18f;     // 2^63: a product of two smaller numbers is finite, with a factor of 4 to spare for sums
 constexpr int kFlushSlabs = 16;
 constexpr int kTileStages = 3;
-constexpr int kScatterThreads = 256, kGroupThreads = 128, kTileThreads = kScatterThreads + 64;
+constexpr int kValueWarps = 4;            // of every CTA, to see whether the values are still those of the tiles
+constexpr int kScatterThreads = 256, kGroupThreads = 128, kTileThreads = kScatterThreads + 64 + 32 * kValueWarps;
 constexpr int kAhead = 8;                 // records a thread holds for its group's next tile
 constexpr int T = 256;
 constexpr int kBands = 4096;
@@ -78,6 +79,56 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
+// What a warp remembers of its share of the values, in fours: the sum modulo 2^64 of products of pairs, every value shifted by a key
+// that depends on its place, and the plain sum modulo 2^32.  One changed value always shows (in the second sum where its partner
+// is zero), several do but for one chance in some 2^32 a share.  Nine instructions for four values: hashing every one by itself
+// cost the MMAs beside it twice as much.
+struct ValueSum {
+    unsigned long long pairs;
+    uint32_t plain, pad;
+};
+__device__ __forceinline__ void add_values(ValueSum& sum, uint4 x, uint32_t at)
+{
+    const uint32_t key = at * 0x9E3779B1u, a = x.x + key, b = x.y + key + 0x85EBCA6Bu, c = x.z + key + 0xC2B2AE35u, d = x.w + key + 0x27D4EB2Fu;
+    sum.pairs += (unsigned long long)a * b;
+    sum.pairs += (unsigned long long)c * d;
+    sum.plain += a + b + c + d;
+}
+__device__ __forceinline__ ValueSum value_sum(const float* __restrict__ val, int64_t nnz, int share, int shares)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t fours = (nnz + 3) / 4, per = (fours + shares - 1) / shares, end = min(fours, (share + 1) * per);
+    int64_t i = min(fours, share * per);
+    ValueSum sum{};
+    if ((reinterpret_cast<uintptr_t>(val) & 15) == 0) {
+        constexpr int kInFlight = 8;
+        for (; i + 32 * kInFlight <= min(end, nnz / 4); i += 32 * kInFlight) {
+            uint4 x[kInFlight];
+#pragma unroll
+            for (int j = 0; j < kInFlight; ++j) x[j] = __ldcs(reinterpret_cast<const uint4*>(val) + i + j * 32 + lane);
+#pragma unroll
+            for (int j = 0; j < kInFlight; ++j) add_values(sum, x[j], (uint32_t)i + j * 32 + lane);
+        }
+    }
+    for (i += lane; i < end; i += 32) {
+        uint32_t x[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = 4 * i + j < nnz ? __float_as_uint(__ldcs(val + 4 * i + j)) : 0u;
+        add_values(sum, make_uint4(x[0], x[1], x[2], x[3]), (uint32_t)i);
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        sum.pairs += __shfl_xor_sync(0xffffffffu, sum.pairs, off);
+        sum.plain += __shfl_xor_sync(0xffffffffu, sum.plain, off);
+    }
+    return sum;
+}
+__global__ void __launch_bounds__(32 * kValueWarps) k_value_sums(const float* __restrict__ val, int64_t nnz, ValueSum* __restrict__ sums)
+{
+    const int share = blockIdx.x * kValueWarps + (threadIdx.x >> 5);
+    const ValueSum sum = value_sum(val, nnz, share, gridDim.x * kValueWarps);
+    if ((threadIdx.x & 31) == 0) sums[share] = sum;
+}
+
 // Slab images of B: [panel][column tile][piece][k octet][n][8] bf16.  One thread makes one 16-byte octet of all three pieces.
 __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B, int64_t ldb, const int32_t* __restrict__ columns, int32_t n_columns,
                                                     int32_t col_tiles, int32_t F, int32_t n_pad, uint16_t* __restrict__ out, int* __restrict__ words)
@@ -115,10 +166,15 @@ struct TileArgs {
     int *status, *device_status;          // the plan's word and the device's
     int* words;                           // dg_plan::status + DG_TILE_WORDS
     int wait_limit;                       // polls of a wait
+    const float* val;                     // the matrix's values, nnz of them, and what the tiles remember of them
+    const ValueSum* value_sums;
+    int64_t nnz;
 };
 
 // blockIdx.x: the CTA's share of the tiles, blockIdx.y: panel of n_pad columns.  Warps 0-3 and 4-7: the two scatter groups
-// (group g fills tiles g, g + 2, ... and drains the 16-column pieces g, g + 2, ... of the accumulators), 8: copies, 9: MMA issue.
+// (group g fills tiles g, g + 2, ... and drains the 16-column pieces g, g + 2, ... of the accumulators), 8: copies, 9: MMA issue, the
+// others see whether the values are still those of the tiles (beside the MMAs, which leave DRAM alone: 504 MB, F = 256 548 -> 579 us,
+// F = 48 321 -> 338; the pass alone would be 77 us.  Half as many warps: 30 to 60 us longer where the tiles are few).
 //
 // A group drains a finished run of tiles two or three tiles after its end, so that the tiles of the next run are being
 // filled meanwhile.  Why nothing deadlocks: filling tile t waits for the MMAs of tile t - 3 (its stage), those of t - 3 wait
@@ -223,6 +279,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
                 }
             }
             await_mmas(done);
+        }
+    } else if (warp > 9) {
+        const int share = blockIdx.x * kValueWarps + warp - 10;
+        if (blockIdx.y == 0 && !unfit) {
+            const ValueSum sum = value_sum(a.val, a.nnz, share, gridDim.x * kValueWarps), then = a.value_sums[share];
+            if (lane == 0 && (sum.pairs != then.pairs || sum.plain != then.plain)) a.words[DG_GATHER_ALL] = 1;
         }
     } else {
         const int group = warp >> 2, q = warp & 3, tid = threadIdx.x & (kGroupThreads - 1);
@@ -677,6 +739,8 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     DG_CUDA(cudaStreamSynchronize(stream));
     if ((rc = dg_pool_alloc((void**)&t->rest_chunks, (size_t)t->n_rest_chunks * sizeof(dg_chunk)))) return rc;
     k_rest_chunks<2><<<row_blocks, T, 0, stream>>>(d_rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, t->rest_chunks);
+    if ((rc = dg_pool_alloc(&t->value_sums, (size_t)t->ctas * kValueWarps * sizeof(ValueSum)))) return rc;
+    k_value_sums<<<t->ctas, 32 * kValueWarps, 0, stream>>>(val, p->nnz, static_cast<ValueSum*>(t->value_sums));
     int h_unfit = 0;
     DG_CUDA(cudaMemcpyAsync(&h_unfit, unfit, sizeof(int), cudaMemcpyDeviceToHost, stream));
     DG_CUDA(cudaStreamSynchronize(stream));
@@ -695,7 +759,7 @@ void dg_tiles_free(dg_tiles* t)
 {
     if (!t) return;
     for (void* b : {(void*)t->records, (void*)t->slabs, (void*)t->segments, (void*)t->cta_segment, (void*)t->columns, (void*)t->parts, (void*)t->rest_col,
-                    (void*)t->rest_val, (void*)t->rest_chunks})
+                    (void*)t->rest_val, (void*)t->rest_chunks, t->value_sums})
         dg_pool_free(b);
     delete t;
 }
@@ -761,7 +825,7 @@ int dg_tiles_launch(const dg_plan* p, const float* B, int64_t ldb, int32_t F, fl
     const int32_t F4 = (F + 3) / 4, panels = panels_of(F), n_pad = panel_width(F);
     uint16_t* images = reinterpret_cast<uint16_t*>(area + (int64_t)t->n_segments * kTileRows * F4 * 4);
     k_tile_columns<<<dim3((unsigned)t->col_tiles, (unsigned)panels), T, 0, stream>>>(B, ldb, t->columns, t->n_columns, t->col_tiles, F, n_pad, images, p->status + DG_TILE_WORDS);
-    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, p->status + DG_TILE_WORDS, wait_limit};
+    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, p->status + DG_TILE_WORDS, wait_limit, t->val, static_cast<const ValueSum*>(t->value_sums), p->nnz};
     const size_t smem = kTileStages * (3 * kTileElems * 2 + (size_t)3 * n_pad * kTileCols * 2) + 24 * kTileStages + 32 + 128;
     static std::atomic<bool> allowed[64];
     if (p->device < 0 || p->device >= 64) return DG_ERR_STATE;

@@ -6,6 +6,9 @@
 // which reads every element the tiles use, sets the plan's word DG_UNFIT_OPERAND; k_tile_mma then sets DG_GATHER_ALL, which
 // k_tile_columns cleared, and does nothing else; k_spmm reads DG_GATHER_ALL and clears the other.  Each word is written by one
 // kernel of the three and read by a later one, so that captured graphs can be replayed.
+//
+// The tiles hold copies of the values.  k_tile_mma compares the values of every product with what they were then, and sets
+// DG_GATHER_ALL where they differ: a product never uses others than those in front of it.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -20,7 +23,8 @@ struct dg_segment {         // consecutive slabs of one row tile that one CTA mu
 };
 
 struct dg_tiles {
-    const float* val;             // the values the records were made from: products with other values do not use the tiles
+    const float* val;             // where the values lay that the records were made from: products with others do not use the tiles
+    void* value_sums;             // what they were: sums, a record per checking warp
     int64_t entries;              // entries in tiles
     int32_t n_slabs, n_segments, n_columns, col_tiles, ctas;
     uint2* records;               // [entries] three bf16 pieces of the value and the position in the tile

@@ -254,8 +254,9 @@ class SpmmPlan:
     def tile(self):
         """Moves the densest part of the block to the tensor cores for the products to come (dg_plan_add_tiles): worth its few
         milliseconds for a block that is multiplied again and again, and done where it pays (at least TILE_NNZ entries, enough
-        of them in dense tiles).  The tiles hold the values as they are now; changing them in place afterwards is noticed by
-        the tensor's version counter, and the products then gather everything again."""
+        of them in dense tiles).  The tiles hold the values as they are now.  Changing them in place afterwards drops the tiles;
+        a change that the tensor's version counter does not see (through .data, by a kernel of the caller's) is found by the
+        products themselves, which then gather everything, at the price of the tiles that they did not use."""
         if self.values.numel() >= TILE_NNZ and self._tiled is None:
             index = self.device.index
             with _on(index):

@@ -73,7 +73,8 @@ int dg_plan_destroy(dg_plan* plan);
 /* Lets products on this plan multiply the densest part of the block - long rows x frequent columns - on the tensor cores
  * (six bf16 passes on three-piece splits: fp32 accuracy).  A one-off step for a block that will be multiplied many times: it
  * makes a second copy of the split rows' entries (8 bytes each) WITH their values `val`; products with another `val` pointer
- * are gathered as before, and a caller that changes the values in place calls this again or dg_plan_drop_tiles.  Returns
+ * are gathered as before, and so is one whose values have been changed in place (the device compares them).  That product pays for
+ * the tiles without using them: a caller that changes values calls this again, or dg_plan_drop_tiles.  Returns
  * DG_OK without doing anything where the block has too few dense tiles, or a value of 2^63 or more, an infinity or a NaN among
  * them.  A product whose operand holds such an element in a column of the tiles is gathered whole, with the bits of a plan
  * without tiles: the device finds out, at no wait.  Synchronises `stream`; no product on the plan may be

@@ -651,3 +651,31 @@ def test_values_that_cannot_be_cut_get_no_tiles(bad):
     assert plan.tiled_entries() == 0
     b = torch.randn(2600, 64, device='cuda')
     assert torch.equal(plan.spmm(b, torch.zeros(3001, 64, device='cuda'), 1.0, 0.0).isnan(), make_plan(A).spmm(b, torch.zeros(3001, 64, device='cuda'), 1.0, 0.0).isnan())
+
+
+@pytest.mark.parametrize('offset', [0, 1])
+def test_values_changed_behind_the_plan(offset):
+    """Values written through .data, one at a time and all of them, at every alignment: every product reads those in front of it."""
+    import spmm_cpp
+    A = skewed_block(15)
+    values = torch.empty(A.nnz + 4, device='cuda')[offset:offset + A.nnz]
+    values.copy_(dev(A.val))
+    keep = spmm_cpp.TILE_NNZ
+    try:
+        spmm_cpp.TILE_NNZ = 0
+        plan = spmm_cpp.SpmmPlan(dev(A.row, torch.int32), dev(A.col, torch.int32), values, *A.shape).tile()
+    finally:
+        spmm_cpp.TILE_NNZ = keep
+    assert plan.tiled_entries() > 0
+    b = torch.randn(2600, 256, device='cuda')
+    product = lambda p, **kw: p.spmm(b, torch.zeros(3001, 256, device='cuda'), 1.0, 0.0, **kw)
+    usual = product(plan)
+    for at in (0, 1, A.nnz // 2, A.nnz - 2, A.nnz - 1):
+        kept = float(values[at])
+        plan.values.data[at] = kept + 1.0
+        assert plan.tiled_entries() > 0
+        assert torch.equal(product(plan), product(make_plan(A), values=plan.values.clone()))
+        plan.values.data[at] = kept
+        assert torch.equal(product(plan), usual)                   # the tiles' values again
+    plan.values.data.mul_(2.0)
+    assert torch.equal(product(plan), product(make_plan(A), values=plan.values.clone()))

@@ -41,7 +41,7 @@ struct dg_split_row {
 
 #define DG_STATUS_WORDS 4
 #define DG_TILE_WORDS 2           // from here: whether the product under way may use its tiles (dg_tiles.h)
-#define DG_UNFIT_OPERAND 0
+#define DG_LARGEST_ELEMENT 0
 #define DG_GATHER_ALL 1
 
 struct dg_tiles;      // dg_tiles.h

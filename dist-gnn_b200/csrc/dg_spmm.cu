@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
             if constexpr (WHOLE) {
                 if (!whole) return;
             } else {
-                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.tile_words[DG_UNFIT_OPERAND] = 0;      // for the next product
+                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.tile_words[DG_LARGEST_ELEMENT] = 0;      // for the next product
                 if (whole && (int)blockIdx.x < chunk_ctas) return;
             }
         }

@@ -36,6 +36,15 @@ constexpr int kTileElems = kTileRows * kTileCols;
 constexpr int kTileMin = 160;             // entries from which a tile is worth multiplying
 constexpr int kMaxColumns = 1 << 16;      // frequent columns considered, at most
 constexpr float kTileBound = 9.2233720e18f;     // 2^63: a product of two smaller numbers is finite, with a factor of 4 to spare for sums
+// The small pieces of numbers far below this fall under the smallest bf16 and the products under the smallest fp32: an operand, or a
+// product of value and operand, that is nowhere larger loses bits (error against float64, whole operand at 2^-110 1.2e-7, at 2^-115
+// 9e-7, at 2^-120 2.8e-5; gathered 1.5e-7).  Small elements beside larger ones do no harm.
+constexpr float kTileLeast = 7.8886091e-31f;    // 2^-100
+// `largest`: bits of the largest magnitude, ordered as the numbers are with infinities and NaN above them
+__device__ __forceinline__ bool unfit_operand(int largest, float least)
+{
+    return largest >= __float_as_int(kTileBound) || (largest > 0 && largest < __float_as_int(least));
+}
 constexpr int kFlushSlabs = 16;
 constexpr int kTileStages = 3;
 constexpr int kValueWarps = 4;            // of every CTA, to see whether the values are still those of the tiles
@@ -134,7 +143,9 @@ __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B,
                                                     int32_t col_tiles, int32_t F, int32_t n_pad, uint16_t* __restrict__ out, int* __restrict__ words)
 {
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) words[DG_GATHER_ALL] = 0;
-    bool fit = true;
+    __shared__ int block_largest;
+    if (threadIdx.x == 0) block_largest = 0;
+    int largest = 0;
     uint16_t* image = out + ((int64_t)blockIdx.y * col_tiles + blockIdx.x) * 3 * n_pad * kTileCols;
     for (int i = threadIdx.x; i < n_pad * (kTileCols / 8); i += T) {
         const int n = i % n_pad, octet = i / n_pad, f = blockIdx.y * n_pad + n;
@@ -143,7 +154,7 @@ __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B,
         for (int j = 0; j < 8; ++j) {
             const int k = blockIdx.x * kTileCols + octet * 8 + j;
             const float x = k < n_columns && f < F ? __ldg(B + (int64_t)__ldg(columns + k) * ldb + f) : 0.f;
-            fit = fit && fabsf(x) < kTileBound;                   // not so for a NaN
+            largest = max(largest, __float_as_int(fabsf(x)));
             split3(x, h[j], m[j], l[j]);
         }
         uint4* at = reinterpret_cast<uint4*>(image) + octet * n_pad + n;
@@ -152,7 +163,11 @@ __global__ void __launch_bounds__(T) k_tile_columns(const float* __restrict__ B,
         at[piece] = make_uint4(m[0] | m[1] << 16, m[2] | m[3] << 16, m[4] | m[5] << 16, m[6] | m[7] << 16);
         at[2 * piece] = make_uint4(l[0] | l[1] << 16, l[2] | l[3] << 16, l[4] | l[5] << 16, l[6] | l[7] << 16);
     }
-    if (!fit) words[DG_UNFIT_OPERAND] = 1;
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) atomicMax(&block_largest, largest);
+    __syncthreads();
+    if (threadIdx.x == 0 && block_largest > __ldcg(words + DG_LARGEST_ELEMENT)) atomicMax(words + DG_LARGEST_ELEMENT, block_largest);
 }
 
 struct TileArgs {
@@ -164,6 +179,7 @@ struct TileArgs {
     float4* partial;                      // [slot][ld4][128]
     int32_t ld4, F4, n_pad, col_tiles;    // 16-byte pieces of a partial row; of those, how many are wanted
     int *status, *device_status;          // the plan's word and the device's
+    float least;                          // an operand without any element of this size is too small
     int* words;                           // dg_plan::status + DG_TILE_WORDS
     int wait_limit;                       // polls of a wait
     const float* val;                     // the matrix's values, nnz of them, and what the tiles remember of them
@@ -216,7 +232,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_mma(const TileArgs a)
     const uint32_t tmem = *tmem_slot, acc_small = tmem + 256;
     bool ok = true;
 
-    const bool unfit = __ldcg(a.words + DG_UNFIT_OPERAND) != 0;   // the whole product will be gathered: no tiles for anybody
+    const bool unfit = unfit_operand(__ldcg(a.words + DG_LARGEST_ELEMENT), a.least);   // the whole product will be gathered: no tiles for anybody
     if (unfit && threadIdx.x == 0) a.words[DG_GATHER_ALL] = 1;
     const int seg0 = a.cta_segment[blockIdx.x], seg1 = unfit ? seg0 : a.cta_segment[blockIdx.x + 1];
     const int slab0 = seg0 < seg1 ? a.segments[seg0].slab0 : 0, total = seg0 < seg1 ? a.segments[seg1 - 1].slab1 - slab0 : 0;
@@ -459,7 +475,7 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
                                                     const float* __restrict__ val, const int32_t* __restrict__ row_rank,
                                                     const int32_t* __restrict__ col_rank, int32_t col_tiles, int32_t* __restrict__ tile,
                                                     int32_t* __restrict__ cursor, int32_t* __restrict__ rest, uint2* __restrict__ records,
-                                                    int32_t* __restrict__ rest_col, float* __restrict__ rest_val, int* __restrict__ unfit)
+                                                    int32_t* __restrict__ rest_col, float* __restrict__ rest_val, int* __restrict__ largest)
 {
     const int32_t c = blockIdx.x * (T / 32) + (threadIdx.x >> 5);
     if (c >= n_chunks) return;
@@ -468,6 +484,7 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
     const int32_t rr = row_rank[ch.heavy];
     int32_t* row_tile = tile + (int64_t)(rr / kTileRows) * col_tiles;
     int32_t left = MODE == 2 ? rest[ch.slot] : 0;
+    int biggest = 0;
     for (int base = 0; base < ch.len; base += 32) {
         const bool valid = base + lane < ch.len;
         int32_t cc = 0, cr = -1;
@@ -486,7 +503,7 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
                     if (slab >= 0) {
                         uint32_t h, m, l;
                         split3(v, h, m, l);
-                        if (!(fabsf(v) < kTileBound)) *unfit = 1;
+                        biggest = max(biggest, __float_as_int(fabsf(v)));       // ordered as the numbers are, a NaN above them
                         records[atomicAdd(cursor + slab, 1)] =
                             make_uint2(h | m << 16, l | (uint32_t)tile_element(rr % kTileRows, cr % kTileCols) << 16);
                     } else {
@@ -500,6 +517,10 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
         }
     }
     if (MODE == 1 && lane == 0) rest[ch.slot] = left;
+    if (MODE == 2) {
+        biggest = __reduce_max_sync(0xffffffffu, biggest);
+        if (lane == 0 && biggest > *(volatile int*)largest) atomicMax(largest, biggest);
+    }
 }
 
 // Exclusive sums in place, one CTA; the total goes behind the last element.
@@ -633,7 +654,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     int64_t columns = h_bins[kWeightBins - 1];
     while (least > 1 + kTileMin / kTileCols && columns + h_bins[least - 1] <= kMaxColumns) columns += h_bins[--least];
     if (columns < kTileCols || columns > kMaxColumns) return DG_OK;
-    int32_t *d_count = bins + kWeightBins, *unfit = d_count + 1;
+    int32_t *d_count = bins + kWeightBins, *largest = d_count + 1;
     k_frequent_columns<<<grid_of(p->k, T), T, 0, stream>>>(weight, p->k, least, frequent, kMaxColumns, d_count);
     std::vector<int2> h_frequent((size_t)columns);
     DG_CUDA(cudaMemcpyAsync(h_frequent.data(), frequent, h_frequent.size() * sizeof(int2), cudaMemcpyDeviceToHost, stream));
@@ -725,7 +746,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
         (rc = upload(&t->segments, segments, stream)) || (rc = upload(&t->cta_segment, cta_segment, stream)) || (rc = upload(&t->parts, parts, stream)))
         return rc;
     k_tile_entries<2><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, cursor, rest, t->records, t->rest_col,
-                                               t->rest_val, unfit);
+                                               t->rest_val, largest);
     // chunks of the rest, in the order of the column band they start in
     int32_t *chunk_first = nullptr, *bands = nullptr;
     if ((rc = tmp.alloc(&chunk_first, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&bands, kBands + 1))) return rc;
@@ -741,11 +762,12 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     k_rest_chunks<2><<<row_blocks, T, 0, stream>>>(d_rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, t->rest_chunks);
     if ((rc = dg_pool_alloc(&t->value_sums, (size_t)t->ctas * kValueWarps * sizeof(ValueSum)))) return rc;
     k_value_sums<<<t->ctas, 32 * kValueWarps, 0, stream>>>(val, p->nnz, static_cast<ValueSum*>(t->value_sums));
-    int h_unfit = 0;
-    DG_CUDA(cudaMemcpyAsync(&h_unfit, unfit, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    float h_largest = 0.f;
+    DG_CUDA(cudaMemcpyAsync(&h_largest, largest, sizeof(float), cudaMemcpyDeviceToHost, stream));
     DG_CUDA(cudaStreamSynchronize(stream));
     DG_CUDA(cudaGetLastError());
-    if (h_unfit) return DG_OK;                                    // an infinity, a NaN or a huge value among them
+    if (!(h_largest < kTileBound) || h_largest < kTileLeast) return DG_OK;
+    t->least_operand = h_largest < 1.f ? kTileLeast / h_largest : kTileLeast;
     t->val = val;
     t->n_slabs = (int32_t)slabs.size();
     t->n_segments = (int32_t)segments.size();
@@ -825,7 +847,7 @@ int dg_tiles_launch(const dg_plan* p, const float* B, int64_t ldb, int32_t F, fl
     const int32_t F4 = (F + 3) / 4, panels = panels_of(F), n_pad = panel_width(F);
     uint16_t* images = reinterpret_cast<uint16_t*>(area + (int64_t)t->n_segments * kTileRows * F4 * 4);
     k_tile_columns<<<dim3((unsigned)t->col_tiles, (unsigned)panels), T, 0, stream>>>(B, ldb, t->columns, t->n_columns, t->col_tiles, F, n_pad, images, p->status + DG_TILE_WORDS);
-    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, p->status + DG_TILE_WORDS, wait_limit, t->val, static_cast<const ValueSum*>(t->value_sums), p->nnz};
+    const TileArgs a{t->slabs, t->segments, t->cta_segment, t->records, images, reinterpret_cast<float4*>(area), F4, F4, n_pad, t->col_tiles, p->status, t->status, t->least_operand, p->status + DG_TILE_WORDS, wait_limit, t->val, static_cast<const ValueSum*>(t->value_sums), p->nnz};
     const size_t smem = kTileStages * (3 * kTileElems * 2 + (size_t)3 * n_pad * kTileCols * 2) + 24 * kTileStages + 32 + 128;
     static std::atomic<bool> allowed[64];
     if (p->device < 0 || p->device >= 64) return DG_ERR_STATE;

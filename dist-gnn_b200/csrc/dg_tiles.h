@@ -1,11 +1,12 @@
 // Dense tiles of a sparse block (dg_tiles.cu): the part of a plan's entries that the tensor cores multiply.
 //
-// A dense tile multiplies its zeros too, and values and operand are cut into bf16 pieces.  Both are right for numbers of a size whose
-// products cannot overflow; an infinity, a NaN or a number beyond kTileBound would reach rows that have no entry there, or turn an
-// infinity into NaN.  So values like that get no tiles, and an operand like that has its whole product gathered: k_tile_columns,
-// which reads every element the tiles use, sets the plan's word DG_UNFIT_OPERAND; k_tile_mma then sets DG_GATHER_ALL, which
-// k_tile_columns cleared, and does nothing else; k_spmm reads DG_GATHER_ALL and clears the other.  Each word is written by one
-// kernel of the three and read by a later one, so that captured graphs can be replayed.
+// A dense tile multiplies its zeros too, and values and operand are cut into bf16 pieces.  Both are right for numbers of a size
+// whose products neither overflow nor vanish; an infinity, a NaN or a number beyond kTileBound would reach rows that have no entry
+// there, or turn an infinity into NaN, and numbers that are all below kTileLeast lose bits.  So values like that get no tiles,
+// and an operand like that has its whole product gathered: k_tile_columns, which reads every element the tiles use, leaves the
+// largest in the plan's word DG_LARGEST_ELEMENT; where that does not fit, k_tile_mma sets DG_GATHER_ALL, which k_tile_columns
+// cleared, and does nothing else; k_spmm reads DG_GATHER_ALL and clears the other.  Each word is written by one kernel of the
+// three and read by a later one, so that captured graphs can be replayed.
 //
 // The tiles hold copies of the values.  k_tile_mma compares the values of every product with what they were then, and sets
 // DG_GATHER_ALL where they differ: a product never uses others than those in front of it.
@@ -25,6 +26,7 @@ struct dg_segment {         // consecutive slabs of one row tile that one CTA mu
 struct dg_tiles {
     const float* val;             // where the values lay that the records were made from: products with others do not use the tiles
     void* value_sums;             // what they were: sums, a record per checking warp
+    float least_operand;          // an operand without any element of this size is too small for the tiles
     int64_t entries;              // entries in tiles
     int32_t n_slabs, n_segments, n_columns, col_tiles, ctas;
     uint2* records;               // [entries] three bf16 pieces of the value and the position in the tile

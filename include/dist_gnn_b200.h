@@ -76,8 +76,9 @@ int dg_plan_destroy(dg_plan* plan);
  * are gathered as before, and so is one whose values have been changed in place (the device compares them).  That product pays for
  * the tiles without using them: a caller that changes values calls this again, or dg_plan_drop_tiles.  Returns
  * DG_OK without doing anything where the block has too few dense tiles, or a value of 2^63 or more, an infinity or a NaN among
- * them.  A product whose operand holds such an element in a column of the tiles is gathered whole, with the bits of a plan
- * without tiles: the device finds out, at no wait.  Synchronises `stream`; no product on the plan may be
+ * them, or none of 2^-100.  A product whose operand holds such an element in a column of the tiles, or only elements under 2^-100
+ * (under 2^-100 over the largest value, if that is below 1), is gathered whole, with the bits of a plan without tiles: the device
+ * finds out, at no wait.  Synchronises `stream`; no product on the plan may be
  * in flight.  dg_plan_tiled_entries: how many entries the tensor cores take (0: no tiles).  Where it fails, for lack of memory
  * (cudaErrorMemoryAllocation) or otherwise, the plan is as it was without tiles; a plan whose scratch finds no memory drops them. */
 int dg_plan_add_tiles(dg_plan* plan, const float* val, void* stream);

@@ -679,3 +679,20 @@ def test_values_changed_behind_the_plan(offset):
         assert torch.equal(product(plan), usual)                   # the tiles' values again
     plan.values.data.mul_(2.0)
     assert torch.equal(product(plan), product(make_plan(A), values=plan.values.clone()))
+
+
+@pytest.mark.parametrize('value_exponent,operand_exponent', [(0, -95), (0, -105), (0, -130), (-40, -55), (-50, -60), (-99, 0), (-105, 0), (60, -99)])
+def test_tiles_of_small_numbers_are_as_exact_as_gathering(value_exponent, operand_exponent):
+    """Whole operands and values down to the smallest normal numbers: the same error against float64 as without tiles."""
+    A = skewed_block(16)
+    A.val *= np.float32(2.0 ** value_exponent)
+    plan, plain = tiled_plan(A), make_plan(A)
+    assert (plan.tiled_entries() > 0) == (value_exponent > -100)
+    b = torch.randn(2600, 64, device='cuda', generator=torch.Generator(device='cuda').manual_seed(1)) * 2.0 ** operand_exponent
+    b[5] = 0.0
+    dense = torch.zeros(3001, 2600, dtype=torch.float64, device='cuda')
+    dense[dev(A.row), dev(A.col)] = dev(A.val).double()
+    want = dense @ b.double()
+    err = lambda p: float((p.spmm(b, torch.empty(3001, 64, device='cuda'), 1.0, 0.0).double() - want).norm() / want.norm())
+    assert err(plan) <= 1.5 * err(plain)
+    assert torch.equal(plan.spmm(torch.zeros_like(b), torch.ones_like(b[:1]).repeat(3001, 1), 1.0, 0.0), torch.zeros(3001, 64, device='cuda'))

@@ -16,6 +16,9 @@
 // with 256), and 256 where rows are long on average (dense graph, F = 256: 5.6 ms against 6.3 with 128).
 static inline int32_t dg_default_chunk(int64_t nnz, int32_t m) { return nnz < (1 << 20) ? 64 : nnz < 128 * (int64_t)m ? 128 : 256; }
 
+// What dg_spmm_csr_static holds against its capacity are chunks of this many entries wherever the plan's own lengths are defaults.
+#define DG_STATIC_CHUNK 256
+
 #define DG_FINISH_TILES 16        // column tiles of one launch: arrival counts are kept per split row and tile
 
 // One chunk of a split (heavy) row: entries [e0, e0 + len) of row `row`; its partial sum lands in scratch row `slot`.
@@ -57,6 +60,7 @@ struct dg_plan {
     int* arrived;             // device, n_heavy * DG_FINISH_TILES, zero between products
     int32_t n_chunks, n_heavy;
     int64_t heavy_nnz, max_row_nnz, touched_columns;
+    int64_t static_chunks;    // chunks that count against the static entry's capacity
     float* scratch;           // device, grown on demand by dg_spmm_prepare
     int64_t scratch_floats;
     bool no_padded_copy;      // there was no memory for one
@@ -78,13 +82,13 @@ int dg_spmm_stream_launch(const dg_plan* plan, const float* val, const float* B,
 
 // Launches the product with an explicit scratch area (at least n_chunks x F floats; room for a padded copy of an odd-width
 // operand behind it is used where it is there); shared by the plan-owned and the fixed-scratch entry points.
-// `check` != 0: C stays as it is if that check has failed (row kernels only).
+// `check` != 0: C stays as it is if that check has failed (row kernels only).  `split` false: no row is split, no scratch used.
 int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                    int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
                    float* scratch, int64_t scratch_floats, cudaStream_t stream, int check = 0);
 int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                         int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                        float* scratch, int64_t scratch_floats, cudaStream_t stream, int check = 0);
+                        float* scratch, int64_t scratch_floats, cudaStream_t stream, int check = 0, bool split = true);
 int dg_plan_build_lean(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k, void* stream, dg_plan** out);
 int dg_plan_ensure_tasks(dg_plan* plan, cudaStream_t stream);
 // Device memory of plans (dg_pool.cu), on the current device.  A block may be freed once the device is done with it.

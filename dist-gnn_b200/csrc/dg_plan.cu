@@ -20,7 +20,7 @@ constexpr int kEntriesPerThread = 4;
 constexpr int kBands = 4096;          // column bands the chunks are ordered by
 
 struct PlanCounts {
-    unsigned long long max_row, heavy_nnz, touched;
+    unsigned long long max_row, heavy_nnz, touched, static_chunks;
     int32_t n_heavy, n_chunks;
     int bad;
     int pad;
@@ -101,9 +101,9 @@ __device__ __forceinline__ int2 split_of(const int64_t* rowptr, int32_t i, int32
     return *e1 - *e0 > threshold ? make_int2(1, (int)((*e1 - *e0 + chunk - 1) / chunk)) : make_int2(0, 0);
 }
 
-// Per 256 rows: how many are split, and into how many chunks.
-__global__ void __launch_bounds__(T) k_row_census(const int64_t* __restrict__ rowptr, int32_t m, int32_t threshold, int32_t chunk,
-                                                  int2* __restrict__ block_sums, PlanCounts* __restrict__ counts)
+// Per 256 rows: how many are split, and into how many chunks; over all, how many chunks the static entry counts.
+__global__ void __launch_bounds__(T) k_row_census(const int64_t* __restrict__ rowptr, int32_t m, int32_t threshold, int32_t chunk, int32_t static_threshold,
+                                                  int32_t static_chunk, int2* __restrict__ block_sums, PlanCounts* __restrict__ counts)
 {
     if (counts->bad) return;
     __shared__ int2 sums[T / 32 + 1];
@@ -111,13 +111,16 @@ __global__ void __launch_bounds__(T) k_row_census(const int64_t* __restrict__ ro
     const int2 s = split_of(rowptr, blockIdx.x * T + threadIdx.x, m, threshold, chunk, &e0, &e1);
     block_scan(s, sums);
     unsigned long long deg = (unsigned long long)(e1 - e0), heavy = s.x ? deg : 0;
+    unsigned long long pieces = e1 - e0 > static_threshold ? (unsigned long long)((e1 - e0 + static_chunk - 1) / static_chunk) : 0;
     for (int off = 16; off > 0; off >>= 1) {
         const unsigned long long o = __shfl_xor_sync(0xffffffffu, deg, off);
         deg = o > deg ? o : deg;
         heavy += __shfl_xor_sync(0xffffffffu, heavy, off);
+        pieces += __shfl_xor_sync(0xffffffffu, pieces, off);
     }
     if ((threadIdx.x & 31) == 0 && deg > 0) atomicMax(&counts->max_row, deg);
     if ((threadIdx.x & 31) == 0 && heavy > 0) atomicAdd(&counts->heavy_nnz, heavy);
+    if ((threadIdx.x & 31) == 0 && pieces > 0) atomicAdd(&counts->static_chunks, pieces);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = sums[T / 32];
 }
 
@@ -339,6 +342,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     if (nnz < 0 || m < 0 || k < 0) return DG_ERR_DIMS;
     if (nnz > 0 && (!row || !col || (sizeof(Id) == 8 && !col32))) return DG_ERR_NULL;
     if (nnz > 0 && (m == 0 || k == 0)) return DG_ERR_DIMS;
+    const int32_t static_threshold = heavy_threshold > 0 ? heavy_threshold : DG_STATIC_CHUNK, static_chunk = chunk > 0 ? chunk : DG_STATIC_CHUNK;
     if (heavy_threshold <= 0) heavy_threshold = dg_default_chunk(nnz, m);
     if (chunk <= 0) chunk = dg_default_chunk(nnz, m);
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -381,7 +385,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     k_ingest<Id><<<(unsigned)((nnz + 1 + per_block - 1) / per_block), T, 0, stream>>>(row, col, nnz, m, k, sizeof(Id) == 8 ? col32 : nullptr, p->rowptr,
                                                                                      bitmap, counts);
     if (row_blocks > 0) {
-        k_row_census<<<row_blocks, T, 0, stream>>>(p->rowptr, m, heavy_threshold, chunk, block_sums, counts);
+        k_row_census<<<row_blocks, T, 0, stream>>>(p->rowptr, m, heavy_threshold, chunk, static_threshold, static_chunk, block_sums, counts);
         if (max_chunks > 0) {
             k_scan_blocks<<<1, 1024, 0, stream>>>(block_sums, row_blocks, counts);
             k_emit_chunks<<<row_blocks, T, 0, stream>>>(p->rowptr, m, k, heavy_threshold, chunk, block_sums, p->col, in_row_order, bands, counts);
@@ -402,6 +406,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     p->touched_columns = lean ? (int64_t)k : (int64_t)h.touched;
     p->n_heavy = h.n_heavy;
     p->n_chunks = h.n_chunks;
+    p->static_chunks = (int64_t)h.static_chunks;
     *out = p;
     return DG_OK;
 }

@@ -483,7 +483,7 @@ int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, in
 
 int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                         int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale, const float* bias,
-                        float* scratch, int64_t scratch_floats, cudaStream_t stream, int check)
+                        float* scratch, int64_t scratch_floats, cudaStream_t stream, int check, bool split)
 {
     if (plan->m == 0 || F == 0) return DG_OK;
     SpmmArgs a{};
@@ -492,7 +492,7 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     a.row_scale = row_scale; a.bias = bias; a.chunks = plan->chunks; a.arrived = plan->arrived; a.scratch = scratch;
     a.chunk_col = plan->col; a.chunk_val = val;
     a.ldb = ldb; a.ldc = ldc; a.lds = F; a.m = plan->m; a.F = F;
-    a.heavy_threshold = plan->heavy_threshold; a.n_chunks = plan->n_chunks;
+    a.heavy_threshold = split ? plan->heavy_threshold : INT32_MAX; a.n_chunks = split ? plan->n_chunks : 0;
     // Rows per CTA: as wide a window as still gives every SM a dozen CTAs (wider windows sort better and share their offsets;
     // 64 rows are best at 150 k rows, 128 at 300 k, 256 from 1 M).
     a.rows_per_cta = 32;

@@ -6,8 +6,11 @@
 // time a plan is used at a wider F; this variant never allocates: the partial sums of split (heavy) rows go to a
 // fixed array that is part of the library image, so every GPU that loads the library carries it until the process ends.
 //
-// Limit: DG_STATIC_SCRATCH_FLOATS floats (16 MiB).  A product needs heavy_chunks * F floats of scratch
-// (dg_plan_get_stats gives heavy_chunks); a larger request is refused with DG_ERR_SCRATCH before anything is launched.
+// Limit: DG_STATIC_SCRATCH_FLOATS floats (16 MiB).  A request counts F floats for every chunk of DG_STATIC_CHUNK entries of the
+// rows longer than that (the plan's own lengths where its maker gave any); a larger one is refused with DG_ERR_SCRATCH before anything
+// is launched.  The chunks that plans really have are two to four times as many where their length is a default, so a product within
+// the limit may not fit in one go: it is then done in pieces of its columns, which change no bit of a column's sums, or,
+// where no row is longer than DG_STATIC_CHUNK (or the chunks leave no room for four columns), without splitting rows.
 //
 // Sharing: all calls on a device use the same array.  Nothing in it has to start at zero - every scratch row is fully
 // written by the chunk kernel before the finishing kernel reads it - so no clearing is done between calls, but two
@@ -67,9 +70,17 @@ extern "C" int dg_spmm_csr_static(const dg_plan* plan, const float* val, const f
 {
     int rc = dg_check_spmm_args(plan, val, B, ldb, C, ldc, F, flags, row_scale, bias);   // also checks the current device
     if (rc) return rc;
-    if ((int64_t)plan->n_chunks * F > DG_STATIC_SCRATCH_FLOATS) return DG_ERR_SCRATCH;
+    const int64_t chunks = plan->n_chunks;
+    const bool fits = chunks * F <= DG_STATIC_SCRATCH_FLOATS;
+    if (!fits && plan->static_chunks * F > DG_STATIC_SCRATCH_FLOATS) return DG_ERR_SCRATCH;
     float* scratch = nullptr;
     if ((rc = static_scratch_address(plan->device, &scratch))) return rc;
-    return dg_spmm_launch_rows(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, scratch, (int64_t)plan->n_chunks * F,
-                               (cudaStream_t)stream);
+    const bool split = fits || (plan->max_row_nnz > DG_STATIC_CHUNK && chunks * 4 <= DG_STATIC_SCRATCH_FLOATS);
+    const int32_t piece = fits || !split ? F : (int32_t)(DG_STATIC_SCRATCH_FLOATS / chunks / 4 * 4);
+    for (int32_t c0 = 0; c0 < F && rc == DG_OK; c0 += piece) {
+        const int32_t width = F - c0 < piece ? F - c0 : piece;
+        rc = dg_spmm_launch_rows(plan, val, B ? B + c0 : B, ldb, C + c0, ldc, width, alpha, beta, flags, row_scale, bias ? bias + c0 : bias, scratch,
+                                 split ? chunks * width : 0, (cudaStream_t)stream, 0, split);
+    }
+    return rc;
 }

@@ -129,7 +129,8 @@ int dg_spmm_csr(const dg_plan* plan, const float* val, const float* B, int64_t l
  * a latency-critical loop that must not take the device-wide synchronisation an allocation implies.  Identical
  * arguments and results to dg_spmm_csr, but the partial sums of split rows go to a fixed 16 MiB array inside the
  * library image (held by every GPU that loads the library, shared by all calls on that GPU).  Returns DG_ERR_SCRATCH
- * when heavy_chunks * F exceeds dg_static_scratch_capacity() floats.  Calls that overlap in time on one GPU race on
+ * when chunks * F exceeds dg_static_scratch_capacity() floats, where `chunks` are heavy_chunks or, if fewer, what they would be with
+ * chunks and a threshold of 256 entries in the place of defaults (a product that needs more than one go is done in column pieces).  Calls that overlap in time on one GPU race on
  * the array.  The array is materialised on a device (16 MiB, by the CUDA module loader) the first time its address is
  * resolved there: dg_static_scratch_prepare() does that for the current device and is meant to be called once where an
  * allocation is still acceptable (beside dg_plan_create, before any stream capture); without it the first

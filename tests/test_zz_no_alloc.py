@@ -80,3 +80,29 @@ def test_static_scratch_entry_refuses_requests_beyond_its_capacity():
     B, C = torch.ones(2, 256, device='cuda'), torch.zeros(m, 256, device='cuda')       # exactly at the limit: accepted
     assert _call(L.dg_spmm_csr_static, plan, B, C, 1.0, 0.0) == 0
     assert torch.equal(C.cpu(), torch.full((m, 256), 2.0))
+
+
+@pytest.mark.parametrize('length,rows,width,taken', [(100, 9000, 512, True), (300, 3300, 256, True), (300, 3300, 621, True), (300, 3300, 635, True),
+                                                     (300, 3300, 636, False), (257, 3800, 300, True)])
+def test_static_scratch_entry_counts_chunks_of_256_entries_under_default_lengths(length, rows, width, taken):
+    """Plans with the default chunk length have more chunks than the limit counts: the product is done in column pieces (rows over
+    256 entries) or without splitting rows, and is refused only beyond the limit."""
+    import spmm_cpp
+    L = spmm_cpp.lib()
+    row = torch.arange(rows, dtype=torch.int32, device='cuda').repeat_interleave(length)
+    col = (torch.arange(rows * length, device='cuda') % length).to(torch.int32)
+    gen = torch.Generator(device='cuda').manual_seed(length)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device='cuda')
+    plan = spmm_cpp.SpmmPlan(row, col, rand(rows * length), rows, length)
+    cap, chunks = L.dg_static_scratch_capacity(), plan.stats()['heavy_chunks']
+    assert chunks * width > cap
+    assert taken == ((0 if length <= 256 else -(-length // 256) * rows) * width <= cap)
+    B, C0, scale, bias = rand(length, width), rand(rows, width), rand(rows), rand(width)
+    got = C0.clone()
+    rc = _call(L.dg_spmm_csr_static, plan, B, got, 1.5, -0.5, 7, scale, bias)
+    if not taken:
+        assert rc == -6 and torch.equal(got, C0)
+        return
+    assert rc == 0
+    want = (1.5 * plan.values.view(rows, length).double() @ B.double() - 0.5 * C0.double()) * scale.double()[:, None] + bias.double()
+    assert_close(got.cpu().numpy(), want.clamp(min=0).cpu().numpy(), TOL, f'{length} entries a row, F={width}')

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <mutex>
 #include "dist_gnn_b200.h"
 
 #define DG_CUDA(expr)                                        \
@@ -72,6 +73,7 @@ struct dg_plan {
     int* status;              // device words: [0] set non-zero by a kernel that gave up on a bounded wait, [1] the last check
                               // (by number) that found other ids than the plan's, then the tiles' (DG_TILE_WORDS)
     int checks;               // checks issued so far
+    std::mutex issue;         // held while a checked product is issued (dg_spmm_csr_checked)
 };
 
 int dg_stream_selected();     // non-zero while dg_select_kernel(2) is in force

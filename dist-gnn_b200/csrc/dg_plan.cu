@@ -349,7 +349,6 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
 
     dg_plan* p = new (std::nothrow) dg_plan();
     if (!p) return (int)cudaErrorMemoryAllocation;
-    *p = dg_plan{};
     p->m = m; p->k = k; p->nnz = nnz;
     p->col = sizeof(Id) == 8 ? col32 : reinterpret_cast<const int32_t*>(col);
     p->heavy_threshold = heavy_threshold; p->chunk = chunk;
@@ -513,6 +512,10 @@ extern "C" int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row,
     if (rc) return rc;
     if (!host_equal || (plan->nnz > 0 && (!plan_row || !plan_col || !row || !col))) return DG_ERR_NULL;
     cudaStream_t stream = (cudaStream_t)stream_;
+    // The scratch grows, and a check and the product behind it are issued, under one lock: the word that the product reads holds one
+    // check's number, and another thread's check between the two could take its place.
+    dg_plan* p = const_cast<dg_plan*>(plan);
+    std::unique_lock<std::mutex> lock(p->issue);
     if ((rc = dg_spmm_prepare(plan, F, stream))) return rc;
     *host_equal = 1;
     auto product = [&](int check) {
@@ -526,16 +529,19 @@ extern "C" int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row,
     *verdict.word = 0;
     int* differ = nullptr;
     DG_CUDA(cudaHostGetDevicePointer((void**)&differ, verdict.word, 0));
-    int& checks = const_cast<dg_plan*>(plan)->checks;
-    checks = checks == INT32_MAX ? 1 : checks + 1;
+    p->checks = p->checks == INT32_MAX ? 1 : p->checks + 1;
     const int64_t blocks = (plan->nnz + T - 1) / T;
-    k_ids_equal<<<(unsigned)std::min<int64_t>(blocks, 148 * 8), T, 0, stream>>>(plan_row, row, plan_col, col, plan->nnz, differ, plan->status + 1, checks);
+    k_ids_equal<<<(unsigned)std::min<int64_t>(blocks, 148 * 8), T, 0, stream>>>(plan_row, row, plan_col, col, plan->nnz, differ, plan->status + 1, p->checks);
     DG_CUDA(cudaGetLastError());
     DG_CUDA(cudaEventRecord(done, stream));
     const bool rows = !dg_spmm_stream_eligible(plan, B, ldb, C, ldc, F);
-    rc = rows ? product(checks) : DG_OK;
+    rc = rows ? product(p->checks) : DG_OK;
+    lock.unlock();
     DG_CUDA(cudaEventSynchronize(done));
     *host_equal = *(volatile int*)verdict.word == 0;
-    if (rc == DG_OK && !rows && *host_equal) rc = product(0);
+    if (rc == DG_OK && !rows && *host_equal) {
+        lock.lock();
+        rc = product(0);
+    }
     return rc;
 }

@@ -92,7 +92,8 @@ int dg_pool_trim(void);
  * more.  A program whose allocator keeps freed memory returns it to the driver there, as spmm_cpp does with PyTorch's.  NULL: none. */
 int dg_on_low_memory(void (*give_back)(void));
 /* dg_spmm_csr if the ids `row`, `col` (plan's nnz entries) equal `plan_row`, `plan_col`, those the plan was built from: *host_equal
- * says so.  Otherwise C is left alone.  Waits on the host for the comparison (one pass over both lists), not for the product. */
+ * says so.  Otherwise C is left alone.  Waits on the host for the comparison (one pass over both lists), not for the product.  Several
+ * threads may call it for one plan on one stream. */
 int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row, const int32_t* plan_col, const int32_t* row, const int32_t* col,
                         const float* val, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t F, float alpha, float beta,
                         int* host_equal, void* stream);

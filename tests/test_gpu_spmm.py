@@ -696,3 +696,39 @@ def test_tiles_of_small_numbers_are_as_exact_as_gathering(value_exponent, operan
     err = lambda p: float((p.spmm(b, torch.empty(3001, 64, device='cuda'), 1.0, 0.0).double() - want).norm() / want.norm())
     assert err(plan) <= 1.5 * err(plain)
     assert torch.equal(plan.spmm(torch.zeros_like(b), torch.ones_like(b[:1]).repeat(3001, 1), 1.0, 0.0), torch.zeros(3001, 64, device='cuda'))
+
+
+def test_checked_products_from_several_threads():
+    """Four host threads on one plan and one stream, two of them with ids that differ: their results stay as they are, every time."""
+    import threading
+    import spmm_cpp
+    rng = np.random.Generator(np.random.PCG64(701))
+    A = random_coo(rng, 500, 333, 4000, heavy=[(17, 300), (499, 90)])
+    plan, F = make_plan(A), 64
+    row, col = dev(A.row, torch.int32), dev(A.col, torch.int32)
+    other = col.clone()
+    other[-1] += 1
+    b = torch.randn(333, F, device='cuda')
+    want = plan.spmm(b, torch.zeros(500, F, device='cuda'), 1.0, 0.0)
+    L, stream, wrong = spmm_cpp.lib(), torch.cuda.current_stream().cuda_stream, []
+    results = [torch.full((500, F), 7.0, device='cuda') for _ in range(4)]
+    plan.spmm(b, torch.empty_like(want), 1.0, 0.0)
+    torch.cuda.synchronize()
+
+    def work(i):
+        ids, C, same = (other if i % 2 else col), results[i], ctypes.c_int(-1)
+        for _ in range(300):
+            rc = L.dg_spmm_csr_checked(plan.handle, row.data_ptr(), col.data_ptr(), row.data_ptr(), ids.data_ptr(), plan.values.data_ptr(), b.data_ptr(), F,
+                                       C.data_ptr(), F, F, 1.0, 0.0, ctypes.byref(same), stream)
+            if rc or same.value != (0 if i % 2 else 1):
+                wrong.append((i, rc, same.value))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong
+    for i in range(4):
+        assert torch.equal(results[i], torch.full_like(want, 7.0) if i % 2 else want)

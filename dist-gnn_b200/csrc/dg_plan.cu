@@ -107,21 +107,30 @@ __global__ void __launch_bounds__(T) k_row_census(const int64_t* __restrict__ ro
 {
     if (counts->bad) return;
     __shared__ int2 sums[T / 32 + 1];
+    __shared__ unsigned long long longest, split, pieces;          // one global atomic a block, not one a warp
+    if (threadIdx.x == 0) longest = split = pieces = 0;
     int64_t e0 = 0, e1 = 0;
     const int2 s = split_of(rowptr, blockIdx.x * T + threadIdx.x, m, threshold, chunk, &e0, &e1);
     block_scan(s, sums);
     unsigned long long deg = (unsigned long long)(e1 - e0), heavy = s.x ? deg : 0;
-    unsigned long long pieces = e1 - e0 > static_threshold ? (unsigned long long)((e1 - e0 + static_chunk - 1) / static_chunk) : 0;
+    uint32_t part = e1 - e0 > static_threshold ? ((uint32_t)(e1 - e0) + (uint32_t)static_chunk - 1) / (uint32_t)static_chunk : 0;
     for (int off = 16; off > 0; off >>= 1) {
         const unsigned long long o = __shfl_xor_sync(0xffffffffu, deg, off);
         deg = o > deg ? o : deg;
         heavy += __shfl_xor_sync(0xffffffffu, heavy, off);
-        pieces += __shfl_xor_sync(0xffffffffu, pieces, off);
     }
-    if ((threadIdx.x & 31) == 0 && deg > 0) atomicMax(&counts->max_row, deg);
-    if ((threadIdx.x & 31) == 0 && heavy > 0) atomicAdd(&counts->heavy_nnz, heavy);
-    if ((threadIdx.x & 31) == 0 && pieces > 0) atomicAdd(&counts->static_chunks, pieces);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = sums[T / 32];
+    part = __reduce_add_sync(0xffffffffu, part);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&longest, deg);
+        if (heavy) atomicAdd(&split, heavy);
+        if (part) atomicAdd(&pieces, (unsigned long long)part);
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    block_sums[blockIdx.x] = sums[T / 32];
+    if (longest) atomicMax(&counts->max_row, longest);
+    if (split) atomicAdd(&counts->heavy_nnz, split);
+    if (pieces) atomicAdd(&counts->static_chunks, pieces);
 }
 
 // One CTA: exclusive sums over the blocks' counts in place, and over the columns' bitmap.

@@ -37,7 +37,7 @@ def command(verbose=False):
 def up_to_date(srcs):
     if not os.path.exists(OUTPUT):
         return False
-    deps = srcs + [os.path.join(HERE, 'dg_internal.h'), os.path.join(HERE, 'dg_comm.h'), os.path.join(HERE, 'dg_tiles.h'), os.path.join(HERE, 'dg_umma.h'), os.path.join(ROOT, 'include', 'dist_gnn_b200.h'), __file__]
+    deps = srcs + [os.path.join(HERE, 'dg_internal.h'), os.path.join(HERE, 'dg_comm.h'), os.path.join(HERE, 'dg_build.h'), os.path.join(HERE, 'dg_tiles.h'), os.path.join(HERE, 'dg_umma.h'), os.path.join(ROOT, 'include', 'dist_gnn_b200.h'), __file__]
     return all(os.path.getmtime(d) <= os.path.getmtime(OUTPUT) for d in deps)
 
 

@@ -10,14 +10,13 @@
 #include <algorithm>
 #include <new>
 #include <vector>
-#include "dg_internal.h"
+#include "dg_build.h"
 #include "dg_tiles.h"
 
 namespace {
 
 constexpr int T = 256;
 constexpr int kEntriesPerThread = 4;
-constexpr int kBands = 4096;          // column bands the chunks are ordered by
 
 struct PlanCounts {
     unsigned long long max_row, heavy_nnz, touched, static_chunks;
@@ -163,8 +162,6 @@ __global__ void k_count_bits(const uint32_t* __restrict__ bitmap, int64_t words,
     if ((threadIdx.x & 31) == 0 && local) atomicAdd(&counts->touched, local);
 }
 
-__device__ __forceinline__ int band_of(int32_t column, int32_t k) { return (int)((int64_t)column * kBands / k); }
-
 // The chunks of every split row, in row order, and how many start in each column band.  The CTA's threads share its rows'
 // chunks out evenly (a row of 100,000 entries has hundreds).
 __global__ void __launch_bounds__(T) k_emit_chunks(const int64_t* __restrict__ rowptr, int32_t m, int32_t k, int32_t threshold, int32_t chunk,
@@ -256,26 +253,6 @@ __global__ void k_split_census(const int64_t* __restrict__ rowptr, int32_t m, in
     if (slot < capacity) out[slot] = dg_split_row{i, (int32_t)t0, (int32_t)t1, 0};
 }
 
-struct PoolTemp {   // gives its blocks back on scope exit; the stream that used them is waited for first
-    cudaStream_t stream;
-    std::vector<void*> ptrs;
-    bool idle = false;                // the stream has been synchronised since the last use
-    explicit PoolTemp(cudaStream_t s) : stream(s) {}
-    ~PoolTemp()
-    {
-        if (!idle && !ptrs.empty()) cudaStreamSynchronize(stream);
-        for (void* p : ptrs) dg_pool_free(p);
-    }
-    template <class X> int alloc(X** out, size_t count)
-    {
-        void* p = nullptr;
-        const int rc = dg_pool_alloc(&p, std::max<size_t>(count, 1) * sizeof(X));
-        if (rc == DG_OK) ptrs.push_back(p);
-        *out = (X*)p;
-        return rc;
-    }
-};
-
 int build_tasks(dg_plan* p, int32_t task_nnz, cudaStream_t stream)
 {
     dg_pool_free(p->task_first_row);
@@ -289,7 +266,7 @@ int build_tasks(dg_plan* p, int32_t task_nnz, cudaStream_t stream)
     int rc = dg_pool_alloc((void**)&p->task_first_row, (size_t)p->n_tasks * sizeof(int32_t));
     if (rc) return rc;
     k_task_first_row<<<(p->n_tasks + T - 1) / T, T, 0, stream>>>(p->rowptr, p->m, task_nnz, p->n_tasks, p->task_first_row);
-    PoolTemp tmp(stream);
+    PoolScope tmp(stream);
     dg_split_row* d_rows = nullptr;
     int32_t* d_count = nullptr;
     const int32_t capacity = p->n_tasks;      // a row can only be cut at one of the n_tasks - 1 task boundaries
@@ -370,7 +347,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     if (max_chunks > INT32_MAX) return fail(DG_ERR_UNSUPPORTED);
     const int64_t words = lean ? 0 : ((int64_t)k + 31) / 32;
     const int32_t row_blocks = (int32_t)(((int64_t)m + T - 1) / T);
-    PoolTemp tmp(stream);
+    PoolScope tmp(stream);
     uint8_t* zeroed = nullptr;            // counts, column bands, column bitmap: cleared by one memset
     int2* block_sums = nullptr;
     dg_chunk* in_row_order = nullptr;

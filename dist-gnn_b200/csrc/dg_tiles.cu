@@ -24,6 +24,7 @@
 #include <atomic>
 #include <new>
 #include <vector>
+#include "dg_build.h"
 #include "dg_tiles.h"
 #include "dg_umma.h"
 
@@ -51,7 +52,6 @@ constexpr int kValueWarps = 4;            // of every CTA, to see whether the va
 constexpr int kScatterThreads = 256, kGroupThreads = 128, kTileThreads = kScatterThreads + 64 + 32 * kValueWarps;
 constexpr int kAhead = 8;                 // records a thread holds for its group's next tile
 constexpr int T = 256;
-constexpr int kBands = 4096;
 
 // Where element (r, c) of a tile lies: core matrices of 8 rows x 8 columns (128 bytes), rows of cores first.
 __host__ __device__ __forceinline__ int tile_element(int r, int c) { return (c >> 3) * (kTileRows * 8) + (r >> 3) * 64 + (r & 7) * 8 + (c & 7); }
@@ -563,8 +563,6 @@ __global__ void __launch_bounds__(1024) k_exclusive_sums(int32_t* __restrict__ v
     if (threadIdx.x == 0) v[n] = carry;
 }
 
-__device__ __forceinline__ int band_of(int32_t column, int32_t k) { return (int)((int64_t)column * kBands / k); }
-
 // Chunks of what is left of every split row, at least one (it may be empty: whoever works on a row's last chunk writes the row).
 // PASS 0: how many per row; 1: how many start in each column band; 2: the chunks, by band.
 template <int PASS>
@@ -592,26 +590,6 @@ __global__ void k_first_slots(const dg_chunk* __restrict__ chunks, int32_t n_chu
     if (c == 0) first_slot[n_rows] = n_chunks;
     if (c < n_chunks && chunks[c].slot == chunks[c].slot0) first_slot[chunks[c].heavy] = chunks[c].slot0;
 }
-
-struct PoolScope {                    // blocks of the pool that are given back unless kept; the stream is waited for first
-    cudaStream_t stream;
-    std::vector<void*> ptrs;
-    explicit PoolScope(cudaStream_t s) : stream(s) {}
-    ~PoolScope()
-    {
-        if (ptrs.empty()) return;
-        cudaStreamSynchronize(stream);
-        for (void* p : ptrs) dg_pool_free(p);
-    }
-    template <class X> int alloc(X** out, size_t count)
-    {
-        void* p = nullptr;
-        const int rc = dg_pool_alloc(&p, std::max<size_t>(count, 1) * sizeof(X));
-        if (rc == DG_OK) ptrs.push_back(p);
-        *out = (X*)p;
-        return rc;
-    }
-};
 
 unsigned grid_of(int64_t n, int per_block) { return (unsigned)((n + per_block - 1) / per_block); }
 

@@ -384,6 +384,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     py::class_<PlanRef, std::shared_ptr<PlanRef>>(m, "PlanRef").def(py::init<int64_t, Tensor, Tensor>());
     m.def("spmm", &spmm);
     m.def("gcn", &gcn);
+    m.def("readable_padded", &readable_padded);
     m.def("row_cross_entropy", &row_cross_entropy);
     m.def("pending_regions", &pending_regions);
     m.def("resolve_regions", &resolve_regions);

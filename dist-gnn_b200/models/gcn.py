@@ -150,10 +150,8 @@ def _product_operand(env, t, constant):
     of whole pieces; the columns beyond w are read and their results dropped), else a padded copy as above."""
     n, true_width = t.shape
     width = true_width + (-true_width) % 4 if PAD_ODD_WIDTHS else true_width
-    ld = t.stride(0)
-    if t.stride(1) == 1 and ld % 4 == 0 and ld >= width and t.data_ptr() % 16 == 0 and (
-            width == true_width or t.storage_offset() + (n - 1) * ld + width <= t.untyped_storage().nbytes() // 4):
-        return t if width == true_width else t.as_strided((n, width), (ld, 1))
+    if spmm_cpp.binding().readable_padded(t, width):
+        return t if width == true_width else t.as_strided((n, width), (t.stride(0), 1))
     if width == true_width:
         return t.contiguous()
     if constant:

@@ -20,6 +20,10 @@ static inline int32_t dg_default_chunk(int64_t nnz, int32_t m) { return nnz < (1
 // What dg_spmm_csr_static holds against its capacity are chunks of this many entries wherever the plan's own lengths are defaults.
 #define DG_STATIC_CHUNK 256
 
+// Nothing throws across the C ABI: entries that use the host's allocator, or call something that does, are function-try-blocks that
+// end in this, with the code of the exception under way.
+int dg_exception() noexcept;
+
 #define DG_FINISH_TILES 16        // column tiles of one launch: arrival counts are kept per split row and tile
 
 // One chunk of a split (heavy) row: entries [e0, e0 + len) of row `row`; its partial sum lands in scratch row `slot`.
@@ -96,7 +100,7 @@ int dg_plan_ensure_tasks(dg_plan* plan, cudaStream_t stream);
 // Device memory of plans (dg_pool.cu), on the current device.  A block may be freed once the device is done with it.
 int dg_pool_alloc(void** out, size_t bytes);
 int dg_device_alloc(void** out, size_t bytes);      // not from the pool, freed with cudaFree
-void dg_pool_free(void* ptr);
+void dg_pool_free(void* ptr) noexcept;
 int* dg_status_word();        // the current device's, or null
 int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream);
 int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, int64_t ldb, const float* C, int64_t ldc,

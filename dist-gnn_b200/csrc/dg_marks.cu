@@ -29,7 +29,7 @@ cudaEvent_t event_of(int id)
 }  // namespace
 
 extern "C" int dg_mark_record(void* stream)
-{
+try {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return DG_ERR_STATE;
     MarkPool& p = pool();
@@ -49,10 +49,12 @@ extern "C" int dg_mark_record(void* stream)
         return DG_ERR_STATE;
     }
     return (dev << kSlotBits) | slot;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_mark_elapsed(int begin, int end, float* host_ms)
-{
+try {
     if (!host_ms) return DG_ERR_NULL;
     MarkPool& p = pool();
     std::lock_guard<std::mutex> lock(p.mu);
@@ -60,13 +62,17 @@ extern "C" int dg_mark_elapsed(int begin, int end, float* host_ms)
     if (!a || !b) return DG_ERR_STATE;
     DG_CUDA(cudaEventElapsedTime(host_ms, a, b));
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_mark_release(int id)
-{
+try {
     MarkPool& p = pool();
     std::lock_guard<std::mutex> lock(p.mu);
     if (!event_of(id)) return DG_ERR_STATE;
     p.unused[id >> kSlotBits].push_back(id & ((1 << kSlotBits) - 1));
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }

@@ -78,7 +78,7 @@ int pull_block(dg_comm* c, float* dst, const float* src, size_t count, int lanes
 }  // namespace
 
 extern "C" int dg_comm_peer_alloc(dg_comm* c, int64_t floats, char host_handles_out[128])
-{
+try {
     if (!c || !host_handles_out) return DG_ERR_NULL;
     if (floats <= 0) return DG_ERR_DIMS;
     if (!c->peer_ptr.empty()) return DG_ERR_STATE;                // peers still mapped: dg_comm_peer_close first
@@ -105,10 +105,12 @@ extern "C" int dg_comm_peer_alloc(dg_comm* c, int64_t floats, char host_handles_
     c->peer_floats = floats;
     c->peer_loops = 0;
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_comm_peer_open(dg_comm* c, const char* host_handles_all)
-{
+try {
     if (!c || !host_handles_all) return DG_ERR_NULL;
     if (!c->peer_send[0] || !c->peer_ptr.empty()) return DG_ERR_STATE;
     DeviceGuard guard(c->device);
@@ -131,14 +133,18 @@ extern "C" int dg_comm_peer_open(dg_comm* c, const char* host_handles_all)
         }
     }
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_comm_peer_close(dg_comm* c)
-{
+try {
     if (!c) return DG_ERR_NULL;
     DeviceGuard guard(c->device);
     DG_CUDA(cudaStreamSynchronize(c->side));
     return peer_release(c);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int64_t dg_comm_peer_capacity(const dg_comm* c)
@@ -392,9 +398,11 @@ extern "C" int dg_peer_spmm(dg_comm* comm, dg_comm* row_comm, int32_t n_stages, 
                             int32_t n_products, const dg_plan* const* plans, const float* const* vals,
                             const float* const* operands, const int32_t* last_stage, const float* x_local, int32_t n,
                             int32_t F, float* z, int timed, void* compute_stream)
-{
+try {
     return peer_loop(comm, row_comm, PeerPacks{}, n_stages, roots, landing, n_products, plans, vals, operands, last_stage, x_local, n, F,
                      z, timed, compute_stream);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_peer_spmm_packed(dg_comm* comm, dg_comm* row_comm, int32_t n_packs, const int32_t* const* pack_rows,
@@ -403,7 +411,7 @@ extern "C" int dg_peer_spmm_packed(dg_comm* comm, dg_comm* row_comm, int32_t n_p
                                    int32_t n_products, const dg_plan* const* plans, const float* const* vals,
                                    const float* const* operands, const int32_t* last_stage, const float* x_local, int32_t n,
                                    int32_t F, float* z, int timed, void* compute_stream)
-{
+try {
     if (!stage_offsets && n_stages > 0) return DG_ERR_NULL;
     PeerPacks packs;
     packs.n_packs = n_packs; packs.rows = pack_rows; packs.counts = pack_counts; packs.offsets = pack_offsets;
@@ -412,6 +420,8 @@ extern "C" int dg_peer_spmm_packed(dg_comm* comm, dg_comm* row_comm, int32_t n_p
     if (!packs.stage_rows) packs.stage_rows = &none;              // marks packed mode even with no stage to pull
     return peer_loop(comm, row_comm, packs, n_stages, roots, landing, n_products, plans, vals, operands, last_stage, x_local, n, F, z,
                      timed, compute_stream);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_peer_spmm_gather(dg_comm* comm, dg_comm* row_comm, int32_t n_stages, const int32_t* roots,
@@ -419,7 +429,7 @@ extern "C" int dg_peer_spmm_gather(dg_comm* comm, dg_comm* row_comm, int32_t n_s
                                    int32_t n_products, const dg_plan* const* plans, const float* const* vals,
                                    const float* const* operands, const int32_t* last_stage, const float* x_local, int32_t n,
                                    int32_t F, float* z, int timed, void* compute_stream)
-{
+try {
     if (n_stages > 0 && (!stage_lists || !stage_rows)) return DG_ERR_NULL;
     PeerPacks packs;
     static const int32_t* const no_lists[1] = {nullptr};
@@ -427,4 +437,6 @@ extern "C" int dg_peer_spmm_gather(dg_comm* comm, dg_comm* row_comm, int32_t n_s
     packs.stage_rows = stage_rows;
     return peer_loop(comm, row_comm, packs, n_stages, roots, landing, n_products, plans, vals, operands, last_stage, x_local, n, F, z,
                      timed, compute_stream);
+} catch (...) {
+    return dg_exception();
 }

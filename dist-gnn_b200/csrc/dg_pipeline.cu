@@ -142,7 +142,7 @@ extern "C" int dg_comm_unique_id(char host_id_out[128])
 }
 
 extern "C" int dg_comm_create(const char host_id[128], int rank, int nranks, dg_comm** out)
-{
+try {
     if (!host_id || !out) return DG_ERR_NULL;
     if (nranks < 1 || rank < 0 || rank >= nranks) return DG_ERR_DIMS;
     *out = nullptr;
@@ -151,10 +151,12 @@ extern "C" int dg_comm_create(const char host_id[128], int rank, int nranks, dg_
     ncclComm_t nc;
     DG_NCCL(ncclCommInitRank(&nc, nranks, id, rank));
     return finish_comm(nc, out);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_comm_split(dg_comm* parent, int color, int key, dg_comm** out)
-{
+try {
     if (!parent || !out) return DG_ERR_NULL;
     *out = nullptr;
     DeviceGuard guard(parent->device);
@@ -162,6 +164,8 @@ extern "C" int dg_comm_split(dg_comm* parent, int color, int key, dg_comm** out)
     DG_NCCL(ncclCommSplit(parent->comm, color < 0 ? NCCL_SPLIT_NOCOLOR : color, key, &nc, nullptr));
     if (!nc) return DG_OK;    // this rank asked to stay out
     return finish_comm(nc, out);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_comm_destroy(dg_comm* c)
@@ -212,19 +216,23 @@ extern "C" int dg_comm_broadcast(dg_comm* c, float* buf, int64_t count, int root
 extern "C" int dg_bcast_spmm_1d(dg_comm* comm, int32_t n_stages, const int32_t* roots, int32_t group,
                                 const dg_plan* const* plans, const float* const* vals, const float* x_local, int32_t n,
                                 int32_t F, float* const* recv, int32_t nbuf, float* z, int timed, void* compute_stream)
-{
+try {
     return stage_loop(comm, n_stages, roots, group, plans, vals, x_local, n, F, recv, nbuf, z, timed, (cudaStream_t)compute_stream);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_bcast_spmm_15d(dg_comm* col_comm, dg_comm* row_comm, int32_t n_stages, const int32_t* roots,
                                  int32_t group, const dg_plan* const* plans, const float* const* vals,
                                  const float* x_local, int32_t n, int32_t F, float* const* recv, int32_t nbuf, float* z,
                                  int timed, void* compute_stream)
-{
+try {
     int rc = stage_loop(col_comm, n_stages, roots, group, plans, vals, x_local, n, F, recv, nbuf, z, timed, (cudaStream_t)compute_stream);
     if (rc) return rc;
     if (row_comm) rc = dg_comm_allreduce_sum(row_comm, z, (int64_t)n * F, compute_stream);
     return rc;
+} catch (...) {
+    return dg_exception();
 }
 
 // Stage loop with a receive area for every remote block: all broadcasts are queued back to back on the side stream
@@ -234,7 +242,7 @@ extern "C" int dg_bcast_spmm_ordered(dg_comm* comm, dg_comm* row_comm, int32_t n
                                      int32_t bcast_group, float* const* landing, int32_t n_products, const dg_plan* const* plans,
                                      const float* const* vals, const float* const* operands, const int32_t* last_stage,
                                      const float* x_local, int32_t n, int32_t F, float* z, int timed, void* compute_stream)
-{
+try {
     cudaStream_t compute = (cudaStream_t)compute_stream;
     if (!comm) return DG_ERR_NULL;
     if (n_stages < 0 || n_products < 0 || n < 0 || F < 0 || bcast_group < 1) return DG_ERR_DIMS;
@@ -316,6 +324,8 @@ extern "C" int dg_bcast_spmm_ordered(dg_comm* comm, dg_comm* row_comm, int32_t n
     }
     issue.done();
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 // 1D distributed product pipelined along the FEATURE dimension instead of along the source rank: the operand is cut
@@ -326,7 +336,7 @@ extern "C" int dg_bcast_spmm_ordered(dg_comm* comm, dg_comm* row_comm, int32_t n
 extern "C" int dg_allgather_spmm(dg_comm* comm, const dg_plan* plan, const float* val, const float* x_local, int32_t n,
                                  int32_t F, int32_t n_chunks, const int32_t* chunk_widths, float* const* pack,
                                  float* const* area, float* z, int timed, void* compute_stream)
-{
+try {
     cudaStream_t compute = (cudaStream_t)compute_stream;
     if (!comm || !plan) return DG_ERR_NULL;
     if (n < 0 || F < 0 || n_chunks < 1 || !chunk_widths) return DG_ERR_DIMS;
@@ -391,10 +401,12 @@ extern "C" int dg_allgather_spmm(dg_comm* comm, const dg_plan* plan, const float
     }
     issue.done();
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_comm_last_times(dg_comm* c, dg_stage_times* out)
-{
+try {
     if (!c || !out) return DG_ERR_NULL;
     *out = dg_stage_times{0.f, 0.f, 0.f, 0};
     if (c->timed_stages == 0) return DG_OK;
@@ -411,4 +423,6 @@ extern "C" int dg_comm_last_times(dg_comm* c, dg_stage_times* out)
     DG_CUDA(cudaEventElapsedTime(&out->total_ms, c->t_begin, c->t_end));
     out->stages = c->timed_stages;
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }

@@ -298,13 +298,15 @@ int dg_plan_ensure_tasks(dg_plan* p, cudaStream_t stream)
 }
 
 extern "C" int dg_plan_set_task_size(dg_plan* p, int32_t task_nnz, void* stream)
-{
+try {
     if (!p) return DG_ERR_NULL;
     if (task_nnz <= 0) task_nnz = DG_DEFAULT_TASK_NNZ;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev != p->device) return DG_ERR_STATE;
     DG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));     // earlier products may still read the old tables
     return build_tasks(p, task_nnz, (cudaStream_t)stream);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_plan_device_status(const dg_plan* p, int* host_status, void* stream)
@@ -339,12 +341,15 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     p->col = sizeof(Id) == 8 ? col32 : reinterpret_cast<const int32_t*>(col);
     p->heavy_threshold = heavy_threshold; p->chunk = chunk;
     int rc = DG_OK;
-    auto fail = [&](int code) { dg_plan_destroy(p); return code; };
-    if ((rc = (int)cudaGetDevice(&p->device)) != 0) return fail(rc);
+    struct Owner {                        // until the plan is handed out
+        dg_plan* plan;
+        ~Owner() { dg_plan_destroy(plan); }
+    } owner{p};
+    if ((rc = (int)cudaGetDevice(&p->device)) != 0) return rc;
 
     // upper bounds: a split row holds more than heavy_threshold entries, and its last chunk may be a short one
     const int64_t max_heavy = std::min<int64_t>(nnz / ((int64_t)heavy_threshold + 1), m), max_chunks = nnz / chunk + max_heavy;
-    if (max_chunks > INT32_MAX) return fail(DG_ERR_UNSUPPORTED);
+    if (max_chunks > INT32_MAX) return DG_ERR_UNSUPPORTED;
     const int64_t words = lean ? 0 : ((int64_t)k + 31) / 32;
     const int32_t row_blocks = (int32_t)(((int64_t)m + T - 1) / T);
     PoolScope tmp(stream);
@@ -354,11 +359,11 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     const size_t zero_bytes = sizeof(PlanCounts) + kBands * sizeof(int32_t) + (size_t)words * sizeof(uint32_t);
     if ((rc = dg_pool_alloc((void**)&p->rowptr, ((size_t)m + 1) * sizeof(int64_t))) || (rc = dg_pool_alloc((void**)&p->status, DG_STATUS_WORDS * sizeof(int))) ||
         (rc = tmp.alloc(&zeroed, zero_bytes)) || (rc = tmp.alloc(&block_sums, (size_t)row_blocks)))
-        return fail(rc);
+        return rc;
     if (max_chunks > 0 && ((rc = dg_pool_alloc((void**)&p->chunks, (size_t)max_chunks * sizeof(dg_chunk))) ||
                            (rc = dg_pool_alloc((void**)&p->arrived, (size_t)max_heavy * DG_FINISH_TILES * sizeof(int))) ||
                            (rc = tmp.alloc(&in_row_order, (size_t)max_chunks))))
-        return fail(rc);
+        return rc;
     PlanCounts* counts = reinterpret_cast<PlanCounts*>(zeroed);
     int32_t* bands = reinterpret_cast<int32_t*>(counts + 1);
     uint32_t* bitmap = words ? reinterpret_cast<uint32_t*>(bands + kBands) : nullptr;
@@ -382,10 +387,10 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     PlanCounts h{};
     if ((rc = (int)cudaMemcpyAsync(&h, counts, sizeof(h), cudaMemcpyDeviceToHost, stream)) || (rc = (int)cudaStreamSynchronize(stream)) ||
         (rc = (int)cudaGetLastError()))
-        return fail(rc);
+        return rc;
     tmp.idle = true;
-    if (h.bad) return fail(DG_ERR_INDEX);
-    if (h.n_heavy > max_heavy || h.n_chunks > max_chunks) return fail(DG_ERR_STATE);      // cannot happen
+    if (h.bad) return DG_ERR_INDEX;
+    if (h.n_heavy > max_heavy || h.n_chunks > max_chunks) return DG_ERR_STATE;      // cannot happen
     p->max_row_nnz = (int64_t)h.max_row;
     p->heavy_nnz = (int64_t)h.heavy_nnz;
     p->touched_columns = lean ? (int64_t)k : (int64_t)h.touched;
@@ -393,6 +398,7 @@ int plan_build(const Id* row, const Id* col, int64_t nnz, int32_t m, int32_t k, 
     p->n_chunks = h.n_chunks;
     p->static_chunks = (int64_t)h.static_chunks;
     *out = p;
+    owner.plan = nullptr;
     return DG_OK;
 }
 
@@ -405,14 +411,18 @@ int dg_plan_build_lean(const int32_t* row, const int32_t* col, int64_t nnz, int3
 
 extern "C" int dg_plan_create_ex(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k,
                                  int32_t heavy_threshold, int32_t chunk, void* stream, dg_plan** out)
-{
+try {
     return plan_build<int32_t>(row, col, nnz, m, k, heavy_threshold, chunk, false, nullptr, stream, out);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_plan_create_i64(const int64_t* row, const int64_t* col, int64_t nnz, int32_t m, int32_t k, int32_t heavy_threshold,
                                   int32_t chunk, int32_t* col32, void* stream, dg_plan** out)
-{
+try {
     return plan_build<int64_t>(row, col, nnz, m, k, heavy_threshold, chunk, false, col32, stream, out);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_plan_create(const int32_t* row, const int32_t* col, int64_t nnz, int32_t m, int32_t k, void* stream,
@@ -493,7 +503,7 @@ struct Verdict {
 extern "C" int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row, const int32_t* plan_col, const int32_t* row, const int32_t* col,
                                    const float* val, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t F, float alpha, float beta,
                                    int* host_equal, void* stream_)
-{
+try {
     int rc = dg_check_spmm_args(plan, val, B, ldb, C, ldc, F, 0u, nullptr, nullptr);
     if (rc) return rc;
     if (!host_equal || (plan->nnz > 0 && (!plan_row || !plan_col || !row || !col))) return DG_ERR_NULL;
@@ -530,4 +540,6 @@ extern "C" int dg_spmm_csr_checked(const dg_plan* plan, const int32_t* plan_row,
         rc = product(0);
     }
     return rc;
+} catch (...) {
+    return dg_exception();
 }

@@ -14,6 +14,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include "dg_internal.h"
 
@@ -88,6 +89,17 @@ int dg_device_alloc(void** out, size_t bytes)
     return (int)e;
 }
 
+int dg_exception() noexcept
+{
+    try {
+        throw;
+    } catch (const std::bad_alloc&) {
+        return (int)cudaErrorMemoryAllocation;
+    } catch (...) {
+        return DG_ERR_STATE;
+    }
+}
+
 // One word per device, zero until a tensor-core kernel gives up on a bounded wait.
 int* dg_status_word()
 {
@@ -133,12 +145,17 @@ int dg_pool_alloc(void** out, size_t bytes)
     }
     const int rc = dg_device_alloc(out, want);
     if (rc) return rc;
-    std::lock_guard<std::mutex> lock(p.mu);
-    p.size[dev][*out] = want;
+    try {
+        std::lock_guard<std::mutex> lock(p.mu);
+        p.size[dev][*out] = want;
+    } catch (...) {
+        cudaFree(*out);
+        throw;
+    }
     return DG_OK;
 }
 
-void dg_pool_free(void* ptr)
+void dg_pool_free(void* ptr) noexcept
 {
     int dev = -1;
     if (!ptr || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
@@ -161,13 +178,20 @@ void dg_pool_free(void* ptr)
         p.size[dev].erase(oldest->second.ptr);
         unused.erase(oldest);
     }
-    unused.emplace(it->second, Idle{ptr, p.clock++});
-    p.unused_bytes[dev] += it->second;
+    try {
+        unused.emplace(it->second, Idle{ptr, p.clock++});
+        p.unused_bytes[dev] += it->second;
+    } catch (...) {                                               // no room on the host to remember it
+        p.size[dev].erase(it);
+        cudaFree(ptr);
+    }
 }
 
 extern "C" int dg_pool_trim(void)
-{
+try {
     int dev = -1;
     DG_CUDA(cudaGetDevice(&dev));
     return trim(dev);
+} catch (...) {
+    return dg_exception();
 }

@@ -575,7 +575,7 @@ int dg_spmm_launch(const dg_plan* plan, const float* val, const float* B, int64_
 }
 
 extern "C" int dg_profile_begin(void)
-{
+try {
     std::lock_guard<std::mutex> lock(g_profile.mu);
     g_profile.open = true;
     g_profile.used = 0;
@@ -583,10 +583,12 @@ extern "C" int dg_profile_begin(void)
     g_profile.products = 0;
     g_kernel_launches.store(0);
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_profile_end(dg_profile* out)
-{
+try {
     if (!out) return DG_ERR_NULL;
     std::lock_guard<std::mutex> lock(g_profile.mu);
     g_profile.open = false;
@@ -601,6 +603,8 @@ extern "C" int dg_profile_end(dg_profile* out)
                       g_kernel_launches.load()};
     g_profile.used = 0;
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 // Grows the plan's scratch to what a product of width F may need (either kernel family); allocates and synchronises
@@ -640,17 +644,19 @@ int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream)
 extern "C" int dg_spmm_csr(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C, int64_t ldc,
                            int32_t F, float alpha, float beta, uint32_t flags, const float* row_scale,
                            const float* bias, void* stream)
-{
+try {
     int rc = dg_check_spmm_args(plan, val, B, ldb, C, ldc, F, flags, row_scale, bias);
     if (rc) return rc;
     if ((rc = dg_spmm_prepare(plan, F, (cudaStream_t)stream))) return rc;      // first use at this width may grow the scratch
     return dg_spmm_launch(plan, val, B, ldb, C, ldc, F, alpha, beta, flags, row_scale, bias, plan->scratch, plan->scratch_floats,
                           (cudaStream_t)stream);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_spmm_coo(const int32_t* row, const int32_t* col, const float* val, int64_t nnz, int32_t m, int32_t k,
                            const float* B, float* C, int32_t F, float alpha, float beta, void* stream)
-{
+try {
     dg_plan* plan = nullptr;
     int rc = dg_plan_build_lean(row, col, nnz, m, k, stream, &plan);
     if (rc) return rc;
@@ -658,6 +664,8 @@ extern "C" int dg_spmm_coo(const int32_t* row, const int32_t* col, const float* 
     if (rc == DG_OK) rc = (int)cudaStreamSynchronize((cudaStream_t)stream);   // the plan's buffers die below
     dg_plan_destroy(plan);
     return rc;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" const char* dg_strerror(int code)

@@ -57,17 +57,19 @@ int static_scratch_address(int device, float** out)
 extern "C" int64_t dg_static_scratch_capacity(void) { return DG_STATIC_SCRATCH_FLOATS; }
 
 extern "C" int dg_static_scratch_prepare(void)
-{
+try {
     int device = -1;
     DG_CUDA(cudaGetDevice(&device));
     float* unused = nullptr;
     return static_scratch_address(device, &unused);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_spmm_csr_static(const dg_plan* plan, const float* val, const float* B, int64_t ldb, float* C,
                                   int64_t ldc, int32_t F, float alpha, float beta, uint32_t flags,
                                   const float* row_scale, const float* bias, void* stream)
-{
+try {
     int rc = dg_check_spmm_args(plan, val, B, ldb, C, ldc, F, flags, row_scale, bias);   // also checks the current device
     if (rc) return rc;
     const int64_t chunks = plan->n_chunks;
@@ -83,4 +85,6 @@ extern "C" int dg_spmm_csr_static(const dg_plan* plan, const float* val, const f
                                  split ? chunks * width : 0, (cudaStream_t)stream, 0, split);
     }
     return rc;
+} catch (...) {
+    return dg_exception();
 }

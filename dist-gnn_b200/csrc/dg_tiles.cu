@@ -765,39 +765,48 @@ void dg_tiles_free(dg_tiles* t)
 }
 
 extern "C" int dg_plan_add_tiles(dg_plan* p, const float* val, void* stream)
-{
+try {
     if (!p || (p->nnz > 0 && !val)) return DG_ERR_NULL;
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev != p->device) return DG_ERR_STATE;
     const int dropped = dg_plan_drop_tiles(p, stream);
     if (dropped) return dropped;
-    dg_tiles* t = new (std::nothrow) dg_tiles();
+    struct Owner {                        // until the plan has them
+        dg_tiles* tiles;
+        cudaStream_t stream;
+        ~Owner()
+        {
+            if (tiles) cudaStreamSynchronize(stream);
+            dg_tiles_free(tiles);
+        }
+    } owner{new (std::nothrow) dg_tiles(), (cudaStream_t)stream};
+    dg_tiles* t = owner.tiles;
     if (!t) return (int)cudaErrorMemoryAllocation;
-    *t = dg_tiles{};
     t->status = dg_status_word();
     const int rc = t->status ? build_tiles(p, val, (cudaStream_t)stream, t) : DG_ERR_STATE;
-    if (rc != DG_OK || t->entries == 0) {
-        cudaStreamSynchronize((cudaStream_t)stream);
-        dg_tiles_free(t);
-        return rc;
-    }
+    if (rc != DG_OK || t->entries == 0) return rc;
     p->tiles = t;
+    owner.tiles = nullptr;
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_plan_drop_tiles(dg_plan* p, void* stream)
-{
+try {
     if (!p) return DG_ERR_NULL;
     if (!p->tiles) return DG_OK;
     DG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     dg_tiles_free(p->tiles);
     p->tiles = nullptr;
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 // The give-up path on purpose: the tensor-core part of a product, with waits of no polls at all.
 extern "C" int dg_tiles_wait_selftest(const dg_plan* p, const float* B, int64_t ldb, int32_t F, void* stream)
-{
+try {
     if (!p || !B) return DG_ERR_NULL;
     if (F < 1 || ldb < F) return DG_ERR_DIMS;
     int rc = dg_spmm_prepare(p, F, (cudaStream_t)stream);
@@ -806,6 +815,8 @@ extern "C" int dg_tiles_wait_selftest(const dg_plan* p, const float* B, int64_t 
     if (need == 0 || need > p->scratch_floats) return DG_ERR_STATE;
     int launches = 0;
     return dg_tiles_launch(p, B, ldb, F, p->scratch, (cudaStream_t)stream, &launches, 0);
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int64_t dg_plan_tiled_entries(const dg_plan* p) { return p && p->tiles ? p->tiles->entries : 0; }

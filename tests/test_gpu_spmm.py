@@ -732,3 +732,82 @@ def test_checked_products_from_several_threads():
     assert not wrong
     for i in range(4):
         assert torch.equal(results[i], torch.full_like(want, 7.0) if i % 2 else want)
+
+
+OUT_OF_HOST_MEMORY = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <new>
+#include <vector>
+#include <cuda_runtime.h>
+#include "dist_gnn_b200.h"
+static long left = -1;                                   // allocations until one is refused; negative: never
+void* operator new(std::size_t n)
+{
+    if (left >= 0 && left-- == 0) throw std::bad_alloc();
+    if (void* p = std::malloc(n)) return p;
+    throw std::bad_alloc();
+}
+void* operator new(std::size_t n, const std::nothrow_t&) noexcept
+{
+    if (left >= 0 && left-- == 0) return nullptr;
+    return std::malloc(n);
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
+
+int main()
+{
+    const int m = 400, each = 300, F = 64;               // every row split, frequent columns: tiles
+    std::vector<int> row, col;
+    std::vector<float> val(m * each, 1.f), b(each * F, 1.f), c(m * F);
+    for (int i = 0; i < m * each; ++i) row.push_back(i / each), col.push_back(i % each);
+    int *d_row, *d_col;
+    float *d_val, *d_b, *d_c;
+    cudaMalloc(&d_row, row.size() * 4), cudaMalloc(&d_col, row.size() * 4), cudaMalloc(&d_val, row.size() * 4), cudaMalloc(&d_b, b.size() * 4), cudaMalloc(&d_c, c.size() * 4);
+    cudaMemcpy(d_row, row.data(), row.size() * 4, cudaMemcpyHostToDevice), cudaMemcpy(d_col, col.data(), row.size() * 4, cudaMemcpyHostToDevice);
+    cudaMemcpy(d_val, val.data(), row.size() * 4, cudaMemcpyHostToDevice), cudaMemcpy(d_b, b.data(), b.size() * 4, cudaMemcpyHostToDevice);
+    int refused = 0, tiled = 0;
+    for (long after = 0; after < 60; ++after) {
+        dg_plan* plan = nullptr;
+        left = after;
+        const int created = dg_plan_create(d_row, d_col, (int64_t)row.size(), m, each, nullptr, &plan);
+        const int tiles = created == 0 ? dg_plan_add_tiles(plan, d_val, nullptr) : 0;
+        const int began = dg_profile_begin();
+        const int product = created == 0 ? dg_spmm_csr(plan, d_val, d_b, F, d_c, F, F, 1.f, 0.f, 0u, nullptr, nullptr, nullptr) : 0;
+        const int mark = dg_mark_record(nullptr);
+        left = -1;
+        dg_profile out;
+        const int ended = dg_profile_end(&out);
+        for (int code : {created, tiles, began, product, ended})
+            if (code == (int)cudaErrorMemoryAllocation) ++refused;
+            else if (code != 0) return std::printf("code %d after %ld\n", code, after), 1;
+        if (mark == (int)cudaErrorMemoryAllocation) ++refused;
+        else if (mark < 0) return std::printf("mark %d after %ld\n", mark, after), 1;
+        if (created != 0) continue;
+        tiled += dg_plan_tiled_entries(plan) > 0;
+        if (dg_spmm_csr(plan, d_val, d_b, F, d_c, F, F, 1.f, 0.f, 0u, nullptr, nullptr, nullptr) != 0) return std::printf("product\n"), 1;
+        cudaMemcpy(c.data(), d_c, c.size() * 4, cudaMemcpyDeviceToHost);
+        for (float x : c)
+            if (x != (float)each) return std::printf("%f after %ld\n", x, after), 1;
+        dg_plan_destroy(plan);
+    }
+    std::printf("refused %d tiled %d\n", refused, tiled);
+    return refused > 3 && tiled > 0 ? 0 : 1;
+}
+"""
+
+
+def test_host_allocations_that_fail_come_back_as_codes(tmp_path):
+    """A program whose operator new refuses the n-th allocation, for every n that plan, tiles and product make: codes, no exception
+    through the C ABI, and right products afterwards."""
+    import os
+    import subprocess
+    from conftest import PKG, ROOT
+    source, program, csrc = tmp_path / 'refuse.cpp', tmp_path / 'refuse', os.path.join(PKG, 'csrc')
+    source.write_text(OUT_OF_HOST_MEMORY)
+    subprocess.run(['g++', '-O1', '-std=c++17', '-I', os.path.join(ROOT, 'include'), '-I/usr/local/cuda/include', str(source), '-o', str(program), '-L', csrc,
+                    '-l:libdist_gnn_b200.so', '-L/usr/local/cuda/lib64', '-lcudart', f'-Wl,-rpath,{csrc}', '-Wl,-rpath,/usr/local/cuda/lib64',
+                    '-Wl,--allow-shlib-undefined'], check=True)
+    done = subprocess.run([str(program)], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, (done.returncode, done.stdout, done.stderr)

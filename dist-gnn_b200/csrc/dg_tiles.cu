@@ -22,8 +22,9 @@
 // rest is waiting for a tile to be filled after an accumulator was drained.
 #include <algorithm>
 #include <atomic>
+#include <cstring>
 #include <new>
-#include <vector>
+#include <utility>
 #include "dg_build.h"
 #include "dg_tiles.h"
 #include "dg_umma.h"
@@ -417,18 +418,32 @@ int panel_width(int32_t F) { const int p = panels_of(F); return ((F + p - 1) / p
 }  // namespace
 
 // ---- finding the tiles -----------------------------------------------------------------------------------------------------
-// One-off, on the device except for sorting the row and column lists (at most some 100,000 keys each) and choosing the tiles.
-// Four passes over the entries of the split rows, one chunk per warp; about 10 ms for 107 M entries.
+// One-off, on the device; the host waits three times, for how many columns are frequent, how many tiles are dense enough and how
+// many segments and chunks came of it.  Four passes over the entries of the split rows, one chunk per warp, and a few over the
+// lists of rows, columns and tiles in between; what bounds it are the atomics on the counts of hub columns and tiles.  With the
+// lists sorted and the tiles chosen on the host, the table of all tiles crossing PCIe twice: 15.8 M entries 7.1 -> 0.9 ms,
+// 40.6 M 12 -> 1.9, 115 M (dense) 17 -> 5.2, 126 M 24 -> 8.0, 260 M 57 -> 15: about what one product of 256 columns takes.
 namespace {
 
 struct SplitRow { int32_t row, len; };
+struct Keyed { int32_t key, id; };
 
-__global__ void k_split_rows(const dg_chunk* __restrict__ chunks, int32_t n_chunks, const int64_t* __restrict__ rowptr, SplitRow* __restrict__ rows)
+struct Found {                            // what the host waits for
+    int32_t columns, least, max_weight;   // frequent columns: how many, from which weight on, the largest
+    int32_t slabs, entries, segments, rest_chunks, rest;
+    int32_t largest;                      // bits of the largest magnitude among the tiled values
+    int32_t pad;
+    long long cost;                       // of all slabs, in half clocks
+};
+
+__global__ void k_split_rows(const dg_chunk* __restrict__ chunks, int32_t n_chunks, const int64_t* __restrict__ rowptr, SplitRow* __restrict__ rows,
+                             Keyed* __restrict__ by_length)
 {
     const int32_t c = blockIdx.x * T + threadIdx.x;
     if (c >= n_chunks || chunks[c].slot != chunks[c].slot0) return;
-    const int32_t r = chunks[c].row;
-    rows[chunks[c].heavy] = SplitRow{r, (int32_t)min((int64_t)INT32_MAX, rowptr[r + 1] - rowptr[r])};
+    const int32_t r = chunks[c].row, h = chunks[c].heavy, len = (int32_t)min((int64_t)INT32_MAX, rowptr[r + 1] - rowptr[r]);
+    rows[h] = SplitRow{r, len};
+    by_length[h] = Keyed{len, h};
 }
 
 // How many entries of split rows every column holds.
@@ -442,29 +457,97 @@ __global__ void __launch_bounds__(T) k_column_weights(const dg_chunk* __restrict
 }
 
 constexpr int kWeightBins = 4096;
-__global__ void __launch_bounds__(T) k_weight_histogram(const int32_t* __restrict__ weight, int32_t k, int32_t* __restrict__ bins)
+__global__ void __launch_bounds__(T) k_weight_histogram(const int32_t* __restrict__ weight, int32_t k, int32_t* __restrict__ bins, Found* __restrict__ found)
 {
     __shared__ int32_t local[kWeightBins];
     for (int i = threadIdx.x; i < kWeightBins; i += T) local[i] = 0;
     __syncthreads();
-    for (int32_t i = blockIdx.x * T + threadIdx.x; i < k; i += gridDim.x * T) atomicAdd(&local[min(weight[i], kWeightBins - 1)], 1);
+    int32_t most = 0;
+    for (int32_t i = blockIdx.x * T + threadIdx.x; i < k; i += gridDim.x * T) {
+        const int32_t w = weight[i];
+        most = max(most, w);
+        atomicAdd(&local[min(w, kWeightBins - 1)], 1);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0) atomicMax(&found->max_weight, most);
     __syncthreads();
     for (int i = threadIdx.x; i < kWeightBins; i += T)
         if (local[i]) atomicAdd(&bins[i], local[i]);
 }
 
-__global__ void k_frequent_columns(const int32_t* __restrict__ weight, int32_t k, int32_t least, int2* __restrict__ out, int32_t capacity, int32_t* __restrict__ count)
+// Columns of at least that weight in the order of their ids.  PASS 0: how many of every T; 1: the columns.
+template <int PASS>
+__global__ void __launch_bounds__(T) k_frequent_columns(const int32_t* __restrict__ weight, int32_t k, int32_t least, int32_t* __restrict__ first,
+                                                        Keyed* __restrict__ out)
 {
     const int32_t i = blockIdx.x * T + threadIdx.x;
-    if (i >= k || weight[i] < least) return;
-    const int32_t at = atomicAdd(count, 1);
-    if (at < capacity) out[at] = make_int2(i, weight[i]);
+    const bool is = i < k && weight[i] >= least;
+    if constexpr (PASS == 0) {
+        const int n = __syncthreads_count(is);
+        if (threadIdx.x == 0) first[blockIdx.x] = n;
+    } else {
+        __shared__ int warp_count[T / 32];
+        const unsigned mine = __ballot_sync(0xffffffffu, is);
+        if ((threadIdx.x & 31) == 0) warp_count[threadIdx.x >> 5] = __popc(mine);
+        __syncthreads();
+        int at = first[blockIdx.x];
+        for (int w = 0; w < (int)threadIdx.x >> 5; ++w) at += warp_count[w];
+        if (is) out[at + __popc(mine & ((1u << (threadIdx.x & 31)) - 1))] = Keyed{weight[i], i};
+    }
 }
 
-__global__ void k_column_ranks(const int32_t* __restrict__ columns, int32_t n, int32_t* __restrict__ rank)
+// One digit of a stable sort, largest keys first.  A CTA takes kSortBlock elements, a warp an eighth of them in strips of 32, in
+// order; equal digits of a strip find one another by __match_any_sync.  PASS 0: how many of every digit, [digit][CTA]; 1: to their places.
+constexpr int kSortBlock = 2048;
+template <int PASS>
+__global__ void __launch_bounds__(T) k_sort_digit(const Keyed* __restrict__ in, Keyed* __restrict__ out, int32_t n, int shift, int32_t* __restrict__ first)
+{
+    constexpr int kWarps = T / 32, kStrips = kSortBlock / T;
+    __shared__ int count[kWarps][256];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < kWarps * 256; i += T) (&count[0][0])[i] = 0;
+    __syncthreads();
+    const int32_t begin = blockIdx.x * kSortBlock + warp * (kSortBlock / kWarps) + lane;
+    Keyed x[kStrips];
+    int place[kStrips];                   // among the warp's elements with this digit
+#pragma unroll
+    for (int s = 0; s < kStrips; ++s) {
+        const int32_t i = begin + s * 32;
+        const bool valid = i < n;
+        if (valid) x[s] = in[i];
+        const int digit = valid ? 255 - (x[s].key >> shift & 255) : 256;
+        const unsigned same = __match_any_sync(0xffffffffu, digit);
+        int before = 0;
+        if (valid) before = count[warp][digit];
+        __syncwarp();
+        place[s] = before + __popc(same & ((1u << lane) - 1));
+        if (valid && lane == __ffs(same) - 1) count[warp][digit] = before + __popc(same);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < 256; d += T) {
+        int sum = PASS == 0 ? 0 : first[(int64_t)d * gridDim.x + blockIdx.x];
+        for (int w = 0; w < kWarps; ++w) {
+            const int c = count[w][d];
+            count[w][d] = sum;
+            sum += c;
+        }
+        if (PASS == 0) first[(int64_t)d * gridDim.x + blockIdx.x] = sum;
+    }
+    if (PASS == 0) return;
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < kStrips; ++s)
+        if (begin + s * 32 < n) out[count[warp][255 - (x[s].key >> shift & 255)] + place[s]] = x[s];
+}
+
+// rank[id] = place in the sorted list; the ids themselves, where wanted.
+__global__ void k_ranks(const Keyed* __restrict__ sorted, int32_t n, int32_t* __restrict__ rank, int32_t* __restrict__ ids)
 {
     const int32_t i = blockIdx.x * T + threadIdx.x;
-    if (i < n) rank[columns[i]] = i;
+    if (i >= n) return;
+    rank[sorted[i].id] = i;
+    if (ids) ids[i] = sorted[i].id;
 }
 
 // MODE 0: how many entries every tile would hold.  MODE 1: how many entries of every chunk lie outside the chosen tiles.
@@ -521,6 +604,172 @@ __global__ void __launch_bounds__(T) k_tile_entries(const dg_chunk* __restrict__
         biggest = __reduce_max_sync(0xffffffffu, biggest);
         if (lane == 0 && biggest > *(volatile int*)largest) atomicMax(largest, biggest);
     }
+}
+
+// The tiles with at least kTileMin entries, in order of row tile and column tile, and what multiplying one costs: 2,400 clocks and
+// 1.5 for every record beyond 1,024 (counted in half clocks).
+struct Chosen { int32_t slabs, entries; long long cost; };
+__device__ __forceinline__ Chosen operator+(const Chosen& a, const Chosen& b) { return Chosen{a.slabs + b.slabs, a.entries + b.entries, a.cost + b.cost}; }
+__device__ __forceinline__ Chosen chosen(int32_t count)
+{
+    return count < kTileMin ? Chosen{0, 0, 0} : Chosen{1, count, 4800 + 3 * (long long)max(0, count - 1024)};
+}
+__device__ __forceinline__ Chosen shift_up(const Chosen& v, int off)
+{
+    return Chosen{__shfl_up_sync(0xffffffffu, v.slabs, off), __shfl_up_sync(0xffffffffu, v.entries, off), __shfl_up_sync(0xffffffffu, v.cost, off)};
+}
+__device__ __forceinline__ Chosen block_before(const Chosen& v, Chosen* warp_sum, Chosen* all)      // sum over the threads before this one
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Chosen s = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const Chosen o = shift_up(s, off);
+        if (lane >= off) s = s + o;
+    }
+    if (lane == 31) warp_sum[warp] = s;
+    Chosen before = shift_up(s, 1);
+    if (lane == 0) before = Chosen{0, 0, 0};
+    __syncthreads();
+    Chosen total{0, 0, 0};
+    for (int w = 0; w < (int)blockDim.x >> 5; ++w) {
+        if (w < warp) before = before + warp_sum[w];
+        total = total + warp_sum[w];
+    }
+    __syncthreads();
+    *all = total;
+    return before;
+}
+
+// One CTA: from which weight on a column is frequent.  The most frequent columns, at most kMaxColumns, and none so rare that a
+// tile could not reach kTileMin with its like.
+__global__ void __launch_bounds__(1024) k_least_weight(const int32_t* __restrict__ bins, Found* __restrict__ found)
+{
+    __shared__ Chosen warp_sum[32];
+    __shared__ int32_t least;
+    if (threadIdx.x == 0) least = kWeightBins;
+    constexpr int kEach = kWeightBins / 1024;
+    Chosen mine{0, 0, 0}, all;
+    int32_t n[kEach];
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) mine.cost += n[j] = bins[kWeightBins - 1 - ((int)threadIdx.x * kEach + j)];
+    long long columns = block_before(mine, warp_sum, &all).cost, kept = 0;
+    int32_t at = kWeightBins;
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        const int32_t w = kWeightBins - 1 - (threadIdx.x * kEach + j);
+        columns += n[j];
+        if (w > kTileMin / kTileCols && columns <= kMaxColumns) at = w, kept = columns;
+    }
+    if (at < kWeightBins) atomicMin(&least, at);
+    __syncthreads();
+    if (at < kWeightBins && at == least) {
+        found->least = at;
+        found->columns = (int32_t)kept;
+    }
+}
+
+constexpr int kChooseBlock = T * 4;
+// PASS 0: sums of every kChooseBlock tiles.  1: the slabs, the table (which slab a tile is, or -1), and which CTA multiplies a slab: equal
+// shares of the cost, in order.
+template <int PASS>
+__global__ void __launch_bounds__(T) k_choose_tiles(int32_t* __restrict__ tile, int64_t tiles, int32_t col_tiles, int32_t ctas, Chosen* __restrict__ sums,
+                                                    dg_slab* __restrict__ slabs, int32_t* __restrict__ cursor, int2* __restrict__ place,
+                                                    const Found* __restrict__ found)
+{
+    __shared__ Chosen warp_sum[T / 32];
+    const int64_t i0 = (int64_t)blockIdx.x * kChooseBlock + threadIdx.x * 4;
+    int32_t count[4];
+    Chosen mine{0, 0, 0}, all;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        count[j] = i0 + j < tiles ? tile[i0 + j] : 0;
+        mine = mine + chosen(count[j]);
+    }
+    Chosen at = block_before(mine, warp_sum, &all);
+    if constexpr (PASS == 0) {
+        if (threadIdx.x == 0) sums[blockIdx.x] = all;
+    } else {
+        at = at + sums[blockIdx.x];
+        const long long cost = found->cost;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (i0 + j >= tiles) break;
+            const Chosen c = chosen(count[j]);
+            tile[i0 + j] = c.slabs ? at.slabs : -1;
+            if (c.slabs) {
+                slabs[at.slabs] = dg_slab{(int32_t)((i0 + j) % col_tiles), at.entries, count[j]};
+                cursor[at.slabs] = at.entries;
+                place[at.slabs] = make_int2((int32_t)((i0 + j) / col_tiles), (int32_t)min((long long)ctas - 1, at.cost * ctas / cost));
+            }
+            at = at + c;
+        }
+    }
+}
+
+// One CTA: exclusive sums over the blocks' sums, in place.
+__global__ void __launch_bounds__(1024) k_sum_chosen(Chosen* __restrict__ sums, int32_t blocks, Found* __restrict__ found)
+{
+    __shared__ Chosen warp_sum[32];
+    Chosen carry{0, 0, 0}, all;
+    for (int32_t b0 = 0; b0 < blocks; b0 += 1024) {
+        const int32_t b = b0 + threadIdx.x;
+        const Chosen before = block_before(b < blocks ? sums[b] : Chosen{0, 0, 0}, warp_sum, &all);
+        if (b < blocks) sums[b] = carry + before;
+        carry = carry + all;
+    }
+    if (threadIdx.x == 0) {
+        found->slabs = carry.slabs;
+        found->entries = carry.entries;
+        found->cost = carry.cost;
+    }
+}
+
+// One CTA: consecutive slabs of one row tile and one CTA are a segment.  `place`: row tile and CTA of every slab.
+__global__ void __launch_bounds__(1024) k_segments(const int2* __restrict__ place, int32_t slabs, int32_t ctas, dg_segment* __restrict__ segments,
+                                                   int32_t* __restrict__ cta_segment, int2* __restrict__ tile_parts, Found* __restrict__ found)
+{
+    __shared__ Chosen warp_sum[32];
+    int32_t carry = 0;
+    for (int32_t s0 = 0; s0 < slabs; s0 += 4 * 1024) {
+        const int32_t b = s0 + threadIdx.x * 4;
+        int2 at[4], before = b > 0 && b <= slabs ? place[b - 1] : make_int2(-1, -1);
+        Chosen mine{0, 0, 0}, all;
+        for (int j = 0; j < 4; ++j) {
+            at[j] = b + j < slabs ? place[b + j] : make_int2(-1, -1);
+            const int2 p = j ? at[j - 1] : before;
+            if (b + j < slabs && (p.x != at[j].x || p.y != at[j].y)) ++mine.slabs;
+        }
+        int32_t g = carry + block_before(mine, warp_sum, &all).slabs;
+        for (int j = 0; j < 4 && b + j < slabs; ++j) {
+            const int2 p = j ? at[j - 1] : before;
+            if (p.x != at[j].x || p.y != at[j].y) {
+                segments[g].slab0 = b + j;
+                segments[g].slot = g;
+                segments[g].pad = 0;
+                if (g > 0) segments[g - 1].slab1 = b + j;
+                for (int c = p.y + 1; c <= at[j].y; ++c) cta_segment[c] = g;
+                if (p.x != at[j].x) tile_parts[at[j].x].x = g;
+                atomicAdd(&tile_parts[at[j].x].y, 1);
+                ++g;
+            }
+            if (b + j == slabs - 1) {
+                segments[g - 1].slab1 = slabs;
+                for (int c = at[j].y + 1; c <= ctas; ++c) cta_segment[c] = g;
+                found->segments = g;
+            }
+        }
+        carry += all.slabs;
+    }
+}
+
+__global__ void k_row_parts(const int32_t* __restrict__ row_rank, int32_t n_rows, const int2* __restrict__ tile_parts, int2* __restrict__ parts)
+{
+    const int32_t h = blockIdx.x * T + threadIdx.x;
+    if (h >= n_rows) return;
+    const int32_t r = row_rank[h];
+    const int2 of = tile_parts[r / kTileRows];
+    parts[h] = make_int2(of.x * kTileRows + r % kTileRows, of.y);
 }
 
 // Exclusive sums in place, one CTA; the total goes behind the last element.
@@ -593,11 +842,17 @@ __global__ void k_first_slots(const dg_chunk* __restrict__ chunks, int32_t n_chu
 
 unsigned grid_of(int64_t n, int per_block) { return (unsigned)((n + per_block - 1) / per_block); }
 
-template <class X> int upload(X** device, const std::vector<X>& host, cudaStream_t stream)
+// `list` sorted by key, largest first, equal keys in the order they have; the result is where the pointer says.
+int sort_keyed(Keyed** list, Keyed** spare, int32_t n, int32_t max_key, int32_t* first, cudaStream_t stream)
 {
-    const int rc = dg_pool_alloc((void**)device, std::max<size_t>(host.size(), 1) * sizeof(X));
-    if (rc) return rc;
-    return host.empty() ? DG_OK : (int)cudaMemcpyAsync(*device, host.data(), host.size() * sizeof(X), cudaMemcpyHostToDevice, stream);
+    const int32_t blocks = (int32_t)grid_of(n, kSortBlock);
+    for (int shift = 0; shift < 32 && (max_key >> shift) > 0; shift += 8) {
+        k_sort_digit<0><<<blocks, T, 0, stream>>>(*list, nullptr, n, shift, first);
+        k_exclusive_sums<<<1, 1024, 0, stream>>>(first, 256 * blocks);
+        k_sort_digit<1><<<blocks, T, 0, stream>>>(*list, *spare, n, shift, first);
+        std::swap(*list, *spare);
+    }
+    return (int)cudaGetLastError();
 }
 
 // Fills `t`; returns DG_OK with t->entries == 0 where tiles would not pay.
@@ -605,151 +860,118 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
 {
     if (p->n_heavy < kTileRows || p->nnz >= ((int64_t)1 << 31)) return DG_OK;
     PoolScope tmp(stream);
-    int rc;
-    SplitRow* d_rows = nullptr;
-    int32_t *first_slot = nullptr, *weight = nullptr, *bins = nullptr, *col_rank = nullptr, *row_rank = nullptr;
-    int2* frequent = nullptr;
-    const size_t bins_n = kWeightBins + 2;
-    if ((rc = tmp.alloc(&d_rows, p->n_heavy)) || (rc = tmp.alloc(&first_slot, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&weight, p->k)) ||
-        (rc = tmp.alloc(&bins, bins_n)) || (rc = tmp.alloc(&col_rank, p->k)) || (rc = tmp.alloc(&row_rank, p->n_heavy)) ||
-        (rc = tmp.alloc(&frequent, kMaxColumns)))
+    int rc, dev = 0, ctas = 0;
+    DG_CUDA(cudaGetDevice(&dev));
+    DG_CUDA(cudaDeviceGetAttribute(&ctas, cudaDevAttrMultiProcessorCount, dev));
+    SplitRow* rows = nullptr;
+    Keyed *by_length = nullptr, *frequent = nullptr, *spare = nullptr;
+    int32_t *first_slot = nullptr, *weight = nullptr, *bins = nullptr, *col_rank = nullptr, *row_rank = nullptr, *first = nullptr;
+    Found* found = nullptr;
+    const int32_t longest_list = std::max(p->n_heavy, kMaxColumns), column_blocks = (int32_t)grid_of(p->k, T);
+    const size_t sums = std::max<size_t>((size_t)256 * grid_of(longest_list, kSortBlock), column_blocks) + 1;
+    if ((rc = tmp.alloc(&rows, p->n_heavy)) || (rc = tmp.alloc(&by_length, p->n_heavy)) || (rc = tmp.alloc(&spare, longest_list)) ||
+        (rc = tmp.alloc(&first, sums)) || (rc = tmp.alloc(&first_slot, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&weight, p->k)) ||
+        (rc = tmp.alloc(&bins, kWeightBins)) || (rc = tmp.alloc(&col_rank, p->k)) || (rc = tmp.alloc(&row_rank, p->n_heavy)) ||
+        (rc = tmp.alloc(&frequent, kMaxColumns)) || (rc = tmp.alloc(&found, 1)))
         return rc;
     DG_CUDA(cudaMemsetAsync(weight, 0, (size_t)p->k * sizeof(int32_t), stream));
-    DG_CUDA(cudaMemsetAsync(bins, 0, bins_n * sizeof(int32_t), stream));
+    DG_CUDA(cudaMemsetAsync(bins, 0, kWeightBins * sizeof(int32_t), stream));
+    DG_CUDA(cudaMemsetAsync(found, 0, sizeof(Found), stream));
     DG_CUDA(cudaMemsetAsync(col_rank, 0xff, (size_t)p->k * sizeof(int32_t), stream));
-    k_split_rows<<<grid_of(p->n_chunks, T), T, 0, stream>>>(p->chunks, p->n_chunks, p->rowptr, d_rows);
+    k_split_rows<<<grid_of(p->n_chunks, T), T, 0, stream>>>(p->chunks, p->n_chunks, p->rowptr, rows, by_length);
     k_first_slots<<<grid_of(p->n_chunks, T), T, 0, stream>>>(p->chunks, p->n_chunks, p->n_heavy, first_slot);
     k_column_weights<<<grid_of(p->n_chunks, T / 32), T, 0, stream>>>(p->chunks, p->n_chunks, p->col, weight);
-    k_weight_histogram<<<148, T, 0, stream>>>(weight, p->k, bins);
-    std::vector<int32_t> h_bins(kWeightBins);
-    std::vector<SplitRow> h_rows((size_t)p->n_heavy);
-    DG_CUDA(cudaMemcpyAsync(h_bins.data(), bins, kWeightBins * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaMemcpyAsync(h_rows.data(), d_rows, h_rows.size() * sizeof(SplitRow), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaStreamSynchronize(stream));
+    k_weight_histogram<<<148, T, 0, stream>>>(weight, p->k, bins, found);
+    k_least_weight<<<1, 1024, 0, stream>>>(bins, found);
+    Found h{};
+    auto read = [&] {
+        const cudaError_t e = cudaMemcpyAsync(&h, found, sizeof(h), cudaMemcpyDeviceToHost, stream);
+        return (int)(e != cudaSuccess ? e : cudaStreamSynchronize(stream));
+    };
+    if ((rc = read())) return rc;
+    if (h.columns < kTileCols) return DG_OK;
 
-    // the most frequent columns, at most kMaxColumns, and none so rare that a tile could not reach kTileMin with its like
-    int32_t least = kWeightBins - 1;
-    int64_t columns = h_bins[kWeightBins - 1];
-    while (least > 1 + kTileMin / kTileCols && columns + h_bins[least - 1] <= kMaxColumns) columns += h_bins[--least];
-    if (columns < kTileCols || columns > kMaxColumns) return DG_OK;
-    int32_t *d_count = bins + kWeightBins, *largest = d_count + 1;
-    k_frequent_columns<<<grid_of(p->k, T), T, 0, stream>>>(weight, p->k, least, frequent, kMaxColumns, d_count);
-    std::vector<int2> h_frequent((size_t)columns);
-    DG_CUDA(cudaMemcpyAsync(h_frequent.data(), frequent, h_frequent.size() * sizeof(int2), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaStreamSynchronize(stream));
-    std::sort(h_frequent.begin(), h_frequent.end(), [](const int2& a, const int2& b) { return a.y != b.y ? a.y > b.y : a.x < b.x; });
-    std::vector<int32_t> h_columns(h_frequent.size());
-    for (size_t i = 0; i < h_columns.size(); ++i) h_columns[i] = h_frequent[i].x;
-    t->n_columns = (int32_t)columns;
-    t->col_tiles = (int32_t)((columns + kTileCols - 1) / kTileCols);
-    // longest rows first
-    std::vector<int32_t> by_length(h_rows.size()), h_rank(h_rows.size());
-    for (size_t i = 0; i < by_length.size(); ++i) by_length[i] = (int32_t)i;
-    std::stable_sort(by_length.begin(), by_length.end(), [&](int32_t a, int32_t b) { return h_rows[a].len > h_rows[b].len; });
-    for (size_t i = 0; i < by_length.size(); ++i) h_rank[by_length[i]] = (int32_t)i;
-
-    const int32_t row_tiles = (p->n_heavy + kTileRows - 1) / kTileRows;
+    // columns by weight, rows by length
+    t->n_columns = h.columns;
+    t->col_tiles = (int32_t)grid_of(h.columns, kTileCols);
+    const int32_t row_tiles = (int32_t)grid_of(p->n_heavy, kTileRows);
     const int64_t tiles = (int64_t)row_tiles * t->col_tiles;
     if (tiles > (int64_t)1 << 26) return DG_OK;
+    const int32_t choose_blocks = (int32_t)grid_of(tiles, kChooseBlock);
     int32_t *tile = nullptr, *rest = nullptr;
-    if ((rc = upload(&t->columns, h_columns, stream)) || (rc = tmp.alloc(&tile, (size_t)tiles)) || (rc = tmp.alloc(&rest, (size_t)p->n_chunks + 1))) return rc;
-    DG_CUDA(cudaMemcpyAsync(row_rank, h_rank.data(), h_rank.size() * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-    k_column_ranks<<<grid_of(columns, T), T, 0, stream>>>(t->columns, t->n_columns, col_rank);
+    Chosen* chosen_sums = nullptr;
+    if ((rc = dg_pool_alloc((void**)&t->columns, (size_t)h.columns * sizeof(int32_t))) || (rc = tmp.alloc(&tile, (size_t)tiles)) ||
+        (rc = tmp.alloc(&rest, (size_t)p->n_chunks + 1)) || (rc = tmp.alloc(&chosen_sums, (size_t)choose_blocks)))
+        return rc;
+    k_frequent_columns<0><<<column_blocks, T, 0, stream>>>(weight, p->k, h.least, first, nullptr);
+    k_exclusive_sums<<<1, 1024, 0, stream>>>(first, column_blocks);
+    k_frequent_columns<1><<<column_blocks, T, 0, stream>>>(weight, p->k, h.least, first, frequent);
+    Keyed* other = spare;                               // the sorted columns are read before the rows are sorted
+    if ((rc = sort_keyed(&frequent, &other, h.columns, h.max_weight, first, stream))) return rc;
+    k_ranks<<<grid_of(h.columns, T), T, 0, stream>>>(frequent, h.columns, col_rank, t->columns);
+    if ((rc = sort_keyed(&by_length, &spare, p->n_heavy, (int32_t)std::min<int64_t>(INT32_MAX, p->max_row_nnz), first, stream))) return rc;
+    k_ranks<<<grid_of(p->n_heavy, T), T, 0, stream>>>(by_length, p->n_heavy, row_rank, nullptr);
+
+    // how full the tiles are, and which of them are worth it
     DG_CUDA(cudaMemsetAsync(tile, 0, (size_t)tiles * sizeof(int32_t), stream));
     const unsigned warps = grid_of(p->n_chunks, T / 32);
     k_tile_entries<0><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
-    std::vector<int32_t> h_tile((size_t)tiles);
-    DG_CUDA(cudaMemcpyAsync(h_tile.data(), tile, h_tile.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaStreamSynchronize(stream));
+    k_choose_tiles<0><<<choose_blocks, T, 0, stream>>>(tile, tiles, t->col_tiles, ctas, chosen_sums, nullptr, nullptr, nullptr, found);
+    k_sum_chosen<<<1, 1024, 0, stream>>>(chosen_sums, choose_blocks, found);
+    if ((rc = read())) return rc;
+    if (h.slabs == 0 || h.entries < p->nnz / 8) return DG_OK;      // the columns' images and another launch cost more than that saves
 
-    std::vector<dg_slab> slabs;
-    std::vector<int32_t> h_cursor, slab_row_tile;
-    int64_t entries = 0;
-    double cost = 0;
-    auto slab_cost = [](int32_t count) { return 2400.0 + 1.5 * std::max(0, count - 1024); };      // clocks, as measured
-    for (int64_t i = 0; i < tiles; ++i) {
-        const int32_t count = h_tile[i];
-        h_tile[i] = -1;
-        if (count < kTileMin) continue;
-        h_tile[i] = (int32_t)slabs.size();
-        slab_row_tile.push_back((int32_t)(i / t->col_tiles));
-        h_cursor.push_back((int32_t)entries);
-        slabs.push_back(dg_slab{(int32_t)(i % t->col_tiles), (int32_t)entries, count});
-        entries += count;
-        cost += slab_cost(count);
-    }
-    if (slabs.empty() || entries < p->nnz / 8) return DG_OK;       // the columns' images and another launch cost more than that saves
+    // the slabs, equal shares of the work for every CTA, cut again where the row tile changes
+    t->n_slabs = h.slabs;
+    t->ctas = ctas;
+    const int64_t left = p->heavy_nnz - h.entries, max_segments = std::min<int64_t>(h.slabs, (int64_t)row_tiles + ctas),
+                  max_rest_chunks = std::min<int64_t>(p->n_chunks, p->n_heavy + left / p->chunk);
+    int32_t *cursor = nullptr, *chunk_first = nullptr, *bands = nullptr;
+    int2 *place = nullptr, *tile_parts = nullptr;
+    if ((rc = tmp.alloc(&cursor, (size_t)h.slabs)) || (rc = tmp.alloc(&place, (size_t)h.slabs)) || (rc = tmp.alloc(&tile_parts, (size_t)row_tiles)) ||
+        (rc = tmp.alloc(&chunk_first, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&bands, kBands + 1)) ||
+        (rc = dg_pool_alloc((void**)&t->slabs, (size_t)h.slabs * sizeof(dg_slab))) ||
+        (rc = dg_pool_alloc((void**)&t->segments, (size_t)max_segments * sizeof(dg_segment))) ||
+        (rc = dg_pool_alloc((void**)&t->cta_segment, ((size_t)ctas + 1) * sizeof(int32_t))) ||
+        (rc = dg_pool_alloc((void**)&t->parts, (size_t)p->n_heavy * sizeof(int2))) ||
+        (rc = dg_pool_alloc((void**)&t->records, (size_t)h.entries * sizeof(uint2))) ||
+        (rc = dg_pool_alloc((void**)&t->rest_col, (size_t)std::max<int64_t>(left, 1) * sizeof(int32_t))) ||
+        (rc = dg_pool_alloc((void**)&t->rest_val, (size_t)std::max<int64_t>(left, 1) * sizeof(float))) ||
+        (rc = dg_pool_alloc((void**)&t->rest_chunks, (size_t)max_rest_chunks * sizeof(dg_chunk))) ||
+        (rc = dg_pool_alloc(&t->value_sums, (size_t)ctas * kValueWarps * sizeof(ValueSum))))
+        return rc;
+    DG_CUDA(cudaMemsetAsync(tile_parts, 0, (size_t)row_tiles * sizeof(int2), stream));
+    DG_CUDA(cudaMemsetAsync(bands, 0, kBands * sizeof(int32_t), stream));
+    k_choose_tiles<1><<<choose_blocks, T, 0, stream>>>(tile, tiles, t->col_tiles, ctas, chosen_sums, t->slabs, cursor, place, found);
+    k_segments<<<1, 1024, 0, stream>>>(place, h.slabs, ctas, t->segments, t->cta_segment, tile_parts, found);
+    k_row_parts<<<grid_of(p->n_heavy, T), T, 0, stream>>>(row_rank, p->n_heavy, tile_parts, t->parts);
 
-    // equal shares of the work for every CTA, cut again where the row tile changes
-    int dev = 0, ctas = 0;
-    DG_CUDA(cudaGetDevice(&dev));
-    DG_CUDA(cudaDeviceGetAttribute(&ctas, cudaDevAttrMultiProcessorCount, dev));
-    std::vector<dg_segment> segments;
-    std::vector<int32_t> cta_segment(1, 0), tile_slot(row_tiles, 0), tile_parts(row_tiles, 0);
-    double done = 0;
-    for (size_t s = 0; s < slabs.size(); ++s) {
-        const bool new_cta = (int)cta_segment.size() < ctas && done >= cost * (double)cta_segment.size() / ctas && s > 0;
-        const bool new_row = s == 0 || slab_row_tile[s] != slab_row_tile[s - 1];
-        if (new_cta) cta_segment.push_back((int32_t)segments.size());
-        if (new_cta || new_row) {
-            if (!segments.empty()) segments.back().slab1 = (int32_t)s;
-            const int32_t rt = slab_row_tile[s], slot = (int32_t)segments.size();
-            if (new_row) tile_slot[rt] = slot;
-            ++tile_parts[rt];
-            segments.push_back(dg_segment{(int32_t)s, (int32_t)slabs.size(), slot, 0});
-        }
-        done += slab_cost(slabs[s].count);
-    }
-    t->ctas = (int32_t)cta_segment.size();
-    cta_segment.push_back((int32_t)segments.size());
-    std::vector<int2> parts(h_rows.size());
-    for (size_t h = 0; h < parts.size(); ++h) {
-        const int32_t rt = h_rank[h] / kTileRows;
-        parts[h] = make_int2(tile_slot[rt] * kTileRows + h_rank[h] % kTileRows, tile_parts[rt]);
-    }
-
-    int32_t* cursor = nullptr;
-    if ((rc = tmp.alloc(&cursor, slabs.size()))) return rc;
-    DG_CUDA(cudaMemcpyAsync(tile, h_tile.data(), h_tile.size() * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-    DG_CUDA(cudaMemcpyAsync(cursor, h_cursor.data(), h_cursor.size() * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+    // the entries into the slabs' records and into what is left of the rows, with its chunks in the order of the column band they start in
     k_tile_entries<1><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, nullptr, rest, nullptr, nullptr, nullptr, nullptr);
     k_exclusive_sums<<<1, 1024, 0, stream>>>(rest, p->n_chunks);
-    int32_t h_rest = 0;
-    DG_CUDA(cudaMemcpyAsync(&h_rest, rest + p->n_chunks, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaStreamSynchronize(stream));
-    if (h_rest != p->heavy_nnz - entries) return DG_ERR_STATE;     // cannot happen
-    if ((rc = dg_pool_alloc((void**)&t->records, (size_t)entries * sizeof(uint2))) ||
-        (rc = dg_pool_alloc((void**)&t->rest_col, std::max<size_t>(h_rest, 1) * sizeof(int32_t))) ||
-        (rc = dg_pool_alloc((void**)&t->rest_val, std::max<size_t>(h_rest, 1) * sizeof(float))) || (rc = upload(&t->slabs, slabs, stream)) ||
-        (rc = upload(&t->segments, segments, stream)) || (rc = upload(&t->cta_segment, cta_segment, stream)) || (rc = upload(&t->parts, parts, stream)))
-        return rc;
     k_tile_entries<2><<<warps, T, 0, stream>>>(p->chunks, p->n_chunks, p->col, val, row_rank, col_rank, t->col_tiles, tile, cursor, rest, t->records, t->rest_col,
-                                               t->rest_val, largest);
-    // chunks of the rest, in the order of the column band they start in
-    int32_t *chunk_first = nullptr, *bands = nullptr;
-    if ((rc = tmp.alloc(&chunk_first, (size_t)p->n_heavy + 1)) || (rc = tmp.alloc(&bands, kBands + 1))) return rc;
-    DG_CUDA(cudaMemsetAsync(bands, 0, kBands * sizeof(int32_t), stream));
+                                               t->rest_val, &found->largest);
     const unsigned row_blocks = grid_of(p->n_heavy, T);
-    k_rest_chunks<0><<<row_blocks, T, 0, stream>>>(d_rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, nullptr);
+    k_rest_chunks<0><<<row_blocks, T, 0, stream>>>(rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, nullptr);
     k_exclusive_sums<<<1, 1024, 0, stream>>>(chunk_first, p->n_heavy);
-    k_rest_chunks<1><<<row_blocks, T, 0, stream>>>(d_rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, nullptr);
+    k_rest_chunks<1><<<row_blocks, T, 0, stream>>>(rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, nullptr);
     k_exclusive_sums<<<1, 1024, 0, stream>>>(bands, kBands);
-    DG_CUDA(cudaMemcpyAsync(&t->n_rest_chunks, chunk_first + p->n_heavy, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaStreamSynchronize(stream));
-    if ((rc = dg_pool_alloc((void**)&t->rest_chunks, (size_t)t->n_rest_chunks * sizeof(dg_chunk)))) return rc;
-    k_rest_chunks<2><<<row_blocks, T, 0, stream>>>(d_rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, t->rest_chunks);
-    if ((rc = dg_pool_alloc(&t->value_sums, (size_t)t->ctas * kValueWarps * sizeof(ValueSum)))) return rc;
-    k_value_sums<<<t->ctas, 32 * kValueWarps, 0, stream>>>(val, p->nnz, static_cast<ValueSum*>(t->value_sums));
-    float h_largest = 0.f;
-    DG_CUDA(cudaMemcpyAsync(&h_largest, largest, sizeof(float), cudaMemcpyDeviceToHost, stream));
-    DG_CUDA(cudaStreamSynchronize(stream));
+    k_rest_chunks<2><<<row_blocks, T, 0, stream>>>(rows, p->n_heavy, first_slot, rest, p->chunk, t->rest_col, p->k, chunk_first, bands, t->rest_chunks);
+    k_value_sums<<<ctas, 32 * kValueWarps, 0, stream>>>(val, p->nnz, static_cast<ValueSum*>(t->value_sums));
+    DG_CUDA(cudaMemcpyAsync(&found->rest_chunks, chunk_first + p->n_heavy, sizeof(int32_t), cudaMemcpyDeviceToDevice, stream));
+    DG_CUDA(cudaMemcpyAsync(&found->rest, rest + p->n_chunks, sizeof(int32_t), cudaMemcpyDeviceToDevice, stream));
+    if ((rc = read())) return rc;
+    tmp.idle = true;
     DG_CUDA(cudaGetLastError());
-    if (!(h_largest < kTileBound) || h_largest < kTileLeast) return DG_OK;
-    t->least_operand = h_largest < 1.f ? kTileLeast / h_largest : kTileLeast;
+    if (h.rest != left || h.rest_chunks > max_rest_chunks || h.segments > max_segments) return DG_ERR_STATE;     // cannot happen
+    float largest;
+    memcpy(&largest, &h.largest, sizeof(float));
+    if (!(largest < kTileBound) || largest < kTileLeast) return DG_OK;
+    t->least_operand = largest < 1.f ? kTileLeast / largest : kTileLeast;
     t->val = val;
-    t->n_slabs = (int32_t)slabs.size();
-    t->n_segments = (int32_t)segments.size();
-    t->entries = entries;
+    t->n_segments = h.segments;
+    t->n_rest_chunks = h.rest_chunks;
+    t->entries = h.entries;
     return DG_OK;
 }
 

@@ -18,7 +18,7 @@ struct PoolScope {
     ~PoolScope()
     {
         if (!idle && !blocks.empty()) cudaStreamSynchronize(stream);
-        for (void* p : blocks) dg_pool_free(p);
+        for (void* p : blocks) dg_pool_free(p, true);
     }
     template <class X> int alloc(X** out, size_t count)
     {

@@ -3,12 +3,22 @@
 // A training step on a small graph is bound by the host: some twenty launches of a few microseconds each, issued through
 // an interpreter that needs ten times that between them (1.2 ms a step on the 10,000-node graph, 0.3 ms of it on the
 // device).  These two functions issue the layers' products and transforms back to back.
+#include <algorithm>
 #include "dg_internal.h"
 
 namespace {
 
 int64_t pad4(int64_t w) { return (w + 3) / 4 * 4; }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// The plan's scratch for every width of the network, the backward pass's among them, before the first product: grown width by
+// width, the first pass waited for the device and went to the allocator up to three times in its middle.
+int prepare(const dg_gcn_net* a, void* stream)
+{
+    int64_t widest = 0;
+    for (int l = 0; l <= a->layers; ++l) widest = std::max(widest, pad4(a->dims[l]));
+    return dg_spmm_prepare(a->plan, (int32_t)widest, (cudaStream_t)stream);
+}
 
 struct Marks {          // ids of the points between the regions of one call; a failed record is reported by its negative id
     int32_t* at;
@@ -45,9 +55,10 @@ int product(const dg_gcn_net* a, const float* b, int64_t ldb, int32_t width, voi
 }  // namespace
 
 extern "C" int dg_gcn_forward(const dg_gcn_net* a, void* stream)
-{
+try {
     int rc = check_net(a, false);
     if (rc || a->n == 0) return rc;
+    if ((rc = prepare(a, stream))) return rc;
     Marks mark{a->marks, stream};
     mark();
     const float* in = a->x;
@@ -66,12 +77,15 @@ extern "C" int dg_gcn_forward(const dg_gcn_net* a, void* stream)
         ld_in = a->ld_act[l];
     }
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }
 
 extern "C" int dg_gcn_backward(const dg_gcn_net* a, void* stream)
-{
+try {
     int rc = check_net(a, true);
     if (rc || a->n == 0) return rc;
+    if ((rc = prepare(a, stream))) return rc;
     Marks mark{a->marks, stream};
     mark();
     const float* g = a->grad;
@@ -95,4 +109,6 @@ extern "C" int dg_gcn_backward(const dg_gcn_net* a, void* stream)
         ld_g = pad4(K);
     }
     return DG_OK;
+} catch (...) {
+    return dg_exception();
 }

@@ -100,7 +100,7 @@ int dg_plan_ensure_tasks(dg_plan* plan, cudaStream_t stream);
 // Device memory of plans (dg_pool.cu), on the current device.  A block may be freed once the device is done with it.
 int dg_pool_alloc(void** out, size_t bytes);
 int dg_device_alloc(void** out, size_t bytes);      // not from the pool, freed with cudaFree
-void dg_pool_free(void* ptr) noexcept;
+void dg_pool_free(void* ptr, bool building = false) noexcept;      // building: a temporary of plan construction
 int* dg_status_word();        // the current device's, or null
 int dg_spmm_prepare(const dg_plan* plan, int32_t F, cudaStream_t stream);
 int dg_check_spmm_args(const dg_plan* plan, const float* val, const float* B, int64_t ldb, const float* C, int64_t ldc,

@@ -3,10 +3,12 @@
 // cudaMalloc and cudaFree cost tens of microseconds at best and, on a device whose memory is mostly mapped, now and then
 // milliseconds; building a plan took 45 of the former and 54 of the latter, most of the 8 to 30 ms that plan construction
 // and one product of a 300 k-row block cost.  Freed blocks are kept per device, at most kKeepBytes of them, and handed out
-// again to requests of a similar size.  A block that does not fit any more pushes out those that have lain idle longest: what
-// earlier, larger plans left behind must not keep the blocks of those in use now from staying (plan and product of a 55,160-node
-// matrix after others had filled the pool: 930 -> 180 us).  A block may come back only when the device is done with it: callers synchronise
-// first (dg_plan_destroy the device, as cudaFree did; plan construction its stream).
+// again to requests of a similar size; twice as many while a plan is being built, whose temporaries come back in the middle of
+// a caller's call, where a cudaFree would wait for the device: dg_plan_destroy brings the pool back to its size.  A block that does
+// not fit any more pushes out those that have lain idle longest: what earlier, larger plans left behind must not keep the blocks of
+// those in use now from staying (plan and product of a 55,160-node matrix after others had filled the pool: 930 -> 180 us).  A
+// block may come back only when the device is done with it: callers synchronise first (dg_plan_destroy the device, as cudaFree did;
+// plan construction its stream).
 //
 // The program around the library usually has a caching allocator of its own, which may hold the whole device without using it.
 // So an allocation that the driver refuses is tried three times: as it is, after the pool has given its idle blocks back, and
@@ -155,8 +157,9 @@ int dg_pool_alloc(void** out, size_t bytes)
     return DG_OK;
 }
 
-void dg_pool_free(void* ptr) noexcept
+void dg_pool_free(void* ptr, bool building) noexcept
 {
+    const size_t keep = building ? 2 * kKeepBytes : kKeepBytes;
     int dev = -1;
     if (!ptr || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
     Pool& p = pool();
@@ -169,7 +172,7 @@ void dg_pool_free(void* ptr) noexcept
         return;
     }
     auto& unused = p.unused[dev];
-    while (p.unused_bytes[dev] + it->second > kKeepBytes) {
+    while (p.unused_bytes[dev] + it->second > keep) {
         auto oldest = unused.begin();
         for (auto u = unused.begin(); u != unused.end(); ++u)
             if (u->second.since < oldest->second.since) oldest = u;

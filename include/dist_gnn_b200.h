@@ -84,7 +84,7 @@ int dg_plan_destroy(dg_plan* plan);
 int dg_plan_add_tiles(dg_plan* plan, const float* val, void* stream);
 int dg_plan_drop_tiles(dg_plan* plan, void* stream);
 int64_t dg_plan_tiled_entries(const dg_plan* plan);
-/* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device; this gives all of it on the current
+/* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device (1 GB until the next plan is destroyed, where one was being built); this gives all of it on the current
  * device back (a failed allocation of the library does so by itself). */
 int dg_pool_trim(void);
 /* `give_back` is called (on the allocating thread, with the allocating device current and none of the library's locks held) when

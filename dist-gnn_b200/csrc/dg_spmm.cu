@@ -493,8 +493,8 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
     a.chunk_col = plan->col; a.chunk_val = val;
     a.ldb = ldb; a.ldc = ldc; a.lds = F; a.m = plan->m; a.F = F;
     a.heavy_threshold = split ? plan->heavy_threshold : INT32_MAX; a.n_chunks = split ? plan->n_chunks : 0;
-    // Rows per CTA: as wide a window as still gives every SM a dozen CTAs (wider windows sort better and share their offsets;
-    // 64 rows are best at 150 k rows, 128 at 300 k, 256 from 1 M).
+    // Rows per CTA: as wide a window as still makes 2,000 of them, 13 for each of the B200's 148 SMs (wider windows sort better and
+    // share their offsets; 64 rows are best at 150 k rows, 128 at 300 k, 256 from 1 M).
     a.rows_per_cta = 32;
     while (a.rows_per_cta < 256 && (int64_t)a.rows_per_cta * 2 * 2000 <= plan->m) a.rows_per_cta *= 2;
     a.alpha = alpha; a.beta = beta; a.flags = flags;

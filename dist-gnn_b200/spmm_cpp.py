@@ -20,8 +20,12 @@ _lib = None
 
 # Blocks of at least TILE_NNZ entries whose plans are kept for many products (plan_for, the joined blocks of the stage loops) get
 # tensor-core tiles: below that the images of the frequent columns and two more launches cost what the tiles save (2.5 M
-# entries: nothing gained; 15.8 M: a fifth).  From TILE_ALWAYS entries on every plan made from a loader's block gets them:
-# normalising and sorting such a block took ten times as long as finding its tiles.
+# entries: nothing gained; 15.8 M: a sixth).  Finding the tiles takes about one product of 256 columns at any size, and it is paid
+# back by 2 to 15 of them (R-MAT, search and saving per product at F = 256: 15.8 M entries 0.9 ms and 0.16, 40.6 M 1.9 and 0.42,
+# 65 M 3.9 and 0.55, 126 M 8.0 and 0.54, 260 M 15 and 1.6; 115 M on few nodes 5.3 and 2.5): what decides is not the size but how
+# often the block will be multiplied, which SpmmPlan.from_coo is not told unless its caller says (`tiles`).  Left to itself it
+# takes a block of TILE_ALWAYS entries for a matrix that its program holds: wrong, that costs one product, once; not taking it would cost
+# 5 to 40 % of every one.  Smaller blocks, which also come one after the other from a loader, are left as they are.
 TILE_NNZ = 8 << 20
 TILE_ALWAYS = 48 << 20
 
@@ -225,15 +229,17 @@ class SpmmPlan:
         self._own(handle)
 
     @classmethod
-    def from_coo(cls, A, heavy_threshold=0, chunk=0):
-        """From a coalesced torch sparse COO tensor on a CUDA device (int64 indices are narrowed once, here)."""
+    def from_coo(cls, A, heavy_threshold=0, chunk=0, tiles=None):
+        """From a coalesced torch sparse COO tensor on a CUDA device (int64 indices are narrowed once, here).  tiles: True for a
+        block that will be multiplied many times (see tile), False for one that will not; None goes by its size."""
         if not A.is_coalesced():
             A = A.coalesce()
         idx, values = A.indices(), A.values().contiguous()
         if max(A.shape) >= 2**31:
             raise RuntimeError('block dimensions must fit int32')
         if not (idx.is_cuda and idx.dtype == torch.int64 and idx.stride(1) == 1):
-            return cls(idx[0].to(torch.int32), idx[1].to(torch.int32).contiguous(), values, A.size(0), A.size(1), heavy_threshold, chunk)
+            self = cls(idx[0].to(torch.int32), idx[1].to(torch.int32).contiguous(), values, A.size(0), A.size(1), heavy_threshold, chunk)
+            return self.tile() if tiles else self
         self = cls.__new__(cls)
         _dev_tensor(values, torch.float32, 'values')
         nnz = values.numel()
@@ -244,7 +250,7 @@ class SpmmPlan:
             check(lib().dg_plan_create_i64(base, base + 8 * idx.stride(0), nnz, self.m, self.k, heavy_threshold, chunk, self.col.data_ptr(),
                                            _raw_stream(index), ctypes.byref(handle)))
         self._own(handle)
-        return self.tile() if nnz >= TILE_ALWAYS else self
+        return self.tile() if (nnz >= TILE_ALWAYS if tiles is None else tiles) else self
 
     def _own(self, handle):
         # the binding's reference destroys the plan when this object and every autograd graph that uses it are gone
@@ -381,7 +387,7 @@ def plan_for(A):
     hit = _plan_cache.get(key)
     if hit is not None and hit[0]() is A:
         return hit[1]
-    plan = SpmmPlan.from_coo(A).tile()
+    plan = SpmmPlan.from_coo(A, tiles=True)
     _plan_cache[key] = (weakref.ref(A, lambda _ref, key=key: _plan_cache.pop(key, None)), plan)
     return plan
 

@@ -811,3 +811,19 @@ def test_host_allocations_that_fail_come_back_as_codes(tmp_path):
                     '-Wl,--allow-shlib-undefined'], check=True)
     done = subprocess.run([str(program)], capture_output=True, text=True, timeout=120)
     assert done.returncode == 0, (done.returncode, done.stdout, done.stderr)
+
+
+@pytest.mark.parametrize('tiles,many', [(None, False), (False, False), (True, True)])
+def test_caller_says_whether_a_block_is_multiplied_often(monkeypatch, tiles, many):
+    """from_coo goes by the size unless its caller knows better; both ends of the size rule."""
+    import spmm_cpp
+    A = skewed_block(17)
+    t = torch.sparse_coo_tensor(torch.from_numpy(np.stack((A.row, A.col))), torch.from_numpy(A.val), A.shape, is_coalesced=True).cuda()
+    monkeypatch.setattr(spmm_cpp, 'TILE_NNZ', A.nnz)
+    assert (spmm_cpp.SpmmPlan.from_coo(t, tiles=tiles).tiled_entries() > 0) == many
+    monkeypatch.setattr(spmm_cpp, 'TILE_ALWAYS', A.nnz)
+    assert (spmm_cpp.SpmmPlan.from_coo(t, tiles=tiles).tiled_entries() > 0) == (tiles is not False)
+    monkeypatch.setattr(spmm_cpp, 'TILE_ALWAYS', A.nnz + 1)
+    assert (spmm_cpp.SpmmPlan.from_coo(t, tiles=tiles).tiled_entries() > 0) == many
+    monkeypatch.setattr(spmm_cpp, 'TILE_NNZ', A.nnz + 1)
+    assert spmm_cpp.SpmmPlan.from_coo(t, tiles=tiles).tiled_entries() == 0

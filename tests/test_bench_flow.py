@@ -75,3 +75,14 @@ def test_failed_parity_of_the_extra_measurement_is_loud():
     assert out.returncode != 0
     assert len(lines) == 1 and lines[0]['config3']['parity']['ok'] is False
     assert 'config3' in out.stderr
+
+
+def test_reference_arm_without_the_reference_says_so(monkeypatch, capsys, tmp_path):
+    """No restatement is timed in the reference's place: one line that says why there is no figure."""
+    import bench
+    monkeypatch.setattr(bench, 'REF_DIR', str(tmp_path / 'absent'))
+    monkeypatch.setattr(bench, 'run_port_sample', lambda *a: pytest.fail('the port was run as the reference'))
+    monkeypatch.setattr(sys, 'argv', ['bench.py', '--impl', 'reference', '--config', 'plumbing'])
+    bench.run_reference(bench.parse())
+    line = json.loads(capsys.readouterr().out)
+    assert line['impl'] == 'reference' and line['unavailable'] and 'value' not in line

@@ -54,10 +54,10 @@ struct SpmmArgs {
     const dg_chunk* chunks;
     const int32_t* chunk_col;   // entries of the chunks: the matrix's own, or what the tiles leave of the split rows
     const float* chunk_val;
-    const int2* parts;          // partial results of the tiles per split row (dg_tiles.h), or null
+    const int2* parts;          // kTiled: partial results of the tiles per split row (dg_tiles.h)
     const float4* part_area;
     int64_t part_ld4;           // 16-byte pieces of a partial row
-    int* tile_words;            // with tiles: dg_plan::status + DG_TILE_WORDS, else null
+    int* tile_words;            // kTiled, kWhole: dg_plan::status + DG_TILE_WORDS
     int* arrived;               // [n_heavy x DG_FINISH_TILES] partial sums of a split row that are in place; zero between products
     float* scratch;
     int64_t ldb, ldc, lds;      // lds: row stride of the partial sums
@@ -117,16 +117,20 @@ __device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const floa
 // the last rows of a CTA are short ones.  The first entries of the next G rows are requested before the current ones are
 // gathered.
 //
-// What bounds it: the gathers.  512-byte rows that miss nothing but the L1 move at 18.8 TB/s (64 bytes a clock and SM), and
-// large graphs run at that rate times their L2 hit rate; small ones and short rows are bound by latency, which the offsets in
-// shared memory, the look-ahead and U hide.  Against separate kernels with a warp per row (B200, us per product):
+// What bounds it: the gathers.  Rows that the L2 holds come at 18 TB/s, 64 bytes a clock and SM (dense graph, F = 256: 41 GB in
+// 2.30 ms with the L2 at 78 % of its throughput, the path from it to the SMs at 49 %, issue slots at 46 %); larger graphs are held
+// up by the L2 and by what misses it (1 M nodes, 49 M entries: L2 64 %, DRAM 48 %, hit rate 63 %); small ones and short rows
+// are bound by latency, which the offsets in shared memory, the look-ahead and U hide.  Against separate kernels with a warp per row (B200, us per product):
 //   10,000 nodes, 210 k entries, F = 64: 74 -> 17      150,001 nodes, 2.6 M entries, F = 256: 263 -> 204; F = 48: 156 -> 79
 //   1 M nodes, 17 M entries, F = 64: 748 -> 400, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 182
 //   2,449,029 nodes, 126 M entries, F = 256: 10,000 -> 8,640, F = 100: 5,760 -> 4,350, F = 48: 3,620 -> 2,230
-// WHOLE: the second launch of a product with tiles.  It does nothing unless the tiles could not be used (dg_tiles.h): then the first
-// one has left the split rows alone, and a few CTAs per SM gather them whole.
+// MODE kTiled: a product with tiles, whose partial results the split rows take in; kWhole: its second launch.  That does nothing
+// unless the tiles could not be used (dg_tiles.h): then the first one has left the split rows alone, and a few CTAs per SM gather
+// them whole.  kPlain is compiled without any of this: with the branches in it, and the registers they take, eight stage blocks (F = 256)
+// took 1 % longer.
 // PADDED: the operand is the padded copy of a matrix whose rows are not 16-byte multiples; C is then written float by float.
-template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED, bool WHOLE>
+enum { kPlain, kTiled, kWhole };
+template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED, int MODE>
 __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int chunk_ctas)
 {
     constexpr int G = 32 / LPR, NG = 256 / LPR;
@@ -288,33 +292,25 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
                 }
             }
         }
-        if constexpr (VEC == 4) {
-            if (a.parts) {
-                const int2 part = a.parts[ch.heavy];
-                const float4* p = a.part_area + ((int64_t)(part.x >> 7) * a.part_ld4 + vec0) * 128 + (part.x & 127);
-                for (int s = 0; s < part.y; ++s, p += a.part_ld4 * 128)
+        if constexpr (MODE == kTiled) {
+            const int2 part = a.parts[ch.heavy];
+            const float4* p = a.part_area + ((int64_t)(part.x >> 7) * a.part_ld4 + vec0) * 128 + (part.x & 127);
+            for (int s = 0; s < part.y; ++s, p += a.part_ld4 * 128)
 #pragma unroll
-                    for (int t = 0; t < TPL; ++t) {
-                        if (!on[t]) continue;
-                        const float4 x = __ldcg(p + t * LPR * 128);
-                        acc[t][0] += x.x; acc[t][1] += x.y; acc[t][2] += x.z; acc[t][3] += x.w;
-                    }
-            }
+                for (int t = 0; t < TPL; ++t) {
+                    if (!on[t]) continue;
+                    const float4 x = __ldcg(p + t * LPR * 128);
+                    acc[t][0] += x.x; acc[t][1] += x.y; acc[t][2] += x.z; acc[t][3] += x.w;
+                }
         }
         store_row(ch.row);
     };
-    if constexpr (VEC == 4) {
-        if (a.tile_words) {                                       // a product with tiles, which it may turn out not to be able to use
-            const bool whole = __ldcg(a.tile_words + DG_GATHER_ALL) != 0;
-            if constexpr (WHOLE) {
-                if (!whole) return;
-            } else {
-                if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.tile_words[DG_LARGEST_ELEMENT] = 0;      // for the next product
-                if (whole && (int)blockIdx.x < chunk_ctas) return;
-            }
-        }
+    if constexpr (MODE == kTiled) {
+        if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) a.tile_words[DG_LARGEST_ELEMENT] = 0;      // for the next product
+        if ((int)blockIdx.x < chunk_ctas && __ldcg(a.tile_words + DG_GATHER_ALL) != 0) return;
     }
-    if constexpr (WHOLE) {
+    if constexpr (MODE == kWhole) {
+        if (__ldcg(a.tile_words + DG_GATHER_ALL) == 0) return;
         for (int id0 = blockIdx.x * NG; id0 < a.n_chunks; id0 += chunk_ctas * NG) run_chunks(id0);
         return;
     }
@@ -401,15 +397,16 @@ int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
     const int64_t row_ctas = ((int64_t)a.m + a.rows_per_cta - 1) / a.rows_per_cta;
     for (; a.vec_first < a.vec_end; a.vec_first += tile * DG_FINISH_TILES) {
         const dim3 grid((unsigned)(chunk_ctas + row_ctas), (unsigned)std::min((a.vec_end - a.vec_first + tile - 1) / tile, DG_FINISH_TILES));
-        k_spmm<VEC, LPR, TPL, U, MINB, PADDED, false><<<grid, 256, 0, stream>>>(a, chunk_ctas);
+        if (!whole) k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kPlain><<<grid, 256, 0, stream>>>(a, chunk_ctas);
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
         if constexpr (VEC == 4) {
             if (!whole) continue;
+            k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kTiled><<<grid, 256, 0, stream>>>(a, chunk_ctas);
             SpmmArgs w = *whole;
             w.vec_first = a.vec_first;
             w.vec_end = a.vec_end;
             const int ctas = std::min((w.n_chunks + NG - 1) / NG, 148 * 4);
-            k_spmm<VEC, LPR, TPL, U, MINB, PADDED, true><<<dim3((unsigned)ctas, grid.y), 256, 0, stream>>>(w, ctas);
+            k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kWhole><<<dim3((unsigned)ctas, grid.y), 256, 0, stream>>>(w, ctas);
             g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
         }
     }

@@ -1,7 +1,7 @@
 // Dense tiles: the hub x hub corner of a power-law block on the tensor cores.
 //
-// A gather moves 4 F bytes through an SM's 64-byte-a-clock port for every entry, which is what bounds k_spmm on large blocks
-// (16 clocks an entry at F = 256).  Sorted by length and by frequency, the split rows and the frequent columns of a
+// A gather moves 4 F bytes from the L2 to an SM for every entry, 64 bytes a clock at best, which is what bounds k_spmm on large
+// blocks (16 clocks an entry at F = 256).  Sorted by length and by frequency, the split rows and the frequent columns of a
 // power-law graph meet in tiles that are 5 to 90 % full: one row of B serves several rows of such a tile, and multiplying
 // the whole 128 x 32 tile, zeros included, costs the SM as much as gathering some 160 of its entries.  So tiles
 // with more than that (kTileMin) are multiplied as dense matrices and the rest of the split rows is gathered as before.
@@ -18,8 +18,8 @@
 // scatter its records into it in turn, one thread issues the MMAs, and the groups drain the accumulators.  Partial results of a
 // row tile that several CTAs share are added by k_spmm where it finishes the row.
 // Measured (B200): 232,965 nodes / 115 M entries, 64 % of the entries in 91,000 tiles: F = 256 6.18 -> 3.3 ms, F = 604
-// 16.6 -> 8.9 ms; 306,128 nodes / 15.8 M entries, F = 256: 1.03 -> 0.84 ms.  The MMAs themselves are half of k_tile_mma's time, the
-// rest is waiting for a tile to be filled after an accumulator was drained.
+// 16.6 -> 8.9 ms; 306,128 nodes / 15.8 M entries, F = 256: 1.03 -> 0.84 ms.  The tensor pipe is busy for 55 to 59 % of k_tile_mma's
+// time, the rest is waiting for a tile to be filled after an accumulator was drained.
 #include <algorithm>
 #include <atomic>
 #include <cstring>

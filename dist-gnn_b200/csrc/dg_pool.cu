@@ -109,16 +109,19 @@ int* dg_status_word()
     static int* word[kMaxDevices] = {};
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!word[dev]) {
-        int* w = nullptr;
-        if (dg_device_alloc((void**)&w, sizeof(int)) != DG_OK) return nullptr;
-        if (cudaMemset(w, 0, sizeof(int)) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
-            cudaFree(w);
-            return nullptr;
-        }
-        word[dev] = w;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (word[dev]) return word[dev];
     }
+    int* w = nullptr;                                             // no lock while the program may be asked for memory
+    if (dg_device_alloc((void**)&w, sizeof(int)) != DG_OK) return nullptr;
+    if (cudaMemset(w, 0, sizeof(int)) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+        cudaFree(w);
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    if (word[dev]) cudaFree(w);                                   // another thread was faster
+    else word[dev] = w;
     return word[dev];
 }
 

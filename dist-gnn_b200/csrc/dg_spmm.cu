@@ -120,14 +120,15 @@ __device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const floa
 // What bounds it: the gathers.  Rows that the L2 holds come at 18 TB/s, 64 bytes a clock and SM (dense graph, F = 256: 41 GB in
 // 2.30 ms with the L2 at 78 % of its throughput, the path from it to the SMs at 49 %, issue slots at 46 %); larger graphs are held
 // up by the L2 and by what misses it (1 M nodes, 49 M entries: L2 64 %, DRAM 48 %, hit rate 63 %); small ones and short rows
-// are bound by latency, which the offsets in shared memory, the look-ahead and U hide.  Against separate kernels with a warp per row (B200, us per product):
+// are bound by latency, which the offsets in shared memory, the look-ahead and U hide.  Against separate kernels with a warp per
+// row (B200, us per product):
 //   10,000 nodes, 210 k entries, F = 64: 74 -> 17      150,001 nodes, 2.6 M entries, F = 256: 263 -> 204; F = 48: 156 -> 79
 //   1 M nodes, 17 M entries, F = 64: 748 -> 400, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 182
 //   2,449,029 nodes, 126 M entries, F = 256: 10,000 -> 8,640, F = 100: 5,760 -> 4,350, F = 48: 3,620 -> 2,230
 // MODE kTiled: a product with tiles, whose partial results the split rows take in; kWhole: its second launch.  That does nothing
 // unless the tiles could not be used (dg_tiles.h): then the first one has left the split rows alone, and a few CTAs per SM gather
-// them whole.  kPlain is compiled without any of this: with the branches in it, and the registers they take, eight stage blocks (F = 256)
-// took 1 % longer.
+// them whole (as last CTAs of the first launch: 4 % faster at F = 100, 1 to 3 % slower at F = 256 and 48, by its registers).  kPlain is
+// compiled without any of this: with the branches in it eight stage blocks (F = 256) took 1 % longer.
 // PADDED: the operand is the padded copy of a matrix whose rows are not 16-byte multiples; C is then written float by float.
 enum { kPlain, kTiled, kWhole };
 template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED, int MODE>

@@ -87,7 +87,8 @@ int64_t dg_plan_tiled_entries(const dg_plan* plan);
 /* Device memory of destroyed plans is kept for the next ones, at most 512 MB per device (1 GB until the next plan is destroyed, where one was being built); this gives all of it on the current
  * device back (a failed allocation of the library does so by itself). */
 int dg_pool_trim(void);
-/* `give_back` is called (on the allocating thread, with the allocating device current and none of the library's locks held) when
+/* `give_back` is called (on the allocating thread, with the allocating device current and no lock of the library held but, inside
+ * dg_spmm_csr_checked, that plan's) when
  * the driver refuses device memory that the library's own idle blocks cannot make up for; then the allocation is tried once
  * more.  A program whose allocator keeps freed memory returns it to the driver there, as spmm_cpp does with PyTorch's.  NULL: none. */
 int dg_on_low_memory(void (*give_back)(void));

@@ -432,7 +432,7 @@ struct Found {                            // what the host waits for
     int32_t columns, least, max_weight;   // frequent columns: how many, from which weight on, the largest
     int32_t slabs, entries, segments, rest_chunks, rest;
     int32_t largest;                      // bits of the largest magnitude among the tiled values
-    int32_t pad;
+    int32_t unordered;                    // some row's columns do not strictly ascend
     long long cost;                       // of all slabs, in half clocks
 };
 
@@ -446,14 +446,21 @@ __global__ void k_split_rows(const dg_chunk* __restrict__ chunks, int32_t n_chun
     by_length[h] = Keyed{len, h};
 }
 
-// How many entries of split rows every column holds.
+// How many entries of split rows every column holds, and whether a row's columns ascend: an entry that comes twice has one place in a
+// tile, so tiles are for rows whose columns strictly ascend, as coalescing leaves them.
 __global__ void __launch_bounds__(T) k_column_weights(const dg_chunk* __restrict__ chunks, int32_t n_chunks, const int32_t* __restrict__ col,
-                                                      int32_t* __restrict__ weight)
+                                                      int32_t* __restrict__ weight, Found* __restrict__ found)
 {
     const int32_t c = blockIdx.x * (T / 32) + (threadIdx.x >> 5);
     if (c >= n_chunks) return;
     const dg_chunk ch = chunks[c];
-    for (int i = threadIdx.x & 31; i < ch.len; i += 32) atomicAdd(&weight[col[ch.e0 + i]], 1);
+    bool ascend = true;
+    for (int i = threadIdx.x & 31; i < ch.len; i += 32) {
+        const int32_t cc = col[ch.e0 + i];
+        if (i > 0 || ch.slot != ch.slot0) ascend = ascend && col[ch.e0 + i - 1] < cc;      // the row's first entry has none before it
+        atomicAdd(&weight[cc], 1);
+    }
+    if (!ascend) found->unordered = 1;
 }
 
 constexpr int kWeightBins = 4096;
@@ -880,7 +887,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
     DG_CUDA(cudaMemsetAsync(col_rank, 0xff, (size_t)p->k * sizeof(int32_t), stream));
     k_split_rows<<<grid_of(p->n_chunks, T), T, 0, stream>>>(p->chunks, p->n_chunks, p->rowptr, rows, by_length);
     k_first_slots<<<grid_of(p->n_chunks, T), T, 0, stream>>>(p->chunks, p->n_chunks, p->n_heavy, first_slot);
-    k_column_weights<<<grid_of(p->n_chunks, T / 32), T, 0, stream>>>(p->chunks, p->n_chunks, p->col, weight);
+    k_column_weights<<<grid_of(p->n_chunks, T / 32), T, 0, stream>>>(p->chunks, p->n_chunks, p->col, weight, found);
     k_weight_histogram<<<148, T, 0, stream>>>(weight, p->k, bins, found);
     k_least_weight<<<1, 1024, 0, stream>>>(bins, found);
     Found h{};
@@ -889,7 +896,7 @@ int build_tiles(const dg_plan* p, const float* val, cudaStream_t stream, dg_tile
         return (int)(e != cudaSuccess ? e : cudaStreamSynchronize(stream));
     };
     if ((rc = read())) return rc;
-    if (h.columns < kTileCols) return DG_OK;
+    if (h.columns < kTileCols || h.unordered) return DG_OK;
 
     // columns by weight, rows by length
     t->n_columns = h.columns;

@@ -75,7 +75,8 @@ int dg_plan_destroy(dg_plan* plan);
  * makes a second copy of the split rows' entries (8 bytes each) WITH their values `val`; products with another `val` pointer
  * are gathered as before, and so is one whose values have been changed in place (the device compares them).  That product pays for
  * the tiles without using them: a caller that changes values calls this again, or dg_plan_drop_tiles.  Returns
- * DG_OK without doing anything where the block has too few dense tiles, or a value of 2^63 or more, an infinity or a NaN among
+ * DG_OK without doing anything where the block has too few dense tiles, split rows whose columns do not strictly ascend (an entry
+ * that comes twice has one place in a tile), or a value of 2^63 or more, an infinity or a NaN among
  * them, or none of 2^-100.  A product whose operand holds such an element in a column of the tiles, or only elements under 2^-100
  * (under 2^-100 over the largest value, if that is below 1), is gathered whole, with the bits of a plan without tiles: the device
  * finds out, at no wait.  Synchronises `stream`; no product on the plan may be

@@ -827,3 +827,62 @@ def test_caller_says_whether_a_block_is_multiplied_often(monkeypatch, tiles, man
     assert (spmm_cpp.SpmmPlan.from_coo(t, tiles=tiles).tiled_entries() > 0) == many
     monkeypatch.setattr(spmm_cpp, 'TILE_NNZ', A.nnz + 1)
     assert spmm_cpp.SpmmPlan.from_coo(t, tiles=tiles).tiled_entries() == 0
+
+
+def tiled_entries_by_numpy(A, threshold):
+    """How many entries lie in 128 x 32 tiles of 160 or more: rows longer than the threshold, longest first, by columns of at least six
+    such entries, most frequent first; ties by id.  0 where they are fewer than an eighth of all."""
+    deg = np.bincount(A.row, minlength=A.shape[0])
+    long_rows = np.flatnonzero(deg > threshold)
+    if long_rows.size < 128:
+        return 0
+    inside = deg[A.row] > threshold
+    weight = np.bincount(A.col[inside], minlength=A.shape[1])
+    columns = np.flatnonzero(weight >= 6)
+    row_rank, col_rank = np.full(A.shape[0], -1), np.full(A.shape[1], -1)
+    row_rank[long_rows[np.argsort(-deg[long_rows], kind='stable')]] = np.arange(long_rows.size)
+    col_rank[columns[np.argsort(-weight[columns], kind='stable')]] = np.arange(columns.size)
+    r, c = row_rank[A.row], col_rank[A.col]
+    both = (r >= 0) & (c >= 0)
+    tiles = np.bincount(r[both] // 128 * (columns.size // 32 + 1) + c[both] // 32)
+    entries = int(tiles[tiles >= 160].sum())
+    return entries if columns.size >= 32 and entries >= A.nnz // 8 else 0
+
+
+@pytest.mark.parametrize('rows', [127, 128, 129, 2047, 2048, 2049, 4200])
+@pytest.mark.parametrize('columns', [80, 96, 97, 700, 9001])
+def test_tile_search_finds_what_numpy_finds(rows, columns):
+    """Lists around the edges of a sort's block and of a tile, with many equal lengths and weights; product and its bits on a second plan."""
+    rng = np.random.Generator(np.random.PCG64(rows * 10000 + columns))
+    length = 65 + rng.integers(0, 12, rows)
+    p = 1.0 / (1 + np.arange(columns)) ** 0.9
+    col = np.concatenate([np.sort(rng.choice(columns, n, replace=False, p=p / p.sum())) for n in length])
+    A = ref_graph.Coo(np.repeat(np.arange(rows), length), col, rng.standard_normal(length.sum(), dtype=np.float32), (rows, columns))
+    plan = tiled_plan(A)
+    assert plan.stats()['heavy_threshold'] == 64 and plan.tiled_entries() == tiled_entries_by_numpy(A, 64)
+    B = rng.standard_normal((columns, 72), dtype=np.float32)
+    C = plan.spmm(dev(B), torch.empty(rows, 72, device='cuda'), 1.0, 0.0)
+    want = np.zeros((rows, 72))
+    np.add.at(want, A.row, A.val[:, None].astype(np.float64) * B[A.col])
+    assert_close(C.cpu().numpy(), want, TOL / 10, f'{plan.tiled_entries()} tiled entries')
+    assert torch.equal(C, tiled_plan(A).spmm(dev(B), torch.empty_like(C), 1.0, 0.0)) and plan.device_status() == 0
+
+
+@pytest.mark.parametrize('where', [0, 63, 64, 200])
+def test_entries_that_come_twice_are_both_multiplied(where):
+    """A row-sorted block that was never coalesced, its repeated entry inside a chunk of a split row, across the border of two, and last;
+    and one whose columns are in no order: no tiles, the product of a plan without them."""
+    A = skewed_block(18)
+    longest = np.bincount(A.row).argmax()
+    at = np.flatnonzero(A.row == longest)[where if where < 200 else -2]
+    twice = ref_graph.Coo(A.row, A.col.copy(), A.val, A.shape)
+    twice.col[at + 1] = twice.col[at]
+    mixed = ref_graph.Coo(A.row, A.col.copy(), A.val.copy(), A.shape)
+    mixed.col[[at, at + 1]], mixed.val[[at, at + 1]] = A.col[[at + 1, at]], A.val[[at + 1, at]]
+    B = np.random.Generator(np.random.PCG64(19)).standard_normal((2600, 64), dtype=np.float32)
+    assert tiled_plan(A).tiled_entries() > 0
+    for block in (twice, mixed):
+        plan = tiled_plan(block)
+        assert plan.tiled_entries() == 0
+        got = plan.spmm(dev(B), torch.empty(3001, 64, device='cuda'), 1.0, 0.0).cpu().numpy()
+        assert_close(got, ref_gcn.spmm_coo(block, B, np.zeros((3001, 64), np.float32), 1.0, 0.0), TOL, 'not coalesced')

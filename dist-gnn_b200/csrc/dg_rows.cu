@@ -105,25 +105,51 @@ __global__ void __launch_bounds__(kLossThreads) k_rows_ce_mean(const double* __r
 }
 
 // grad[row, c] = (softmax(x[row])[c] - [c == target]) * upstream / count, zero for rows without a target and beyond C.
+// The softmax is taken from the row's maximum and sum anew: against a stored logsumexp it would carry that number's rounding, which
+// grows with the logits (error of the gradient against float64, 47 classes: around 0 1.6e-7, 100 1.3e-6, 10,000 1.6e-4; this way
+// 5e-8 everywhere, as PyTorch's).  A lane's exponentials stay in registers up to
+// kKept classes a lane, so an exponential a class is all it takes, as with the logsumexp.
 template <int LPR>
 __global__ void __launch_bounds__(kLossThreads) k_rows_ce_backward(const float* __restrict__ x, int64_t ld, int64_t n, int32_t C,
-                                                                   const int32_t* __restrict__ target, const float* __restrict__ lse,
-                                                                   const float* __restrict__ upstream, float inv_count,
-                                                                   float* __restrict__ grad, int64_t ldg)
+                                                                   const int32_t* __restrict__ target, const float* __restrict__ upstream,
+                                                                   float inv_count, float* __restrict__ grad, int64_t ldg)
 {
-    constexpr int RPB = kLossThreads / LPR;
+    constexpr int RPB = kLossThreads / LPR, kKept = 4;
     const int lane = threadIdx.x % LPR;
     const float scale = __ldg(upstream) * inv_count;
-    for (int64_t row = (int64_t)blockIdx.x * RPB + threadIdx.x / LPR; row < n; row += (int64_t)gridDim.x * RPB) {
-        const int32_t t = __ldg(target + row);
-        const float l = t >= 0 ? __ldg(lse + row) : 0.f;
+    for (int64_t base = (int64_t)blockIdx.x * RPB; base < n; base += (int64_t)gridDim.x * RPB) {
+        const int64_t row = base + threadIdx.x / LPR;
+        const int32_t t = row < n ? __ldg(target + row) : -1;
+        const bool on = t >= 0;
         const float* r = x + row * ld;
-        float* g = grad + row * ldg;
-        for (int c = lane; c < ldg; c += LPR) {
-            float v = 0.f;
-            if (t >= 0 && c < C) v = (expf(__ldg(r + c) - l) - (c == t ? 1.f : 0.f)) * scale;
-            g[c] = v;
+        float e[kKept], mx = __int_as_float(0xff800000);
+#pragma unroll
+        for (int j = 0; j < kKept; ++j) {
+            e[j] = on && lane + j * LPR < C ? __ldg(r + lane + j * LPR) : __int_as_float(0xff800000);
+            mx = e[j] > mx || e[j] != e[j] ? e[j] : mx;           // a NaN stays
         }
+        if (on)
+            for (int c = lane + kKept * LPR; c < C; c += LPR) {
+                const float v = __ldg(r + c);
+                mx = v > mx || v != v ? v : mx;
+            }
+        mx = group_max<LPR>(mx);
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < kKept; ++j)
+            if (on && lane + j * LPR < C) sum += e[j] = expf(e[j] - mx);
+        if (on)
+            for (int c = lane + kKept * LPR; c < C; c += LPR) sum += expf(__ldg(r + c) - mx);
+        const float inv = 1.f / group_sum<LPR>(sum);
+        if (row >= n) continue;
+        float* g = grad + row * ldg;
+#pragma unroll
+        for (int j = 0; j < kKept; ++j) {
+            const int c = lane + j * LPR;
+            if (c < ldg) g[c] = on && c < C ? (e[j] * inv - (c == t ? 1.f : 0.f)) * scale : 0.f;
+        }
+        for (int c = lane + kKept * LPR; c < ldg; c += LPR)
+            g[c] = on && c < C ? (expf(__ldg(r + c) - mx) * inv - (c == t ? 1.f : 0.f)) * scale : 0.f;
     }
 }
 
@@ -166,10 +192,10 @@ extern "C" int dg_rows_cross_entropy_grad(const float* x, int64_t ld, int64_t n,
     const unsigned blocks = loss_blocks(n, lpr);
     const float inv = (float)(1.0 / (double)count);
     switch (lpr) {
-        case 4: k_rows_ce_backward<4><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
-        case 8: k_rows_ce_backward<8><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
-        case 16: k_rows_ce_backward<16><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
-        default: k_rows_ce_backward<32><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, upstream, inv, grad, ldg); break;
+        case 4: k_rows_ce_backward<4><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
+        case 8: k_rows_ce_backward<8><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
+        case 16: k_rows_ce_backward<16><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
+        default: k_rows_ce_backward<32><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
     }
     return (int)cudaGetLastError();
 }

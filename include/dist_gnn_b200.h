@@ -378,7 +378,7 @@ int dg_pad_rows(const float* src, int64_t ld_src, int64_t n, int32_t cols, float
 
 /* Mean cross-entropy over the rows with a target (replaces the loss of light_dist_gnn/dist_train.py:39-43 on the local train
  * rows): loss = sum over rows with target[i] >= 0 of (logsumexp(x[i, 0..C)) - x[i, target[i]]) / count, where count is the
- * number of such rows and every target is below C.  lse (n floats) keeps the rows' logsumexp for the gradient; scratch holds
+ * number of such rows and every target is below C.  lse (n floats) receives the logsumexp of the rows with a target (the gradient takes its softmax from the logits themselves); scratch holds
  * dg_rows_loss_scratch() doubles.  The gradient is (softmax - onehot) * upstream / count (upstream: one float on the device),
  * zero in rows without a target and in columns C..ldg.  Bit-reproducible. */
 int32_t dg_rows_loss_scratch(void);

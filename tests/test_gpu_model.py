@@ -411,3 +411,19 @@ def test_one_call_network_equals_chained_layers(golden, env1, dims):
     assert torch.equal(h, out)
     for a, w in zip(got, weights):
         assert (a is None) == (w.grad is None) and (a is None or torch.equal(a, w.grad))
+
+
+@pytest.mark.parametrize('C', [2, 16, 41, 47, 64, 128, 129, 300])
+def test_row_cross_entropy_gradient_of_large_logits(C):
+    """Logits around 100 and 10,000: the gradient is the softmax of differences, whose rounding does not grow with the logits.  Against
+    float64, within ten roundings of a probability (the library's loss: 5 to 7e-8)."""
+    import spmm_cpp
+    gen = torch.Generator(device='cuda').manual_seed(C)
+    for offset in (100.0, -10000.0):
+        x = (torch.randn(3001, C, generator=gen, device='cuda') * 4 + offset).requires_grad_()
+        t = torch.randint(-1, C, (3001,), generator=gen, device='cuda').to(torch.int32)
+        rows = torch.nonzero(t >= 0).squeeze(1)
+        spmm_cpp.row_cross_entropy(x, t, rows.numel()).backward()
+        xd = x.detach().double().requires_grad_()
+        torch.nn.functional.cross_entropy(xd[rows], t[rows].long()).backward()
+        assert float((x.grad.double() - xd.grad).norm() / xd.grad.norm()) < 10 * 2.0 ** -24

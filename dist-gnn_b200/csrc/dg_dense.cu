@@ -14,8 +14,8 @@
 // through a 2-stage ring; warps 2-5 split A and later drain the accumulator (tcgen05.ld) to global memory with the
 // optional ReLU / ReLU-backward mask; one thread of warp 1 issues the tcgen05.mma instructions (kind::tf32, 128 x N x 8,
 // operands described by shared-memory matrix descriptors, accumulator in TMEM columns) and commits them to the mbarriers
-// that recycle the stages.  k_dense_nt_persistent: one CTA per SM walks the tiles with two accumulators and separate
-// epilogue warps (used for results wider than 128 columns).  k_dense_tn (further down): the weight gradient X^T * G,
+// that recycle the stages.  k_dense_nt_pair: a CTA pair on every TPC walks over tiles of 256 rows with two accumulators and separate
+// epilogue warps (used for results wider than 64 columns).  k_dense_tn (further down): the weight gradient X^T * G,
 // both operands MN-major, split-K over the CTAs with periodic accumulator flushes.
 // Every mbarrier wait is bounded; a role that gives up sets the status word and the CTA still frees its TMEM.
 #include <cuda.h>
@@ -269,164 +269,262 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
 }
 
-// The same product with one CTA per SM walking over the row tiles (tile, tile + grid, ...): two accumulators in tensor
-// memory (columns 0 and 256) and separate warps for the operand split and for the epilogue, so that tile t is read out
-// of tensor memory and stored while tile t+1 is already being loaded, split and multiplied.
-// Warps: 0 TMA, 1 MMA issue + tensor-memory allocation, 2-5 split A, 6-9 epilogue (warp w reads lane quarter w % 4).
-// The ring holds four half slabs of 16 columns (64-byte rows, 64B swizzle) instead of two slabs of 32: a stage is refilled
-// from the L2 (Bt's 512 KB come back for every tile), split and multiplied one after the other, and with two stages in that
-// circle the tensor cores waited for it more than half of the time.  A slab's MMAs keep their order - both head passes of its
-// four k-steps, then the tail passes - so the sums are the same bits.
-constexpr int kThreadsPersistent = 320;
-constexpr int PK = 16, PSTAGES = 4;
+// The same product by CTA pairs (cta_group::2), one pair on the two SMs of every TPC, that walk over tiles of 256 rows: a CTA holds
+// 128 rows of A and half the rows of Bt, the tensor cores of both read both halves of Bt, and each CTA's tensor memory receives its 128
+// rows of the result.  Two accumulators (columns 0 / 256) and separate warps for the operand split and the epilogue, so that tile t is
+// read out and stored while tile t+1 is loaded, split and multiplied.
+// Warps: 0 TMA, 1 MMA issue (even CTA) + tensor-memory allocation, 2-5 split A, 6-13 epilogue (lane quarter w % 4; two warps a quarter take
+// its 32-column pieces in turn).
+// The ring holds half slabs of 16 columns (64-byte rows, 64B swizzle), as many as fit (6 at 256 columns, 10 at most).
+// Barriers: full (own CTA, TMA), ready (even CTA: the split warps of both), empty and acc_full (both CTAs, by commit), acc_empty (even CTA:
+// the epilogue warps of both).
+//
+// What bounds it: at 256 x 256 the MMAs (tensor pipe 73 %; a single CTA's shared memory was busy with fetching both operands' 12 KB for
+// every MMA and refilling Bt's 512 KB for every 128 rows, which a pair halves), below some 100 columns of A DRAM and the epilogue.
+// 2,449,029 rows (us, one CTA per SM with four epilogue warps -> pair): 256 -> 256 1,600 -> 1,535, with the mask 1,930 -> 1,720;
+// 100 -> 256 1,100 -> 895; 47 -> 256 with the mask 1,600 -> 1,110; 602 -> 256 4,280 -> 3,540; 256 -> 128 1,540 -> 1,065 (one tile per
+// CTA).  150,001 rows: 256 -> 256 102 -> 100, with the mask 126 -> 109; 100 -> 256 76 -> 61.
+// Up to 64 columns k_dense_nt stays: two of its CTAs fit an SM, and an MMA takes some 130 clocks however few columns it has (256 -> 47
+// 860 us against 895; 10,000 rows 12.3 against 14.2).
+constexpr int PK = 16, kMaxPairStages = 10, kSplitWarps = 4, kEpilogueWarps = 8;
+constexpr int kThreadsPair = 32 * (2 + kSplitWarps + kEpilogueWarps);
+constexpr int kPieceBytes = 32 * 32 * 4;                          // staging of an epilogue warp: 32 rows x 32 columns
+constexpr int kPairBarBytes = 8 * (3 * kMaxPairStages + 5) + 8;
 
-__global__ void __launch_bounds__(kThreadsPersistent, 1)
-k_dense_nt_persistent(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
-                      const __grid_constant__ CUtensorMap tmBt, const DenseArgs a, const int n_tiles)
+__device__ __forceinline__ void umma_tf32_pair(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+template <bool MASK>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsPair, 1)
+k_dense_nt_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBh,
+                const __grid_constant__ CUtensorMap tmBt, const DenseArgs a, const int n_tiles, const int stages)
 {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* gbase = smem_raw + (base - raw);
     constexpr int a_bytes = BM * PK * 4;
-    const int b_bytes = a.n_pad * PK * 4;
+    const int half_n = a.n_pad / 2, b_bytes = half_n * PK * 4;
     const int stage_bytes = 2 * a_bytes + 2 * b_bytes;            // A head, A tail, Bt head, Bt tail
-    const int staging = PSTAGES * stage_bytes;                    // the epilogue warps' row pieces
-    const uint32_t bars = base + staging + 4 * kStageBytes;
-    const uint32_t full0 = bars, ready0 = bars + 8 * PSTAGES, empty0 = bars + 16 * PSTAGES;
-    const uint32_t acc_full0 = bars + 24 * PSTAGES, acc_empty0 = acc_full0 + 16, done = acc_empty0 + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + staging + 4 * kStageBytes + 24 * PSTAGES + 40);
+    const int staging = stages * stage_bytes;                     // the epilogue warps' row pieces
+    const uint32_t bars = base + staging + kEpilogueWarps * kPieceBytes;
+    const uint32_t full0 = bars, ready0 = bars + 8 * kMaxPairStages, empty0 = bars + 16 * kMaxPairStages;
+    const uint32_t acc_full0 = bars + 24 * kMaxPairStages, acc_empty0 = acc_full0 + 16, done = acc_empty0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + staging + kEpilogueWarps * kPieceBytes + 24 * kMaxPairStages + 40);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int nhalves = (a.K + PK - 1) / PK;
     constexpr int kTmemCols = 512;                                // two accumulators of up to 256 columns
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < PSTAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
-            mbar_init(ready0 + 8 * s, 128);
+            mbar_init(ready0 + 8 * s, 2 * kSplitWarps);
             mbar_init(empty0 + 8 * s, 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(acc_full0 + 8 * b, 1);
-            mbar_init(acc_empty0 + 8 * b, 128);
+            mbar_init(acc_empty0 + 8 * b, 2 * min(kEpilogueWarps, a.n_pad / 32 * 4));      // a result of 32 columns leaves half of them idle
         }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    cluster_sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
 
     if (warp == 0) {
         if (lane == 0) {                                          // TMA producer: one ring of stages across all tiles
-            int it = 0;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            int it = 0, s = 0, phase = 1;
+            for (int tile = pair; tile < n_tiles && ok; tile += pairs) {
+                const int row0 = (int)((int64_t)tile * (2 * BM) + rank * BM);      // rows beyond the matrix arrive as zeros
                 for (int i = 0; i < nhalves; ++i, ++it) {
-                    const int s = it % PSTAGES, u = it / PSTAGES;
-                    if (u > 0) ok = mbar_wait(empty0 + 8 * s, (u - 1) & 1);
+                    if (it >= stages) ok = mbar_wait(empty0 + 8 * s, phase);
                     if (!ok) break;
                     const uint32_t st = base + s * stage_bytes;
                     mbar_expect_tx(full0 + 8 * s, a_bytes + 2 * b_bytes);
-                    tma_load_2d(st, &tmA, i * PK, tile * BM, full0 + 8 * s);
-                    tma_load_2d(st + 2 * a_bytes, &tmBh, i * PK, 0, full0 + 8 * s);
-                    tma_load_2d(st + 2 * a_bytes + b_bytes, &tmBt, i * PK, 0, full0 + 8 * s);
+                    tma_load_2d(st, &tmA, i * PK, row0, full0 + 8 * s);
+                    tma_load_2d(st + 2 * a_bytes, &tmBh, i * PK, rank * half_n, full0 + 8 * s);
+                    tma_load_2d(st + 2 * a_bytes + b_bytes, &tmBt, i * PK, rank * half_n, full0 + 8 * s);
+                    if (++s == stages) s = 0, phase ^= 1;
                 }
             }
-            await_loads(full0, it, PSTAGES);
+            await_loads(full0, it, stages);
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                          // MMA issuer
-            const uint32_t idesc = umma_idesc_tf32(a.n_pad);
-            int it = 0, lt = 0;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++lt) {
+        if (lane == 0 && rank == 0) {                             // MMA issuer
+            const uint32_t idesc = umma_idesc_tf32(a.n_pad) + ((uint32_t)(BM >> 4) << 24);      // 2 * BM rows
+            int s = 0, phase = 0, lt = 0;
+            for (int tile = pair; tile < n_tiles && ok; tile += pairs, ++lt) {
                 const int b = lt & 1, v = lt >> 1;
-                if (lt >= 2) ok = mbar_wait(acc_empty0 + 8 * b, (v - 1) & 1);     // the epilogue has drained this accumulator
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (lt >= 2) ok = mbar_wait(acc_empty0 + 8 * b, (v - 1) & 1);     // both epilogues have drained this accumulator
                 const uint32_t acc = tmem + (uint32_t)(b * 256);
-                for (int i = 0; i < nhalves && ok; i += 2, it += 2) {
-                    const int halves = min(2, nhalves - i);
+                for (int i = 0; i < nhalves && ok; i += 2) {
                     // The tensor cores read a TF32 operand from a 32-bit container and ignore its low 13 bits (verified: identical
-                    // bits with a masked copy), so the tile as TMA delivered it IS the head: both head passes go out as soon as
-                    // the data has landed, and only the tail pass waits for the split warps.
+                    // bits with a masked copy), so the tile as TMA delivered it is the head.  The order of the additions decides the last
+                    // bits, and those the sign of a ReLU's input: over a slab of two halves, the tail passes come behind the head
+                    // passes (wide results) or beside them (narrow ones), as in the kernels of one CTA.
+                    const int s0 = s, halves = min(2, nhalves - i);
+                    const bool tails_last = a.n_pad > 128;
                     for (int h = 0; h < halves && ok; ++h) {
-                        const int s = (it + h) % PSTAGES, u = (it + h) / PSTAGES;
-                        ok = mbar_wait(full0 + 8 * s, u & 1);
+                        ok = mbar_wait(ready0 + 8 * s, phase);
                         if (!ok) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t st = base + s * stage_bytes;
-                        const uint64_t a_head = umma_desc_sw64(st), b_head = umma_desc_sw64(st + 2 * a_bytes), b_tail = umma_desc_sw64(st + 2 * a_bytes + b_bytes);
+                        const uint64_t a_head = umma_desc_sw64(st), a_tail = umma_desc_sw64(st + a_bytes);
+                        const uint64_t b_head = umma_desc_sw64(st + 2 * a_bytes), b_tail = umma_desc_sw64(st + 2 * a_bytes + b_bytes);
 #pragma unroll
                         for (int k = 0; k < PK / 8; ++k) {        // 8 TF32 columns = 32 bytes per MMA: +2 in 16-byte units
-                            umma_tf32(acc, a_head + 2 * k, b_tail + 2 * k, idesc, (i + h > 0 || k > 0) ? 1u : 0u);
-                            umma_tf32(acc, a_head + 2 * k, b_head + 2 * k, idesc, 1u);
+                            const uint32_t add = i > 0 || h > 0 || k > 0 ? 1u : 0u;
+                            if (!tails_last) umma_tf32_pair(acc, a_tail + 2 * k, b_head + 2 * k, idesc, add);
+                            umma_tf32_pair(acc, a_head + 2 * k, b_tail + 2 * k, idesc, tails_last ? add : 1u);
+                            umma_tf32_pair(acc, a_head + 2 * k, b_head + 2 * k, idesc, 1u);
                         }
+                        if (!tails_last) umma_commit_pair(empty0 + 8 * s);
+                        if (++s == stages) s = 0, phase ^= 1;
                     }
-                    for (int h = 0; h < halves && ok; ++h) {
-                        const int s = (it + h) % PSTAGES, u = (it + h) / PSTAGES;
-                        ok = mbar_wait(ready0 + 8 * s, u & 1);
-                        if (!ok) break;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t st = base + s * stage_bytes;
+                    for (int h = 0, t = s0; tails_last && h < halves && ok; ++h) {
+                        const uint32_t st = base + t * stage_bytes;
                         const uint64_t a_tail = umma_desc_sw64(st + a_bytes), b_head = umma_desc_sw64(st + 2 * a_bytes);
 #pragma unroll
-                        for (int k = 0; k < PK / 8; ++k) umma_tf32(acc, a_tail + 2 * k, b_head + 2 * k, idesc, 1u);
-                        umma_commit(empty0 + 8 * s);
+                        for (int k = 0; k < PK / 8; ++k) umma_tf32_pair(acc, a_tail + 2 * k, b_head + 2 * k, idesc, 1u);
+                        umma_commit_pair(empty0 + 8 * t);
+                        if (++t == stages) t = 0;
                     }
-                    if (halves == 1) --it;                        // the last slab of an odd count takes one stage
                 }
-                if (ok) umma_commit(acc_full0 + 8 * b);
+                if (ok) umma_commit_pair(acc_full0 + 8 * b);
             }
-            await_mmas(done);
+            await_mmas_pair(done);
+        } else if (lane == 0) {
+            mbar_wait(done, 0);
         }
-    } else if (warp < 6) {
-        const int t = threadIdx.x - 64;                           // 0..127: split the A half slab of every stage
-        int it = 0;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            for (int i = 0; i < nhalves; ++i, ++it) {
-                const int s = it % PSTAGES, u = it / PSTAGES;
-                ok = mbar_wait(full0 + 8 * s, u & 1);
+    } else if (warp < 2 + kSplitWarps) {
+        const int t = threadIdx.x - 64;                           // split the A half slab of every stage
+        const uint32_t leader_ready0 = in_leader(ready0);
+        int s = 0, phase = 0;
+        for (int tile = pair; tile < n_tiles && ok; tile += pairs) {
+            for (int i = 0; i < nhalves; ++i) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase));
                 if (!ok) break;
-                const float4* head = reinterpret_cast<const float4*>(gbase + (size_t)s * stage_bytes);
-                float4* tail = reinterpret_cast<float4*>(gbase + (size_t)s * stage_bytes + a_bytes);
+                const float4* head = reinterpret_cast<const float4*>(gbase + (size_t)s * stage_bytes) + t;
+                float4* tail = reinterpret_cast<float4*>(gbase + (size_t)s * stage_bytes + a_bytes) + t;
+                float4 x[a_bytes / 16 / (32 * kSplitWarps)];
 #pragma unroll
-                for (int j = t; j < a_bytes / 16; j += 128) {
-                    const float4 x = head[j];
+                for (int j = 0; j < a_bytes / 16 / (32 * kSplitWarps); ++j) x[j] = head[j * 32 * kSplitWarps];
+#pragma unroll
+                for (int j = 0; j < a_bytes / 16 / (32 * kSplitWarps); ++j) {
                     float4 h;
-                    h.x = __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u); h.y = __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
-                    h.z = __uint_as_float(__float_as_uint(x.z) & 0xFFFFE000u); h.w = __uint_as_float(__float_as_uint(x.w) & 0xFFFFE000u);
-                    tail[j] = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
+                    h.x = __uint_as_float(__float_as_uint(x[j].x) & 0xFFFFE000u); h.y = __uint_as_float(__float_as_uint(x[j].y) & 0xFFFFE000u);
+                    h.z = __uint_as_float(__float_as_uint(x[j].z) & 0xFFFFE000u); h.w = __uint_as_float(__float_as_uint(x[j].w) & 0xFFFFE000u);
+                    tail[j * 32 * kSplitWarps] = make_float4(x[j].x - h.x, x[j].y - h.y, x[j].z - h.z, x[j].w - h.w);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                mbar_arrive(ready0 + 8 * s);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leader_ready0 + 8 * s);
+                if (++s == stages) s = 0, phase ^= 1;
             }
         }
     } else {
-        const int q = warp & 3;                                   // a warp may only read its own quarter of the TMEM lanes
+        const int q = warp & 3, first = (warp - 2 - kSplitWarps) / 4 * 32;      // a warp may only read its own quarter of the TMEM lanes
+        constexpr int step = kEpilogueWarps / 4 * 32;
+        const uint32_t leader_acc_empty0 = in_leader(acc_empty0);
+        float4* stage = reinterpret_cast<float4*>(gbase + staging + (warp - 2 - kSplitWarps) * kPieceBytes);
+        const bool vec = a.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0 &&
+                         (!MASK || (a.ldm % 4 == 0 && (reinterpret_cast<uintptr_t>(a.mask) & 15) == 0));
+        const int r4 = lane >> 3, piece = lane & 7;
         int lt = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++lt) {
+        for (int tile = first < a.n_pad ? pair : n_tiles; tile < n_tiles; tile += pairs, ++lt) {
             const int b = lt & 1, v = lt >> 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * b, v & 1));     // tcgen05.ld is warp-collective
+            const int64_t row0 = (int64_t)tile * (2 * BM) + rank * BM + q * 32;
+            const int rows = (int)max((int64_t)0, min((int64_t)32, a.M - row0));
+            const uint32_t acc = tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16);
+            for (int c0 = first; c0 < a.n_pad; c0 += step) {
+                const bool whole = vec && c0 + 32 <= a.N;         // 128-byte pieces of every row, four rows an instruction
+                [[maybe_unused]] float4 mk[8];
+                if (MASK && whole) {                              // under way while the accumulator is waited for and read
+                    const float* m = a.mask + (row0 + r4) * a.ldm + c0 + piece * 4;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i, m += 4 * a.ldm)
+                        if (i * 4 + r4 < rows) mk[i] = __ldg(reinterpret_cast<const float4*>(m));
+                }
+                if (c0 == first) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * b, v & 1));     // tcgen05.ld is warp-collective
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                }
+                {
+                    uint32_t r[32];
+                    tmem_ld16(acc + (uint32_t)c0, r);
+                    tmem_ld16(acc + (uint32_t)c0 + 16, r + 16);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (c0 + step >= a.n_pad) {                   // the accumulator has been read: its next tile may start
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(leader_acc_empty0 + 8 * b);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)                   // a lane holds one row: through shared memory, conflict-free both ways
+                        stage[lane * 8 + (j ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+                }
+                __syncwarp();
+                if (whole) {
+                    float4 x[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) x[i] = stage[(i * 4 + r4) * 8 + (piece ^ ((i * 4 + r4) & 7))];
+                    float* c = a.C + (row0 + r4) * a.ldc + c0 + piece * 4;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i, c += 4 * a.ldc) {
+                        if (a.relu) x[i] = make_float4(fmaxf(x[i].x, 0.f), fmaxf(x[i].y, 0.f), fmaxf(x[i].z, 0.f), fmaxf(x[i].w, 0.f));
+                        if (MASK) {
+                            if (!(mk[i].x > 0.f)) x[i].x = 0.f;
+                            if (!(mk[i].y > 0.f)) x[i].y = 0.f;
+                            if (!(mk[i].z > 0.f)) x[i].z = 0.f;
+                            if (!(mk[i].w > 0.f)) x[i].w = 0.f;
+                        }
+                        if (i * 4 + r4 < rows) __stcs(reinterpret_cast<float4*>(c), x[i]);
+                    }
+                } else if (c0 + lane < a.N) {                     // odd strides and the last columns: a row's floats side by side
+                    const float* flat = reinterpret_cast<const float*>(stage);
+                    for (int i0 = 0; i0 < rows; i0 += 8) {        // eight rows' mask values in flight
+                        [[maybe_unused]] float mrow[8];
+                        if (MASK) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                if (i0 + i < rows) mrow[i] = __ldg(a.mask + (row0 + i0 + i) * a.ldm + c0 + lane);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            if (i0 + i >= rows) break;
+                            float x = flat[((i0 + i) * 8 + ((lane >> 2) ^ ((i0 + i) & 7))) * 4 + (lane & 3)];
+                            if (a.relu) x = fmaxf(x, 0.f);
+                            if (MASK && !(mrow[i] > 0.f)) x = 0.f;
+                            __stcs(a.C + (row0 + i0 + i) * a.ldc + c0 + lane, x);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
             if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int64_t row0 = (int64_t)tile * BM + q * 32;
-            if (row0 < a.M)
-                store_rows(a, tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16), reinterpret_cast<float*>(gbase + staging + q * kStageBytes), row0, lane);
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(acc_empty0 + 8 * b);
         }
     }
     if (!ok) atomicExch(a.status, 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    cluster_sync();                                               // no CTA leaves while the other's MMAs read its operands or arrive at its barriers
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 1)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
 __global__ void k_tf32_split(const float* __restrict__ src, float* __restrict__ head, float* __restrict__ tail, int64_t count)
@@ -606,31 +704,33 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
     a.mask = mask; a.ldm = ldm;
     a.status = dg_status_word();
     if (!a.status) return DG_ERR_STATE;
-    const int n_tiles = (int)((M + BM - 1) / BM);
-    // two kernels: one tile per CTA, or one persistent CTA per SM walking the tiles
-    // Narrow results leave room for two one-tile CTAs per SM, which overlap each other's load latency better than the
-    // persistent CTA's stages do (2,449,029 x 256 -> 47: 1.09 ms against 1.28 ms; -> 256: 2.16 against 1.88, before either
-    // kernel stored whole row pieces).
-    const bool per_tile = a.n_pad <= 128;
-    const int box = per_tile ? BK : PK;
+    const bool pair = a.n_pad > 64;
     CUtensorMap tmA, tmBh, tmBt;
     int rc;
-    if ((rc = make_map(&tmA, A, M, K, lda, BM, box)) || (rc = make_map(&tmBh, Bt_head, N, K, ldb, a.n_pad, box)) ||
-        (rc = make_map(&tmBt, Bt_tail, N, K, ldb, a.n_pad, box)))
-        return rc;
-    const size_t stage = (size_t)box * 4 * (2 * BM + 2 * a.n_pad);
-    const size_t smem = per_tile ? STAGES * stage + 24 * STAGES + 48 + 1024 : PSTAGES * stage + 4 * kStageBytes + 24 * PSTAGES + 64 + 1024;
-    if (per_tile) {
+    if (!pair) {
+        const size_t smem = STAGES * (size_t)BK * 4 * (2 * BM + 2 * a.n_pad) + 24 * STAGES + 48 + 1024;
+        if ((rc = make_map(&tmA, A, M, K, lda, BM)) || (rc = make_map(&tmBh, Bt_head, N, K, ldb, a.n_pad)) ||
+            (rc = make_map(&tmBt, Bt_tail, N, K, ldb, a.n_pad)))
+            return rc;
         static std::atomic<bool> granted[64];
         if ((rc = allow_smem((const void*)k_dense_nt, granted))) return rc;
-        k_dense_nt<<<(unsigned)n_tiles, kThreads, smem, (cudaStream_t)stream>>>(tmA, tmBh, tmBt, a);
+        k_dense_nt<<<(unsigned)((M + BM - 1) / BM), kThreads, smem, (cudaStream_t)stream>>>(tmA, tmBh, tmBt, a);
         return (int)cudaGetLastError();
     }
-    static std::atomic<bool> granted[64];
+    a.n_pad = (N + 31) / 32 * 32;                                 // both CTAs hold whole groups of 16 of its rows
+    if ((rc = make_map(&tmA, A, M, K, lda, BM, PK)) || (rc = make_map(&tmBh, Bt_head, N, K, ldb, a.n_pad / 2, PK)) ||
+        (rc = make_map(&tmBt, Bt_tail, N, K, ldb, a.n_pad / 2, PK)))
+        return rc;
     const int sms = sm_count();
     if (sms <= 0) return DG_ERR_STATE;
-    if ((rc = allow_smem((const void*)k_dense_nt_persistent, granted))) return rc;
-    k_dense_nt_persistent<<<(unsigned)(n_tiles < sms ? n_tiles : sms), kThreadsPersistent, smem, (cudaStream_t)stream>>>(tmA, tmBh, tmBt, a, n_tiles);
+    const size_t stage = (size_t)PK * 4 * (2 * BM + a.n_pad), rest = kEpilogueWarps * kPieceBytes + kPairBarBytes + 1024;
+    const int stages = (int)std::min<size_t>(kMaxPairStages, (227 * 1024 - rest) / stage);
+    static std::atomic<bool> granted[64];
+    static std::atomic<bool> granted_masked[64];
+    if ((rc = mask ? allow_smem((const void*)k_dense_nt_pair<true>, granted_masked) : allow_smem((const void*)k_dense_nt_pair<false>, granted))) return rc;
+    const int n_tiles = (int)((M + 2 * BM - 1) / (2 * BM));
+    (mask ? k_dense_nt_pair<true> : k_dense_nt_pair<false>)<<<2u * (unsigned)std::min(n_tiles, sms / 2), kThreadsPair, stages * stage + rest, (cudaStream_t)stream>>>(
+        tmA, tmBh, tmBt, a, n_tiles, stages);
     return (int)cudaGetLastError();
 }
 

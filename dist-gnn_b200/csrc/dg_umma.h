@@ -45,6 +45,29 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// ---- CTA pairs: two CTAs of a cluster, on the two SMs of a TPC, that the tensor cores treat as one (cta_group::2) ------------------
+// The address of the even CTA's barrier in the cluster's shared memory, given this CTA's own.
+__device__ __forceinline__ uint32_t in_leader(uint32_t bar)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(bar), "r"(0));
+    return r;
+}
+// Without a release at cluster scope, which costs some 1,900 clocks: what it reports is what the tensor cores, not another CTA's threads,
+// touch next - operands behind fence.proxy.async, or an accumulator whose tcgen05.ld has been waited for.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar)
+{
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar)      // arrives at the barrier of that offset in both CTAs
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // What a role waits for before it leaves the CTA, whether its loop came to its end or gave up: a copy that lands, or an MMA that
 // reads, after the CTA is gone would do so in the shared and tensor memory of the next one.
 // The loads of stages 0 .. issued - 1 of a ring (one full barrier a stage): the last round of every stage.
@@ -56,6 +79,11 @@ __device__ __forceinline__ void await_loads(uint32_t full0, int issued, int stag
 __device__ __forceinline__ void await_mmas(uint32_t done)
 {
     umma_commit(done);
+    mbar_wait(done, 0);
+}
+__device__ __forceinline__ void await_mmas_pair(uint32_t done)      // by the issuing CTA; the other one leaves after it, behind a cluster barrier
+{
+    umma_commit_pair(done);
     mbar_wait(done, 0);
 }
 

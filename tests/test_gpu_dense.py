@@ -177,3 +177,23 @@ def test_dense_kernels_take_column_slices_of_padded_buffers():
 def test_dense_tn_unsupported_shapes_fall_back():
     import spmm_cpp
     assert spmm_cpp.dense_tn(torch.randn(100, 47, device='cuda'), torch.randn(100, 16, device='cuda')) is None      # 188-byte rows
+
+
+@pytest.mark.parametrize('M', [1, 127, 129, 256, 257, 19073])
+@pytest.mark.parametrize('N,K', [(65, 4), (96, 16), (97, 20), (255, 36), (256, 100), (130, 8)])
+def test_dense_nt_by_cta_pairs(M, N, K):
+    """Results wider than 64 columns: tiles of 256 rows with a half that has few rows or none, more tiles than pairs, columns that end inside
+    a 32-column piece, rows of C and of the mask that are no 16-byte multiples, depths below and beside a half slab of 16."""
+    import spmm_cpp
+    g = torch.Generator(device='cuda').manual_seed(M + 1000 * N + K)
+    a = torch.randn(M, K, device='cuda', generator=g)
+    bt = torch.randn(N, K, device='cuda', generator=g)
+    want = a.double() @ bt.double().t()
+    plain = spmm_cpp.dense_nt(a, bt)
+    assert_close(plain.cpu().numpy(), want.cpu().numpy(), TOL, f'{M}x{N}x{K}')
+    assert torch.equal(spmm_cpp.dense_nt(a, bt, relu=True), plain.clamp(min=0))
+    act = torch.relu(torch.randn(M, N, device='cuda', generator=g))
+    assert torch.equal(spmm_cpp.dense_nt(a, bt, mask=act), plain * (act > 0))
+    wide = torch.nn.functional.pad(act, (0, (-N) % 4))[:, :N]
+    assert torch.equal(spmm_cpp.dense_nt(a, bt, mask=wide), plain * (act > 0))
+    assert spmm_cpp.dense_status() == 0

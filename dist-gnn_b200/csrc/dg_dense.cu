@@ -803,28 +803,38 @@ extern "C" int dg_dense_wait_selftest(int* host_gave_up, void* stream)
 // The reduction runs over the n rows of the block, so both operands are read "MN-major": a TMA box of 32 columns x 16
 // rows lands as 16 rows of 128 bytes in the 32-byte-atom variant of the 128B swizzle, which is the one layout the tensor
 // cores accept for 32-bit MN-major operands (the plain 128B swizzle makes them read zeros); the boxes of one operand lie
-// 2048 bytes apart (leading byte offset), 4-row groups 512 bytes.  Each CTA streams a contiguous range
-// of rows through a 3-stage ring, splits BOTH operands into TF32 head and tail in shared memory, accumulates the three
-// passes into one or two 128 x Nn fp32 accumulators in tensor memory, and writes its partial D to scratch; a second
-// kernel adds the partials of all CTAs in CTA order (deterministic).
+// 2048 bytes apart (leading byte offset), 4-row groups 512 bytes.  The rows are cut into as many ranges as there are CTAs; a range is
+// streamed through a ring, BOTH operands are split into TF32 head and tail in shared memory, the three
+// passes are accumulated into fp32 accumulators in tensor memory, and the range's partial D goes to scratch; a second
+// kernel adds the partials of all ranges in order (deterministic).
+//
+// One operand, P, lies along the 128 rows of an MMA, the other, Q, along its up to 256 columns.  An MMA with 32-bit operands takes
+// some 130 clocks for 128 rows however few columns it has, so P is the narrower operand (256 x 47: 47 columns padded to 128 rows, once
+// over Q's 256, instead of twice over 48) and D comes out transposed where that is G.  Where both are wider than 128 the
+// CTAs of a pair (cta_group::2) hold 128 columns of P and half of Q each, and take two ranges, one after the other.  An element of D is
+// the same sum in the same order either way.
 namespace {
 
 constexpr int TN_ROWS = 16;                     // rows of X / G per stage (two MMA k-steps of 8)
-constexpr int TN_STAGES = 3;
 constexpr int TN_BOX_BYTES = TN_ROWS * 128;     // one 32-column box
+constexpr int TN_P_BYTES = 4 * TN_BOX_BYTES;    // the 128 columns of P that a CTA holds
+constexpr int kTnSplitWarps = 8, kTnThreads = 32 * (2 + kTnSplitWarps + 4);
+constexpr int kMaxTnStages = 8, kTnBarBytes = 8 * (3 * kMaxTnStages + 5) + 8;
 
 struct DenseTnArgs {
-    float* partial;                             // [gridDim.x][m_halves][n_pad / 16][4][128][4]
+    float4* partial;                            // [range][CTA of the pair][q_store / 4][p_store]: four columns of Q, rows side by side
     int64_t n;                                  // rows to reduce over
-    int64_t rows_per_cta;                       // multiple of TN_ROWS
-    int32_t Km, Nn, n_pad, m_halves;            // n_pad: Nn rounded up to 16; m_halves: 1 (Km <= 128) or 2
+    int64_t rows_per_range;                     // multiple of TN_ROWS
+    int32_t ranges;
+    int32_t p_cols, q_cols;                     // columns of P and Q
+    int32_t q_pad;                              // columns of the MMA: a multiple of 16, of 64 for a pair
+    int32_t p_store, q_store;                   // rows and columns of a CTA's partial: multiples of 16
     int32_t flush_slabs;                        // slabs accumulated in tensor memory between two flushes
+    int32_t stages;
+    int32_t swapped;                            // P is G
     int* status;
 };
 
-// A CTA's partial D: the 128 rows of an accumulator half are the fastest index above a float4 of columns,
-// [half][16-column group][float4][row][4], so that a warp that holds 32 rows of tensor memory moves 512 contiguous bytes per
-// access.
 // MN-major tile of 32-bit elements.  The tensor cores read such operands only in the "128B swizzle with 32-byte atoms"
 // layout (32-byte chunks of a 128-byte row XOR-ed with the row index modulo 4), which TMA writes in its
 // SWIZZLE_128B_ATOM_32B mode: 4-row groups are 512 bytes apart (stride byte offset), the 32-column boxes 2048 bytes
@@ -839,182 +849,245 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr)
     d |= (uint64_t)1 << 61;                                   // layout type: SWIZZLE_128B_BASE32B
     return d;
 }
-__device__ __forceinline__ uint32_t umma_idesc_tf32_mn(int n_pad)
-{
-    return umma_idesc_tf32(n_pad) | (1u << 15) | (1u << 16);  // A and B are MN-major
-}
 
-__global__ void __launch_bounds__(kThreads, 1)
-k_dense_tn(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, const DenseTnArgs a)
+// What bounds it: shared memory (MN-major 32-bit operands are read at half its rate) for wide operands, the MMAs' 130 clocks for narrow
+// ones.  2,449,029 rows (us; four warps that split and flush in turn, two accumulators of one CTA -> this): 256 x 256 1,830 -> 1,660,
+// 100 x 256 1,205 -> 940, 256 x 47 1,017 -> 787, 256 x 128 1,280 -> 970; 150,001 rows: 127 -> 120, 91 -> 73, 78 -> 66, 96 -> 71.
+// Warps: 0 TMA, 1 MMA issue + tensor-memory allocation, 2-9 split, 10-13 flush.  Two accumulators (columns 0 / 256): while one is added to
+// the partial result the other takes the next rows.
+template <bool PAIR>
+__device__ __forceinline__ void dense_tn(const CUtensorMap& tmP, const CUtensorMap& tmQ, const DenseTnArgs& a)
 {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* gbase = smem_raw + (base - raw);
-    const int x_boxes = a.m_halves * 4;                           // 32-column boxes covering the (padded) Km
-    const int g_boxes = (a.n_pad + 31) / 32;
-    const int x_bytes = x_boxes * TN_BOX_BYTES, g_bytes = g_boxes * TN_BOX_BYTES;
-    const int stage_bytes = 2 * x_bytes + 2 * g_bytes;            // X head, X tail, G head, G tail
-    const uint32_t bars = base + TN_STAGES * stage_bytes;
-    const uint32_t full0 = bars, ready0 = bars + 8 * TN_STAGES, empty0 = bars + 16 * TN_STAGES, acc_full = bars + 24 * TN_STAGES;
-    const uint32_t acc_empty = acc_full + 8, done = acc_full + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + TN_STAGES * stage_bytes + 24 * TN_STAGES + 24);
+    const int rank = PAIR ? blockIdx.x & 1 : 0;
+    const int range0 = PAIR ? blockIdx.x & ~1 : blockIdx.x, range1 = min(a.ranges, range0 + (PAIR ? 2 : 1));
+    const int p0 = rank * 128, q0 = rank * (a.q_pad / 2);         // first columns of this CTA
+    const int p_boxes = max(0, min(4, (a.p_cols - p0 + 31) / 32)), q_boxes = (PAIR ? a.q_pad / 2 : a.q_pad + 31) / 32;
+    const int q_bytes = q_boxes * TN_BOX_BYTES;
+    const int stage_bytes = 2 * TN_P_BYTES + 2 * q_bytes;         // P head, P tail, Q head, Q tail
+    const uint32_t bars = base + a.stages * stage_bytes;
+    const uint32_t full0 = bars, ready0 = bars + 8 * kMaxTnStages, empty0 = bars + 16 * kMaxTnStages, acc_full0 = bars + 24 * kMaxTnStages;
+    const uint32_t acc_empty0 = acc_full0 + 16, done = acc_empty0 + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + a.stages * stage_bytes + 24 * kMaxTnStages + 40);
     const int T = a.flush_slabs;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t r_begin = (int64_t)blockIdx.x * a.rows_per_cta;
-    const int64_t r_end = min(r_begin + a.rows_per_cta, a.n);
-    const int nslabs = r_end > r_begin ? (int)((r_end - r_begin + TN_ROWS - 1) / TN_ROWS) : 0;
-    int tmem_cols = 32;
-    while (tmem_cols < (a.m_halves == 2 ? 256 + a.n_pad : a.n_pad)) tmem_cols <<= 1;
+    auto slabs_of = [&](int range) { return (int)((max((int64_t)0, min(a.rows_per_range, a.n - range * a.rows_per_range)) + TN_ROWS - 1) / TN_ROWS); };
+    constexpr int kTmemCols = 512;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TN_STAGES; ++s) {
+        for (int s = 0; s < a.stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
-            mbar_init(ready0 + 8 * s, 128);
+            mbar_init(ready0 + 8 * s, (PAIR ? 2 : 1) * kTnSplitWarps);
             mbar_init(empty0 + 8 * s, 1);
         }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_empty, 128);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(acc_full0 + 8 * b, 1);
+            mbar_init(acc_empty0 + 8 * b, (PAIR ? 2 : 1) * 4);
+        }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    auto sync_unit = [&] {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if constexpr (PAIR) cluster_sync();
+        else __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    };
+    sync_unit();
     const uint32_t tmem = *tmem_slot;
     bool ok = true;
+    auto commit = [](uint32_t bar) {
+        if constexpr (PAIR) umma_commit_pair(bar);
+        else umma_commit(bar);
+    };
+    auto arrive = [](uint32_t bar) {                              // `bar`: of the CTA that issues the MMAs
+        if constexpr (PAIR) mbar_arrive_cluster(bar);
+        else mbar_arrive(bar);
+    };
+    uint32_t issuer_ready0 = ready0, issuer_acc_empty0 = acc_empty0;
+    if constexpr (PAIR) {
+        issuer_ready0 = in_leader(ready0);
+        issuer_acc_empty0 = in_leader(acc_empty0);
+    }
 
     if (warp == 0) {
         if (lane == 0) {                                          // TMA producer
-            int i = 0;
-            for (; i < nslabs && ok; ++i) {
-                const int s = i % TN_STAGES, u = i / TN_STAGES;
-                if (u > 0) ok = mbar_wait(empty0 + 8 * s, (u - 1) & 1);
-                if (!ok) break;
-                const uint32_t st = base + s * stage_bytes;
-                const int r0 = (int)(r_begin + (int64_t)i * TN_ROWS);
-                mbar_expect_tx(full0 + 8 * s, x_bytes + g_bytes);
-                for (int j = 0; j < x_boxes; ++j) tma_load_2d(st + j * TN_BOX_BYTES, &tmX, 32 * j, r0, full0 + 8 * s);
-                for (int j = 0; j < g_boxes; ++j) tma_load_2d(st + 2 * x_bytes + j * TN_BOX_BYTES, &tmG, 32 * j, r0, full0 + 8 * s);
+            int it = 0, s = 0, phase = 1;
+            for (int range = range0; range < range1; ++range) {
+                const int nslabs = slabs_of(range);
+                for (int i = 0; i < nslabs && ok; ++i, ++it) {
+                    if (it >= a.stages) ok = mbar_wait(empty0 + 8 * s, phase);
+                    if (!ok) break;
+                    const uint32_t st = base + s * stage_bytes;
+                    const int r0 = (int)(range * a.rows_per_range + (int64_t)i * TN_ROWS);
+                    mbar_expect_tx(full0 + 8 * s, (p_boxes + q_boxes) * TN_BOX_BYTES);
+                    for (int j = 0; j < p_boxes; ++j) tma_load_2d(st + j * TN_BOX_BYTES, &tmP, p0 + 32 * j, r0, full0 + 8 * s);
+                    for (int j = 0; j < q_boxes; ++j) tma_load_2d(st + 2 * TN_P_BYTES + j * TN_BOX_BYTES, &tmQ, q0 + 32 * j, r0, full0 + 8 * s);
+                    if (++s == a.stages) s = 0, phase ^= 1;
+                }
             }
-            await_loads(full0, i, TN_STAGES);
+            await_loads(full0, it, a.stages);
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                          // MMA issuer
-            const uint32_t idesc = umma_idesc_tf32_mn(a.n_pad);
-            for (int i = 0; i < nslabs && ok; ++i) {
-                const int s = i % TN_STAGES, u = i / TN_STAGES;
-                const int grp = i / T, in_grp = i % T;            // the accumulators restart with every flush group
-                if (in_grp == 0 && grp > 0) ok = mbar_wait(acc_empty, (grp - 1) & 1);
-                if (!ok) break;
-                const uint32_t st = base + s * stage_bytes;
-                const uint64_t g_head = umma_desc_mn_sw128(st + 2 * x_bytes), g_tail = umma_desc_mn_sw128(st + 2 * x_bytes + g_bytes);
-                ok = mbar_wait(ready0 + 8 * s, u & 1);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int h = 0; h < a.m_halves; ++h) {
-                    const uint64_t x_head = umma_desc_mn_sw128(st + h * 4 * TN_BOX_BYTES);
-                    const uint64_t x_tail = umma_desc_mn_sw128(st + x_bytes + h * 4 * TN_BOX_BYTES);
-                    const uint32_t acc = tmem + (uint32_t)(h * 256);
+        if (lane == 0 && rank == 0) {                             // MMA issuer
+            // A and B MN-major, 128 rows per CTA
+            const uint32_t idesc = (umma_idesc_tf32(a.q_pad) + (PAIR ? (uint32_t)(BM >> 4) << 24 : 0u)) | (1u << 15) | (1u << 16);
+            int s = 0, phase = 0, group = 0;
+            for (int range = range0; range < range1; ++range) {
+                const int nslabs = slabs_of(range);
+                for (int i = 0; i < nslabs && ok; ++i) {
+                    const int b = group & 1, in_group = i % T;    // the accumulators change, and restart, with every flush group
+                    if (in_group == 0 && group >= 2) ok = mbar_wait(acc_empty0 + 8 * b, ((group >> 1) - 1) & 1);
+                    ok = ok && mbar_wait(ready0 + 8 * s, phase);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t st = base + s * stage_bytes, acc = tmem + (uint32_t)(b * 256);
+                    const uint64_t p_head = umma_desc_mn_sw128(st), p_tail = umma_desc_mn_sw128(st + TN_P_BYTES);
+                    const uint64_t q_head = umma_desc_mn_sw128(st + 2 * TN_P_BYTES), q_tail = umma_desc_mn_sw128(st + 2 * TN_P_BYTES + q_bytes);
+                    auto multiply = [&](uint64_t p, uint64_t q, uint32_t add) {
+                        if constexpr (PAIR) umma_tf32_pair(acc, p, q, idesc, add);
+                        else umma_tf32(acc, p, q, idesc, add);
+                    };
 #pragma unroll
-                    for (int k = 0; k < TN_ROWS / 8; ++k) {       // one 8-row group (1024 bytes) per MMA
+                    for (int k = 0; k < TN_ROWS / 8; ++k) {       // one 8-row group (1024 bytes) per MMA; the tail of X comes first
                         const uint64_t adv = (uint64_t)(k * (1024 >> 4));
-                        umma_tf32(acc, x_tail + adv, g_head + adv, idesc, (in_grp > 0 || k > 0) ? 1u : 0u);
-                        umma_tf32(acc, x_head + adv, g_tail + adv, idesc, 1u);
-                        umma_tf32(acc, x_head + adv, g_head + adv, idesc, 1u);
+                        multiply((a.swapped ? p_head : p_tail) + adv, (a.swapped ? q_tail : q_head) + adv, (in_group > 0 || k > 0) ? 1u : 0u);
+                        multiply((a.swapped ? p_tail : p_head) + adv, (a.swapped ? q_head : q_tail) + adv, 1u);
+                        multiply(p_head + adv, q_head + adv, 1u);
                     }
+                    commit(empty0 + 8 * s);
+                    if (in_group == T - 1 || i == nslabs - 1) {
+                        commit(acc_full0 + 8 * b);
+                        ++group;
+                    }
+                    if (++s == a.stages) s = 0, phase ^= 1;
                 }
-                umma_commit(empty0 + 8 * s);
-                if (in_grp == T - 1 || i == nslabs - 1) umma_commit(acc_full);
             }
-            await_mmas(done);
+            if constexpr (PAIR) await_mmas_pair(done);
+            else await_mmas(done);
+        } else if (lane == 0) {
+            mbar_wait(done, 0);
         }
-    } else {
-        const int t = threadIdx.x - 64;
-        const int q = warp & 3;                                   // the quarter of the tensor-memory lanes this warp may read
-        float4* part4 = reinterpret_cast<float4*>(a.partial + (size_t)blockIdx.x * a.m_halves * 128 * a.n_pad) + q * 32 + lane;
-        for (int i = 0; i < nslabs && ok; ++i) {
-            const int s = i % TN_STAGES, u = i / TN_STAGES;
-            ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, u & 1));        // warp-uniform: tcgen05.ld below is .aligned
+    } else if (warp < 2 + kTnSplitWarps) {
+        // The tile as loaded serves as head, its tail goes behind it.  Half the warps take the even boxes, half the odd ones.  Columns of P
+        // that it does not have are neither loaded nor split: what lies there reaches rows of the accumulators that nobody reads.
+        const int t = threadIdx.x - 64, half = t >> 7, boxes = p_boxes + q_boxes;
+        int s = 0, phase = 0, slabs = 0;
+        for (int range = range0; range < range1; ++range) slabs += slabs_of(range);
+        for (int i = 0; i < slabs; ++i) {
+            ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, phase));
             if (!ok) break;
-            unsigned char* st = gbase + (size_t)s * stage_bytes;
-            for (int part = 0; part < 2; ++part) {                // X then G: the tile as loaded serves as head, its tail goes behind it
-                float4* head = reinterpret_cast<float4*>(st + (part ? 2 * x_bytes : 0));
-                const int count = (part ? g_bytes : x_bytes) / 16;
-                float4* tail = head + count;
-                for (int j = t; j < count; j += 128) {
-                    const float4 x = head[j];
+            unsigned char* st = gbase + (size_t)s * stage_bytes + (t & 127) * 16;
+            auto at = [&](int box) { return st + (box < p_boxes ? box * TN_BOX_BYTES : 2 * TN_P_BYTES + (box - p_boxes) * TN_BOX_BYTES); };
+            for (int b0 = half; b0 < boxes; b0 += 8) {
+                float4 x[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (b0 + 2 * j < boxes) x[j] = *reinterpret_cast<const float4*>(at(b0 + 2 * j));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int box = b0 + 2 * j;
+                    if (box >= boxes) break;
                     float4 h;
-                    h.x = __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u); h.y = __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
-                    h.z = __uint_as_float(__float_as_uint(x.z) & 0xFFFFE000u); h.w = __uint_as_float(__float_as_uint(x.w) & 0xFFFFE000u);
-                    tail[j] = make_float4(x.x - h.x, x.y - h.y, x.z - h.z, x.w - h.w);
+                    h.x = __uint_as_float(__float_as_uint(x[j].x) & 0xFFFFE000u); h.y = __uint_as_float(__float_as_uint(x[j].y) & 0xFFFFE000u);
+                    h.z = __uint_as_float(__float_as_uint(x[j].z) & 0xFFFFE000u); h.w = __uint_as_float(__float_as_uint(x[j].w) & 0xFFFFE000u);
+                    *reinterpret_cast<float4*>(at(box) + (box < p_boxes ? TN_P_BYTES : q_bytes)) = make_float4(x[j].x - h.x, x[j].y - h.y, x[j].z - h.z, x[j].w - h.w);
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive(ready0 + 8 * s);
-            if (i % T != T - 1 && i != nslabs - 1) continue;
-            // Flush: the tensor cores add into their accumulator with truncation, an error that grows with the length
-            // of the chain, so after T slabs the accumulators are added - rounded to nearest - into this CTA's partial
-            // result (which stays in L2) and restart from zero.
-            const int grp = i / T;
-            ok = __all_sync(0xffffffffu, mbar_wait(acc_full, grp & 1));
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            for (int h = 0; h < a.m_halves; ++h) {
-                for (int c0 = 0; c0 < a.n_pad; c0 += 32) {        // two 16-column reads in flight per wait
-                    const int two = c0 + 16 < a.n_pad;            // warp-uniform
+            __syncwarp();
+            if (lane == 0) arrive(issuer_ready0 + 8 * s);
+            if (++s == a.stages) s = 0, phase ^= 1;
+        }
+    } else {
+        // Flush: the tensor cores add into their accumulator with truncation, an error that grows with the length
+        // of the chain, so after T slabs an accumulator is added - rounded to nearest - into this CTA's partial
+        // result (which stays in L2) and restarts from zero.
+        const int q = warp & 3, row = q * 32 + lane;              // a warp may only read its own quarter of the TMEM lanes
+        const bool stored = row < a.p_store;
+        int group = 0;
+        for (int range = range0; range < range1 && ok; ++range) {
+            float4* part = a.partial + (int64_t)((PAIR ? 2 : 1) * range + rank) * (a.q_store / 4) * a.p_store + row;
+            const int groups = (slabs_of(range) + T - 1) / T;
+            for (int g = 0; g < groups; ++g, ++group) {
+                const int b = group & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(acc_full0 + 8 * b, (group >> 1) & 1));        // tcgen05.ld is warp-collective
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int c0 = 0; c0 < a.q_store; c0 += 32) {      // two 16-column reads in flight per wait
+                    const int two = c0 + 16 < a.q_store;          // warp-uniform
                     uint32_t r[32];
-                    tmem_ld16(tmem + (uint32_t)(h * 256) + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-                    if (two) tmem_ld16(tmem + (uint32_t)(h * 256) + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + 16), r + 16);
+                    const uint32_t acc = tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
+                    tmem_ld16(acc, r);
+                    if (two) tmem_ld16(acc + 16, r + 16);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    float4* p = part4 + (size_t)(h * (a.n_pad >> 4) + (c0 >> 4)) * 4 * 128;
+                    float4* p = part + (int64_t)(c0 / 4) * a.p_store;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        if (j >= 4 && !two) break;
+                        if (!stored || (j >= 4 && !two)) break;
                         // Only this thread ever touches these 16 bytes, in program order, so the sum order is fixed; the
                         // reduction is sent to L2 and not waited for.
-                        if (grp == 0)
-                            __stcg(p + j * 128, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                                            __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
+                        if (g == 0)
+                            __stcg(p + j * a.p_store, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                                  __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
                         else
-                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + j * 128), "f"(__uint_as_float(r[4 * j])),
+                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + j * a.p_store), "f"(__uint_as_float(r[4 * j])),
                                          "f"(__uint_as_float(r[4 * j + 1])), "f"(__uint_as_float(r[4 * j + 2])), "f"(__uint_as_float(r[4 * j + 3]))
                                          : "memory");
                     }
                 }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) arrive(issuer_acc_empty0 + 8 * b);
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            mbar_arrive(acc_empty);
-        }
-        if (nslabs == 0) {                                        // a CTA without rows contributes zeros
-            for (int j = 0; j < a.m_halves * a.n_pad / 4; ++j) __stcg(part4 + (size_t)j * 128, make_float4(0.f, 0.f, 0.f, 0.f));
+            if (groups == 0 && stored)                            // a range without rows contributes zeros
+                for (int j = 0; j < a.q_store / 4; ++j) __stcg(part + (int64_t)j * a.p_store, make_float4(0.f, 0.f, 0.f, 0.f));
         }
     }
     if (!ok) atomicExch(a.status, 1);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 1)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
+    sync_unit();                                                  // no CTA leaves while the other's MMAs read its operands or arrive at its barriers
+    if (warp == 1) {
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    }
+}
+__global__ void __launch_bounds__(kTnThreads, 1)
+k_dense_tn(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, const DenseTnArgs a)
+{
+    dense_tn<false>(tmP, tmQ, a);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTnThreads, 1)
+k_dense_tn_pair(const __grid_constant__ CUtensorMap tmP, const __grid_constant__ CUtensorMap tmQ, const DenseTnArgs a)
+{
+    dense_tn<true>(tmP, tmQ, a);
 }
 
-// One thread per slot of the partial layout (coalesced over the CTAs' partials); slots of the padding are skipped.
-__global__ void k_dense_tn_reduce(const float* __restrict__ partial, int n_parts, int64_t slots, float* __restrict__ D, int64_t ldd,
-                                  int32_t Km, int32_t Nn, int32_t n_pad)
+// One thread per slot of the partial layout (coalesced over the ranges' partials); slots of the padding are skipped.
+__global__ void k_dense_tn_reduce(const float* __restrict__ partial, int ranges, int64_t slots, float* __restrict__ D, int64_t ldd,
+                                  int32_t p_cols, int32_t q_cols, int32_t p_store, int32_t q_store, int transposed)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= slots) return;
-    const int e = (int)(i & 3), r = (int)((i >> 2) & 127);
-    const int64_t blk = i >> 9;                                   // (half, 16-column group, float4 within the group)
-    const int j4 = (int)(blk & 3), c16 = (int)((blk >> 2) % (n_pad >> 4)), h = (int)((blk >> 2) / (n_pad >> 4));
-    const int m = h * 128 + r, c = c16 * 16 + j4 * 4 + e;
-    if (m >= Km || c >= Nn) return;
+    const int half_slots = p_store * q_store;
+    const int half = (int)(i / half_slots), in_half = (int)(i % half_slots), c4 = in_half / (4 * p_store), rest = in_half % (4 * p_store);
+    const int p = half * 128 + rest / 4, q = c4 * 4 + rest % 4;
+    if (p >= p_cols || q >= q_cols) return;
     float sum = 0.f;
-    for (int p = 0; p < n_parts; ++p) sum += partial[(size_t)p * slots + i];
-    D[(int64_t)m * ldd + c] = sum;
+#pragma unroll 32                                                 // in flight at a time: what there is to do is wait for the L2
+    for (int r = 0; r < ranges; ++r) sum += partial[(int64_t)r * slots + i];
+    D[transposed ? (int64_t)q * ldd + p : (int64_t)p * ldd + q] = sum;
 }
 
 int make_map_box(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int64_t ld, int box_cols, int box_rows)
@@ -1056,25 +1129,34 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
             }
         return DG_OK;
     }
+    const bool pair = std::min(Km, Nn) > 128, swapped = !pair && Nn < Km;
     DenseTnArgs a{};
-    a.n = n; a.Km = Km; a.Nn = Nn; a.n_pad = (Nn + 15) / 16 * 16; a.m_halves = Km > 128 ? 2 : 1;
+    a.n = n;
+    a.p_cols = swapped ? Nn : Km;
+    a.q_cols = swapped ? Km : Nn;
+    a.q_store = (a.q_cols + 15) / 16 * 16;
+    a.q_pad = pair ? (a.q_cols + 63) / 64 * 64 : a.q_store;       // a pair's halves are whole boxes
+    a.p_store = pair ? 128 : (a.p_cols + 15) / 16 * 16;
     const int64_t slabs = (n + TN_ROWS - 1) / TN_ROWS;
-    const int ctas = (int)std::min<int64_t>(max_ctas, slabs);
-    a.rows_per_cta = (slabs + ctas - 1) / ctas * TN_ROWS;
-    const int64_t slots = (int64_t)a.m_halves * 128 * a.n_pad;    // one CTA's partial, padding included
-    if (ctas * slots > scratch_floats) return DG_ERR_SCRATCH;
+    a.ranges = (int)std::min<int64_t>(max_ctas, slabs);
+    a.rows_per_range = (slabs + a.ranges - 1) / a.ranges * TN_ROWS;
+    a.swapped = swapped;
+    const int64_t slots = (int64_t)(pair ? 2 : 1) * a.p_store * a.q_store;     // a range's partial, padding included
+    if (a.ranges * slots > scratch_floats) return DG_ERR_SCRATCH;
     a.flush_slabs = 16;                                           // 256 rows = 96 tensor-core accumulations per chain
-    a.partial = scratch;
+    a.partial = reinterpret_cast<float4*>(scratch);
     a.status = dg_status_word();
     if (!a.status) return DG_ERR_STATE;
     CUtensorMap tmX, tmG;
     int rc;
     if ((rc = make_map_box(&tmX, X, n, Km, ldx, 32, TN_ROWS)) || (rc = make_map_box(&tmG, G, n, Nn, ldg, 32, TN_ROWS))) return rc;
-    const int x_bytes = a.m_halves * 4 * TN_BOX_BYTES, g_bytes = (a.n_pad + 31) / 32 * TN_BOX_BYTES;
-    const size_t smem = (size_t)TN_STAGES * (2 * x_bytes + 2 * g_bytes) + 24 * TN_STAGES + 32 + 1024;
-    static std::atomic<bool> granted[64];
-    if ((rc = allow_smem((const void*)k_dense_tn, granted))) return rc;
-    k_dense_tn<<<ctas, kThreads, smem, (cudaStream_t)stream>>>(tmX, tmG, a);
-    k_dense_tn_reduce<<<(unsigned)((slots + 255) / 256), 256, 0, (cudaStream_t)stream>>>(scratch, ctas, slots, D, ldd, Km, Nn, a.n_pad);
+    const size_t stage = 2 * TN_P_BYTES + 2 * (((pair ? a.q_pad / 2 : a.q_pad) + 31) / 32) * TN_BOX_BYTES;
+    a.stages = (int)std::min<size_t>(kMaxTnStages, (227 * 1024 - kTnBarBytes - 1024) / stage);
+    const size_t smem = a.stages * stage + kTnBarBytes + 1024;
+    const CUtensorMap &tmP = swapped ? tmG : tmX, &tmQ = swapped ? tmX : tmG;
+    static std::atomic<bool> granted[64], granted_pair[64];
+    if ((rc = pair ? allow_smem((const void*)k_dense_tn_pair, granted_pair) : allow_smem((const void*)k_dense_tn, granted))) return rc;
+    (pair ? k_dense_tn_pair : k_dense_tn)<<<pair ? (a.ranges + 1) / 2 * 2 : a.ranges, kTnThreads, smem, (cudaStream_t)stream>>>(tmP, tmQ, a);
+    k_dense_tn_reduce<<<(unsigned)((slots + 255) / 256), 256, 0, (cudaStream_t)stream>>>(scratch, a.ranges, slots, D, ldd, a.p_cols, a.q_cols, a.p_store, a.q_store, swapped);
     return (int)cudaGetLastError();
 }

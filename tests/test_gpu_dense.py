@@ -197,3 +197,24 @@ def test_dense_nt_by_cta_pairs(M, N, K):
     wide = torch.nn.functional.pad(act, (0, (-N) % 4))[:, :N]
     assert torch.equal(spmm_cpp.dense_nt(a, bt, mask=wide), plain * (act > 0))
     assert spmm_cpp.dense_status() == 0
+
+
+@pytest.mark.parametrize('n', [1, 15, 17, 257, 4096 + 5, 148 * 256 + 1])
+@pytest.mark.parametrize('Km,Nn', [(129, 130), (256, 193), (256, 128), (128, 256), (10, 200), (200, 5), (1, 40), (96, 96)])
+@pytest.mark.parametrize('ctas', [1, 5, 148])
+def test_dense_tn_roles_and_ranges(n, Km, Nn, ctas):
+    """Either operand along the rows of the MMAs, alone or by CTA pairs; ranges without rows, an odd number of them for the last pair, fewer
+    rows than a slab, several flushes in a range; the scratch exactly as large as documented, with a guard behind it.  An element's error
+    goes with sqrt(n) (1.2e-6 of it; TOL leaves 8 times that), so results are compared over at least 40 elements: one that cancels to a
+    fourteenth of sqrt(n) is 1.6e-5 off by itself."""
+    import spmm_cpp
+    g = torch.Generator(device='cuda').manual_seed(n + 1000 * Km + Nn)
+    x = torch.randn(n, Km + (-Km) % 4, device='cuda', generator=g)
+    y = torch.randn(n, Nn + (-Nn) % 4, device='cuda', generator=g)
+    need = min(ctas, (n + 15) // 16) * (-(-Km // 128) * 128) * (-(-Nn // 16) * 16)
+    scratch = torch.full((need + 1024,), 3.5, device='cuda')
+    d = torch.full((Km, Nn + 3), -1.0, device='cuda')
+    spmm_cpp.check(spmm_cpp.lib().dg_dense_tn(x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), d.data_ptr(), Nn + 3, n, Km, Nn, scratch.data_ptr(), need,
+                                              ctas, spmm_cpp._stream()))
+    assert_close(d[:, :Nn].cpu().numpy(), (x[:, :Km].double().t() @ y[:, :Nn].double()).cpu().numpy(), TOL, f'{n}x{Km}x{Nn} on {ctas}')
+    assert bool((d[:, Nn:] == -1).all()) and bool((scratch[need:] == 3.5).all()) and spmm_cpp.dense_status() == 0

@@ -72,9 +72,13 @@ struct SpmmArgs {
     const int* failed_check;
 };
 
+// VEC floats side by side, aligned to as many (8: 32 bytes).  A gathered row comes by way of the L1, which holds the most frequent ones.
 template <int VEC> __device__ __forceinline__ void load_vec(const float* p, float (&out)[VEC])
 {
-    if constexpr (VEC == 4) {
+    if constexpr (VEC == 8) {
+        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(out[0]), "=f"(out[1]), "=f"(out[2]), "=f"(out[3]), "=f"(out[4]), "=f"(out[5]), "=f"(out[6]), "=f"(out[7]) : "l"(p));
+    } else if constexpr (VEC == 4) {
         const float4 v = __ldg(reinterpret_cast<const float4*>(p));
         out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
     } else if constexpr (VEC == 2) {
@@ -84,6 +88,29 @@ template <int VEC> __device__ __forceinline__ void load_vec(const float* p, floa
         out[0] = __ldg(p);
     }
 }
+// Pieces of at most 16 bytes, by the given access.
+template <int VEC, class Use> __device__ __forceinline__ void each_piece(Use use)
+{
+    if constexpr (VEC == 8) {
+        use(0);
+        use(4);
+    } else {
+        use(0);
+    }
+}
+template <int VEC> struct Piece { using type = float4; };
+template <> struct Piece<2> { using type = float2; };
+template <> struct Piece<1> { using type = float; };
+template <int VEC> using piece_t = typename Piece<VEC>::type;
+__device__ __forceinline__ void set_scaled(float* acc, float scale, float4 v) { acc[0] = scale * v.x; acc[1] = scale * v.y; acc[2] = scale * v.z; acc[3] = scale * v.w; }
+__device__ __forceinline__ void set_scaled(float* acc, float scale, float2 v) { acc[0] = scale * v.x; acc[1] = scale * v.y; }
+__device__ __forceinline__ void set_scaled(float* acc, float scale, float v) { acc[0] = scale * v; }
+__device__ __forceinline__ void add(float* acc, float4 v) { acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w; }
+__device__ __forceinline__ void add(float* acc, float2 v) { acc[0] += v.x; acc[1] += v.y; }
+__device__ __forceinline__ void add(float* acc, float v) { acc[0] += v; }
+__device__ __forceinline__ void pack(float4& v, const float* acc) { v = make_float4(acc[0], acc[1], acc[2], acc[3]); }
+__device__ __forceinline__ void pack(float2& v, const float* acc) { v = make_float2(acc[0], acc[1]); }
+__device__ __forceinline__ void pack(float& v, const float* acc) { v = acc[0]; }
 
 // What is left to do with a sum before it is stored: alpha * sum + beta * C (alpha == 1 has beta * C in the sum already), row
 // scale, bias, ReLU.
@@ -157,7 +184,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
                 c_next = __ldcs(col + e + base + LPR);            // streamed once: keep it from displacing rows of B in cache
                 v_next = __ldcs(val + e + base + LPR);
             }
-            const int cnt = len - base, steps = min(LPR, longest - base);
+            const int cnt = LPR % U ? min(LPR, len - base) : len - base, steps = min(LPR, longest - base);
 #pragma unroll 1
             for (int k = 0; k < steps; k += U) {
                 float x[U][TPL][VEC], w[U];
@@ -165,6 +192,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
                 for (int u = 0; u < U; ++u) {
                     const int j = __shfl_sync(0xffffffffu, c, k + u, LPR);
                     w[u] = __shfl_sync(0xffffffffu, v, k + u, LPR);          // 0 beyond the last entry
+                    if (LPR % U && k + u >= LPR) w[u] = 0.f;                 // the next set's
                     const float* row = bl + j * ldb;
 #pragma unroll
                     for (int t = 0; t < TPL; ++t) {
@@ -201,14 +229,8 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
 #pragma unroll
                 for (int q = 0; q < VEC; ++q)
                     if ((vec0 + t * LPR) * VEC + q < a.F) acc[t][q] = a.beta * __ldcs(p + q);
-            } else if constexpr (VEC == 4) {
-                const float4 o = __ldcs(reinterpret_cast<const float4*>(p));
-                acc[t][0] = a.beta * o.x; acc[t][1] = a.beta * o.y; acc[t][2] = a.beta * o.z; acc[t][3] = a.beta * o.w;
-            } else if constexpr (VEC == 2) {
-                const float2 o = __ldcs(reinterpret_cast<const float2*>(p));
-                acc[t][0] = a.beta * o.x; acc[t][1] = a.beta * o.y;
             } else {
-                acc[t][0] = a.beta * __ldcs(p);
+                each_piece<VEC>([&](int at) { set_scaled(acc[t] + at, a.beta, __ldcs(reinterpret_cast<const piece_t<VEC>*>(p + at))); });
             }
         }
     };
@@ -229,12 +251,12 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
 #pragma unroll
                 for (int q = 0; q < VEC; ++q)
                     if (c0 + q < a.F) __stcs(p + q, acc[t][q]);
-            } else if constexpr (VEC == 4) {
-                __stcs(reinterpret_cast<float4*>(p), make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]));
-            } else if constexpr (VEC == 2) {
-                __stcs(reinterpret_cast<float2*>(p), make_float2(acc[t][0], acc[t][1]));
             } else {
-                __stcs(p, acc[t][0]);
+                each_piece<VEC>([&](int at) {
+                    piece_t<VEC> v;
+                    pack(v, acc[t] + at);
+                    __stcs(reinterpret_cast<piece_t<VEC>*>(p + at), v);
+                });
             }
         }
     };
@@ -260,9 +282,11 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
             for (int t = 0; t < TPL; ++t) {
                 if (!on[t]) continue;
                 float* p = sp + t * LPR * VEC;
-                if constexpr (VEC == 4) __stcg(reinterpret_cast<float4*>(p), make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]));
-                else if constexpr (VEC == 2) __stcg(reinterpret_cast<float2*>(p), make_float2(acc[t][0], acc[t][1]));
-                else __stcg(p, acc[t][0]);
+                each_piece<VEC>([&](int at) {
+                    piece_t<VEC> v;
+                    pack(v, acc[t] + at);
+                    __stcg(reinterpret_cast<piece_t<VEC>*>(p + at), v);
+                });
             }
         }
         __threadfence();                                          // the partial sum is in place before the count says so
@@ -282,26 +306,17 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
 #pragma unroll 4
             for (int s = 0; s < ch.nchunks; ++s) {
                 const float* ps = p + s * a.lds;
-                if constexpr (VEC == 4) {
-                    const float4 x = __ldcg(reinterpret_cast<const float4*>(ps));
-                    acc[t][0] += x.x; acc[t][1] += x.y; acc[t][2] += x.z; acc[t][3] += x.w;
-                } else if constexpr (VEC == 2) {
-                    const float2 x = __ldcg(reinterpret_cast<const float2*>(ps));
-                    acc[t][0] += x.x; acc[t][1] += x.y;
-                } else {
-                    acc[t][0] += __ldcg(ps);
-                }
+                each_piece<VEC>([&](int at) { add(acc[t] + at, __ldcg(reinterpret_cast<const piece_t<VEC>*>(ps + at))); });
             }
         }
         if constexpr (MODE == kTiled) {
             const int2 part = a.parts[ch.heavy];
-            const float4* p = a.part_area + ((int64_t)(part.x >> 7) * a.part_ld4 + vec0) * 128 + (part.x & 127);
+            const float4* p = a.part_area + ((int64_t)(part.x >> 7) * a.part_ld4 + vec0 * (VEC / 4)) * 128 + (part.x & 127);
             for (int s = 0; s < part.y; ++s, p += a.part_ld4 * 128)
 #pragma unroll
                 for (int t = 0; t < TPL; ++t) {
                     if (!on[t]) continue;
-                    const float4 x = __ldcg(p + t * LPR * 128);
-                    acc[t][0] += x.x; acc[t][1] += x.y; acc[t][2] += x.z; acc[t][3] += x.w;
+                    each_piece<VEC>([&](int at) { add(acc[t] + at, __ldcg(p + (t * LPR * (VEC / 4) + at / 4) * 128)); });
                 }
         }
         store_row(ch.row);
@@ -400,7 +415,7 @@ int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
         const dim3 grid((unsigned)(chunk_ctas + row_ctas), (unsigned)std::min((a.vec_end - a.vec_first + tile - 1) / tile, DG_FINISH_TILES));
         if (!whole) k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kPlain><<<grid, 256, 0, stream>>>(a, chunk_ctas);
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-        if constexpr (VEC == 4) {
+        if constexpr (VEC >= 4) {
             if (!whole) continue;
             k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kTiled><<<grid, 256, 0, stream>>>(a, chunk_ctas);
             SpmmArgs w = *whole;
@@ -422,21 +437,51 @@ int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
 // have too few rows for that and want a row spread over more lanes.  us per product, this form against twice the lanes:
 //   F = 256: 1 M nodes / 17 M entries 1,545 -> 1,296, 2.4 M / 126 M 9,850 -> 8,640; 10,000 nodes / 210 k entries 27 -> 41 (not taken)
 //   F = 100: 936 -> 717, 5,540 -> 4,350, 150 k nodes / 2.6 M entries 131 -> 115; F = 48: 470 -> 389, 2,750 -> 2,250
+// Where rows are whole, aligned 32-byte pieces (`octets`) the wide form reads those: half the load instructions, with 24 warps
+// instead of 32 (F = 256: 2.4 M / 126 M with tiles 7,810 -> 7,550, 1 M / 17 M 1,291 -> 1,274, 300 k / 15 M 876 -> 855; F = 512: 2,860 -> 2,800).
+// Small matrices, wide rows: three gathers in flight (with four, 72 bytes of spills: eight 306 k-row stage blocks 1,459 -> 1,409,
+// 150 k / 2.6 M F = 256 204 -> 197, F = 200 197 -> 190).
+// 65 to 96 floats, from 4 M entries: 8 lanes of three vectors, of which at most 7 idle (16 x 2: up to 15).  1 M / 17 M F = 96 676 -> 618, 600 k /
+// 21 M 676 -> 622, 2.4 M / 126 M 4,190 -> 3,920, 300 k / 15 M 471 -> 447, 2.4 M / 42 M 1,758 -> 1,798 (F = 72 1,700 -> 1,680); 150 k / 2.6 M 111 -> 119 (not taken).
+// 33 to 48 floats, from 1 M entries, without tiles: 4 lanes of three, eight rows a warp, as long as the L2 holds the operand, or three
+// eighths of it where rows straddle sectors.  200 k / 10 M F = 48 223 -> 184, F = 44 (35 MB) 232 -> 214, 300 k / 15 M 300 -> 279, 150 k / 2.6 M 74 -> 66,
+// 600 k / 21 M (115 MB) 394 -> 393.  Not taken: F = 44 300 k / 15 M (53 MB) 320 -> 324; 1.5 M / 62 M (288 MB) 1,125 -> 1,190; 40 k / 840 k 31 -> 41;
+// with tiles 306 k / 16 M 303 -> 310.
+constexpr int64_t kL2Bytes = (int64_t)126 << 20;
 template <int VEC, bool PADDED>
-int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, cudaStream_t stream)
+int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, int32_t k, bool octets, cudaStream_t stream)
 {
     const bool large = nnz >= (int64_t)4 << 20, small = nnz < (int64_t)1 << 20;
     const int end = a.vec_end, wide = end % 64 > 48 ? end : end / 64 * 64;
     int rc = DG_OK;
     if (wide > 0) {
         a.vec_end = wide;
-        rc = large ? launch<VEC, 16, 4, 2, 4, PADDED>(a, whole, stream) : launch<VEC, 32, 2, 4, 4, PADDED>(a, whole, stream);
+        if constexpr (VEC == 4 && !PADDED) {
+            if (large && octets) {
+                SpmmArgs o = a;
+                o.vec_end = wide / 2;
+                rc = launch<8, 16, 2, 2, 3, PADDED>(o, whole, stream);
+                a.vec_first = wide;
+            }
+        }
+        if (a.vec_first == 0) rc = large ? launch<VEC, 16, 4, 2, 4, PADDED>(a, whole, stream) : launch<VEC, 32, 2, VEC == 4 ? 3 : 4, 4, PADDED>(a, whole, stream);
         a.vec_first = wide;
     }
     while (rc == DG_OK && a.vec_first < end) {
         a.vec_end = std::min(end, a.vec_first + 32);
         const int nvec = a.vec_end - a.vec_first;
-        if (nvec <= 4) rc = launch<VEC, 4, 1, 4, 5, PADDED>(a, whole, stream);
+        bool thirds = false;
+        if constexpr (VEC == 4) {
+            if (nvec > 8 && nvec <= 12 && !small && !whole && k * a.ldb * 4 <= (a.ldb % 8 ? kL2Bytes * 3 / 8 : kL2Bytes)) {
+                rc = launch<VEC, 4, 3, 4, 4, PADDED>(a, whole, stream);
+                thirds = true;
+            } else if (nvec > 16 && nvec <= 24 && large) {
+                rc = launch<VEC, 8, 3, 4, 3, PADDED>(a, whole, stream);
+                thirds = true;
+            }
+        }
+        if (thirds) {}
+        else if (nvec <= 4) rc = launch<VEC, 4, 1, 4, 5, PADDED>(a, whole, stream);
         else if (nvec <= 8) rc = launch<VEC, 8, 1, 8, 4, PADDED>(a, whole, stream);
         else if (nvec <= 16) rc = large ? launch<VEC, 8, 2, 8, 3, PADDED>(a, whole, stream) : launch<VEC, 16, 1, 4, 5, PADDED>(a, whole, stream);
         else rc = small ? launch<VEC, 32, 1, 4, 5, PADDED>(a, whole, stream) : launch<VEC, 16, 2, 4, 4, PADDED>(a, whole, stream);
@@ -530,11 +575,11 @@ int dg_spmm_launch_rows(const dg_plan* plan, const float* val, const float* B, i
         whole.parts = nullptr;
     }
     const SpmmArgs* w = tiles ? &whole : nullptr;
-    if (padded) return launch_vec<4, true>(a, w, plan->nnz, stream);
+    if (padded) return launch_vec<4, true>(a, w, plan->nnz, plan->k, false, stream);
     switch (vec) {
-        case 4: return launch_vec<4, false>(a, w, plan->nnz, stream);
-        case 2: return launch_vec<2, false>(a, w, plan->nnz, stream);
-        default: return launch_vec<1, false>(a, w, plan->nnz, stream);
+        case 4: return launch_vec<4, false>(a, w, plan->nnz, plan->k, F % 8 == 0 && ldb % 8 == 0 && aligned(B, 32), stream);
+        case 2: return launch_vec<2, false>(a, w, plan->nnz, plan->k, false, stream);
+        default: return launch_vec<1, false>(a, w, plan->nnz, plan->k, false, stream);
     }
 }
 

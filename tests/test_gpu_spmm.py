@@ -886,3 +886,56 @@ def test_entries_that_come_twice_are_both_multiplied(where):
         assert plan.tiled_entries() == 0
         got = plan.spmm(dev(B), torch.empty(3001, 64, device='cuda'), 1.0, 0.0).cpu().numpy()
         assert_close(got, ref_gcn.spmm_coo(block, B, np.zeros((3001, 64), np.float32), 1.0, 0.0), TOL, 'not coalesced')
+
+
+def lengths_block(lengths, k, seed):
+    """Rows of the given lengths with random columns, on the device: row ids, column ids, values."""
+    g = torch.Generator(device='cuda').manual_seed(seed)
+    lengths = torch.as_tensor(lengths, device='cuda')
+    row = torch.repeat_interleave(torch.arange(lengths.numel(), device='cuda'), lengths).to(torch.int32)
+    col = torch.randint(0, k, (row.numel(),), device='cuda', generator=g, dtype=torch.int32)
+    return row, col, torch.randn(row.numel(), device='cuda', generator=g)
+
+
+@pytest.mark.parametrize('nnz', [200_000, 1_100_000, 4_300_000])
+def test_forms_by_size_and_width(nnz):
+    """Every form a width and size of a matrix choose: widths around 8 / 12 / 16 / 24 / 32 vectors and whole tiles, rows of 32-byte pieces
+    read as such and the same operand one vector off them, odd widths through the padded copy, an operand beyond the L2, products
+    added to C and the fused epilogue; rows with no entry, around the sets of 4 to 32 entries, and split ones.  Against float64, within 64
+    roundings of a sum of the magnitudes."""
+    import spmm_cpp
+    edges = torch.tensor([0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 30, 31, 32, 33, 34, 35, 63, 64, 65, 66, 67, 127, 128, 129, 130, 300, 1025])
+    k = 40_000
+    lengths = edges.repeat(nnz // int(edges.sum()) + 1)
+    row, col, val = lengths_block(lengths, k, nnz)
+    m = lengths.numel()
+    plan = spmm_cpp.SpmmPlan(row, col, val, m, k)
+    sparse = torch.sparse_coo_tensor(torch.stack((row, col)).long(), val.double(), (m, k)).to_sparse_csr()
+    magnitudes = torch.sparse_csr_tensor(sparse.crow_indices(), sparse.col_indices(), sparse.values().abs(), (m, k))
+    g = torch.Generator(device='cuda').manual_seed(7)
+    for F in (33, 36, 41, 44, 48, 49, 52, 65, 68, 93, 96, 97, 100, 200, 256, 264, 320):
+        b = torch.randn(k, F, device='cuda', generator=g)
+        c0 = torch.randn(m, F, device='cuda', generator=g)
+        scale, bias = torch.rand(m, device='cuda', generator=g) + 0.5, torch.randn(F, device='cuda', generator=g)
+        want, bound = torch.sparse.mm(sparse, b.double()), torch.sparse.mm(magnitudes, b.double().abs()) + c0.abs()
+        close = lambda got, exact: bool(((got.double() - exact).abs() <= 64 * 2.0 ** -24 * (bound + 1) * 2).all())
+        out = plan.spmm(b, torch.empty_like(c0), 1.0, 0.0)
+        assert close(out, want), (nnz, F)
+        assert close(plan.spmm(b, c0.clone(), 1.0, 1.0), want + c0), (nnz, F)
+        assert close(plan.spmm(b, c0.clone(), 0.5, -1.0, row_scale=scale, bias=bias, relu=True), ((0.5 * want - c0) * scale[:, None] + bias).clamp(min=0)), (nnz, F)
+        if F % 8 == 0:
+            apart = torch.empty(k, F + 4, device='cuda')[:, 4:]            # rows 16 bytes off a 32-byte piece
+            apart.copy_(b)
+            assert torch.equal(plan.spmm(apart, torch.empty_like(c0), 1.0, 0.0), out), (nnz, F)
+
+
+def test_infinite_values_beside_short_batches():
+    """Three gathers at a time do not divide a set of 32 entries: what the last step reads beyond it must not touch the row."""
+    import spmm_cpp
+    lengths = [31, 32, 33, 64] * 3
+    row, col, val = lengths_block(lengths, 500, 3)
+    first = torch.cat((torch.zeros(1, dtype=torch.long), torch.tensor(lengths).cumsum(0)[:-1])).cuda()
+    val[first[4:8]] = float('inf')
+    b = torch.rand(500, 256, device='cuda') + 0.5
+    out = spmm_cpp.SpmmPlan(row, col, val, len(lengths), 500).spmm(b, torch.empty(len(lengths), 256, device='cuda'), 1.0, 0.0)
+    assert bool(torch.isinf(out[4:8]).all()) and bool(torch.isfinite(out[:4]).all()) and bool(torch.isfinite(out[8:]).all())

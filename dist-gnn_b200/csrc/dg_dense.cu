@@ -1074,19 +1074,35 @@ k_dense_tn_pair(const __grid_constant__ CUtensorMap tmP, const __grid_constant__
     dense_tn<true>(tmP, tmQ, a);
 }
 
-// One thread per slot of the partial layout (coalesced over the ranges' partials); slots of the padding are skipped.
-__global__ void k_dense_tn_reduce(const float* __restrict__ partial, int ranges, int64_t slots, float* __restrict__ D, int64_t ldd,
-                                  int32_t p_cols, int32_t q_cols, int32_t p_store, int32_t q_store, int transposed)
+// Adds the ranges' partials slot by slot, in order; slots of the padding are skipped.  A CTA takes 128 slots, eight warps fetch 40 ranges'
+// at a time, 512 bytes each, and four add them (one thread a slot, loads and adds of its own, took 7.6 to 17 us: now 4.5 to 5.7, 256 x 256 7.1 to 8.6).
+__global__ void __launch_bounds__(256) k_dense_tn_reduce(const float* __restrict__ partial, int ranges, int32_t slots, float* __restrict__ D, int64_t ldd,
+                                                         int32_t p_cols, int32_t q_cols, int32_t p_store, int32_t q_store, int transposed)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= slots) return;
-    const int half_slots = p_store * q_store;
-    const int half = (int)(i / half_slots), in_half = (int)(i % half_slots), c4 = in_half / (4 * p_store), rest = in_half % (4 * p_store);
+    constexpr int kEach = 5, kChunk = 8 * kEach;
+    __shared__ float4 part[2][kChunk][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float4* from = reinterpret_cast<const float4*>(partial) + blockIdx.x * 32 + lane;      // slots are a multiple of 256
+    float sum = 0.f;
+    for (int r0 = 0, b = 0; r0 < ranges; r0 += kChunk, b ^= 1) {
+        const int n = min(kChunk, ranges - r0);
+        float4 x[kEach];
+#pragma unroll
+        for (int j = 0; j < kEach; ++j)
+            if (warp + 8 * j < n) x[j] = __ldcg(from + (int64_t)(r0 + warp + 8 * j) * (slots / 4));
+#pragma unroll
+        for (int j = 0; j < kEach; ++j)
+            if (warp + 8 * j < n) part[b][warp + 8 * j][lane] = x[j];
+        __syncthreads();                                          // whoever fills this buffer next has passed the next one of these
+        if (threadIdx.x < 128)
+#pragma unroll 8
+            for (int r = 0; r < n; ++r) sum += reinterpret_cast<const float*>(part[b][r])[threadIdx.x];
+    }
+    if (threadIdx.x >= 128) return;
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    const int half_slots = p_store * q_store, half = i / half_slots, in_half = i % half_slots, c4 = in_half / (4 * p_store), rest = in_half % (4 * p_store);
     const int p = half * 128 + rest / 4, q = c4 * 4 + rest % 4;
     if (p >= p_cols || q >= q_cols) return;
-    float sum = 0.f;
-#pragma unroll 32                                                 // in flight at a time: what there is to do is wait for the L2
-    for (int r = 0; r < ranges; ++r) sum += partial[(int64_t)r * slots + i];
     D[transposed ? (int64_t)q * ldd + p : (int64_t)p * ldd + q] = sum;
 }
 
@@ -1157,6 +1173,6 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
     static std::atomic<bool> granted[64], granted_pair[64];
     if ((rc = pair ? allow_smem((const void*)k_dense_tn_pair, granted_pair) : allow_smem((const void*)k_dense_tn, granted))) return rc;
     (pair ? k_dense_tn_pair : k_dense_tn)<<<pair ? (a.ranges + 1) / 2 * 2 : a.ranges, kTnThreads, smem, (cudaStream_t)stream>>>(tmP, tmQ, a);
-    k_dense_tn_reduce<<<(unsigned)((slots + 255) / 256), 256, 0, (cudaStream_t)stream>>>(scratch, a.ranges, slots, D, ldd, a.p_cols, a.q_cols, a.p_store, a.q_store, swapped);
+    k_dense_tn_reduce<<<(unsigned)(slots / 128), 256, 0, (cudaStream_t)stream>>>(scratch, a.ranges, (int32_t)slots, D, ldd, a.p_cols, a.q_cols, a.p_store, a.q_store, swapped);
     return (int)cudaGetLastError();
 }

@@ -32,9 +32,9 @@ import torch  # noqa: E402
 METRIC, UNIT = 'gcn_epoch_ms', 'ms'
 # DRAM traffic of the local products (dram__bytes_read + dram__bytes_write, ncu, one pass, --clock-control none):
 #   the N = 1 default workload itself, one epoch of `bench.py --steps 1 --warmup 3 --no-cpu-baseline --profiler-range`:
-#   161.7 GB for 147.87 G (stored entry x float) = 1.094 B each; no capture of these kernels on the blocks of several ranks.
-MEASURED_TRAFFIC = {('sparse2m', 1, 3): 161.7e9}      # (config, ranks, layers) -> bytes per step, captured on that very workload
-TRAFFIC_PER_ENTRY_FLOAT = 1.094
+#   160.1 GB for 147.87 G (stored entry x float) = 1.083 B each; no capture of these kernels on the blocks of several ranks.
+MEASURED_TRAFFIC = {('sparse2m', 1, 3): 160.1e9}      # (config, ranks, layers) -> bytes per step, captured on that very workload
+TRAFFIC_PER_ENTRY_FLOAT = 1.083
 CONFIG3_DEADLINE_S = 150      # the extra 1.5D measurement of an 8-GPU default run gives up after this long (it takes about 20 s)
 
 

@@ -279,7 +279,7 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 // Barriers: full (own CTA, TMA), ready (even CTA: the split warps of both), empty and acc_full (both CTAs, by commit), acc_empty (even CTA:
 // the epilogue warps of both).
 //
-// What bounds it: at 256 x 256 the MMAs (tensor pipe 73 %; a single CTA's shared memory was busy with fetching both operands' 12 KB for
+// What bounds it: at 256 x 256 the MMAs (tensor pipe 60 % with the mask, DRAM 53 %; a single CTA's shared memory was busy with fetching both operands' 12 KB for
 // every MMA and refilling Bt's 512 KB for every 128 rows, which a pair halves), below some 100 columns of A DRAM and the epilogue.
 // 2,449,029 rows (us, one CTA per SM with four epilogue warps -> pair): 256 -> 256 1,600 -> 1,535, with the mask 1,930 -> 1,720;
 // 100 -> 256 1,100 -> 895; 47 -> 256 with the mask 1,600 -> 1,110; 602 -> 256 4,280 -> 3,540; 256 -> 128 1,540 -> 1,065 (one tile per

@@ -443,10 +443,11 @@ int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
 // 150 k / 2.6 M F = 256 204 -> 197, F = 200 197 -> 190).
 // 65 to 96 floats, from 4 M entries: 8 lanes of three vectors, of which at most 7 idle (16 x 2: up to 15).  1 M / 17 M F = 96 676 -> 618, 600 k /
 // 21 M 676 -> 622, 2.4 M / 126 M 4,190 -> 3,920, 300 k / 15 M 471 -> 447, 2.4 M / 42 M 1,758 -> 1,798 (F = 72 1,700 -> 1,680); 150 k / 2.6 M 111 -> 119 (not taken).
-// 33 to 48 floats, from 1 M entries, without tiles: 4 lanes of three, eight rows a warp, as long as the L2 holds the operand, or three
-// eighths of it where rows straddle sectors.  200 k / 10 M F = 48 223 -> 184, F = 44 (35 MB) 232 -> 214, 300 k / 15 M 300 -> 279, 150 k / 2.6 M 74 -> 66,
-// 600 k / 21 M (115 MB) 394 -> 393.  Not taken: F = 44 300 k / 15 M (53 MB) 320 -> 324; 1.5 M / 62 M (288 MB) 1,125 -> 1,190; 40 k / 840 k 31 -> 41;
-// with tiles 306 k / 16 M 303 -> 310.
+// 33 to 48 floats, from 4 M entries, or from 1 M with 64 k rows or more where the operand is read as it is, without tiles: 4 lanes of
+// three, eight rows a warp, as long as the L2 holds the operand, or three eighths of it where rows straddle sectors.  F = 48: 200 k rows / 10 M
+// 223 -> 184, 250 k / 8 M 199 -> 170, 30 k / 8 M 161 -> 149, 250 k / 1.4 M 78 -> 70, 80 k / 1.2 M 53 -> 52, 600 k / 21 M (115 MB) 394 -> 393;
+// padded from 41: 200 k / 10 M 232 -> 214, 30 k / 8 M 168 -> 165.  Not taken: 30 k / 3 M 70 -> 72, 30 k / 1.1 M 35 -> 46 (too few rows for so many
+// groups); padded 80 k / 1.2 M 62 -> 66; F = 44 300 k / 15 M (53 MB) 320 -> 324; 1.5 M / 62 M (288 MB) 1,125 -> 1,190; with tiles 306 k / 16 M 303 -> 310.
 constexpr int64_t kL2Bytes = (int64_t)126 << 20;
 template <int VEC, bool PADDED>
 int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, int32_t k, bool octets, cudaStream_t stream)
@@ -472,7 +473,8 @@ int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, int32_t k, bool o
         const int nvec = a.vec_end - a.vec_first;
         bool thirds = false;
         if constexpr (VEC == 4) {
-            if (nvec > 8 && nvec <= 12 && !small && !whole && k * a.ldb * 4 <= (a.ldb % 8 ? kL2Bytes * 3 / 8 : kL2Bytes)) {
+            const bool many = large || (!small && !PADDED && a.m >= 1 << 16);
+            if (nvec > 8 && nvec <= 12 && many && !whole && k * a.ldb * 4 <= (a.ldb % 8 ? kL2Bytes * 3 / 8 : kL2Bytes)) {
                 rc = launch<VEC, 4, 3, 4, 4, PADDED>(a, whole, stream);
                 thirds = true;
             } else if (nvec > 16 && nvec <= 24 && large) {

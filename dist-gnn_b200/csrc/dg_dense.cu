@@ -1145,7 +1145,12 @@ extern "C" int dg_dense_tn(const float* X, int64_t ldx, const float* G, int64_t 
             }
         return DG_OK;
     }
+    if (max_ctas == 1 && Km > 128 && Nn > 128) {      // no CTA to pair with: both halves of X, one after the other (the same sums in the same order)
+        const int rc = dg_dense_tn(X, ldx, G, ldg, D, ldd, n, 128, Nn, scratch, scratch_floats, 1, stream);
+        return rc ? rc : dg_dense_tn(X + 128, ldx, G, ldg, D + (int64_t)128 * ldd, ldd, n, Km - 128, Nn, scratch, scratch_floats, 1, stream);
+    }
     const bool pair = std::min(Km, Nn) > 128, swapped = !pair && Nn < Km;
+    if (pair) max_ctas &= ~1;                                     // whole pairs, and no more CTAs than allowed
     DenseTnArgs a{};
     a.n = n;
     a.p_cols = swapped ? Nn : Km;

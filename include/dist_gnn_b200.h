@@ -309,9 +309,9 @@ int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_head, const 
                        int64_t ldc, int64_t M, int32_t N, int32_t K, int32_t relu, const float* mask, int64_t ldm,
                        void* stream);
 /* Weight-gradient product D[Km x Nn] = X[n x Km]^T * G[n x Nn] (torch.mm at models/gcn.py:50), same arithmetic (three
- * TF32 passes, fp32 accumulator in tensor memory) with BOTH operands split inside the kernel.  The n rows are cut
- * into at most max_ctas ranges, one for every CTA (two for a pair of CTAs, which share operands wider than 128 columns each).  The tensor cores truncate when they add into their accumulator, an error that grows
- * with the number of rows, so every 256 rows the
+ * TF32 passes, fp32 accumulator in tensor memory) with BOTH operands split inside the kernel.  At most max_ctas CTAs run, and the
+ * n rows are cut into no more ranges than that: one for every CTA, or two for a pair of CTAs, which shares operands wider than 128
+ * columns each.  The tensor cores truncate when they add into their accumulator, an error that grows with the number of rows, so every 256 rows the
  * accumulators are added, rounded to nearest, into the range's partial result in `scratch` and restarted; a second kernel adds the
  * partials in order of the ranges, so the result is bit-reproducible and within about 6e-6 of the exact product for any n.
  * `scratch` is 16-byte aligned and holds ranges * roundup(min(Km, 256), 128) * roundup(min(Nn, 256), 16) floats

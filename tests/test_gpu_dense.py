@@ -218,3 +218,26 @@ def test_dense_tn_roles_and_ranges(n, Km, Nn, ctas):
                                               ctas, spmm_cpp._stream()))
     assert_close(d[:, :Nn].cpu().numpy(), (x[:, :Km].double().t() @ y[:, :Nn].double()).cpu().numpy(), TOL, f'{n}x{Km}x{Nn} on {ctas}')
     assert bool((d[:, Nn:] == -1).all()) and bool((scratch[need:] == 3.5).all()) and spmm_cpp.dense_status() == 0
+
+
+@pytest.mark.parametrize('ctas,floats', [(1, 128 * 256), (3, 2 * 256 * 256), (5, 4 * 256 * 256)])
+def test_dense_tn_runs_no_more_ctas_than_it_may(ctas, floats):
+    """Operands that CTA pairs would share, with an odd number of CTAs allowed: the partial results of whole pairs (of one CTA's half of X
+    at a time) have to do, so that no further CTA can have written any; the same bits as two halves multiplied one by one."""
+    import spmm_cpp
+    n, Km, Nn = 5000, 256, 256
+    g = torch.Generator(device='cuda').manual_seed(ctas)
+    x, y = torch.randn(n, Km, device='cuda', generator=g), torch.randn(n, Nn, device='cuda', generator=g)
+    scratch = torch.full((floats + 1024,), 3.5, device='cuda')
+
+    def product(a, allowed, room):
+        d = torch.empty(a.size(1), Nn, device='cuda')
+        spmm_cpp.check(spmm_cpp.lib().dg_dense_tn(a.data_ptr(), a.stride(0), y.data_ptr(), Nn, d.data_ptr(), Nn, n, a.size(1), Nn, scratch.data_ptr(), room, allowed,
+                                                  spmm_cpp._stream()))
+        return d
+
+    d = product(x, ctas, floats)
+    assert_close(d.cpu().numpy(), (x.double().t() @ y.double()).cpu().numpy(), TOL, f'{ctas} CTAs')
+    ranges = max(1, ctas & ~1)
+    assert torch.equal(d, torch.cat([product(x[:, h:h + 128], ranges, ranges * 128 * 256) for h in (0, 128)]))
+    assert bool((scratch[floats:] == 3.5).all()) and spmm_cpp.dense_status() == 0

@@ -145,6 +145,19 @@ Tensor padded_copy(const Tensor& t)
     return wide;
 }
 
+// ---- partial results of weight gradients ------------------------------------------------------------------------------------
+// A product's own, from torch's allocator: products on two streams may run at the same time, and the memory serves the next one on its stream.
+int tn_ctas(const Tensor& x) { return at::cuda::getDeviceProperties(x.get_device())->multiProcessorCount; }
+int64_t tn_floats(int64_t Km, int64_t Nn, int ctas)
+{
+    return ctas * ((std::min<int64_t>(Km, 256) + 127) / 128 * 128) * ((std::min<int64_t>(Nn, 256) + 15) / 16 * 16);
+}
+std::pair<Tensor, int> tn_scratch(const Tensor& x, int64_t Km, int64_t Nn)
+{
+    const int ctas = tn_ctas(x);
+    return {at::empty({tn_floats(Km, Nn, ctas)}, x.options()), ctas};
+}
+
 // ---- the whole GCN on one rank ----------------------------------------------------------------------------------------------
 struct Net {                              // shapes and buffers of one call
     std::vector<int32_t> dims;
@@ -173,11 +186,10 @@ struct GcnNode : public torch::autograd::Node {
     std::shared_ptr<PlanRef> plan;
     SavedVariable features;               // only to notice that they were changed in place
     std::vector<SavedVariable> weights;
-    Tensor x, hidden, splits, tn_scratch;
+    Tensor x, hidden, splits;
     std::vector<int32_t> dims;
     std::vector<int64_t> act_start, bwd_split;
     int64_t timer = 0;
-    int ctas = 0;
 
     std::string name() const override { return "OneRankGcnBackward"; }
     void release_variables() override
@@ -226,8 +238,13 @@ struct GcnNode : public torch::autograd::Node {
         call.net.ld_grad = n > 1 ? g.stride(0) : width;
         call.net.dw = dw.data();
         call.net.bwd_split = split.data();
-        call.net.tn_scratch = tn_scratch.data_ptr<float>();
-        call.net.tn_scratch_floats = tn_scratch.numel();
+        const int ctas = tn_ctas(x);
+        int64_t partials = 0;
+        for (int l = 0; l < L; ++l)
+            if (dw[l]) partials = std::max(partials, tn_floats(dims[l], dims[l + 1], ctas));
+        Tensor partial = at::empty({std::max<int64_t>(partials, 1)}, x.options());
+        call.net.tn_scratch = partial.data_ptr<float>();
+        call.net.tn_scratch_floats = partial.numel();
         call.net.max_ctas = ctas;
         check(dg_gcn_backward(&call.net, stream_of(x)));
         g_launches += launches;
@@ -236,8 +253,7 @@ struct GcnNode : public torch::autograd::Node {
     }
 };
 
-Tensor gcn(const std::shared_ptr<PlanRef>& plan, const Tensor& features, const Tensor& x, const std::vector<Tensor>& weights, const Tensor& tn_scratch,
-           int64_t ctas, int64_t timer)
+Tensor gcn(const std::shared_ptr<PlanRef>& plan, const Tensor& features, const Tensor& x, const std::vector<Tensor>& weights, int64_t timer)
 {
     const int L = (int)weights.size();
     const int64_t n = x.size(0);
@@ -309,12 +325,10 @@ Tensor gcn(const std::shared_ptr<PlanRef>& plan, const Tensor& features, const T
         node->x = x.detach();
         node->hidden = hidden;
         node->splits = splits;
-        node->tn_scratch = tn_scratch;
         node->dims = dims;
         node->act_start = act_start;
         node->bwd_split = bwd_split;
         node->timer = timer;
-        node->ctas = (int)ctas;
         torch::autograd::set_history(out, node);
     }
     return out;
@@ -385,6 +399,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
     m.def("spmm", &spmm);
     m.def("gcn", &gcn);
     m.def("readable_padded", &readable_padded);
+    m.def("tn_scratch", &tn_scratch);
     m.def("row_cross_entropy", &row_cross_entropy);
     m.def("pending_regions", &pending_regions);
     m.def("resolve_regions", &resolve_regions);

@@ -522,9 +522,8 @@ class GCN(nn.Module):
         same order on the same operands, the same bits, without the host's work between them."""
         env = DistEnv.env
         plan.value_ptr()                                    # values changed in place: their tiles go first
-        scratch, ctas = spmm_cpp.tn_scratch(features.device.index)
         timer = env.timer
-        out = spmm_cpp.binding().gcn(plan.ref, features, _product_operand(env, features, True), weights, scratch, ctas, timer.ident)
+        out = spmm_cpp.binding().gcn(plan.ref, features, _product_operand(env, features, True), weights, timer.ident)
         timer.bound_regions()
         return out
 

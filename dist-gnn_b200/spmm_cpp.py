@@ -786,21 +786,10 @@ def dense_nt(a, b, transposed=False, relu=False, mask=None, cache_key=None):
     return c
 
 
-_tn_scratch = {}
-
-
-def tn_scratch(index):
-    """(partial-result area of dense_tn on CUDA device `index`, number of CTAs it serves)."""
-    hit = _tn_scratch.get(index)
-    if hit is None:
-        ctas = torch.cuda.get_device_properties(index).multi_processor_count
-        hit = _tn_scratch[index] = (torch.empty(ctas * 256 * 256, dtype=torch.float32, device=torch.device('cuda', index)), ctas)
-    return hit
-
-
 def dense_tn(x, g):
     """x[n x Km]^T @ g[n x Nn] on the tensor cores with fp32 accuracy (dg_dense_tn), or None when the shapes or strides
-    are outside what the kernel takes.  Both operands are streamed once; per-CTA partial results are added in CTA order."""
+    are outside what the kernel takes.  Both operands are streamed once; the partial results of the ranges of rows are added in
+    their order."""
     ldx, ldg = _row_major(x, 'x'), _row_major(g, 'g')
     lib()
     n, Km = x.shape
@@ -810,9 +799,9 @@ def dense_tn(x, g):
     if not lib().dg_dense_tn_supported(n, Km, Nn, ldx, ldg, x.data_ptr(), g.data_ptr()):
         return None
     index = x.device.index
-    scratch, ctas = tn_scratch(index)
+    scratch, ctas = binding().tn_scratch(x, Km, Nn)
     global dense_launches
-    dense_launches += 2 * ((Km + 255) // 256) * ((Nn + 255) // 256)      # per 256 x 256 panel: the product and the reduction over the CTAs' partials
+    dense_launches += 2 * ((Km + 255) // 256) * ((Nn + 255) // 256)      # per 256 x 256 panel: the product and the reduction over the ranges' partials
     d = torch.empty((Km, Nn), dtype=torch.float32, device=x.device)
     with _on(index):
         check(_lib.dg_dense_tn(x.data_ptr(), ldx, g.data_ptr(), ldg, d.data_ptr(), Nn, n, Km, Nn, scratch.data_ptr(), scratch.numel(),

@@ -241,3 +241,25 @@ def test_dense_tn_runs_no_more_ctas_than_it_may(ctas, floats):
     ranges = max(1, ctas & ~1)
     assert torch.equal(d, torch.cat([product(x[:, h:h + 128], ranges, ranges * 128 * 256) for h in (0, 128)]))
     assert bool((scratch[floats:] == 3.5).all()) and spmm_cpp.dense_status() == 0
+
+
+@pytest.mark.parametrize('n,Km,Nn', [(1500, 256, 256), (2300, 100, 47)])
+def test_dense_tn_on_two_streams_at_once(n, Km, Nn):
+    """Weight gradients that are under way at the same time on two streams, with SMs left for each other, are what each is alone: their
+    partial results share no memory."""
+    import spmm_cpp
+    g = torch.Generator(device='cuda').manual_seed(n)
+    pairs = [(torch.randn(n, Km + (-Km) % 4, device='cuda', generator=g)[:, :Km], torch.randn(n, Nn + (-Nn) % 4, device='cuda', generator=g)[:, :Nn]) for _ in range(2)]
+    alone = [spmm_cpp.dense_tn(x, y) for x, y in pairs]
+    for (x, y), d in zip(pairs, alone):
+        assert_close(d.cpu().numpy(), (x.double().t() @ y.double()).cpu().numpy(), TOL, f'{n}x{Km}x{Nn}')
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], [[], []]
+    for _ in range(40):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(spmm_cpp.dense_tn(*pairs[i]))
+    torch.cuda.synchronize()
+    for d, same in zip(alone, got):
+        assert all(torch.equal(d, e) for e in same)
+    assert spmm_cpp.dense_status() == 0

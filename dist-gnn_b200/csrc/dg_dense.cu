@@ -15,7 +15,7 @@
 // optional ReLU / ReLU-backward mask; one thread of warp 1 issues the tcgen05.mma instructions (kind::tf32, 128 x N x 8,
 // operands described by shared-memory matrix descriptors, accumulator in TMEM columns) and commits them to the mbarriers
 // that recycle the stages.  k_dense_nt_pair: a CTA pair on every TPC walks over tiles of 256 rows with two accumulators and separate
-// epilogue warps (used for results wider than 64 columns).  k_dense_tn (further down): the weight gradient X^T * G,
+// epilogue warps (wider results; by_pairs).  k_dense_tn (further down): the weight gradient X^T * G,
 // both operands MN-major, split-K over the CTAs with periodic accumulator flushes.
 // Every mbarrier wait is bounded; a role that gives up sets the status word and the CTA still frees its TMEM.
 #include <cuda.h>
@@ -289,8 +289,6 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 // CTA -> pair, tails behind -> together: 150,001 rows 256 -> 160 77 -> 83 -> 68, 256 -> 192 84 -> 87 -> 75, 256 -> 256 99 -> 95 -> 87; 3,000 rows
 // 256 -> 160 13.4 -> 14.7 -> 12.3.  2,449,029 rows (in turn, 20 ms between launches) 256 -> 256 1,448 -> 1,343, with the mask 1,603 -> 1,470,
 // 602 -> 256 3,346 -> 3,145, 256 -> 128 988 -> 912.  Error against float64: 256 -> 256 2.30e-6 -> 2.15e-6, 64 -> 192 9.0e-7 -> 7.9e-7.
-// Up to 64 columns k_dense_nt stays: two of its CTAs fit an SM, and an MMA takes some 130 clocks however few columns it has (256 -> 47
-// 860 us against 895; 10,000 rows 12.3 against 14.2).
 constexpr int PK = 16, kMaxPairStages = 10, kSplitWarps = 4, kEpilogueWarps = 8;
 constexpr int kThreadsPair = 32 * (2 + kSplitWarps + kEpilogueWarps);
 constexpr int kPieceBytes = 32 * 32 * 4;                          // staging of an epilogue warp: 32 rows x 32 columns
@@ -624,6 +622,23 @@ int make_map(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int
     return r == CUDA_SUCCESS ? DG_OK : DG_ERR_UNSUPPORTED;
 }
 
+// Which of the two kernels multiplies; an element is the same sum in the same order in both.  n_pad: columns rounded up to 16.
+// One tile per CTA wins while its CTAs are all resident at once and there is no next tile to overlap with: up to 80 columns two of them
+// fit an SM, above one.  A pair costs it some 0.5 us of cluster barriers and remote arrivals, an MMA takes 130 clocks however few columns it
+// has, and half slabs spare it the padding of a depth such as 100 or 16.  us, one tile per CTA against pair:
+//   10,000 rows: 64 -> 96 6.1 and 6.8, 256 -> 80 11.6 and 12.2; 100 -> 128 9.0 and 8.5 (pair), 384 -> 128 16.1 and 15.4 (pair)
+//   25,000 rows: 64 -> 80 8.1 and 9.6, 256 -> 72 15.0 and 19.1; 64 -> 96 10.8 and 8.7 (pair: a second wave)
+// With more rows than that the pair's overlap pays, up to 80 columns only where two CTAs an SM do not overlap as well themselves: 150,001
+// rows 100 -> 72 39.1 and 31.9 (pair), 64 -> 80 with the mask 45.7 and 48.6, 602 -> 72 114 and 129, 256 -> 80 with the mask 71.9 and 64.9 (pair).
+bool by_pairs(int64_t M, int n_pad, int K, bool masked, int sms)
+{
+    if (n_pad <= 64) return false;
+    const int64_t tiles = (M + BM - 1) / BM;
+    const bool half_slab = (K - 1) % BK < BK / 2;
+    if (tiles <= sms) return n_pad > 128 || half_slab || (K > 192 && n_pad > 96);
+    return n_pad > 80 || (tiles > 2 * sms && (masked ? K > 64 : K <= 192));
+}
+
 }  // namespace
 
 extern "C" int dg_dense_split(const float* src, float* head, float* tail, int64_t count, void* stream)
@@ -694,7 +709,9 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
     a.mask = mask; a.ldm = ldm;
     a.status = dg_status_word();
     if (!a.status) return DG_ERR_STATE;
-    const bool pair = a.n_pad > 64;
+    const int sms = sm_count();
+    if (sms <= 0) return DG_ERR_STATE;
+    const bool pair = by_pairs(M, a.n_pad, K, mask != nullptr, sms);
     CUtensorMap tmA, tmBh, tmBt;
     int rc;
     if (!pair) {
@@ -711,8 +728,6 @@ extern "C" int dg_dense_nt_masked(const float* A, int64_t lda, const float* Bt_h
     if ((rc = make_map(&tmA, A, M, K, lda, BM, PK)) || (rc = make_map(&tmBh, Bt_head, N, K, ldb, a.n_pad / 2, PK)) ||
         (rc = make_map(&tmBt, Bt_tail, N, K, ldb, a.n_pad / 2, PK)))
         return rc;
-    const int sms = sm_count();
-    if (sms <= 0) return DG_ERR_STATE;
     const size_t stage = (size_t)PK * 4 * (2 * BM + a.n_pad), rest = kEpilogueWarps * kPieceBytes + kPairBarBytes + 1024;
     const int stages = (int)std::min<size_t>(kMaxPairStages, (227 * 1024 - rest) / stage);
     static std::atomic<bool> granted[64];

@@ -199,6 +199,25 @@ def test_dense_nt_by_cta_pairs(M, N, K):
     assert spmm_cpp.dense_status() == 0
 
 
+@pytest.mark.parametrize('K', [16, 64, 100, 192, 196, 256, 604])
+@pytest.mark.parametrize('N', [64, 65, 80, 81, 96, 128, 129])
+def test_dense_nt_rows_do_not_depend_on_the_kernel(N, K):
+    """One tile per CTA or CTA pairs, by rows, columns, depth and mask: on either side of every limit a row is the same bits."""
+    import spmm_cpp
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    counts = [128 * sms, 128 * sms + 1, 256 * sms, 256 * sms + 1]
+    g = torch.Generator(device='cuda').manual_seed(1000 * N + K)
+    a = torch.randn(counts[-1], K, device='cuda', generator=g)
+    bt = torch.randn(N, K, device='cuda', generator=g)
+    act = torch.randn(counts[-1], N, device='cuda', generator=g)
+    plain, masked = spmm_cpp.dense_nt(a, bt), spmm_cpp.dense_nt(a, bt, mask=act)
+    assert_close(plain.cpu().numpy(), (a.double() @ bt.double().t()).cpu().numpy(), TOL, f'{N}x{K}')
+    assert torch.equal(masked, plain * (act > 0))
+    for M in counts[:-1]:
+        assert torch.equal(spmm_cpp.dense_nt(a[:M], bt), plain[:M]) and torch.equal(spmm_cpp.dense_nt(a[:M], bt, mask=act[:M]), masked[:M])
+    assert spmm_cpp.dense_status() == 0
+
+
 @pytest.mark.parametrize('n', [1, 15, 17, 257, 4096 + 5, 148 * 256 + 1])
 @pytest.mark.parametrize('Km,Nn', [(129, 130), (256, 193), (256, 128), (128, 256), (10, 200), (200, 5), (1, 40), (96, 96)])
 @pytest.mark.parametrize('ctas', [1, 5, 148])

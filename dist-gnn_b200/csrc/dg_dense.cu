@@ -629,7 +629,7 @@ int make_map(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int
 //   10,000 rows: 64 -> 96 6.1 and 6.8, 256 -> 80 11.6 and 12.2; 100 -> 128 9.0 and 8.5 (pair), 384 -> 128 16.1 and 15.4 (pair)
 //   25,000 rows: 64 -> 80 8.1 and 9.6, 256 -> 72 15.0 and 19.1; 64 -> 96 10.8 and 8.7 (pair: a second wave)
 // With more rows than that the pair's overlap pays, up to 80 columns only where two CTAs an SM do not overlap as well themselves: 150,001
-// rows 100 -> 72 39.1 and 31.9 (pair), 64 -> 80 with the mask 45.7 and 48.6, 602 -> 72 114 and 129, 256 -> 80 with the mask 71.9 and 64.9 (pair).
+// rows 256 -> 47 59 and 62, 100 -> 72 39.1 and 31.9 (pair), 64 -> 80 with the mask 45.7 and 48.6, 602 -> 72 114 and 129, 256 -> 80 with the mask 71.9 and 64.9 (pair).
 bool by_pairs(int64_t M, int n_pad, int K, bool masked, int sms)
 {
     if (n_pad <= 64) return false;

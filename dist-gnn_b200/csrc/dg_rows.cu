@@ -25,16 +25,13 @@ __global__ void __launch_bounds__(256) k_pad_rows(const float* __restrict__ src,
 }
 
 // ---- mean cross-entropy over the rows that carry a target --------------------------------------------------------------
-// The step's loss reads the logits of the train rows once and its gradient reads them once more and writes n x C floats:
-// memory bound, 12 bytes per row and class.  As separate passes (row gather, log-softmax, a one-CTA loss reduction, its
+// The step's loss reads the logits of the train rows once and its gradient reads them once more and writes n x C floats: 12 bytes per row
+// and class.  As separate passes (row gather, log-softmax, a one-CTA loss reduction, its
 // backward, the softmax backward, a scatter into zeros) it took 5.5 ms of a 66 ms step at 2,449,029 x 47.
-// What bounds them is instructions: a group of few lanes with up to kKept classes a lane shares row, target, shuffles and logarithm among
-// more rows of a warp, and a class is loaded and exponentiated once (up to four classes a lane -> up to eight, 2,449,029 x 47: forward
-// 286 -> 251 us, gradient 374 -> 337).  The next row's classes are requested before this one's are worked on, its target a row earlier (251 -> 203,
-// 337 -> 291).
+// What bounds them is instructions, and the wait for a row: loss_form.
 // A group of LPR lanes owns a row; lanes read neighbouring classes.  Sums are taken in a fixed order (rows of a thread in
 // order, lanes and warps by a tree, CTAs in order), so the loss is bit-reproducible.
-constexpr int kLossThreads = 256, kKept = 8;
+constexpr int kLossThreads = 256;
 
 template <int LPR> __device__ __forceinline__ float group_max(float v)
 {
@@ -52,44 +49,55 @@ template <int LPR> __device__ __forceinline__ float group_sum(float v)
     return v;
 }
 
-// The rows a group works on, one after the other: a row's target is requested two rows ahead, its first kKept * LPR classes one row ahead.
-template <int LPR> struct RowAhead {
+// The rows a group works on, one after the other, their first KEPT * LPR classes in registers.  AHEAD: a row's target is requested two rows
+// ahead, its classes one row ahead.
+template <int LPR, int KEPT, bool AHEAD> struct Rows {
     const float* x;
     const int32_t* target;
     int64_t ld, n, row, step;
     int32_t C, t, t_next;
-    float v[kKept];
-    __device__ __forceinline__ void fetch(const float* r, bool on)
+    float v[AHEAD ? KEPT : 1];
+    __device__ __forceinline__ int32_t target_of(int64_t r) const { return r < n ? __ldg(target + r) : -1; }
+    __device__ __forceinline__ void fetch(float* to)
     {
         const int lane = threadIdx.x % LPR;
+        const float* r = x + row * ld;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j) v[j] = on && lane + j * LPR < C ? __ldg(r + lane + j * LPR) : __int_as_float(0xff800000);
+        for (int j = 0; j < KEPT; ++j) to[j] = t >= 0 && lane + j * LPR < C ? __ldg(r + lane + j * LPR) : __int_as_float(0xff800000);
     }
-    __device__ __forceinline__ RowAhead(const float* x_, int64_t ld_, int64_t n_, int32_t C_, const int32_t* target_) : x(x_), target(target_), ld(ld_), n(n_), C(C_)
+    __device__ __forceinline__ Rows(const float* x_, int64_t ld_, int64_t n_, int32_t C_, const int32_t* target_) : x(x_), target(target_), ld(ld_), n(n_), C(C_)
     {
         constexpr int RPB = kLossThreads / LPR;
         row = (int64_t)blockIdx.x * RPB + threadIdx.x / LPR;
         step = (int64_t)gridDim.x * RPB;
-        t = row < n ? __ldg(target + row) : -1;
-        t_next = row + step < n ? __ldg(target + row + step) : -1;
-        fetch(x + row * ld, t >= 0);
+        if constexpr (AHEAD) {
+            t = target_of(row);
+            t_next = target_of(row + step);
+            fetch(v);
+        }
     }
-    // Moves on: `e` and `of` receive the row it was at, the one behind it is under way.
-    __device__ __forceinline__ int64_t next(float (&e)[kKept], int32_t& of)
+    // Moves on: `e` and `of` receive the row it was at.
+    __device__ __forceinline__ int64_t next(float* e, int32_t& of)
     {
         const int64_t was = row;
-        of = t;
+        if constexpr (AHEAD) {
+            of = t;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j) e[j] = v[j];
-        row += step;
-        t = t_next;
-        t_next = row + step < n ? __ldg(target + row + step) : -1;
-        fetch(x + row * ld, t >= 0);
+            for (int j = 0; j < KEPT; ++j) e[j] = v[j];
+            row += step;
+            t = t_next;
+            t_next = target_of(row + step);
+            fetch(v);
+        } else {
+            of = t = target_of(row);
+            fetch(e);
+            row += step;
+        }
         return was;
     }
 };
 
-template <int LPR>
+template <int LPR, int KEPT, bool AHEAD>
 __global__ void __launch_bounds__(kLossThreads) k_rows_ce_forward(const float* __restrict__ x, int64_t ld, int64_t n, int32_t C,
                                                                   const int32_t* __restrict__ target, float* __restrict__ lse,
                                                                   double* __restrict__ partial)
@@ -97,27 +105,27 @@ __global__ void __launch_bounds__(kLossThreads) k_rows_ce_forward(const float* _
     constexpr int RPB = kLossThreads / LPR;
     const int lane = threadIdx.x % LPR;
     double loss = 0.0;
-    RowAhead<LPR> rows(x, ld, n, C, target);
+    Rows<LPR, KEPT, AHEAD> rows(x, ld, n, C, target);
     for (int64_t base = (int64_t)blockIdx.x * RPB; base < n; base += (int64_t)gridDim.x * RPB) {
-        float e[kKept], mx = __int_as_float(0xff800000);
+        float e[KEPT ? KEPT : 1], mx = __int_as_float(0xff800000);
         int32_t t;
         const int64_t row = rows.next(e, t);
         const bool on = t >= 0;                                   // the same in every lane of a row's group
         const float* r = x + row * ld;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j) mx = e[j] > mx || e[j] != e[j] ? e[j] : mx;           // a NaN stays
+        for (int j = 0; j < KEPT; ++j) mx = e[j] > mx || e[j] != e[j] ? e[j] : mx;           // a NaN stays
         if (on)
-            for (int c = lane + kKept * LPR; c < C; c += LPR) {
+            for (int c = lane + KEPT * LPR; c < C; c += LPR) {
                 const float v = __ldg(r + c);
                 mx = v > mx || v != v ? v : mx;
             }
         mx = group_max<LPR>(mx);
         float sum = 0.f;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j)
+        for (int j = 0; j < KEPT; ++j)
             if (on && lane + j * LPR < C) sum += expf(e[j] - mx);
         if (on)
-            for (int c = lane + kKept * LPR; c < C; c += LPR) sum += expf(__ldg(r + c) - mx);
+            for (int c = lane + KEPT * LPR; c < C; c += LPR) sum += expf(__ldg(r + c) - mx);
         sum = group_sum<LPR>(sum);
         if (on && lane == 0) {
             const float l = logf(sum);
@@ -155,8 +163,8 @@ __global__ void __launch_bounds__(kLossThreads) k_rows_ce_mean(const double* __r
 // The softmax is taken from the row's maximum and sum anew: against a stored logsumexp it would carry that number's rounding, which
 // grows with the logits (error of the gradient against float64, 47 classes: around 0 1.6e-7, 100 1.3e-6, 10,000 1.6e-4; this way
 // 5e-8 everywhere, as PyTorch's).  A lane's exponentials stay in registers up to
-// kKept classes a lane, so an exponential a class is all it takes, as with the logsumexp.
-template <int LPR>
+// KEPT classes a lane, so an exponential a class is all it takes, as with the logsumexp.
+template <int LPR, int KEPT, bool AHEAD>
 __global__ void __launch_bounds__(kLossThreads) k_rows_ce_backward(const float* __restrict__ x, int64_t ld, int64_t n, int32_t C,
                                                                    const int32_t* __restrict__ target, const float* __restrict__ upstream,
                                                                    float inv_count, float* __restrict__ grad, int64_t ldg)
@@ -164,42 +172,83 @@ __global__ void __launch_bounds__(kLossThreads) k_rows_ce_backward(const float* 
     constexpr int RPB = kLossThreads / LPR;
     const int lane = threadIdx.x % LPR;
     const float scale = __ldg(upstream) * inv_count;
-    RowAhead<LPR> rows(x, ld, n, C, target);
+    Rows<LPR, KEPT, AHEAD> rows(x, ld, n, C, target);
     for (int64_t base = (int64_t)blockIdx.x * RPB; base < n; base += (int64_t)gridDim.x * RPB) {
-        float e[kKept], mx = __int_as_float(0xff800000);
+        float e[KEPT ? KEPT : 1], mx = __int_as_float(0xff800000);
         int32_t t;
         const int64_t row = rows.next(e, t);
         const bool on = t >= 0;
         const float* r = x + row * ld;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j) mx = e[j] > mx || e[j] != e[j] ? e[j] : mx;           // a NaN stays
+        for (int j = 0; j < KEPT; ++j) mx = e[j] > mx || e[j] != e[j] ? e[j] : mx;           // a NaN stays
         if (on)
-            for (int c = lane + kKept * LPR; c < C; c += LPR) {
+            for (int c = lane + KEPT * LPR; c < C; c += LPR) {
                 const float v = __ldg(r + c);
                 mx = v > mx || v != v ? v : mx;
             }
         mx = group_max<LPR>(mx);
         float sum = 0.f;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j)
+        for (int j = 0; j < KEPT; ++j)
             if (on && lane + j * LPR < C) sum += e[j] = expf(e[j] - mx);
         if (on)
-            for (int c = lane + kKept * LPR; c < C; c += LPR) sum += expf(__ldg(r + c) - mx);
+            for (int c = lane + KEPT * LPR; c < C; c += LPR) sum += expf(__ldg(r + c) - mx);
         const float inv = 1.f / group_sum<LPR>(sum);
         if (row >= n) continue;
         float* g = grad + row * ldg;
 #pragma unroll
-        for (int j = 0; j < kKept; ++j) {
+        for (int j = 0; j < KEPT; ++j) {
             const int c = lane + j * LPR;
             if (c < ldg) g[c] = on && c < C ? (e[j] * inv - (c == t ? 1.f : 0.f)) * scale : 0.f;
         }
-        for (int c = lane + kKept * LPR; c < ldg; c += LPR)
+        for (int c = lane + KEPT * LPR; c < ldg; c += LPR)
             g[c] = on && c < C ? (expf(__ldg(r + c) - mx) * inv - (c == t ? 1.f : 0.f)) * scale : 0.f;
     }
 }
 
-// Lanes per row: the least power of two that leaves a lane no more than kKept classes, 4 to 32.
-int lanes_per_row(int32_t C) { return C <= 32 ? 4 : C <= 64 ? 8 : C <= 128 ? 16 : 32; }
+// The kernel that a loss takes: lanes a row, classes a lane keeps in registers, and whether the next row is requested ahead.
+// Eight classes a lane share row, target, shuffles and logarithm among more rows of a warp than four do, as long as there are rows enough
+// for so few lanes.  The look-ahead pays where the rows come from DRAM; out of the L2 its registers cost more than it hides.  Up to
+// 16 classes four lanes keep one class or four: eight slots would be idle.  Beyond 128 classes the forward pass reads a row
+// twice, out of the L1.  us, forward and gradient, four a lane -> eight -> eight and ahead (C > 128: none kept -> four -> eight):
+//   2,449,029 x 47 (460 MB) 282 329 -> 191 265 -> 182 257; x 16 (157 MB) 81 92 (ahead 71 88) -> 93 121 -> 85 117; x 2 57 67 -> 71 93 -> 73 97
+//   150,001 x 47 (28 MB) 19.6 20.6 -> 15.1 16.9 -> 15.8 18.3; x 10 7.8 6.6 -> 8.7 8.3 -> 9.6 9.2; 10,000 x 32 4.3 2.7 -> 4.4 3.3 -> 4.5 3.3
+//   150,001 x 130 36 - -> 41 54 -> 41 59, x 200 42 - -> 48 72 -> 47 65
+struct LossForm {
+    int lanes, kept;
+    bool ahead;
+};
+LossForm loss_form(int64_t n, int32_t C, int64_t ld, bool backward)
+{
+    if (C > 128) return {32, !backward ? 0 : C <= 160 ? 4 : 8, false};
+    const bool ahead = n * ld * 4 > (int64_t)64 << 20;            // half of the L2: what else passes through it needs the rest
+    if (C <= 4) return {4, 1, false};
+    if (C <= 16) return {4, 4, ahead};
+    const int few = C <= 32 ? 4 : C <= 64 ? 8 : 16;
+    if (n * few < 1 << 16) return {2 * few, 4, false};
+    return {few, 8, ahead};
+}
+
+// `use` is called with the form's lanes, classes and look-ahead as constants.
+template <int N> using Int = std::integral_constant<int, N>;
+template <bool BACKWARD, class Use> void with_form(const LossForm& f, Use use)
+{
+    auto either = [&](auto lanes, auto kept) {
+        if (f.ahead) use(lanes, kept, std::true_type{});
+        else use(lanes, kept, std::false_type{});
+    };
+    switch (f.lanes) {
+        case 4: f.kept == 1 ? use(Int<4>{}, Int<1>{}, std::false_type{}) : f.kept == 4 ? either(Int<4>{}, Int<4>{}) : either(Int<4>{}, Int<8>{}); break;
+        case 8: f.kept == 4 ? use(Int<8>{}, Int<4>{}, std::false_type{}) : either(Int<8>{}, Int<8>{}); break;
+        case 16: f.kept == 4 ? use(Int<16>{}, Int<4>{}, std::false_type{}) : either(Int<16>{}, Int<8>{}); break;
+        default:
+            if constexpr (!BACKWARD) {
+                f.kept == 4 ? use(Int<32>{}, Int<4>{}, std::false_type{}) : use(Int<32>{}, Int<0>{}, std::false_type{});
+            } else {
+                f.kept == 4 ? use(Int<32>{}, Int<4>{}, std::false_type{}) : use(Int<32>{}, Int<8>{}, std::false_type{});
+            }
+    }
+}
 
 unsigned loss_blocks(int64_t n, int lpr)
 {
@@ -215,14 +264,11 @@ extern "C" int dg_rows_cross_entropy(const float* x, int64_t ld, int64_t n, int3
     if (n <= 0 || C <= 0 || count <= 0 || ld < C) return DG_ERR_DIMS;
     if (!x || !target || !lse || !scratch || !loss) return DG_ERR_NULL;
     cudaStream_t s = (cudaStream_t)stream;
-    const int lpr = lanes_per_row(C);
-    const unsigned blocks = loss_blocks(n, lpr);
-    switch (lpr) {
-        case 4: k_rows_ce_forward<4><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
-        case 8: k_rows_ce_forward<8><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
-        case 16: k_rows_ce_forward<16><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
-        default: k_rows_ce_forward<32><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch); break;
-    }
+    const LossForm form = loss_form(n, C, ld, false);
+    const unsigned blocks = loss_blocks(n, form.lanes);
+    with_form<false>(form, [&](auto lanes, auto kept, auto ahead) {
+        k_rows_ce_forward<lanes(), kept(), ahead()><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, lse, scratch);
+    });
     k_rows_ce_mean<<<1, kLossThreads, 0, s>>>(scratch, (int)blocks, 1.0 / (double)count, loss);
     return (int)cudaGetLastError();
 }
@@ -233,15 +279,12 @@ extern "C" int dg_rows_cross_entropy_grad(const float* x, int64_t ld, int64_t n,
     if (n <= 0 || C <= 0 || count <= 0 || ld < C || ldg < C) return DG_ERR_DIMS;
     if (!x || !target || !lse || !upstream || !grad) return DG_ERR_NULL;
     cudaStream_t s = (cudaStream_t)stream;
-    const int lpr = lanes_per_row(C);
-    const unsigned blocks = loss_blocks(n, lpr);
+    const LossForm form = loss_form(n, C, ld, true);
+    const unsigned blocks = loss_blocks(n, form.lanes);
     const float inv = (float)(1.0 / (double)count);
-    switch (lpr) {
-        case 4: k_rows_ce_backward<4><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
-        case 8: k_rows_ce_backward<8><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
-        case 16: k_rows_ce_backward<16><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
-        default: k_rows_ce_backward<32><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg); break;
-    }
+    with_form<true>(form, [&](auto lanes, auto kept, auto ahead) {
+        k_rows_ce_backward<lanes(), kept(), ahead()><<<blocks, kLossThreads, 0, s>>>(x, ld, n, C, target, upstream, inv, grad, ldg);
+    });
     return (int)cudaGetLastError();
 }
 

@@ -427,3 +427,31 @@ def test_row_cross_entropy_gradient_of_large_logits(C):
         xd = x.detach().double().requires_grad_()
         torch.nn.functional.cross_entropy(xd[rows], t[rows].long()).backward()
         assert float((x.grad.double() - xd.grad).norm() / xd.grad.norm()) < 10 * 2.0 ** -24
+
+
+@pytest.mark.parametrize('n,C,ld', [(227333, 3, 3), (227333, 10, 10), (227333, 10, 80), (227333, 30, 30), (227333, 30, 80), (113669, 47, 47), (113669, 47, 150),
+                                    (56837, 100, 100), (56837, 128, 300), (28421, 130, 130), (28421, 161, 161), (28421, 300, 300), (16383, 32, 32), (16384, 17, 17),
+                                    (8191, 64, 64), (4095, 128, 128)])
+def test_row_cross_entropy_over_several_rows_of_a_group(n, C, ld):
+    """Every form of the loss - lanes a row, classes kept, the next row requested ahead (operands beyond 64 MB) - with more than three rows for
+    most of its groups where its sizes allow that, among them some of which every row, the middle one or the first and last have no target.
+    Against float64: the loss to 1e-6, the gradient within ten roundings of a probability."""
+    import spmm_cpp
+    gen = torch.Generator(device='cuda').manual_seed(n + C + ld)
+    x = (torch.randn(n, ld, device='cuda', generator=gen) * 3)[:, :C].requires_grad_(True)
+    t = torch.randint(0, C, (n,), device='cuda', generator=gen, dtype=torch.int32)
+    t[torch.rand(n, device='cuda', generator=gen) < 0.4] = -1
+    groups = n // 3                                               # the rows of a group are as far apart, where it has several
+    for first, off in ((100, (0, 1, 2, 3)), (300, (1,)), (500, (0, 2))):
+        for k in off:
+            t[k * groups + first:k * groups + first + 100] = -1
+    rows = (t >= 0).nonzero().squeeze(1)
+    loss = spmm_cpp.row_cross_entropy(x, t, rows.numel())
+    grad, = torch.autograd.grad(loss * 2.5, x)
+    xd = x.detach().double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(xd[rows], t[rows].long())
+    want_grad, = torch.autograd.grad(want * 2.5, xd)
+    assert abs(loss.item() - want.item()) <= 1e-6 * max(1.0, abs(want.item()))
+    assert float((grad.double() - want_grad).norm() / want_grad.norm()) < 10 * 2.0 ** -24
+    assert bool((grad[t < 0] == 0).all())
+    assert torch.equal(loss, spmm_cpp.row_cross_entropy(x, t, rows.numel()))

@@ -441,8 +441,12 @@ int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
 // instead of 32 (F = 256: 2.4 M / 126 M with tiles 7,810 -> 7,550, 1 M / 17 M 1,291 -> 1,274, 300 k / 15 M 876 -> 855; F = 512: 2,860 -> 2,800).
 // Small matrices, wide rows: three gathers in flight (with four, 72 bytes of spills: eight 306 k-row stage blocks 1,459 -> 1,409,
 // 150 k / 2.6 M F = 256 204 -> 197, F = 200 197 -> 190).
-// 65 to 96 floats, from 4 M entries: 8 lanes of three vectors, of which at most 7 idle (16 x 2: up to 15).  1 M / 17 M F = 96 676 -> 618, 600 k /
-// 21 M 676 -> 622, 2.4 M / 126 M 4,190 -> 3,920, 300 k / 15 M 471 -> 447, 2.4 M / 42 M 1,758 -> 1,798 (F = 72 1,700 -> 1,680); 150 k / 2.6 M 111 -> 119 (not taken).
+// 65 to 96 floats, from 4 M entries: 8 lanes of three vectors, of which at most 7 idle (16 x 2: up to 15).  1 M / 17 M F = 96 675 -> 618, F = 68
+// 655 -> 583, 600 k / 21 M 676 -> 622, 2.4 M / 126 M 4,190 -> 3,920, 300 k / 15 M 471 -> 447, 2.4 M / 42 M 1,727 -> 1,727 (F = 68 1,668 -> 1,631); 150 k / 2.6 M
+// 111 -> 119 (not taken).  Not taken either beside tiles in windows of 64 rows, which leave too few rows for four groups a warp (200 k / 10 M F = 96
+// 308 -> 325, F = 68 297 -> 306; windows of 128: 300 k / 12 M F = 96 388 -> 387, F = 68 377 -> 364), nor for short rows out of DRAM, read as they
+// are: fewer than eight entries a row and an operand of four times the L2 (2.4 M / 16 M F = 96 1,009 -> 1,108, 4 M / 20 M 1,475 -> 1,615;
+// 2.4 M / 22 M 1,189 -> 1,094, 1.5 M / 7.5 M 540 -> 516, padded F = 65 2.4 M / 12 M 1,081 -> 1,033).
 // 33 to 48 floats, from 4 M entries, or from 1 M with 64 k rows or more where the operand is read as it is, without tiles: 4 lanes of
 // three, eight rows a warp, as long as the L2 holds the operand, or three eighths of it where rows straddle sectors.  F = 48: 200 k rows / 10 M
 // 223 -> 184, 250 k / 8 M 199 -> 170, 30 k / 8 M 161 -> 149, 250 k / 1.4 M 78 -> 70, 80 k / 1.2 M 53 -> 52, 600 k / 21 M (115 MB) 394 -> 393;
@@ -477,7 +481,8 @@ int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, int32_t k, bool o
             if (nvec > 8 && nvec <= 12 && many && !whole && k * a.ldb * 4 <= (a.ldb % 8 ? kL2Bytes * 3 / 8 : kL2Bytes)) {
                 rc = launch<VEC, 4, 3, 4, 4, PADDED>(a, whole, stream);
                 thirds = true;
-            } else if (nvec > 16 && nvec <= 24 && large) {
+            } else if (nvec > 16 && nvec <= 24 && large && !(whole && a.rows_per_cta < 128) &&
+                       (PADDED || nnz >= 8 * (int64_t)a.m || k * a.ldb <= kL2Bytes)) {
                 rc = launch<VEC, 8, 3, 4, 3, PADDED>(a, whole, stream);
                 thirds = true;
             }

@@ -897,36 +897,104 @@ def lengths_block(lengths, k, seed):
     return row, col, torch.randn(row.numel(), device='cuda', generator=g)
 
 
+class Exact:
+    """Products of a block in float64, and the bound on a product's error: 128 roundings of the sum of the magnitudes, and of one."""
+
+    def __init__(self, row, col, val, m, k):
+        self.m, self.k = m, k
+        self.sparse = torch.sparse_coo_tensor(torch.stack((row, col)).long(), val.double(), (m, k)).to_sparse_csr()
+        self.magnitudes = torch.sparse_csr_tensor(self.sparse.crow_indices(), self.sparse.col_indices(), self.sparse.values().abs(), (m, k))
+
+    def check(self, plan, b, g):
+        """The product alone, added to C, and with the fused epilogue; returns the first."""
+        F = b.size(1)
+        c0 = torch.randn(self.m, F, device='cuda', generator=g)
+        scale, bias = torch.rand(self.m, device='cuda', generator=g) + 0.5, torch.randn(F, device='cuda', generator=g)
+        want, bound = torch.sparse.mm(self.sparse, b.double()), torch.sparse.mm(self.magnitudes, b.double().abs()) + c0.abs()
+        close = lambda got, exact: bool(((got.double() - exact).abs() <= 128 * 2.0 ** -24 * (bound + 1)).all())
+        out = plan.spmm(b, torch.empty_like(c0), 1.0, 0.0)
+        assert close(out, want), (self.m, F)
+        assert close(plan.spmm(b, c0.clone(), 1.0, 1.0), want + c0), (self.m, F)
+        assert close(plan.spmm(b, c0.clone(), 0.5, -1.0, row_scale=scale, bias=bias, relu=True), ((0.5 * want - c0) * scale[:, None] + bias).clamp(min=0)), (self.m, F)
+        return out
+
+
 @pytest.mark.parametrize('nnz', [200_000, 1_100_000, 4_300_000])
 def test_forms_by_size_and_width(nnz):
-    """Every form a width and size of a matrix choose: widths around 8 / 12 / 16 / 24 / 32 vectors and whole tiles, rows of 32-byte pieces
-    read as such and the same operand one vector off them, odd widths through the padded copy, an operand beyond the L2, products
-    added to C and the fused epilogue; rows with no entry, around the sets of 4 to 32 entries, and split ones.  Against float64, within 64
-    roundings of a sum of the magnitudes."""
+    """The forms that widths and the number of entries choose for an operand that the L2 holds: widths around 8 / 12 / 16 / 24 / 32 vectors and
+    whole tiles, rows of 32-byte pieces read as such and the same operand one vector off them, odd widths through the padded copy, products
+    added to C and the fused epilogue; rows with no entry, around the sets of 4 to 32 entries, and split ones."""
     import spmm_cpp
     edges = torch.tensor([0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 30, 31, 32, 33, 34, 35, 63, 64, 65, 66, 67, 127, 128, 129, 130, 300, 1025])
     k = 40_000
     lengths = edges.repeat(nnz // int(edges.sum()) + 1)
     row, col, val = lengths_block(lengths, k, nnz)
     m = lengths.numel()
-    plan = spmm_cpp.SpmmPlan(row, col, val, m, k)
-    sparse = torch.sparse_coo_tensor(torch.stack((row, col)).long(), val.double(), (m, k)).to_sparse_csr()
-    magnitudes = torch.sparse_csr_tensor(sparse.crow_indices(), sparse.col_indices(), sparse.values().abs(), (m, k))
+    plan, exact = spmm_cpp.SpmmPlan(row, col, val, m, k), Exact(row, col, val, m, k)
     g = torch.Generator(device='cuda').manual_seed(7)
     for F in (33, 36, 41, 44, 48, 49, 52, 65, 68, 93, 96, 97, 100, 200, 256, 264, 320):
         b = torch.randn(k, F, device='cuda', generator=g)
-        c0 = torch.randn(m, F, device='cuda', generator=g)
-        scale, bias = torch.rand(m, device='cuda', generator=g) + 0.5, torch.randn(F, device='cuda', generator=g)
-        want, bound = torch.sparse.mm(sparse, b.double()), torch.sparse.mm(magnitudes, b.double().abs()) + c0.abs()
-        close = lambda got, exact: bool(((got.double() - exact).abs() <= 64 * 2.0 ** -24 * (bound + 1) * 2).all())
-        out = plan.spmm(b, torch.empty_like(c0), 1.0, 0.0)
-        assert close(out, want), (nnz, F)
-        assert close(plan.spmm(b, c0.clone(), 1.0, 1.0), want + c0), (nnz, F)
-        assert close(plan.spmm(b, c0.clone(), 0.5, -1.0, row_scale=scale, bias=bias, relu=True), ((0.5 * want - c0) * scale[:, None] + bias).clamp(min=0)), (nnz, F)
+        out = exact.check(plan, b, g)
         if F % 8 == 0:
             apart = torch.empty(k, F + 4, device='cuda')[:, 4:]            # rows 16 bytes off a 32-byte piece
             apart.copy_(b)
-            assert torch.equal(plan.spmm(apart, torch.empty_like(c0), 1.0, 0.0), out), (nnz, F)
+            assert torch.equal(plan.spmm(apart, torch.empty_like(out), 1.0, 0.0), out), (nnz, F)
+
+
+@pytest.mark.parametrize('m,nnz,k,widths', [(100_000, 1_500_000, 40_000, (33, 36, 40, 48)), (150_000, 4_400_000, 300_000, (36, 41, 44, 48)),
+                                            (150_000, 4_400_000, 750_000, (48,)), (600_000, 4_400_000, 2_000_000, (68, 93, 96)),
+                                            (600_000, 4_900_000, 2_000_000, (68,))])
+def test_forms_by_rows_and_operand(m, nnz, k, widths):
+    """What the number of rows and the size of the operand add to that: medium matrices with many rows, operands on either side of what the
+    L2 holds and of three eighths of it (rows that straddle sectors), short rows of an operand of more than four times the L2."""
+    import spmm_cpp
+    lengths = torch.arange(m) % (2 * nnz // m + 1)
+    lengths[::1000] += 600                                        # split rows
+    row, col, val = lengths_block(lengths, k, m + nnz)
+    plan, exact = spmm_cpp.SpmmPlan(row, col, val, m, k), Exact(row, col, val, m, k)
+    g = torch.Generator(device='cuda').manual_seed(8)
+    for F in widths:
+        exact.check(plan, torch.randn(k, F, device='cuda', generator=g), g)
+
+
+@pytest.mark.parametrize('m', [200_000, 262_145])
+@pytest.mark.parametrize('F', [72, 93, 96, 200, 256, 264, 320])
+def test_tiles_beside_the_forms_of_large_matrices(F, m):
+    """A block of more than 4.2 M entries with tiles, in windows of 64 and of 128 rows: whole, incomplete and several column tiles of rows of 32-byte
+    pieces, thirds, the padded copy.  Then with a value that was changed without the version counter's notice, and with an operand
+    element that the tiles cannot take: the launch behind the tiles gathers the split rows whole."""
+    import spmm_cpp
+    g = torch.Generator(device='cuda').manual_seed(F + m)
+    k, dense_rows = 6000, 1200
+    lengths = torch.full((m,), 6, device='cuda')
+    mask = torch.rand(dense_rows, k, device='cuda', generator=g) < 0.45
+    at = torch.randperm(m, device='cuda', generator=g)[:dense_rows].sort().values
+    lengths[at] = mask.sum(1)
+    row = torch.repeat_interleave(torch.arange(m, device='cuda'), lengths).to(torch.int32)
+    first = lengths.cumsum(0) - lengths
+    place = torch.arange(row.numel(), device='cuda') - first[row.long()]
+    col = (place * 1000 + torch.randint(0, 1000, (row.numel(),), device='cuda', generator=g)).to(torch.int32)      # ascending, one of every thousand
+    in_dense = torch.isin(row, at.to(torch.int32))
+    col[in_dense] = mask.nonzero()[:, 1].to(torch.int32)
+    val = torch.randn(row.numel(), device='cuda', generator=g)
+    assert row.numel() > 4_200_000
+    keep = spmm_cpp.TILE_NNZ
+    try:
+        spmm_cpp.TILE_NNZ = 0
+        plan = spmm_cpp.SpmmPlan(row, col, val, m, k).tile()
+    finally:
+        spmm_cpp.TILE_NNZ = keep
+    assert plan.tiled_entries() > row.numel() // 4
+    b = torch.randn(k, F, device='cuda', generator=g)
+    Exact(row, col, val, m, k).check(plan, b, g)
+    assert plan.device_status() == 0
+    b[17, F // 2] = 1e19
+    Exact(row, col, val, m, k).check(plan, b, g)
+    b[17, F // 2] = 1.0
+    changed = int(first[at[5]]) + 1000
+    val.data[changed] = 300.0
+    Exact(row, col, val, m, k).check(plan, b, g)
+    assert plan.device_status() == 0
 
 
 def test_infinite_values_beside_short_batches():

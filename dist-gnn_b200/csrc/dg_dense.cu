@@ -333,7 +333,7 @@ k_dense_nt_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(acc_full0 + 8 * b, 1);
-            mbar_init(acc_empty0 + 8 * b, 2 * min(kEpilogueWarps, a.n_pad / 32 * 4));      // a result of 32 columns leaves half of them idle
+            mbar_init(acc_empty0 + 8 * b, 2 * kEpilogueWarps);
         }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -433,7 +433,7 @@ k_dense_nt_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                          (!MASK || (a.ldm % 4 == 0 && (reinterpret_cast<uintptr_t>(a.mask) & 15) == 0));
         const int r4 = lane >> 3, piece = lane & 7;
         int lt = 0;
-        for (int tile = first < a.n_pad ? pair : n_tiles; tile < n_tiles; tile += pairs, ++lt) {
+        for (int tile = pair; tile < n_tiles; tile += pairs, ++lt) {
             const int b = lt & 1, v = lt >> 1;
             const int64_t row0 = (int64_t)tile * (2 * BM) + rank * BM + q * 32;
             const int rows = (int)max((int64_t)0, min((int64_t)32, a.M - row0));
@@ -987,7 +987,8 @@ __device__ __forceinline__ void dense_tn(const CUtensorMap& tmP, const CUtensorM
         }
     } else if (warp < 2 + kTnSplitWarps) {
         // The tile as loaded serves as head, its tail goes behind it.  Half the warps take the even boxes, half the odd ones.  Columns of P
-        // that it does not have are neither loaded nor split: what lies there reaches rows of the accumulators that nobody reads.
+        // that it does not have are neither loaded nor split: what lies there reaches rows of the accumulators, and of a pair's partial
+        // results, that k_dense_tn_reduce leaves out.
         const int t = threadIdx.x - 64, half = t >> 7, boxes = p_boxes + q_boxes;
         int s = 0, phase = 0, slabs = 0;
         for (int range = range0; range < range1; ++range) slabs += slabs_of(range);

@@ -130,7 +130,7 @@ __device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const floa
 // ---- the product -------------------------------------------------------------------------------------------------------
 // A warp is G = 32 / LPR groups of LPR lanes, and every group works on an item of its own: a row, or a chunk of a split
 // row.  Lane gl of a group owns the TPL vectors (VEC floats each) gl, gl + LPR, ... of the column tile blockIdx.y, so a
-// gathered row of B is read with coalesced loads of up to 128 bits; the group reads LPR (col, val) pairs at a time, the next
+// gathered row of B is read with coalesced loads of up to 256 bits; the group reads LPR (col, val) pairs at a time, the next
 // LPR while it works on these, and hands them out by shuffle, U gathers in flight before the first FMA.  A row is summed
 // in entry order by one group, whatever LPR is.
 //
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256, MINB) k_spmm(const SpmmArgs a, const int 
     }
 }
 
-template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED>
+template <int VEC, int LPR, int TPL, int U, int MINB, bool PADDED, bool TILES = VEC >= 4>
 int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
 {
     constexpr int NG = 256 / LPR, tile = LPR * TPL;
@@ -415,7 +415,7 @@ int launch(const SpmmArgs& args, const SpmmArgs* whole, cudaStream_t stream)
         const dim3 grid((unsigned)(chunk_ctas + row_ctas), (unsigned)std::min((a.vec_end - a.vec_first + tile - 1) / tile, DG_FINISH_TILES));
         if (!whole) k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kPlain><<<grid, 256, 0, stream>>>(a, chunk_ctas);
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-        if constexpr (VEC >= 4) {
+        if constexpr (TILES) {
             if (!whole) continue;
             k_spmm<VEC, LPR, TPL, U, MINB, PADDED, kTiled><<<grid, 256, 0, stream>>>(a, chunk_ctas);
             SpmmArgs w = *whole;
@@ -479,7 +479,7 @@ int launch_vec(SpmmArgs a, const SpmmArgs* whole, int64_t nnz, int32_t k, bool o
         if constexpr (VEC == 4) {
             const bool many = large || (!small && !PADDED && a.m >= 1 << 16);
             if (nvec > 8 && nvec <= 12 && many && !whole && k * a.ldb * 4 <= (a.ldb % 8 ? kL2Bytes * 3 / 8 : kL2Bytes)) {
-                rc = launch<VEC, 4, 3, 4, 4, PADDED>(a, whole, stream);
+                rc = launch<VEC, 4, 3, 4, 4, PADDED, false>(a, nullptr, stream);
                 thirds = true;
             } else if (nvec > 16 && nvec <= 24 && large && !(whole && a.rows_per_cta < 128) &&
                        (PADDED || nnz >= 8 * (int64_t)a.m || k * a.ldb <= kL2Bytes)) {

@@ -46,19 +46,28 @@ _padded_rows = {}
 def _rows(t, keep=False):
     """t itself when its rows are dense and start on 16-byte boundaries (a column slice of a padded buffer is fine), else
     the first t.size(1) columns of a copy whose rows are padded to a multiple of 4 floats.  keep=True caches that copy for
-    as long as t lives and is not modified in place (the input features: 602 floats per row -> 604)."""
+    as long as t lives and is not modified in place (the input features: 602 floats per row -> 604); a stream that did not
+    make it waits until it has been made (a captured one cannot: captures begin on an idle device)."""
     if t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 4 == 0 and t.stride(0) >= t.size(1) and t.data_ptr() % 16 == 0:
         return t
     if keep:
         hit = _padded_rows.get(id(t))
         if hit is not None and hit[0]() is t and hit[1] == t._version:
-            return hit[2]
+            _, _, view, stream, made = hit
+            if made is not None and stream != spmm_cpp.current_stream(t) and not torch.cuda.is_current_stream_capturing():
+                now = torch.cuda.current_stream(t.device)
+                now.wait_event(made)
+                view.record_stream(now)
+            return view
     rows, cols = t.shape
     wide = torch.empty((rows, cols + (-cols) % 4), dtype=t.dtype, device=t.device)
     view = _pad_into(t, wide)[:, :cols]
-    if keep:
-        key = id(t)
-        _padded_rows[key] = (weakref.ref(t, lambda _r, key=key: _padded_rows.pop(key, None)), t._version, view)
+    if keep and not (t.is_cuda and torch.cuda.is_current_stream_capturing()):      # a captured copy is not made before the graph runs
+        key, stream, made = id(t), None, None
+        if t.is_cuda:
+            stream, made = spmm_cpp.current_stream(t), torch.cuda.Event()
+            made.record(torch.cuda.current_stream(t.device))
+        _padded_rows[key] = (weakref.ref(t, lambda _r, key=key: _padded_rows.pop(key, None)), t._version, view, stream, made)
     return view
 
 
@@ -157,7 +166,7 @@ def _product_operand(env, t, constant):
     if constant:
         kept = _rows(t, keep=True)
         return kept.as_strided((n, width), (kept.stride(0), 1))
-    return _pad_into(t, env.recv_buffers(n, width, nbuf=1, tag='padded')[0])
+    return _pad_into(t, torch.empty((n, width), dtype=torch.float32, device=t.device))
 
 
 def _local_products(env, adj_parts, t, constant):

@@ -193,6 +193,11 @@ def _stream(index=None):
     return _raw_stream(index)
 
 
+def current_stream(t):
+    """torch's current stream of t's CUDA device as a plain number."""
+    return _raw_stream(t.device.index)
+
+
 def _dev_tensor(t, dtype, what):
     if not (isinstance(t, torch.Tensor) and t.is_cuda):
         raise RuntimeError(f'{what} must be a CUDA tensor: this library has no CPU path')
@@ -701,7 +706,7 @@ def dense_split(w):
     return head, tail
 
 
-_split_cache = {}       # id(weight object) -> (weak reference to it, {transposed flag: (version, buffer, head, tail, ldb)})
+_split_cache = {}       # id(weight object) -> (weak reference to it, {(transposed flag, stream): (version, buffer, head, tail, ldb)})
 
 
 def split_operands(requests):
@@ -709,8 +714,8 @@ def split_operands(requests):
     tail, all of them by one launch.  requests: (w, transposed, cache_key) each; transposed=True takes w as [K x N] and
     transposes it.  With a cache_key (the weight object the caller holds, e.g. the nn.Parameter) the result is kept until
     that tensor is modified in place - its version counter moves with every optimiser step - so a weight is transposed and
-    split once per step, not once per product.  Returns (buffer that holds them, head address, tail address, row stride)
-    per request; the tail lies right behind the head."""
+    split once per step and stream, not once per product; the work of a stream only reads what that stream split.  Returns
+    (buffer that holds them, head address, tail address, row stride) per request; the tail lies right behind the head."""
     out, stale, floats = [None] * len(requests), [], 0
     for i, (w, transposed, cache_key) in enumerate(requests):
         slot = None
@@ -720,7 +725,7 @@ def split_operands(requests):
             if entry is None or entry[0]() is not cache_key:   # tensors compare element-wise, so the table is keyed by identity
                 entry = _split_cache[ident] = (weakref.ref(cache_key, lambda _r, ident=ident: _split_cache.pop(ident, None)), {})
             slot = entry[1]
-            hit = slot.get(transposed)
+            hit = slot.get((transposed, _raw_stream(w.device.index)))
             if hit is not None and hit[0] == cache_key._version and hit[1].device == w.device:
                 out[i] = hit[1:]
                 continue
@@ -731,26 +736,30 @@ def split_operands(requests):
         if transposed:
             N, K = K, N
         ldb = K + (-K) % 4
-        stale.append((i, w, transposed, cache_key, slot, N, K, ldb, floats))
+        stale.append((i, w, transposed, None if cache_key is None else cache_key._version, slot, N, K, ldb, floats))
         floats += 2 * N * ldb
     if stale:
         device = stale[0][1].device
         buffer = torch.empty(floats, dtype=torch.float32, device=device)
         base = buffer.data_ptr()
         jobs = (SplitJob * len(stale))()
-        for job, (i, w, transposed, cache_key, slot, N, K, ldb, first) in zip(jobs, stale):
+        for job, (i, w, transposed, version, slot, N, K, ldb, first) in zip(jobs, stale):
             head = base + 4 * first
             tail = head + 4 * N * ldb
             job.w, job.ldw, job.head, job.tail, job.ldb = w.data_ptr(), w.stride(0), head, tail, ldb
             job.N, job.K, job.transposed = N, K, transposed
             out[i] = (buffer, head, tail, ldb)
-            if cache_key is not None:
-                slot[transposed] = (cache_key._version,) + out[i]
         global dense_launches
         dense_launches += 1
         index = device.index
+        stream = _raw_stream(index)
         with _on(index):
-            check(lib().dg_dense_split_operands(jobs, len(stale), _raw_stream(index)))
+            check(lib().dg_dense_split_operands(jobs, len(stale), stream))
+        for i, w, transposed, version, slot, *_ in stale:          # only now that the copies are under way may another thread find them
+            if slot is not None:
+                for old in [key for key, kept in list(slot.items()) if kept[0] != version]:
+                    slot.pop(old, None)                            # of streams that have not come back since the weight changed
+                slot[transposed, stream] = (version,) + out[i]
     return out
 
 

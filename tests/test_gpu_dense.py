@@ -282,3 +282,54 @@ def test_dense_tn_on_two_streams_at_once(n, Km, Nn):
     for d, same in zip(alone, got):
         assert all(torch.equal(d, e) for e in same)
     assert spmm_cpp.dense_status() == 0
+
+
+def test_copies_that_are_kept_are_ready_on_every_stream():
+    """A weight's split copy and an input's padded copy, made on a stream that is held up, and used meanwhile on another one."""
+    import spmm_cpp
+    from models.gcn import _rows
+    g = torch.Generator(device='cuda').manual_seed(3)
+    a = torch.randn(500, 100, device='cuda', generator=g)
+    weight = torch.nn.Parameter(torch.randn(100, 64, device='cuda', generator=g))
+    x = torch.randn(70001, 41, device='cuda', generator=g)
+    want = spmm_cpp.dense_nt(a, weight, transposed=True)
+    junk = [torch.full((1 << 20,), float('nan'), device='cuda') for _ in range(24)]
+    torch.cuda.synchronize()
+    del junk                                                      # what an early reader would find
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(20_000_000)                             # some ten milliseconds
+        one = spmm_cpp.dense_nt(a, weight, transposed=True, cache_key=weight)
+        kept = _rows(x, keep=True)
+    with torch.cuda.stream(second):
+        two = spmm_cpp.dense_nt(a, weight, transposed=True, cache_key=weight)
+        other = _rows(x, keep=True)
+        copy = other.clone()
+    torch.cuda.synchronize()
+    assert torch.equal(one, want) and torch.equal(two, want)
+    assert other.data_ptr() == kept.data_ptr() and torch.equal(copy, x)
+    with torch.no_grad():
+        weight.mul_(2.0)
+    assert torch.equal(spmm_cpp.dense_nt(a, weight, transposed=True, cache_key=weight), 2 * want)
+
+
+@pytest.mark.parametrize('warm', [False, True])
+def test_kept_copies_under_capture(warm):
+    """A captured product that reads a kept padded copy, made before on another stream or not at all; the copy of a capture is not kept."""
+    import spmm_cpp
+    from models.gcn import dense_mm
+    g = torch.Generator(device='cuda').manual_seed(4)
+    x = torch.randn(3001, 41, device='cuda', generator=g)
+    y = torch.randn(3001, 64, device='cuda', generator=g)
+    if warm:
+        dense_mm(x, y, ta=True, constant_a=True)
+    else:
+        dense_mm(x.clone(), y, ta=True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = dense_mm(x, y, ta=True, constant_a=True)
+    eager = dense_mm(x, y, ta=True, constant_a=True)
+    graph.replay()
+    assert torch.equal(out, eager)
+    assert_close(eager.cpu().numpy(), (x.double().t() @ y.double()).cpu().numpy(), TOL, 'captured')
+    assert spmm_cpp.dense_status() == 0

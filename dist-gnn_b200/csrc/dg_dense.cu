@@ -284,11 +284,11 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 // 2,449,029 rows (us, one CTA per SM with four epilogue warps -> pair): 256 -> 256 1,600 -> 1,535, with the mask 1,930 -> 1,720;
 // 100 -> 256 1,100 -> 895; 47 -> 256 with the mask 1,600 -> 1,110; 602 -> 256 4,280 -> 3,540; 256 -> 128 1,540 -> 1,065 (one tile per
 // CTA).  150,001 rows: 256 -> 256 102 -> 100, with the mask 126 -> 109; 100 -> 256 76 -> 61.
-// A half slab's six MMAs are issued together.  With the tail passes behind the head passes of two half slabs, as above 128 columns before, an
-// MMA took 177 clocks instead of 139 whatever its width, and results of 160 to 200 columns were slower than with one CTA per SM.  us, one
-// CTA -> pair, tails behind -> together: 150,001 rows 256 -> 160 77 -> 83 -> 68, 256 -> 192 84 -> 87 -> 75, 256 -> 256 99 -> 95 -> 87; 3,000 rows
-// 256 -> 160 13.4 -> 14.7 -> 12.3.  2,449,029 rows (in turn, 20 ms between launches) 256 -> 256 1,448 -> 1,343, with the mask 1,603 -> 1,470,
-// 602 -> 256 3,346 -> 3,145, 256 -> 128 988 -> 912.  Error against float64: 256 -> 256 2.30e-6 -> 2.15e-6, 64 -> 192 9.0e-7 -> 7.9e-7.
+// The warp that issues the MMAs walks through its loop together and one lane issues (elect_one).  With one lane in the whole loop the issue
+// itself was the limit: 125 clocks an MMA, 197 with the tail passes behind the head passes, whatever the width and however many stages.  ns per
+// half slab, 3,000 rows: 96 columns 386 -> 320, 160 600 -> 293, 256 599 -> 446.  us, one CTA -> pair -> this: 150,001 rows 256 -> 160 76 -> 84 -> 68,
+// 256 -> 192 82 -> 85 -> 74, 256 -> 256 98 -> 94 -> 90; 3,000 rows 256 -> 160 13.6 -> 15.0 -> 12.1; 2,449,029 rows (in turn, 20 ms between launches)
+// 256 -> 256 1,492 -> 1,428, with the mask 1,678 -> 1,574, 602 -> 256 3,423 -> 3,238, 256 -> 128 1,017 -> 904.
 constexpr int PK = 16, kMaxPairStages = 10, kSplitWarps = 4, kEpilogueWarps = 8;
 constexpr int kThreadsPair = 32 * (2 + kSplitWarps + kEpilogueWarps);
 constexpr int kPieceBytes = 32 * 32 * 4;                          // staging of an epilogue warp: 32 rows x 32 columns
@@ -367,34 +367,58 @@ k_dense_nt_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             await_loads(full0, it, stages);
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {                             // MMA issuer
+        if (rank == 0) {                                          // MMA issuer: the warp waits and counts together, one lane issues
+            const bool issuer = elect_one(), tails_last = a.n_pad > 128;
+            // the issuing lane polls: all of them polling held the epilogue up (306,128 rows 32 -> 112 45.1 us, 46.7)
+            auto wait = [&](uint32_t bar, int parity) { return __any_sync(0xffffffffu, issuer && mbar_wait(bar, parity)) != 0; };
             const uint32_t idesc = umma_idesc_tf32(a.n_pad) + ((uint32_t)(BM >> 4) << 24);      // 2 * BM rows
+            const uint64_t desc0 = umma_desc_sw64(base);
+            const uint32_t next_stage = (uint32_t)stage_bytes >> 4, tail = a_bytes >> 4, b_head = 2 * tail, b_tail = b_head + ((uint32_t)b_bytes >> 4);
             int s = 0, phase = 0, lt = 0;
             for (int tile = pair; tile < n_tiles && ok; tile += pairs, ++lt) {
                 const int b = lt & 1, v = lt >> 1;
-                if (lt >= 2) ok = mbar_wait(acc_empty0 + 8 * b, (v - 1) & 1);     // both epilogues have drained this accumulator
+                if (lt >= 2) ok = wait(acc_empty0 + 8 * b, (v - 1) & 1);     // both epilogues have drained this accumulator
                 const uint32_t acc = tmem + (uint32_t)(b * 256);
-                for (int i = 0; i < nhalves; ++i) {
-                    ok = ok && mbar_wait(ready0 + 8 * s, phase);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int i = 0; i < nhalves && ok; i += 2) {
                     // The tensor cores read a TF32 operand from a 32-bit container and ignore its low 13 bits (verified: identical
-                    // bits with a masked copy), so the tile as TMA delivered it is the head.  The tail comes first, as in the kernel of one CTA.
-                    const uint32_t st = base + s * stage_bytes;
-                    const uint64_t a_head = umma_desc_sw64(st), a_tail = umma_desc_sw64(st + a_bytes);
-                    const uint64_t b_head = umma_desc_sw64(st + 2 * a_bytes), b_tail = umma_desc_sw64(st + 2 * a_bytes + b_bytes);
+                    // bits with a masked copy), so the tile as TMA delivered it is the head.  The order of the additions decides the last
+                    // bits, and those the sign of a ReLU's input: over a slab of two halves, the tail passes come behind the head
+                    // passes (wide results) or beside them (narrow ones), as in the kernels of one CTA.
+                    const int s0 = s, halves = min(2, nhalves - i);
+                    for (int h = 0; h < halves && ok; ++h) {
+                        ok = wait(ready0 + 8 * s, phase);
+                        if (!ok) break;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint64_t d = desc0 + (uint32_t)s * next_stage;
+                        if (issuer) {
 #pragma unroll
-                    for (int k = 0; k < PK / 8; ++k) {            // 8 TF32 columns = 32 bytes per MMA: +2 in 16-byte units
-                        umma_tf32_pair(acc, a_tail + 2 * k, b_head + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
-                        umma_tf32_pair(acc, a_head + 2 * k, b_tail + 2 * k, idesc, 1u);
-                        umma_tf32_pair(acc, a_head + 2 * k, b_head + 2 * k, idesc, 1u);
+                            for (int k = 0; k < PK / 8; ++k) {    // 8 TF32 columns = 32 bytes per MMA: +2 in 16-byte units
+                                const uint32_t add = i > 0 || h > 0 || k > 0 ? 1u : 0u;
+                                if (!tails_last) umma_tf32_pair(acc, d + tail + 2 * k, d + b_head + 2 * k, idesc, add);
+                                umma_tf32_pair(acc, d + 2 * k, d + b_tail + 2 * k, idesc, tails_last ? add : 1u);
+                                umma_tf32_pair(acc, d + 2 * k, d + b_head + 2 * k, idesc, 1u);
+                            }
+                            if (!tails_last) umma_commit_pair(empty0 + 8 * s);
+                        }
+                        __syncwarp();
+                        if (++s == stages) s = 0, phase ^= 1;
                     }
-                    umma_commit_pair(empty0 + 8 * s);
-                    if (++s == stages) s = 0, phase ^= 1;
+                    for (int h = 0, t = s0; tails_last && h < halves && ok; ++h) {
+                        const uint64_t d = desc0 + (uint32_t)t * next_stage;
+                        if (issuer) {
+#pragma unroll
+                            for (int k = 0; k < PK / 8; ++k) umma_tf32_pair(acc, d + tail + 2 * k, d + b_head + 2 * k, idesc, 1u);
+                            umma_commit_pair(empty0 + 8 * t);
+                        }
+                        __syncwarp();
+                        if (++t == stages) t = 0;
+                    }
                 }
-                if (ok) umma_commit_pair(acc_full0 + 8 * b);
+                if (ok && issuer) umma_commit_pair(acc_full0 + 8 * b);
+                __syncwarp();
             }
-            await_mmas_pair(done);
+            if (issuer) await_mmas_pair(done);
+            __syncwarp();
         } else if (lane == 0) {
             mbar_wait(done, 0);
         }

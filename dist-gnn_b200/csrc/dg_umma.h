@@ -45,6 +45,14 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// One lane of a converged warp.  A warp that walks through its work together and lets this lane alone issue keeps the addresses of MMAs and
+// barriers in uniform registers; with a single lane in the whole loop they had to be moved there for every MMA, 60 to 100 ns each.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
 // ---- CTA pairs: two CTAs of a cluster, on the two SMs of a TPC, that the tensor cores treat as one (cta_group::2) ------------------
 // The address of the even CTA's barrier in the cluster's shared memory, given this CTA's own.
 __device__ __forceinline__ uint32_t in_leader(uint32_t bar)

@@ -647,20 +647,21 @@ int make_map(CUtensorMap* map, const float* ptr, int64_t rows, int64_t cols, int
 }
 
 // Which of the two kernels multiplies; an element is the same sum in the same order in both.  n_pad: columns rounded up to 16.
-// One tile per CTA wins while its CTAs are all resident at once and there is no next tile to overlap with: up to 80 columns two of them
-// fit an SM, above one.  A pair costs it some 0.5 us of cluster barriers and remote arrivals, an MMA takes 130 clocks however few columns it
-// has, and half slabs spare it the padding of a depth such as 100 or 16.  us, one tile per CTA against pair:
-//   10,000 rows: 64 -> 96 6.1 and 6.8, 256 -> 80 11.6 and 12.2; 100 -> 128 9.0 and 8.5 (pair), 384 -> 128 16.1 and 15.4 (pair)
-//   25,000 rows: 64 -> 80 8.1 and 9.6, 256 -> 72 15.0 and 19.1; 64 -> 96 10.8 and 8.7 (pair: a second wave)
-// With more rows than that the pair's overlap pays, up to 80 columns only where two CTAs an SM do not overlap as well themselves: 150,001
-// rows 256 -> 47 59 and 62, 100 -> 72 39.1 and 31.9 (pair), 64 -> 80 with the mask 45.7 and 48.6, 602 -> 72 114 and 129, 256 -> 80 with the mask 71.9 and 64.9 (pair).
+// Up to 80 columns two one-tile CTAs fit an SM.  While all of them are resident at once, and for no more than one wave of those of up to 128
+// columns, there is no next tile for a pair to overlap with, and its cluster barriers and remote arrivals are not won back
+// unless the depth is large or ends in a half slab, which spares it padding.  us, one tile per CTA against pair:
+//   10,000 rows 64 -> 96 6.0 and 6.5, 64 -> 80 6.6 and 7.1, 128 -> 80 8.2 and 8.6; 100 -> 128 9.0 and 8.0 (pair), 128 -> 96 7.8 and 7.6 (pair), 256 -> 80 11.5 and 10.9 (pair)
+//   25,000 rows 64 -> 80 8.0 and 9.7, 256 -> 72 14.9 and 17.1; 64 -> 96 10.8 and 8.5 (pair: a second wave)
+// With more rows the pair wins (150,001 rows 100 -> 72 40.6 and 31.7, 256 -> 80 58 and 53, 256 -> 128 96 and 59) but for shallow products up to 80
+// columns with the mask, which wait for its rows and have more warps to do so as two CTAs (150,001 rows 64 -> 65 57 and 61, 100,000 rows
+// 64 -> 80 26.8 and 30.7).  Up to 64 columns the line was drawn when a pair issued its MMAs more slowly (256 -> 47 860 and 895; now 830 and 701).
 bool by_pairs(int64_t M, int n_pad, int K, bool masked, int sms)
 {
     if (n_pad <= 64) return false;
     const int64_t tiles = (M + BM - 1) / BM;
     const bool half_slab = (K - 1) % BK < BK / 2;
-    if (tiles <= sms) return n_pad > 128 || half_slab || (K > 192 && n_pad > 96);
-    return n_pad > 80 || (tiles > 2 * sms && (masked ? K > 64 : K <= 192));
+    if (tiles <= sms) return n_pad > 128 || half_slab || K > (n_pad > 80 ? 96 : 128);
+    return n_pad > 80 || (tiles > 2 * sms && (!masked || K > 64));
 }
 
 }  // namespace

@@ -279,7 +279,7 @@ k_dense_nt(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
 // Barriers: full (own CTA, TMA), ready (even CTA: the split warps of both), empty and acc_full (both CTAs, by commit), acc_empty (even CTA:
 // the epilogue warps of both).
 //
-// What bounds it: at 256 x 256 the MMAs (tensor pipe 60 % with the mask, DRAM 53 %; a single CTA's shared memory was busy with fetching both operands' 12 KB for
+// What bounds it: at 256 x 256 the MMAs (tensor pipe 68 %, with the mask 64 and DRAM 60 %; a single CTA's shared memory was busy with fetching both operands' 12 KB for
 // every MMA and refilling Bt's 512 KB for every 128 rows, which a pair halves), below some 100 columns of A DRAM and the epilogue.
 // 2,449,029 rows (us, one CTA per SM with four epilogue warps -> pair): 256 -> 256 1,600 -> 1,535, with the mask 1,930 -> 1,720;
 // 100 -> 256 1,100 -> 895; 47 -> 256 with the mask 1,600 -> 1,110; 602 -> 256 4,280 -> 3,540; 256 -> 128 1,540 -> 1,065 (one tile per
@@ -838,8 +838,8 @@ extern "C" int dg_dense_wait_selftest(int* host_gave_up, void* stream)
 // passes are accumulated into fp32 accumulators in tensor memory, and the range's partial D goes to scratch; a second
 // kernel adds the partials of all ranges in order (deterministic).
 //
-// One operand, P, lies along the 128 rows of an MMA, the other, Q, along its up to 256 columns.  An MMA with 32-bit operands takes
-// some 130 clocks for 128 rows however few columns it has, so P is the narrower operand (256 x 47: 47 columns padded to 128 rows, once
+// One operand, P, lies along the 128 rows of an MMA, the other, Q, along its up to 256 columns.  As one lane alone issues them here, an MMA
+// takes some 130 clocks for 128 rows however few columns it has, so P is the narrower operand (256 x 47: 47 columns padded to 128 rows, once
 // over Q's 256, instead of twice over 48) and D comes out transposed where that is G.  Where both are wider than 128 the
 // CTAs of a pair (cta_group::2) hold 128 columns of P and half of Q each, and take two ranges, one after the other.  An element of D is
 // the same sum in the same order either way.

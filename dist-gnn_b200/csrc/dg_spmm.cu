@@ -144,10 +144,11 @@ __device__ __forceinline__ float finish(const SpmmArgs& a, float sum, const floa
 // the last rows of a CTA are short ones.  The first entries of the next G rows are requested before the current ones are
 // gathered.
 //
-// What bounds it: the gathers.  Rows that the L2 holds come at 18 TB/s, 64 bytes a clock and SM (dense graph, F = 256: 41 GB in
-// 2.30 ms with the L2 at 78 % of its throughput, the path from it to the SMs at 49 %, issue slots at 46 %); larger graphs are held
-// up by the L2 and by what misses it (1 M nodes, 49 M entries: L2 64 %, DRAM 48 %, hit rate 63 %); small ones and short rows
-// are bound by latency, which the offsets in shared memory, the look-ahead and U hide.  Against separate kernels with a warp per
+// What bounds it: the gathers.  Wide rows that the L2 holds come at 18 TB/s, 64 bytes a clock and SM (dense graph, F = 256: 41 GB in
+// 2.27 ms with the L2 at 79 % of its throughput, issue slots at 36 %); larger graphs are held
+// up by the L2 and by what misses it (1 M nodes, 49 M entries: L2 65 %, DRAM 49 %, hit rate 63 %); narrow rows by the L1's data pipe, issue
+// and latency (300 k nodes, F = 100: 11 TB/s, L1 data pipe 75 %, issue 61 %, L2 50 %; 1 M nodes, F = 64: 10 TB/s, 56, 53, 43 %); small graphs and
+// short rows by latency, which the offsets in shared memory, the look-ahead and U hide.  Against separate kernels with a warp per
 // row (B200, us per product):
 //   10,000 nodes, 210 k entries, F = 64: 74 -> 17      150,001 nodes, 2.6 M entries, F = 256: 263 -> 204; F = 48: 156 -> 79
 //   1 M nodes, 17 M entries, F = 64: 748 -> 400, F = 16: 582 -> 194        306 k-row stage block, 1.9 M entries, F = 256: 281 -> 182

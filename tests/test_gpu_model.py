@@ -455,3 +455,32 @@ def test_row_cross_entropy_over_several_rows_of_a_group(n, C, ld):
     assert float((grad.double() - want_grad).norm() / want_grad.norm()) < 10 * 2.0 ** -24
     assert bool((grad[t < 0] == 0).all())
     assert torch.equal(loss, spmm_cpp.row_cross_entropy(x, t, rows.numel()))
+
+
+def test_two_networks_backward_on_two_streams(golden, env1):
+    """Two networks, each with its graph, train at the same time on two streams: every weight gradient is what it is alone, bit for bit."""
+    from coo_graph import COO_Graph, Parted_COO_Graph
+    from models import GCN
+    z = golden('graph_small')
+    models, ups = [], []
+    for i in range(2):
+        g = Parted_COO_Graph.from_full(COO_Graph.from_dict('gsmall', _fixture_dataset(z), device='cuda'), 0, 1)
+        gen = torch.Generator(device='cuda').manual_seed(90 + i)
+        g.features = torch.randn(g.local_num_nodes, 200, device='cuda', generator=gen)
+        g.num_classes = 47
+        models.append(GCN(g, env1, hidden_dim=256, num_layers=3))
+        ups.append(torch.randn(g.local_num_nodes, 47, device='cuda', generator=gen))
+
+    def step(i):
+        return torch.autograd.grad(models[i](models[i].g.features), models[i].weights(), ups[i])
+
+    alone = [step(i) for i in range(2)]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], [[], []]
+    for _ in range(20):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(step(i))
+    torch.cuda.synchronize()
+    for want, steps in zip(alone, got):
+        assert all(torch.equal(a, b) for grads in steps for a, b in zip(want, grads))
